@@ -1,4 +1,5 @@
-"""ctypes binding of libdualquant_b200.so (the C ABI declared in include/dualquant_b200.h).
+"""ctypes binding of libdualquant_b200.so (the C ABI declared in include/dualquant_b200.h), and the loader of
+the native torch binding (csrc/torch_host.cpp) that the hot wrappers of ops.py go through.
 
 The library is the only compute path: if it cannot be loaded, or the device is not sm_100,
 every op raises -- there is no fallback.
@@ -11,6 +12,7 @@ import threading
 
 _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.environ.get("DUALQUANT_B200_LIB", os.path.join(_PKG, "lib", "libdualquant_b200.so"))
+HOST_PATH = os.path.join(_PKG, "lib", "_torch_host.so")
 
 DQ_OK = 0
 DQ_ERR_TIMEOUT = 9
@@ -113,6 +115,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_host = None
 _lock = threading.Lock()
 _inited = set()
 
@@ -137,6 +140,30 @@ def load():
             fn.argtypes = args
         _lib = lib
     return _lib
+
+
+def host():
+    """The native torch binding (loaded once, on top of the library)."""
+    global _host
+    if _host is not None:
+        return _host
+    load()
+    with _lock:
+        if _host is not None:
+            return _host
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError(f"{HOST_PATH} is missing: build it with `python -m dualquant_b200.build`")
+        import importlib.machinery
+        import importlib.util
+
+        import torch  # noqa: F401  (the binding resolves its symbols in the loaded torch)
+
+        loader = importlib.machinery.ExtensionFileLoader("_torch_host", HOST_PATH)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_torch_host", loader))
+        loader.exec_module(mod)
+        mod.setup(LIB_PATH, check, ensure_init)
+        _host = mod
+    return _host
 
 
 def last_error() -> str:

@@ -45,6 +45,8 @@ class PermLinear(nn.Module):
         self._packed_fp4: Optional[ops.PackedFp4Weight] = None
         self._hadamard_cache = None
         self._scratch: Optional[torch.Tensor] = None
+        # what the native forward needs, made by _make_plan; None = to be made by the next call
+        self._plan = None
         # None = not examined yet; False = the weight is not on the W4 grid of the activation
         # format, the layer keeps the reference's fake-quant formulation
         self._weight_on_grid: Optional[bool] = None
@@ -179,7 +181,34 @@ class PermLinear(nn.Module):
             out = ops.hadamard_f32(x32, had) if had is not None else x32
         return out.to(self.dtype).reshape(x.shape)
 
+    def _make_plan(self, x) -> None:
+        """Called when a packed path has taken a bf16 call: prepares the native forward for the next ones
+        (torch_host.cpp: it answers None, and the Python code below runs, whenever an attribute the plan was
+        made from has been replaced)."""
+        self._plan = None
+        if self.quantize_bmm_input or self.dtype not in (torch.bfloat16, torch.float32) or x.dtype != torch.bfloat16:
+            return
+        x2 = x.reshape(-1, x.shape[-1])
+        if self._int4_path():
+            kind, packed = 0, self._packed
+        elif self._fp4_fmt() is not None:
+            kind, packed = 1, self._packed_fp4
+            if packed is not None and packed.fmt != self._fp4_fmt():
+                return
+        elif not self.act_quant_enabled and self.dtype == torch.bfloat16 and self._a16w4_ready():
+            kind, packed = 2, self._packed
+        else:
+            return
+        if packed is not None:
+            had = self._hadamard(x.device) if kind == 0 else None
+            self._plan = _lib.host().make_plan(self, kind, had, 2 if self._bf16_arith(x2) else 0, self.dtype)
+            self._scratch = None  # the plan keeps its own
+
     def forward(self, x):
+        out = _lib.host().perm_forward(self, x)
+        return out if out is not None else self._forward(x)
+
+    def _forward(self, x):
         if not x.is_cuda:
             raise RuntimeError("dualquant_b200.PermLinear runs on CUDA (sm_100a) tensors only")
         use_int4 = self._int4_path()
@@ -242,6 +271,7 @@ class PermLinear(nn.Module):
                 out = ops.fakequant_act_int4_bf16(out.reshape(-1, out.shape[-1])).reshape(out.shape)
             else:
                 out = self.act_fmt.cast(out.to(torch.float32)).to(self.dtype)
+        self._make_plan(x)
         return out
 
 

@@ -1,4 +1,4 @@
-"""Builds libdualquant_b200.so (sm_100a only) with nvcc, in-tree.
+"""Builds libdualquant_b200.so (sm_100a only, nvcc) and the torch binding _torch_host.so (g++), in-tree.
 
 Usage: python -m dualquant_b200.build [--force] [--verbose]
 """
@@ -12,6 +12,8 @@ PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_DIR = os.path.join(PKG_DIR, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libdualquant_b200.so")
+HOST_SOURCE = "torch_host.cpp"
+HOST_PATH = os.path.join(LIB_DIR, "_torch_host.so")
 
 SOURCES = [
     "dq_runtime.cu",
@@ -59,11 +61,30 @@ def _newest_source_mtime() -> float:
 
 
 def needs_build() -> bool:
-    return not os.path.exists(LIB_PATH) or os.path.getmtime(LIB_PATH) < _newest_source_mtime()
+    newest = _newest_source_mtime()
+    return any(not os.path.exists(p) or os.path.getmtime(p) < newest for p in (LIB_PATH, HOST_PATH))
+
+
+def _host_command() -> list:
+    """The binding against this interpreter's torch; its symbols come from the torch that is already loaded
+    when the module is imported."""
+    import sysconfig
+
+    import torch
+    from torch.utils.cpp_extension import include_paths, library_paths
+
+    cuda = os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")
+    dirs = [*include_paths(), sysconfig.get_paths()["include"], cuda]
+    return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wall",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            *(f"-isystem{d}" for d in dirs), os.path.join(CSRC, HOST_SOURCE), "-o", HOST_PATH,
+            *(f"-L{d}" for d in library_paths()), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda",
+            "-ltorch_python", "-ldl"]
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile every .cu under csrc/ into one shared library; returns its path."""
+    """Compile every .cu under csrc/ into one shared library, and the torch binding next to it; returns the
+    library's path."""
     if not force and not needs_build():
         return LIB_PATH
     os.makedirs(LIB_DIR, exist_ok=True)
@@ -77,6 +98,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
             print(" ".join(cmd), flush=True)
         procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
         objs.append(obj)
+    procs.append((HOST_SOURCE, subprocess.Popen(_host_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT,
+                                                text=True)))
     failed = False
     for src, p in procs:
         out, _ = p.communicate()
@@ -84,7 +107,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
             sys.stderr.write(f"--- {src}\n{out}\n")
         failed |= p.returncode != 0
     if failed:
-        raise RuntimeError("nvcc failed; see output above")
+        raise RuntimeError("the compiler failed; see output above")
     link = [_nvcc(), "-shared", "-o", LIB_PATH, *objs, "-gencode", "arch=compute_100a,code=sm_100a",
             "-Xcompiler", "-fPIC"]
     subprocess.run(link, check=True)

@@ -1,5 +1,6 @@
 """Tensor-level wrappers over the C ABI: torch supplies device memory and the stream, the
-shared library does all the work."""
+shared library does all the work.  The wrappers of the per-call path (activation quantisers, GEMMs, one-call
+linears) check and call through the native binding, csrc/torch_host.cpp; the rest goes through ctypes."""
 from __future__ import annotations
 
 import ctypes
@@ -124,59 +125,21 @@ def quant_act_int4(x: torch.Tensor, a: Optional[torch.Tensor] = None,
                    e4m3: bool = False):
     """bf16 or fp32 [M,K] -> (codes int8 [M,K], sx fp32 [M]); e4m3: the codes as E4M3 bytes (uint8),
     the operand of gemm_w4a4_int4_e4m3."""
-    lib = _prep(x)
-    if x.dtype not in (torch.bfloat16, torch.float32):
-        raise ValueError("quant_act_int4 expects bf16 or fp32 activations")
-    if x.stride(-1) != 1:
-        x = x.contiguous()
-    M, K = x.shape
-    codes = torch.empty(M, K, dtype=torch.uint8 if e4m3 else torch.int8, device=x.device)
-    sx = torch.empty(M, dtype=torch.float32, device=x.device)
-    desc = had.desc() if had is not None else None
-    fn, what = ((lib.dq_quant_act_int4, "dq_quant_act_int4") if x.dtype == torch.bfloat16
-                else (lib.dq_quant_act_int4_f32, "dq_quant_act_int4_f32"))
-    _lib.check(fn(_ptr(x), x.stride(0) if M > 1 else K, _ptr(a), desc, M, K, _ptr(codes), _ptr(sx),
-                  _scale_mode(scale_fp16, bf16_arith) | (_lib.CODES_E4M3 if e4m3 else 0), _stream(x.device)), what)
-    return codes, sx
+    return _lib.host().quant_act_int4(x, a, had, _scale_mode(scale_fp16, bf16_arith), bool(e4m3))
 
 
 def quant_act_int4_gated(gate: torch.Tensor, up: torch.Tensor, a: Optional[torch.Tensor] = None,
                          had: Optional[Hadamard] = None, scale_fp16: bool = False, e4m3: bool = False):
     """codes/scales of bf16(bf16(SiLU(gate)) * up); gate and up are bf16 [M,K] views with the same
     row stride (typically the two halves of a fused gate+up projection output)."""
-    lib = _prep(gate)
-    if gate.dtype != torch.bfloat16 or up.dtype != torch.bfloat16:
-        raise ValueError("quant_act_int4_gated expects bf16 inputs")
-    if gate.shape != up.shape or gate.stride() != up.stride() or gate.stride(-1) != 1:
-        raise ValueError("gate and up must have the same shape and strides (unit inner stride)")
-    M, K = gate.shape
-    codes = torch.empty(M, K, dtype=torch.uint8 if e4m3 else torch.int8, device=gate.device)
-    sx = torch.empty(M, dtype=torch.float32, device=gate.device)
-    desc = had.desc() if had is not None else None
-    _lib.check(lib.dq_quant_act_int4_gated(_ptr(gate), _ptr(up), gate.stride(0) if M > 1 else K, _ptr(a),
-                                           desc, M, K, _ptr(codes), _ptr(sx),
-                                           int(scale_fp16) | (_lib.CODES_E4M3 if e4m3 else 0),
-                                           _stream(gate.device)), "dq_quant_act_int4_gated")
-    return codes, sx
+    return _lib.host().quant_act_int4_gated(gate, up, a, had, int(scale_fp16), bool(e4m3))
 
 
 def quant_act_int4_rmsnorm(x: torch.Tensor, norm_weight: Optional[torch.Tensor], eps: float,
                            a: Optional[torch.Tensor] = None, scale_fp16: bool = False, e4m3: bool = False):
     """RMSNorm (bf16 result, optional bf16 weight) + column scale + per-token int4 quantiser in
     one pass: bf16 [M,K] -> (codes int8 [M,K], sx fp32 [M])."""
-    lib = _prep(x)
-    if x.dtype != torch.bfloat16 or x.stride(-1) != 1:
-        raise ValueError("quant_act_int4_rmsnorm expects bf16 rows with unit inner stride")
-    if norm_weight is not None and (norm_weight.dtype != torch.bfloat16 or norm_weight.numel() != x.shape[1]):
-        raise ValueError("norm_weight must be bf16 with one entry per input channel")
-    M, K = x.shape
-    codes = torch.empty(M, K, dtype=torch.uint8 if e4m3 else torch.int8, device=x.device)
-    sx = torch.empty(M, dtype=torch.float32, device=x.device)
-    _lib.check(lib.dq_quant_act_int4_rmsnorm(_ptr(x), x.stride(0) if M > 1 else K, _ptr(norm_weight),
-                                             float(eps), _ptr(a), M, K, _ptr(codes), _ptr(sx),
-                                             int(scale_fp16) | (_lib.CODES_E4M3 if e4m3 else 0), _stream(x.device)),
-               "dq_quant_act_int4_rmsnorm")
-    return codes, sx
+    return _lib.host().quant_act_int4_rmsnorm(x, norm_weight, float(eps), a, int(scale_fp16), bool(e4m3))
 
 
 def fakequant_act_int4(x: torch.Tensor, a: Optional[torch.Tensor] = None,
@@ -262,26 +225,7 @@ def gemm_w4a4_int4(codes: torch.Tensor, sx: torch.Tensor, pw: PackedInt4Weight,
                    residual: Optional[torch.Tensor] = None) -> torch.Tensor:
     """residual: [M, N] of the output's dtype -> out = residual + linear (fused into the epilogue;
     may be the output tensor itself)."""
-    lib = _prep(codes)
-    M, K = codes.shape
-    if K != pw.K:
-        raise ValueError(f"K mismatch: activations {K}, weight {pw.K}")
-    if out is None:
-        out = torch.empty(M, pw.N, dtype=residual.dtype if residual is not None else out_dtype,
-                          device=codes.device)
-    ydt = _lib.DTYPE_BF16 if out.dtype == torch.bfloat16 else _lib.DTYPE_F32
-    if residual is not None:
-        if residual.dtype != out.dtype or tuple(residual.shape) != (M, pw.N) or not residual.is_contiguous():
-            raise ValueError("residual must be a contiguous [M, N] tensor of the output's dtype")
-        _lib.check(lib.dq_gemm_w4a4_int4_residual(_ptr(codes), _ptr(sx), _ptr(pw.w_packed), _ptr(pw.sw_t),
-                                                  _ptr(r), _ptr(residual), M, pw.N, K, pw.group, _ptr(out),
-                                                  ydt, _stream(codes.device)), "dq_gemm_w4a4_int4_residual")
-        return out
-    _lib.check(lib.dq_gemm_w4a4_int4_ex(_ptr(codes), _ptr(sx), _ptr(pw.w_packed), _ptr(pw.sw_t), _ptr(r),
-                                        M, pw.N, K, pw.group, _ptr(out), ydt, None, 0,
-                                        _stream(codes.device), token_tile, split_k),
-               "dq_gemm_w4a4_int4")
-    return out
+    return _lib.host().gemm_w4a4_int4(codes, sx, pw, r, out_dtype, token_tile, split_k, out, residual)
 
 
 def expand_w_e4m3(pw: PackedInt4Weight) -> torch.Tensor:
@@ -308,20 +252,7 @@ def gemm_w4a4_int4_e4m3(x8: torch.Tensor, sx: torch.Tensor, w8: torch.Tensor, pw
                         out: Optional[torch.Tensor] = None,
                         residual: Optional[torch.Tensor] = None) -> torch.Tensor:
     """The int4 GEMM on the FP8 tensor-core path (prefill); same bits as gemm_w4a4_int4."""
-    lib = _prep(x8)
-    M, K = x8.shape
-    if K != pw.K or tuple(w8.shape) != (pw.N, pw.K) or not x8.is_contiguous() or not w8.is_contiguous():
-        raise ValueError("x8 [M, K] and w8 [N, K] must be contiguous and match the packed weight")
-    if out is None:
-        out = torch.empty(M, pw.N, dtype=residual.dtype if residual is not None else out_dtype, device=x8.device)
-    if residual is not None and (residual.dtype != out.dtype or tuple(residual.shape) != (M, pw.N)
-                                 or not residual.is_contiguous()):
-        raise ValueError("residual must be a contiguous [M, N] tensor of the output's dtype")
-    ydt = _lib.DTYPE_BF16 if out.dtype == torch.bfloat16 else _lib.DTYPE_F32
-    _lib.check(lib.dq_gemm_w4a4_int4_e4m3(_ptr(x8), _ptr(sx), _ptr(w8), _ptr(pw.sw_t), _ptr(r), M, pw.N, K,
-                                          pw.group, _ptr(out), ydt, _ptr(residual), _stream(x8.device)),
-               "dq_gemm_w4a4_int4_e4m3")
-    return out
+    return _lib.host().gemm_w4a4_int4_e4m3(x8, sx, w8, pw, r, out_dtype, out, residual)
 
 
 class AllReduceContext:
@@ -494,27 +425,10 @@ def linear_w4a4_int4(x: torch.Tensor, a: Optional[torch.Tensor], had: Optional[H
                      pw: PackedInt4Weight, r: Optional[torch.Tensor], out_dtype=torch.float32,
                      scale_fp16: bool = False, scratch: Optional[torch.Tensor] = None,
                      out: Optional[torch.Tensor] = None, bf16_arith: bool = False) -> torch.Tensor:
-    """Whole PermLinear.forward on the int4 path in one C call."""
-    lib = _prep(x)
-    if x.dtype != torch.bfloat16:
-        raise ValueError("linear_w4a4_int4 expects bf16 activations (quantise fp32 rows with "
-                         "quant_act_int4 and call gemm_w4a4_int4)")
-    if x.stride(-1) != 1:
-        x = x.contiguous()
-    M, K = x.shape
-    # a caller's scratch is used as it is when it covers the plain path; the C side takes the
-    # FP8-path GEMM for prefill batches only if the scratch also has room for the weight's byte form
-    if scratch is None or scratch.numel() < linear_scratch_bytes(M, pw.N, K, prefill=False):
-        scratch = torch.empty(max(linear_scratch_bytes(M, pw.N, K), 256), dtype=torch.uint8, device=x.device)
-    if out is None:
-        out = torch.empty(M, pw.N, dtype=out_dtype, device=x.device)
-    ydt = _lib.DTYPE_BF16 if out.dtype == torch.bfloat16 else _lib.DTYPE_F32
-    desc = had.desc() if had is not None else None
-    _lib.check(lib.dq_linear_w4a4_int4(_ptr(x), x.stride(0) if M > 1 else K, _ptr(a), desc,
-                                       _ptr(pw.w_packed), _ptr(pw.sw_t), _ptr(r), M, pw.N, K, pw.group,
-                                       _ptr(out), ydt, _scale_mode(scale_fp16, bf16_arith), _ptr(scratch),
-                                       scratch.numel(), _stream(x.device)), "dq_linear_w4a4_int4")
-    return out
+    """Whole PermLinear.forward on the int4 path in one C call.  A caller's scratch is used as it is when it
+    covers the plain path; prefill batches take the FP8-path GEMM when it also has room for the weight's byte
+    form (linear_scratch_bytes)."""
+    return _lib.host().linear_w4a4_int4(x, a, had, pw, r, out_dtype, _scale_mode(scale_fp16, bf16_arith), scratch, out)
 
 
 def linear_a16w4(x: torch.Tensor, a: Optional[torch.Tensor], pw: PackedInt4Weight,
@@ -522,25 +436,7 @@ def linear_a16w4(x: torch.Tensor, a: Optional[torch.Tensor], pw: PackedInt4Weigh
                  scratch: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """bf16 activations (times the column scale a, rounded to fp16) against the int4 weight
     artefact on the 16-bit tensor cores: Y = r * (fp16(x * a) @ fp16(codes * group scale)^T)."""
-    lib = _prep(x)
-    if x.dtype != torch.bfloat16:
-        raise ValueError("linear_a16w4 expects bf16 activations")
-    if x.stride(-1) != 1:
-        x = x.contiguous()
-    M, K = x.shape
-    if K != pw.K:
-        raise ValueError(f"K mismatch: activations {K}, weight {pw.K}")
-    need = int(lib.dq_linear_a16w4_scratch_bytes(M, pw.N, K))
-    if scratch is None or scratch.numel() < need:
-        scratch = torch.empty(max(need, 256), dtype=torch.uint8, device=x.device)
-    if out is None:
-        out = torch.empty(M, pw.N, dtype=out_dtype, device=x.device)
-    ydt = _lib.DTYPE_BF16 if out.dtype == torch.bfloat16 else _lib.DTYPE_F32
-    _lib.check(lib.dq_linear_a16w4(_ptr(x), x.stride(0) if M > 1 else K, _ptr(a), _ptr(pw.w_packed), _ptr(r),
-                                   M, pw.N, K, pw.group, _ptr(out), ydt, _ptr(scratch),
-                                   0 if scratch is None else scratch.numel(), _stream(x.device)),
-               "dq_linear_a16w4")
-    return out
+    return _lib.host().linear_a16w4(x, a, pw, r, out_dtype, scratch, out)
 
 
 # ---------------------------------------------------------------------------------------------
@@ -653,8 +549,7 @@ def gemm_w4a4_fp4(x_codes: torch.Tensor, x_sf_atoms: torch.Tensor, x_scale: Opti
 def linear_w4a4_fp4(x: torch.Tensor, a: Optional[torch.Tensor], pw: PackedFp4Weight,
                     r: Optional[torch.Tensor] = None, out_dtype=torch.float32) -> torch.Tensor:
     """Quantise activations (per-token second-level scale for NVFP4) and run the FP4 GEMM."""
-    codes, sf_atoms, row_scale = quant_fp4(x, pw.fmt, a, None, atoms=True)
-    return gemm_w4a4_fp4(codes, sf_atoms, row_scale, pw, r, out_dtype)
+    return _lib.host().linear_w4a4_fp4(x, a, pw, r, out_dtype)
 
 
 def mma_peak(kind: int, iters: int = 4096, device=None) -> float:

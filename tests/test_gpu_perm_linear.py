@@ -213,3 +213,48 @@ def test_bf16_arithmetic_branch_bit_exact_against_the_reference(golden):
     qw, sw = O.quant_w_int4(w)
     exact = O.dequant_matmul(q, s, qw, sw)
     assert ((y.double() - exact).abs().max() / exact.abs().max()) < 8e-3
+
+
+@pytest.mark.parametrize("name", ["rtn_int4", "mxfp4", "nvfp4", "off"])
+def test_native_forward_equals_the_python_forward_and_follows_changes(name):
+    """The second call of a packed layer runs through the native forward; it returns the Python forward's
+    bits, and a replaced scale, bias, weight artefact or switch takes effect at the next call."""
+    import copy
+
+    K, N = 1024, 384
+    torch.manual_seed(7)
+    lin = nn.Linear(K, N, bias=True).to(torch.bfloat16).to(DEV)
+    w = synthetic.make_w(N, K, 4).to(DEV)
+    if name in ("mxfp4", "nvfp4"):
+        fmt = formats.make_format(name, block_size=32 if name == "mxfp4" else 16)
+        lin.weight.data = fmt.cast(w)
+    else:
+        fmt = formats.make_format("rtn_int4", block_size=-1)
+        lin.weight.data = O.dequant_w(*O.quant_w_int4(w.cpu())).to(torch.bfloat16).to(DEV)
+    lin.requires_grad_(False)
+    pl = PermLinear(lin, fmt)
+    pl.set_act_scale(torch.rand(K, device=DEV) + 0.5)
+    if name == "off":
+        pl.set_act_quant_enabled(False)
+    pl._packed_fp4 is None and name in ("mxfp4", "nvfp4") and pl.pack_fp4(pl._fp4_fmt(), force=True)
+    for shape in ((1, K), (2, 3, K), (1, 40, K), (1100, K)):
+        x = torch.randn(*shape, device=DEV).to(torch.bfloat16)
+        ref = pl._forward(x)
+        assert pl._plan is not None
+        y = pl(x)
+        assert y.shape == ref.shape and torch.equal(y, ref)
+    xs = torch.randn(5, 2 * K, device=DEV).to(torch.bfloat16)[:, :K]  # rows with a gap between them
+    assert torch.equal(pl(xs), pl._forward(xs))
+    x = torch.randn(3, K, device=DEV).to(torch.bfloat16)
+    before = pl(x)
+    pl.set_act_scale(torch.rand(K, device=DEV) + 0.5)
+    changed = pl(x)
+    assert not torch.equal(changed, before) and torch.equal(changed, pl._forward(x))
+    lin.bias.data.zero_()
+    assert torch.equal(pl(x), pl._forward(x)) and not torch.equal(pl(x), changed)
+    if name == "rtn_int4":
+        pl.online_full_had, (pl.had_K, pl.K) = True, quarot.get_hadK(K)
+        pl._hadamard_cache = None
+        assert torch.equal(pl(x), pl._forward(x))
+    twin = copy.deepcopy(pl)
+    assert twin._plan is None and torch.equal(twin(x), pl(x))
