@@ -73,6 +73,10 @@ SIGNATURES = {
     "dq_pack_w_int4": (_i, [_vp, _vp, _vp, _i, _i, _i, _vp, _vp, _vp]),
     "dq_unpack_w_int4": (_i, [_vp, _i, _i, _vp, _vp]),
     "dq_quant_w_int4": (_i, [_vp, _i, _i, _i, _vp, _vp, _vp]),
+    "dq_quant_pack_w_int4": (_i, [_vp, _i, _i, _i, _i, _vp, _vp, _vp]),
+    "dq_dualquant_workspace_bytes": (_sz, [_i, _i]),
+    "dq_dualquant_search": (_i, [_vp, _i, _i, _i, _i, _i, _i, _i, _i, ctypes.c_float, ctypes.c_float, _vp, _vp, _vp,
+                                 _vp, _vp, _sz, _vp]),
     "dq_quant_act_int4": (_i, [_vp, _i64, _vp, _hp, _i, _i, _vp, _vp, _i, _vp]),
     "dq_quant_act_int4_f32": (_i, [_vp, _i64, _vp, _hp, _i, _i, _vp, _vp, _i, _vp]),
     "dq_quant_act_int4_rmsnorm": (_i, [_vp, _i64, _vp, ctypes.c_float, _vp, _i, _i, _vp, _vp, _i, _vp]),

@@ -8,8 +8,8 @@ dualquant_with_beta_only (:344-368) or dualquant_with_alpha_only (:371-394) foll
 _reconstruct_block_* (:403-420).  A block only ever sees its own rows x block_size columns, so all
 blocks of a matrix are independent: here they are one batch - the weight is viewed as
 [rows, blocks, block_size], the row scales alpha as [rows, blocks], the column scales beta as
-[blocks, block_size] - and every step of the iteration is a handful of element-wise / reduction
-launches over the whole matrix on its own device.  Same formulas, same initialisations, same scale
+[blocks, block_size].  On a CUDA device one kernel pass over the matrix is an iteration (csrc/bcd.cu); CPU
+tensors, and block sizes that have no kernel, take the same steps as tensor expressions.  Same formulas, same initialisations, same scale
 roundings; what differs from the reference's result is the order in which fp32 sums are formed
 (and therefore, rarely, a code at a rounding boundary).
 
@@ -30,6 +30,31 @@ _E4M3_TINY = float(torch.finfo(torch.float8_e4m3fn).tiny)
 _E4M3_MAX = float(torch.finfo(torch.float8_e4m3fn).max)
 
 _QRANGE = {"rtn_int4": (-8.0, 7.0), "rtn_int8": (-128.0, 127.0)}
+
+# argument codes of dq_dualquant_search
+_OPTIONS = {"row_column": 0, "only_column": 1, "only_row": 2}
+_ROW_INITS = {"max_abs": 0, "all_one": 1}
+_COL_INITS = {"l1_norm": 0, "l2_norm": 1, "all_one": 2, "max_abs": 3}
+_SCALE_FORMATS = {"none": 0, "e8m0": 1, "e4m3": 2}
+
+
+def _on_device(weight: torch.Tensor, block_size: int, num_iter: int, scale_option: str, row_init: str, col_init: str,
+               scale_format: str, quant_method: str, stored_weight: bool):
+    """The search in the library's kernels, or None where they do not apply (CPU tensors, other block sizes, no
+    iteration; unknown options are left to the tensor form, which says what is wrong with them)."""
+    R, C = weight.shape
+    if (not weight.is_cuda or block_size not in (32, 64, 128, 256) or C % block_size or num_iter < 1 or R < 1
+            or quant_method not in _QRANGE or scale_option not in _OPTIONS or row_init not in _ROW_INITS
+            or col_init not in _COL_INITS or scale_format not in _SCALE_FORMATS):
+        return None
+    from . import ops
+
+    w = weight.detach().to(torch.float32).contiguous()
+    if w.data_ptr() % 16:
+        w = w.clone()
+    return ops.dualquant_search(w, block_size, num_iter, _OPTIONS[scale_option], _ROW_INITS[row_init],
+                                _COL_INITS[col_init], _SCALE_FORMATS[scale_format], *_QRANGE[quant_method],
+                                stored_weight)
 
 
 def _quantize_scale(scale: torch.Tensor, scale_format: str) -> torch.Tensor:
@@ -83,6 +108,9 @@ def dualquant_scales(weight: torch.Tensor, *, block_size: int = 128, num_iter: i
     """The scale search for every column block of `weight` [rows, cols] at once, on its device.
     Returns (alpha [rows, blocks], beta [blocks, block_size]), the forward scales: the quantiser
     sees alpha * W * beta."""
+    done = _on_device(weight, block_size, num_iter, scale_option, row_init, col_init, scale_format, quant_method, False)
+    if done is not None:
+        return done[:2]
     if quant_method not in _QRANGE:
         raise NotImplementedError(f"quant_method {quant_method!r} is not restated (supported: {sorted(_QRANGE)})")
     qmin, qmax = _QRANGE[quant_method]
@@ -131,6 +159,9 @@ def dualquant_weight(weight: torch.Tensor, *, block_size: int = 128, num_iter: i
     scale per (row, block) - and column_scales [cols] = 1 / beta is the vector the activations are
     divided by at run time (W ~ mat_q * column_scales).  `wrap.pack_from_dualquant(mat_q,
     column_scales)` turns the pair into the packed int4 artefact."""
+    done = _on_device(weight, block_size, num_iter, scale_option, row_init, col_init, scale_format, quant_method, True)
+    if done is not None:
+        return done[2:]
     qmin, qmax = _QRANGE.get(quant_method, (None, None))
     alpha, beta = dualquant_scales(weight, block_size=block_size, num_iter=num_iter, scale_option=scale_option,
                                    row_init=row_init, col_init=col_init, scale_format=scale_format,

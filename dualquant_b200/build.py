@@ -18,6 +18,7 @@ HOST_PATH = os.path.join(LIB_DIR, "_torch_host.so")
 SOURCES = [
     "dq_runtime.cu",
     "weights_int4.cu",
+    "bcd.cu",
     "act_quant_int4.cu",
     "act_quant_had_bf16.cu",
     "act_quant_had_f32.cu",

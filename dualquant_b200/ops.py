@@ -104,6 +104,35 @@ def pack_w_int4(codes: Optional[torch.Tensor], sw: torch.Tensor, group: int = GR
     return PackedInt4Weight(w_packed, sw_t, N, K, group)
 
 
+def quant_pack_w_int4(w: torch.Tensor, group: int = GROUP) -> PackedInt4Weight:
+    """pack_w_int4(*quant_w_int4(w)) in one pass over w (bf16, or fp32 rounded to bf16 on the way in)."""
+    lib = _prep(w)
+    w = (w if w.dtype in (torch.bfloat16, torch.float32) else w.to(torch.bfloat16)).contiguous()
+    N, K = w.shape
+    w_packed = torch.empty(int(lib.dq_packed_w_bytes(N, K)), dtype=torch.uint8, device=w.device)
+    sw_t = torch.empty((N + 127) // 128 * 128 * (K // group), dtype=torch.float16, device=w.device)
+    _lib.check(lib.dq_quant_pack_w_int4(_ptr(w), int(w.dtype == torch.float32), N, K, group, _ptr(w_packed),
+                                        _ptr(sw_t), _stream(w.device)), "dq_quant_pack_w_int4")
+    return PackedInt4Weight(w_packed, sw_t, N, K, group)
+
+
+def dualquant_search(w: torch.Tensor, block_size: int, num_iter: int, scale_option: int, row_init: int, col_init: int,
+                     scale_format: int, qmin: float, qmax: float, weight: bool):
+    """dq_dualquant_search on fp32 w [R, C] -> (alpha [R, blocks], beta [blocks, block_size], mat_q [R, C] or None,
+    column_scales [C] or None); weight: also form the stored weight and 1 / beta."""
+    lib = _prep(w)
+    R, C = w.shape
+    alpha = torch.empty(R, C // block_size, dtype=torch.float32, device=w.device)
+    beta = torch.empty(C // block_size, block_size, dtype=torch.float32, device=w.device)
+    mat_q = torch.empty_like(w) if weight else None
+    cs = torch.empty(C, dtype=torch.float32, device=w.device) if weight else None
+    ws = torch.empty(int(lib.dq_dualquant_workspace_bytes(R, C)), dtype=torch.uint8, device=w.device)
+    _lib.check(lib.dq_dualquant_search(_ptr(w), R, C, block_size, num_iter, scale_option, row_init, col_init,
+                                       scale_format, qmin, qmax, _ptr(alpha), _ptr(beta), _ptr(mat_q), _ptr(cs),
+                                       _ptr(ws), ws.numel(), _stream(w.device)), "dq_dualquant_search")
+    return alpha, beta, mat_q, cs
+
+
 def unpack_w_int4(pw: PackedInt4Weight) -> torch.Tensor:
     lib = _prep(pw.w_packed)
     codes = torch.empty(pw.N, pw.K, dtype=torch.int8, device=pw.w_packed.device)

@@ -28,13 +28,12 @@ def pack_from_dualquant(mat_q: torch.Tensor,
         raise RuntimeError("pack_from_dualquant needs mat_q on a CUDA device (no CPU path)")
     if mat_q.dim() != 2 or mat_q.shape[1] % 128 != 0:
         raise ValueError(f"mat_q must be [N, K] with K % 128 == 0, got {tuple(mat_q.shape)}")
-    codes, sw = ops.quant_w_int4(mat_q.detach().to(torch.bfloat16).contiguous())
     a = None
     if column_scales is not None:
         if column_scales.numel() != mat_q.shape[1]:
             raise ValueError("column_scales must have one entry per input channel")
         a = column_scales.detach().to(device=mat_q.device, dtype=torch.float32).contiguous()
-    return ops.pack_w_int4(codes, sw), a
+    return ops.quant_pack_w_int4(mat_q.detach()), a
 
 
 def load_wrap_cache(path: str) -> dict:

@@ -130,6 +130,30 @@ DQ_API int dq_unpack_w_int4(const uint8_t* w_packed, int N, int K, int8_t* codes
 DQ_API int dq_quant_w_int4(const void* w_bf16, int N, int K, int G, int8_t* codes, void* sw,
                     void* stream);
 
+/* dq_quant_w_int4 on bf16(w) and dq_pack_w_int4 in one pass over w (bf16, or fp32 when w_is_f32 != 0), without the
+ * row-major codes and scales in between: what becomes of DualQuant's stored weight
+ * (ablation/real_int4_kernel/validate_real_kernel.py:95-98). */
+DQ_API int dq_quant_pack_w_int4(const void* w, int w_is_f32, int N, int K, int G, uint8_t* w_packed, void* sw_t,
+                                void* stream);
+
+/*
+ * DualQuant's offline scale search and block quantisation of a whole weight, every block of block_size columns
+ * (32, 64, 128 or 256) at once: wrap_dualquant_layer of layer_wrapper_dualquant.py:423-533 (search :300-394,
+ * initial scales :246-277, row-scale formats :84-147, block quantisation :403-420) for the integer formats.
+ *   w fp32 [R, C]; num_iter >= 1
+ *   scale_option 0 row_column, 1 only_column, 2 only_row;  row_init 0 max_abs, 1 all_one;
+ *   col_init 0 l1_norm, 1 l2_norm, 2 all_one, 3 max_abs;  scale_format 0 none, 1 e8m0, 2 e4m3
+ *   alpha [R, C / block_size] and beta [C] receive the forward scales (the quantiser sees alpha * w * beta);
+ *   mat_q [R, C] (may be null) the stored weight (1 / alpha) * RTN(alpha * w * beta), one RTN scale per row of a
+ *   block; column_scales [C] (may be null) 1 / beta.
+ * workspace: dq_dualquant_workspace_bytes(R, C) bytes.
+ */
+DQ_API size_t dq_dualquant_workspace_bytes(int R, int C);
+DQ_API int dq_dualquant_search(const float* w, int R, int C, int block_size, int num_iter, int scale_option,
+                               int row_init, int col_init, int scale_format, float qmin, float qmax, float* alpha,
+                               float* beta, float* mat_q, float* column_scales, void* workspace,
+                               size_t workspace_bytes, void* stream);
+
 /* ---- activations ------------------------------------------------------------------------- */
 
 /*

@@ -126,3 +126,38 @@ def test_full_size_layer_on_the_gpu():
         mq_b, cs_b = bcd.dualquant_weight(W[:, b * 128:(b + 1) * 128].contiguous(), block_size=128, **cfg)
         assert torch.allclose(mq_b, mat_q[:, b * 128:(b + 1) * 128], rtol=1e-5, atol=1e-9)
         assert torch.allclose(cs_b, cs[b * 128:(b + 1) * 128], rtol=1e-5, atol=0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,cols,bs", [(1, 128, 128), (7, 256, 32), (33, 192, 64), (130, 512, 256), (1025, 384, 128)])
+@pytest.mark.parametrize("option", ["row_column", "only_column", "only_row"])
+@pytest.mark.parametrize("fmt", ["none", "e8m0", "e4m3"])
+def test_search_kernels_against_the_tensor_form(rows, cols, bs, option, fmt):
+    """Ragged row counts (chunk and warp remainders) and every block size: one iteration agrees with the tensor
+    expressions on the CPU to the order of fp32 sums (more iterations would compare a scale or code that stepped at
+    a rounding boundary); the fused quantise-and-pack gives the bytes of the two separate steps."""
+    from dualquant_b200 import ops, wrap
+
+    g = torch.Generator().manual_seed(rows + cols)
+    W = torch.randn(rows, cols, generator=g) * 0.02
+    for col_init, row_init in (("l1_norm", "max_abs"), ("l2_norm", "max_abs"), ("max_abs", "all_one"), ("all_one", "max_abs")):
+        cfg = dict(block_size=bs, num_iter=1, scale_option=option, row_init=row_init, col_init=col_init, scale_format=fmt)
+        ref_q, ref_c = bcd.dualquant_weight(W, **cfg)
+        ref_a, ref_b = bcd.dualquant_scales(W, **cfg)
+        mat_q, cs = bcd.dualquant_weight(W.cuda(), **cfg)
+        alpha, beta = bcd.dualquant_scales(W.cuda(), **cfg)
+        for got, ref in ((alpha, ref_a), (beta, ref_b), (cs, ref_c)):
+            assert got.shape == ref.shape
+            off = (got.cpu() - ref).abs() > 1e-5 * ref.abs()
+            assert torch.equal(torch.isfinite(got.cpu()), torch.isfinite(ref))
+            assert (off & torch.isfinite(ref)).float().mean() <= (0.02 if rows > 1 else 0.1)
+        same = torch.isfinite(ref_q)
+        assert torch.equal(torch.isfinite(mat_q.cpu()), same)  # a column whose codes are all zero has no scale
+        bad = (mat_q.cpu() - ref_q).abs()[same] > 1e-4 * ref_q.abs().nan_to_num(0.0, 0.0, 0.0).max()
+        assert bad.numel() == 0 or bad.float().mean() < 0.02
+    if cols % 128 == 0:
+        mat_q = W.cuda()
+        for w in (mat_q, mat_q.to(torch.bfloat16)):
+            a, b = ops.quant_pack_w_int4(w), ops.pack_w_int4(*ops.quant_w_int4(w))
+            assert torch.equal(a.w_packed, b.w_packed) and torch.equal(a.sw_t.view(torch.int16), b.sw_t.view(torch.int16))
+        assert torch.equal(wrap.pack_from_dualquant(mat_q)[0].w_packed, a.w_packed)
