@@ -33,6 +33,10 @@ SOURCES = [
     "gemm_a16w4.cu",
     "decoder_ops.cu",
     "gemm_w4a4_int4_f8.cu",
+    "gemm_w4a4_int4_f8_out0.cu",
+    "gemm_w4a4_int4_f8_out1.cu",
+    "gemm_w4a4_int4_f8_out2.cu",
+    "gemm_w4a4_int4_f8_out3.cu",
     "gemm_fp4_persist.cu",
     "exchange.cu",
 ]

@@ -90,7 +90,8 @@ enum {
   DQ_TUNE_FUSED_SPLIT = 2,      // its split of K
   DQ_TUNE_FUSED_EXTRA_CTA = 3,  // CTAs' worth of shared memory left free per SM for the next launch
   DQ_TUNE_AR_WAIT_LOG2 = 4,     // fused all-reduce: a peer's flag is waited for 2^value SM cycles (0 = 30)
-  DQ_TUNE_COUNT = 5
+  DQ_TUNE_F8_TILE = 5,          // token tile of the FP8-path GEMM (32 .. 256 in steps of 32)
+  DQ_TUNE_COUNT = 6
 };
 int tuning(int key);
 

@@ -1,5 +1,5 @@
 // Thin inline-PTX wrappers for the sm_100a features the kernels use: mbarrier, TMA
-// (cp.async.bulk.tensor, no multicast), tcgen05 (TMEM allocation, UMMA issue, commit, load)
+// (cp.async.bulk.tensor, no multicast), tcgen05 (TMEM allocation, UMMA issue, commit, load; CTA pairs)
 // and cluster barriers / distributed shared memory.
 #pragma once
 #include <cuda.h>
@@ -70,6 +70,36 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
 #pragma unroll 1
     for (int i = 0; i < 256; ++i) {
       if (mbar_try_wait(bar, parity)) return true;
+    }
+    if (*abort_flag != 0) return false;
+    if (clock64() - t0 > (1ll << 31)) {
+      *abort_flag = site;
+      return false;
+    }
+  }
+}
+
+// mbar_wait on a shared-memory address (loops that step through a ring keep the address in a register).
+__device__ __forceinline__ bool mbar_wait_addr(uint32_t addr, uint32_t parity, volatile int* abort_flag, int site) {
+  auto ready = [&]() -> bool {
+    uint32_t ok;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.b32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok)
+        : "r"(addr), "r"(parity)
+        : "memory");
+    return ok != 0;
+  };
+  if (ready()) return true;
+  const long long t0 = clock64();
+  for (;;) {
+#pragma unroll 1
+    for (int i = 0; i < 256; ++i) {
+      if (ready()) return true;
     }
     if (*abort_flag != 0) return false;
     if (clock64() - t0 > (1ll << 31)) {
@@ -280,6 +310,46 @@ __device__ __forceinline__ void tmem_ld_x32(uint32_t taddr, uint32_t* v) {
 }
 __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// ---------------------------------------------------------------------------------------
+// CTA pairs (tcgen05 cta_group::2): two CTAs of a cluster work on one 256-row tile.  Every CTA keeps its own 128
+// rows of A and of the accumulator and one half of B; one thread of the even-ranked CTA issues for both.
+// ---------------------------------------------------------------------------------------
+// One warp of EACH CTA of the pair executes these.
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_out, uint32_t ncols) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_out)), "r"(ncols)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish_pair() {
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+// Completes `bar` (same offset in both CTAs of the pair) in both once all UMMAs issued so far by this thread have finished.
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+          smem_u32(bar)),
+      "h"(static_cast<unsigned short>(3))
+      : "memory");
+}
+// Tile of this GPU's memory into the issuing CTA's shared memory; the bytes are counted on `bar_addr`, a barrier of
+// either CTA of the pair (a shared::cluster address).
+__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* tm, int x, int y, uint32_t bar_addr,
+                                                 uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2.L2::cache_hint"
+      " [%0], [%1, {%2, %3}], [%4], %5;" ::"r"(smem_u32(smem_dst)),
+      "l"(reinterpret_cast<uint64_t>(tm)), "r"(x), "r"(y), "r"(bar_addr), "l"(policy)
+      : "memory");
+}
+// Arrival on a barrier of either CTA of the cluster (a shared::cluster address).  It hands over tensor memory only,
+// which tcgen05.fence orders; with explicit release.cluster here and acquire.cluster waits on the other side - meant
+// for ordinary memory - every group of a K loop took three times as long.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar_addr) : "memory");
 }
 
 // ---------------------------------------------------------------------------------------

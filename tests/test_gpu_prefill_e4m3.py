@@ -247,3 +247,30 @@ def test_exchange_sum_and_push(world):
         assert torch.equal(sxg[p, rank * tq:(rank + 1) * tq], smine)
         assert int(codes[p].sum().item()) == int(mine.sum().item())  # nothing outside the slice
     _lib.device_status(0)
+
+
+@pytest.mark.parametrize("tile", [32, 64, 96, 128, 160, 192, 224, 256])
+@pytest.mark.parametrize("M,N,K", [(1, 128, 128), (33, 136, 256), (255, 384, 1152), (257, 1280, 640), (700, 2056, 512)])
+def test_every_token_tile_equals_the_integer_kernel(tile, M, N, K):
+    """The CTA-pair kernel at each of its token tiles: ragged tokens, an odd number of 128-row tiles (the pair's
+    second CTA past the last row), one group, K loops shorter and longer than the ring; all output modes."""
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    pw = ops.pack_w_int4(*ops.quant_w_int4((torch.randn(N, K, generator=g, device=DEV) * 0.02).to(torch.bfloat16)))
+    x = torch.randn(M, K, generator=g, device=DEV).to(torch.bfloat16)
+    r = torch.rand(N, generator=g, device=DEV) + 0.5
+    codes, sx = ops.quant_act_int4(x)
+    x8, _ = ops.quant_act_int4(x, e4m3=True)
+    res = torch.randn(M, N, generator=g, device=DEV).to(torch.bfloat16)
+    try:
+        _lib.set_tuning("f8_tile", tile)
+        for kw in (dict(out_dtype=torch.float32), dict(out_dtype=torch.bfloat16), dict(residual=res)):
+            ref = ops.gemm_w4a4_int4(codes, sx, pw, r, token_tile=1128, split_k=1,
+                                     **{k: v for k, v in kw.items() if k != "residual"}) if "residual" not in kw else \
+                res + ops.gemm_w4a4_int4(codes, sx, pw, r, token_tile=1128, split_k=1, out_dtype=torch.bfloat16)
+            assert torch.equal(ops.gemm_w4a4_int4_e4m3(x8, sx, pw.bytes_e4m3(), pw, r, **kw), ref)
+        odd = ops.pack_w_int4(*ops.quant_w_int4((torch.randn(N + 3, K, generator=g, device=DEV) * 0.02).to(torch.bfloat16)))
+        y = ops.gemm_w4a4_int4_e4m3(x8, sx, odd.bytes_e4m3(), odd, out_dtype=torch.bfloat16)  # direct stores
+        assert torch.equal(y, ops.gemm_w4a4_int4(codes, sx, odd, token_tile=1128, split_k=1, out_dtype=torch.bfloat16))
+    finally:
+        _lib.set_tuning("f8_tile", 0)
+    _lib.device_status(0)
