@@ -34,14 +34,22 @@ cudaError_t init_out3();
 
 // Four two's-complement nibbles (bits 0-15 of sel) -> four E4M3 bytes of the same integers.
 // Non-negative codes 0..7: 00 38 40 44 48 4A 4C 4E; negative codes -8..-1: D0 CE CC CA C8 C4 C0 B8.
+// The byte permute takes the nibbles as selectors: its low three bits look up a magnitude, and where the fourth (the
+// sign) is set it replicates the sign bit of the byte looked up - so one permute over bytes of 0x80 gives 0x80 for a
+// non-negative code and 0xFF for a negative one, and that selects between the two tables and makes the sign bit.
 __device__ __forceinline__ uint32_t e4m3x4_of_nibbles(uint32_t sel) {
   const uint32_t s3 = sel & 0x7777u;
   const uint32_t pos = __byte_perm(0x44403800u, 0x4E4C4A48u, s3);
-  const uint32_t neg = __byte_perm(0xCACCCED0u, 0xB8C0C4C8u, s3);
-  const uint32_t m = sel & 0x8888u;
-  const uint32_t msb = ((m & 0x8u) << 4) | ((m & 0x80u) << 8) | ((m & 0x800u) << 12) | ((m & 0x8000u) << 16);
-  const uint32_t mask = (msb >> 7) * 0xFFu;  // 0xFF in the bytes of negative codes
-  return (pos & ~mask) | (neg & mask);
+  const uint32_t neg = __byte_perm(0x4A4C4E50u, 0x38404448u, s3);  // magnitudes
+  uint32_t r;
+  asm("prmt.b32 %0, %1, %1, %2;" : "=r"(r) : "r"(0x80808080u), "r"(sel));
+  return (pos & ~r) | (neg & r & 0x7F7F7F7Fu) | ((r << 7) & 0x80808080u);
+}
+// A packed word of the artefact (low nibbles: four consecutive k, high nibbles: the four sixteen further on) -> both fours
+__device__ __forceinline__ void e4m3_of_word(uint32_t w, uint32_t& lo, uint32_t& hi) {
+  const uint32_t a = e4m3x4_of_nibbles(w), b = e4m3x4_of_nibbles(w >> 16);  // lo0 hi0 lo1 hi1 | lo2 hi2 lo3 hi3
+  lo = __byte_perm(a, b, 0x6420);
+  hi = __byte_perm(a, b, 0x7531);
 }
 // the low nibbles of the four bytes of v, packed into bits 0-15
 __device__ __forceinline__ uint32_t low_nibbles(uint32_t v) {
@@ -67,10 +75,7 @@ __global__ void __launch_bounds__(256) expand_w_e4m3_kernel(const uint8_t* __res
   const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
   uint32_t lo[4], hi[4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    lo[j] = e4m3x4_of_nibbles(low_nibbles(w[j]));       // k = 4j .. 4j+3 of the chunk
-    hi[j] = e4m3x4_of_nibbles(low_nibbles(w[j] >> 4));  // k = 16 + 4j ..
-  }
+  for (int j = 0; j < 4; ++j) e4m3_of_word(w[j], lo[j], hi[j]);  // k = 4j .. 4j+3 of the chunk, k = 16 + 4j ..
   uint8_t* dst = w8 + row * K + (g * 4 + ch) * 32;
   *reinterpret_cast<uint4*>(dst) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
   *reinterpret_cast<uint4*>(dst + 16) = make_uint4(hi[0], hi[1], hi[2], hi[3]);

@@ -16,6 +16,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/ops/add.h>
 #include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -49,7 +50,7 @@ uint64_t g_inited = 0;              // devices ensure_init has been called for
 // attribute names, interned once
 #define DQ_NAMES(X)                                                                                   \
   X(kind) X(had_k) X(had_dim) X(scale) X(had_mat) X(w_packed) X(sw_t) X(N) X(K) X(group) X(codes)       \
-  X(sf_atoms) X(tensor_scale) X(fmt) X(_plan) X(act_quant_enabled) X(online_full_had)                  \
+  X(sf_atoms) X(tensor_scale) X(w8) X(bytes_e4m3) X(fmt) X(_plan) X(act_quant_enabled) X(online_full_had)                  \
   X(online_partial_had) X(had_K) X(act_fmt) X(quantize_bmm_input) X(dtype) X(_buffers) X(act_scale)    \
   X(_modules) X(layer) X(_parameters) X(bias) X(_packed) X(_packed_fp4)
 #define DQ_DECLARE(n) PyObject* n = nullptr;
@@ -371,6 +372,46 @@ PyObject* gemm_w4a4_int4_e4m3(PyObject*, PyObject* const* v, Py_ssize_t n) {
   });
 }
 
+// The weight's byte form (ops.PackedInt4Weight.w8, kept with the packed weight once it exists) for a batch that the
+// FP8-path GEMM serves better, or null.  Made by the first such batch: N * K bytes that used to be expanded into scratch
+// on every call.  From 256 tokens on that GEMM is the faster one on every layer shape measured (4096 -> 28672: 88 -> 68 us
+// at 300 tokens, 120 -> 76 at 500; 14336 -> 4096: 58 -> 55).  While a graph is being captured nothing is made: an
+// expansion recorded there would not have run when the next call reads it.
+constexpr int kByteFormTokens = 256;
+const uint8_t* byte_form(PyObject* pw, int M, int group) {
+  if (M < kByteFormTokens || group != 128) return nullptr;
+  {
+    Ref w8(PyObject_GetAttr(pw, names.w8));
+    if (w8.p != Py_None) return static_cast<const uint8_t*>(tensor(w8.p, "w8").data_ptr());
+  }
+  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return nullptr;
+  Ref w8(PyObject_CallMethodNoArgs(pw, names.bytes_e4m3));
+  return static_cast<const uint8_t*>(tensor(w8.p, "w8").data_ptr());
+}
+// Scratch of linear_int4 below.
+int64_t int4_scratch_bytes(const uint8_t* w8, int M, int N, int K) {
+  return static_cast<int64_t>(w8 != nullptr ? abi.dq_linear_w4a4_int4_scratch_bytes(M, N, K)
+                                            : abi.dq_linear_w4a4_int4_prefill_scratch_bytes(M, N, K));
+}
+// Activation quantiser + GEMM of one linear: with the weight's byte form on the FP8 path, else as the library chooses.
+void linear_int4(const void* x, int64_t ldx, const float* a, const dq_hadamard_desc* had, const PackedInt4& w,
+                 const uint8_t* w8, const float* r, int M, const at::Tensor& out, int mode, const at::Tensor& scratch,
+                 int idx) {
+  void* stream = stream_of(idx);
+  if (w8 == nullptr) {
+    check(abi.dq_linear_w4a4_int4(x, ldx, a, had, w.w_packed, w.sw_t, r, M, w.N, w.K, w.group, out.data_ptr(),
+                                  y_dtype_of(out), mode, scratch.data_ptr(), static_cast<size_t>(scratch.numel()), stream),
+          "dq_linear_w4a4_int4");
+    return;
+  }
+  int8_t* codes = static_cast<int8_t*>(scratch.data_ptr());
+  float* sx = reinterpret_cast<float*>(codes + (static_cast<int64_t>(M) * w.K + 255) / 256 * 256);
+  check(abi.dq_quant_act_int4(x, ldx, a, had, M, w.K, codes, sx, mode | DQ_CODES_E4M3, stream), "dq_quant_act_int4");
+  check(abi.dq_gemm_w4a4_int4_e4m3(reinterpret_cast<const uint8_t*>(codes), sx, w8, w.sw_t, r, M, w.N, w.K, w.group,
+                                   out.data_ptr(), y_dtype_of(out), nullptr, stream),
+        "dq_gemm_w4a4_int4_e4m3");
+}
+
 // linear_w4a4_int4(x, a, had, pw, r, out_dtype, scale_mode, scratch, out) -> out
 PyObject* linear_w4a4_int4(PyObject*, PyObject* const* v, Py_ssize_t n) {
   DQ_ARGS(9, "linear_w4a4_int4");
@@ -388,22 +429,18 @@ PyObject* linear_w4a4_int4(PyObject*, PyObject* const* v, Py_ssize_t n) {
       PyErr_Format(PyExc_ValueError, "K mismatch: activations %d, weight %d", K, w.K);
       throw PyError();
     }
-    // a caller's scratch is used as it is when it covers the plain path; the C side takes the
-    // FP8-path GEMM for prefill batches only if the scratch also has room for the weight's byte form
+    // a caller's scratch is used as it is when it covers the plain path
+    const uint8_t* w8 = byte_form(v[3], M, w.group);
     at::Tensor scratch;
     if (v[7] != Py_None && tensor(v[7], "scratch").numel() >=
                                static_cast<int64_t>(abi.dq_linear_w4a4_int4_scratch_bytes(M, w.N, K)))
       scratch = tensor(v[7], "scratch");
     else
-      scratch = empty({std::max<int64_t>(static_cast<int64_t>(abi.dq_linear_w4a4_int4_prefill_scratch_bytes(M, w.N, K)), 256)},
-                      at::kByte, idx);
+      scratch = empty({std::max<int64_t>(int4_scratch_bytes(w8, M, w.N, K), 256)}, at::kByte, idx);
     at::Tensor out = output(v[8], Py_None, v[5], M, w.N, idx);
     const dq_hadamard_desc d = hadamard(v[2]);
-    check(abi.dq_linear_w4a4_int4(x.data_ptr(), row_stride(x), static_cast<const float*>(ptr_or_null(v[1], "a")), desc(d),
-                                  w.w_packed, w.sw_t, static_cast<const float*>(ptr_or_null(v[4], "r")), M, w.N, K, w.group,
-                                  out.data_ptr(), y_dtype_of(out), static_cast<int>(as_long(v[6])), scratch.data_ptr(),
-                                  static_cast<size_t>(scratch.numel()), stream_of(idx)),
-          "dq_linear_w4a4_int4");
+    linear_int4(x.data_ptr(), row_stride(x), static_cast<const float*>(ptr_or_null(v[1], "a")), desc(d), w, w8,
+                static_cast<const float*>(ptr_or_null(v[4], "r")), M, out, static_cast<int>(as_long(v[6])), scratch, idx);
     return wrap(std::move(out));
   });
 }
@@ -630,8 +667,9 @@ PyObject* perm_forward(PyObject*, PyObject* const* v, Py_ssize_t n) {
     if (bias == nullptr) Py_RETURN_NONE;
     const int idx = prep(x);
     const int M = static_cast<int>(x.numel() / K);
+    const uint8_t* w8 = p->kind == PLAN_INT4 ? byte_form(p->packed, M, p->w4.group) : nullptr;
     int64_t need;
-    if (p->kind == PLAN_INT4) need = static_cast<int64_t>(abi.dq_linear_w4a4_int4_prefill_scratch_bytes(M, N, K));
+    if (p->kind == PLAN_INT4) need = int4_scratch_bytes(w8, M, N, K);
     else if (p->kind == PLAN_FP4) need = fp4_scratch_bytes(M, K, p->w_fp4.fmt);
     else need = static_cast<int64_t>(abi.dq_linear_a16w4_scratch_bytes(M, N, K));
     if (!p->scratch->defined() || p->scratch->numel() < need)
@@ -640,10 +678,7 @@ PyObject* perm_forward(PyObject*, PyObject* const* v, Py_ssize_t n) {
     sizes.back() = N;
     at::Tensor out = empty(sizes, p->out_dtype, idx);
     if (p->kind == PLAN_INT4) {
-      check(abi.dq_linear_w4a4_int4(x.data_ptr(), ldx, a, desc(p->had), p->w4.w_packed, p->w4.sw_t, nullptr, M, N, K,
-                                    p->w4.group, out.data_ptr(), y_dtype_of(out), p->scale_mode, p->scratch->data_ptr(),
-                                    static_cast<size_t>(p->scratch->numel()), stream_of(idx)),
-            "dq_linear_w4a4_int4");
+      linear_int4(x.data_ptr(), ldx, a, desc(p->had), p->w4, w8, nullptr, M, out, p->scale_mode, *p->scratch, idx);
     } else if (p->kind == PLAN_FP4) {
       linear_fp4(x.data_ptr(), false, K, M, a, p->w_fp4, nullptr, out, *p->scratch, idx);
     } else {

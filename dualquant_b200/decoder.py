@@ -77,8 +77,9 @@ class W4A4Linear:
         return buf
 
     # From this many tokens on the linears run on the FP8-path GEMM with the weight's byte form kept
-    # next to the 4-bit artefact (N * K bytes more per weight; same results bit for bit).
-    PREFILL_TOKENS = 512
+    # next to the 4-bit artefact (N * K bytes more per weight; same results bit for bit, faster on every
+    # linear of a layer).
+    PREFILL_TOKENS = 256
 
     def _gemm(self, codes, sx, out_dtype=torch.bfloat16, residual=None):
         if codes.dtype == torch.uint8:
