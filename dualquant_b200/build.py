@@ -37,6 +37,7 @@ SOURCES = [
     "gemm_w4a4_int4_f8_out1.cu",
     "gemm_w4a4_int4_f8_out2.cu",
     "gemm_w4a4_int4_f8_out3.cu",
+    "gemm_w4a4_int4_f8_out5.cu",
     "gemm_fp4_persist.cu",
     "exchange.cu",
 ]

@@ -24,6 +24,12 @@ struct DeviceState {
   int* status_dev = nullptr;  // device word written by kernels whose bounded waits expire
 };
 
+// What a GEMM epilogue adds to the linear's result: a residual [M, N] (ld = N) or a bias [N] (ld = 0); none: p null.
+struct Addend {
+  const void* p = nullptr;
+  int ld = 0;
+};
+
 DeviceState* device_state(int device);
 // State of the current device, or nullptr (and the error text set) if dq_init has not run.
 DeviceState* current_state();
@@ -111,25 +117,28 @@ int launch_gemm_fp4_persist(const uint8_t* x_codes, const uint8_t* x_sf_atoms, c
                             int M, int N, int K, int nvfp4, void* y, int y_dtype, int row_tiles, cudaStream_t stream,
                             DeviceState* st);
 int launch_gemm_int4_e4m3(const uint8_t* x8, const float* sx, const uint8_t* w8, const void* sw_t, const float* r,
-                          int M, int N, int K, void* y, int y_dtype, const void* residual, cudaStream_t stream,
+                          int M, int N, int K, void* y, int y_dtype, Addend add, cudaStream_t stream,
                           DeviceState* st);
 
 // One-launch decode linear (quantiser inside the GEMM kernel), defined in gemv_w4a4_int4_fused.cu.
 bool gemv_fused_covers(int M, int N, int K, const DeviceState* st);
 int launch_gemv_fused(const void* x_bf16, int64_t ldx, const float* a, const uint8_t* w_packed,
                       const float* r, int M, int N, int K, void* y, int y_dtype, int scale_fp16,
-                      cudaStream_t stream, DeviceState* st, const void* residual = nullptr);
+                      cudaStream_t stream, DeviceState* st, Addend add = {});
 
 // Decode-batch (register-path) variant of the int4 linear, defined in gemv_w4a4_int4.cu.
 int launch_gemm_int4_tm(const int8_t* codes, const float* sx, const uint8_t* w_packed,
                         const void* sw_t, const float* r, int M, int N, int K, void* y, int y_dtype,
                         int32_t* acc_dump, int tn, int split, cudaStream_t s, DeviceState* st,
-                        const void* residual = nullptr, bool grouped_sx = false);
+                        Addend add = {}, bool grouped_sx = false);
+// dq_gemm_w4a4_int4 with a residual or bias.
+int gemm_w4a4_int4_addend(const int8_t* codes, const float* sx, const uint8_t* w_packed, const void* sw_t, const float* r,
+                          Addend add, int M, int N, int K, int G, void* y, int y_dtype, void* stream);
 int gemv_pick_split(int tiles, int total_groups, int tok, int sm_count);
 int launch_gemv_int4(const int8_t* codes, const float* sx, const uint8_t* w_packed,
                      const void* sw_t, const float* r, int M, int N, int K, void* y, int y_dtype,
                      int tok, int split, cudaStream_t stream, DeviceState* st,
-                     const dq_allreduce_ctx* ctx = nullptr, const void* residual = nullptr,
+                     const dq_allreduce_ctx* ctx = nullptr, Addend add = {},
                      bool grouped_sx = false);
 
 }  // namespace dq

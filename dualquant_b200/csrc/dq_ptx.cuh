@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "dq_common.h"
+
 namespace dq {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -353,24 +355,25 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_addr) {
 }
 
 // ---------------------------------------------------------------------------------------
-// output element with the optional fused residual
+// output element with the optional fused addend
 // ---------------------------------------------------------------------------------------
-// Stores Y[idx] = val, or, with a residual matrix of Y's own element type, Y[idx] = residual[idx]
-// + the value a plain store would have written (for bf16 outputs the linear's result is rounded
-// to bf16 first and the sum rounded again: what a bf16 "x = x + linear(h)" computes).
-__device__ __forceinline__ void store_y(void* y, const void* residual, int y_bf16, size_t idx, float val) {
+// Stores Y[m, n] = val, or, with an addend of Y's own element type, Y[m, n] = addend + the value a plain store would
+// have written (for bf16 outputs the linear's result is rounded to bf16 first and the sum rounded again: what a bf16
+// "x = x + linear(h)" or "linear(h) + bias" computes).
+__device__ __forceinline__ void store_y(void* y, const Addend& add, int y_bf16, int m, int n, int N, float val) {
+  const size_t idx = static_cast<size_t>(m) * N + n, at = static_cast<size_t>(m) * add.ld + n;
   if (y_bf16) {
     unsigned short bits;
     asm("cvt.rn.bf16.f32 %0, %1;" : "=h"(bits) : "f"(val));
-    if (residual != nullptr) {
+    if (add.p != nullptr) {
       const float lin = __uint_as_float(static_cast<uint32_t>(bits) << 16);
-      const float res = __uint_as_float(static_cast<uint32_t>(reinterpret_cast<const unsigned short*>(residual)[idx]) << 16);
+      const float res = __uint_as_float(static_cast<uint32_t>(reinterpret_cast<const unsigned short*>(add.p)[at]) << 16);
       asm("cvt.rn.bf16.f32 %0, %1;" : "=h"(bits) : "f"(__fadd_rn(lin, res)));
     }
     reinterpret_cast<unsigned short*>(y)[idx] = bits;
   } else {
     // (an explicit add: the product that formed val must not be contracted into an FMA with it)
-    if (residual != nullptr) val = __fadd_rn(val, reinterpret_cast<const float*>(residual)[idx]);
+    if (add.p != nullptr) val = __fadd_rn(val, reinterpret_cast<const float*>(add.p)[at]);
     reinterpret_cast<float*>(y)[idx] = val;
   }
 }

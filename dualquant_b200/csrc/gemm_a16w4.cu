@@ -265,7 +265,7 @@ gemm_a16w4_kernel(const uint8_t* __restrict__ w_packed, const __grid_constant__ 
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
               const int m = t0 + c0 + j;
-              if (m < M) store_y(y, nullptr, y_bf16, static_cast<size_t>(m) * N + n, __uint_as_float(v[j]) * rn);
+              if (m < M) store_y(y, Addend{}, y_bf16, m, n, N, __uint_as_float(v[j]) * rn);
             }
           }
         }

@@ -114,7 +114,7 @@ gemm_w4a4_int4_kernel(const uint8_t* __restrict__ w_packed,
                       const __grid_constant__ CUtensorMap tm_x,
                       const __half* __restrict__ sw_t, const float* __restrict__ r,
                       const float* __restrict__ sx, void* __restrict__ y, int y_bf16,
-                      const void* __restrict__ residual, int M, int N, int K, int groups_per_split,
+                      const Addend add, int M, int N, int K, int groups_per_split,
                       int split_k, int w_stream_once, int* status) {
   using C = Cfg<TN>;
   // The 128-byte swizzle of the UMMA operands needs the buffers on 1 KB boundaries.  The kernel has
@@ -349,12 +349,10 @@ gemm_w4a4_int4_kernel(const uint8_t* __restrict__ w_packed,
           const int m0 = t0 + h * C::CPW;
           const int cnt = (M - m0 < C::CPW) ? (M - m0) : C::CPW;  // tokens of this slice that exist
           const float* sxp = sx + m0;
-          if (residual != nullptr) {
-            size_t idx = static_cast<size_t>(m0) * N + n;
+          if (add.p != nullptr) {
 #pragma unroll
             for (int j = 0; j < C::CPW; ++j) {
-              if (j < cnt) store_y(y, residual, y_bf16, idx, run[j] * (rn * __ldg(sxp + j)));
-              idx += N;
+              if (j < cnt) store_y(y, add, y_bf16, m0 + j, n, N, run[j] * (rn * __ldg(sxp + j)));
             }
           } else if (y_bf16) {
             __nv_bfloat16* yp = reinterpret_cast<__nv_bfloat16*>(y) + static_cast<size_t>(m0) * N + n;
@@ -469,7 +467,7 @@ gemm_w4a4_int4_kernel(const uint8_t* __restrict__ w_packed,
             const int n = n0 + c4 * 4 + u;
             if (n < N) {
               const float rn = (r != nullptr) ? r[n] : 1.f;
-              store_y(y, residual, y_bf16, static_cast<size_t>(m) * N + n, vals[u] * (rn * sm));
+              store_y(y, add, y_bf16, m, n, N, vals[u] * (rn * sm));
             }
           }
         }
@@ -520,10 +518,8 @@ static int pick_token_tile(int M) {
   return 128;
 }
 
-// Smallest power-of-two split (<= 8, <= TN so every rank finishes at least one token row, and
-// leaving at least two groups per CTA) that fills roughly 60% of the CTA slots of the machine;
-// beyond that the cluster reduction costs more than the extra CTAs bring (measured on the
-// Llama-3.1-8B shapes).
+// Smallest power-of-two split (<= 8, <= TN so every rank finishes at least one token row, and leaving at least two
+// groups per CTA) that fills roughly 60% of the CTA slots of the machine (for a token tile the caller has fixed).
 static int pick_split(int tiles, int total_groups, int tn, int sm_count) {
   const int target = (sm_count * ((tn <= 64) ? 2 : 1) * 6) / 10;
   int s = 1;
@@ -531,10 +527,47 @@ static int pick_split(int tiles, int total_groups, int tn, int sm_count) {
   return s;
 }
 
+// Token tile and split of K for 17 tokens and more: the cheapest by this estimate, in microseconds as measured on B200
+// with the weights streaming from HBM.  A CTA spends group_us per weight group (more where two share an SM) and 4 to 7 us
+// outside its K loop, the exchange between the CTAs of a split 0.6 us per doubling.  What matters most is whether all
+// clusters of a split fit on the chip at once: a cluster needs its slots in one GPC, which leaves about a tenth of the
+// slots unused - 32 clusters of eight or 64 of four run together, 36 or 72 take two rounds (3584 -> 4608 at 48 tokens:
+// split eight ways 12.8 us, four ways 8.0).  Before, the batch size fixed the token tile and the split filled 60 % of
+// the chip: 3584 -> 4608 at 100 tokens 18.9 us, now 12.0.
+struct Shape {
+  int tn, split;
+};
+static Shape pick_shape(int M, int row_tiles, int total_groups, int sm_count) {
+  static const struct { int tn; float group_us; } kTiles[] = {{32, 0.34f}, {64, 0.38f}, {128, 0.435f}};
+  Shape best = {128, 1};
+  float best_cost = 1e30f;
+  for (const auto& t : kTiles) {
+    if (t.tn == 32 && M > 64) continue;
+    const int clusters = row_tiles * ((M + t.tn - 1) / t.tn);
+    for (int lg = 0; lg < 4; ++lg) {
+      const int split = 1 << lg;
+      if (split > 1 && total_groups / split < 2) break;
+      const int gps = (total_groups + split - 1) / split;
+      const int slots = sm_count * (t.tn <= 64 ? 2 : 1);
+      const int fit = split == 1 ? slots : slots * 9 / 10 / split;
+      const int rounds = (clusters + fit - 1) / fit;
+      const float shared = (t.tn <= 64 && clusters * split > sm_count) ? 1.45f : 1.0f;
+      const float once = (t.tn == 128 && split > 1 ? 6.5f : 4.0f) + 0.6f * lg;
+      const float outside = t.tn == 128 && split == 1 ? once : rounds * once;  // (128 unsplit: persistent CTAs)
+      const float cost = rounds * gps * t.group_us * shared + outside;
+      if (cost < best_cost) {
+        best_cost = cost;
+        best = {t.tn, split};
+      }
+    }
+  }
+  return best;
+}
+
 template <int TN>
 static int launch(const int8_t* codes, const float* sx, const uint8_t* w_packed, const __half* sw_t,
                   const float* r, int M, int N, int K, void* y, int y_dtype, int split,
-                  cudaStream_t stream, DeviceState* st, const void* residual) {
+                  cudaStream_t stream, DeviceState* st, Addend add) {
   CUtensorMap tm_x;
   int rc = make_tmap_x_groups(&tm_x, codes, K, M, TN, Cfg<TN>::XC);
   if (rc != DQ_OK) return rc;
@@ -566,7 +599,7 @@ static int launch(const int8_t* codes, const float* sx, const uint8_t* w_packed,
   cfg.numAttrs = 2;
   const int w_stream_once = (tok_tiles == 1) ? 1 : 0;
   cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_w4a4_int4_kernel<TN>, w_packed, tm_x, sw_t, r, sx,
-                                     y, y_dtype == DQ_DTYPE_BF16 ? 1 : 0, residual, M, N, K, gps,
+                                     y, y_dtype == DQ_DTYPE_BF16 ? 1 : 0, add, M, N, K, gps,
                                      split, w_stream_once, st->status_dev);
   if (e != cudaSuccess)
     return set_error(DQ_ERR_CUDA, "gemm_w4a4_int4 launch failed (TN=%d split=%d): %s", TN, split,
@@ -591,7 +624,7 @@ using namespace dq;
 extern "C" size_t dq_gemm_w4a4_int4_workspace_bytes(int, int, int) { return 0; }
 
 static int gemm_int4_dispatch(const int8_t* codes, const float* sx, const uint8_t* w_packed,
-                              const void* sw_t, const float* r, const void* residual, int M, int N,
+                              const void* sw_t, const float* r, Addend add, int M, int N,
                               int K, int G, void* y, int y_dtype, void* stream, int token_tile,
                               int split_k, bool grouped_sx = false) {
   DeviceState* st = current_state();
@@ -618,17 +651,20 @@ static int gemm_int4_dispatch(const int8_t* codes, const float* sx, const uint8_
     DQ_REQUIRE(split <= tok && split <= total_groups, DQ_ERR_SHAPE,
                "split_k=%d too large for %d tokens / %d groups", split, tok, total_groups);
     return launch_gemv_int4(codes, sx, w_packed, sw_t, r, M, N, K, y, y_dtype, tok, split,
-                            static_cast<cudaStream_t>(stream), st, nullptr, residual, grouped_sx);
+                            static_cast<cudaStream_t>(stream), st, nullptr, add, grouped_sx);
   }
   // 1000 + tile / 2000 + tile force the shared-memory-operand / tensor-memory-operand kernel
   int forced = 0;
   if (token_tile >= 2000) { forced = 2; token_tile -= 2000; }
   else if (token_tile >= 1000) { forced = 1; token_tile -= 1000; }
-  const int tn = token_tile ? token_tile : pick_token_tile(M);
+  const int row_tiles = (N + kBN - 1) / kBN;
+  Shape shape = {token_tile ? token_tile : pick_token_tile(M), split_k};
+  if (token_tile == 0 && split_k == 0 && !grouped_sx) shape = pick_shape(M, row_tiles, total_groups, st->sm_count);
+  const int tn = shape.tn;
   DQ_REQUIRE(tn == 16 || tn == 32 || tn == 64 || tn == 128, DQ_ERR_SHAPE,
              "token tile must be 16/32/64/128 (got %d)", tn);
-  const int tiles = ((N + kBN - 1) / kBN) * ((M + tn - 1) / tn);
-  int split = split_k ? split_k : pick_split(tiles, total_groups, tn, st->sm_count);
+  const int tiles = row_tiles * ((M + tn - 1) / tn);
+  const int split = shape.split ? shape.split : pick_split(tiles, total_groups, tn, st->sm_count);
   DQ_REQUIRE(split == 1 || split == 2 || split == 4 || split == 8, DQ_ERR_SHAPE,
              "split_k must be 1/2/4/8 (got %d)", split);
   DQ_REQUIRE(split <= tn && split <= total_groups, DQ_ERR_SHAPE,
@@ -643,12 +679,12 @@ static int gemm_int4_dispatch(const int8_t* codes, const float* sx, const uint8_
   const bool use_tm = grouped_sx || (forced ? (forced == 2) : (tn <= 64));
   if (use_tm)
     return launch_gemm_int4_tm(codes, sx, w_packed, sw_t, r, M, N, K, y, y_dtype, nullptr, tn, split, s, st,
-                               residual, grouped_sx);
+                               add, grouped_sx);
   switch (tn) {
-    case 16: return launch<16>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, split, s, st, residual);
-    case 32: return launch<32>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, split, s, st, residual);
-    case 64: return launch<64>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, split, s, st, residual);
-    default: return launch<128>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, split, s, st, residual);
+    case 16: return launch<16>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, split, s, st, add);
+    case 32: return launch<32>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, split, s, st, add);
+    case 64: return launch<64>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, split, s, st, add);
+    default: return launch<128>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, split, s, st, add);
   }
 }
 
@@ -657,7 +693,7 @@ extern "C" int dq_gemm_w4a4_int4_ex(const int8_t* codes, const float* sx, const 
                                     void* y, int y_dtype, void* /*workspace*/,
                                     size_t /*workspace_bytes*/, void* stream, int token_tile,
                                     int split_k) {
-  return gemm_int4_dispatch(codes, sx, w_packed, sw_t, r, nullptr, M, N, K, G, y, y_dtype, stream,
+  return gemm_int4_dispatch(codes, sx, w_packed, sw_t, r, Addend{}, M, N, K, G, y, y_dtype, stream,
                             token_tile, split_k);
 }
 
@@ -667,14 +703,21 @@ extern "C" int dq_gemm_w4a4_int4_residual(const int8_t* codes, const float* sx,
                                           int y_dtype, void* stream) {
   DQ_REQUIRE(residual != nullptr, DQ_ERR_NULL, "null residual");
   DQ_REQUIRE(aligned(residual, y_dtype == DQ_DTYPE_BF16 ? 2 : 4), DQ_ERR_ALIGN, "misaligned residual");
-  return gemm_int4_dispatch(codes, sx, w_packed, sw_t, r, residual, M, N, K, G, y, y_dtype, stream, 0, 0);
+  return gemm_int4_dispatch(codes, sx, w_packed, sw_t, r, Addend{residual, N}, M, N, K, G, y, y_dtype, stream, 0, 0);
 }
+
+namespace dq {
+int gemm_w4a4_int4_addend(const int8_t* codes, const float* sx, const uint8_t* w_packed, const void* sw_t, const float* r,
+                          Addend add, int M, int N, int K, int G, void* y, int y_dtype, void* stream) {
+  return gemm_int4_dispatch(codes, sx, w_packed, sw_t, r, add, M, N, K, G, y, y_dtype, stream, 0, 0);
+}
+}  // namespace dq
 
 extern "C" int dq_gemm_w4a4_int4_grouped(const int8_t* codes, const float* sx_groups,
                                          const uint8_t* w_packed, const void* sw_t, const float* r,
                                          int M, int N, int K, int G, void* y, int y_dtype,
                                          void* stream) {
-  return gemm_int4_dispatch(codes, sx_groups, w_packed, sw_t, r, nullptr, M, N, K, G, y, y_dtype, stream,
+  return gemm_int4_dispatch(codes, sx_groups, w_packed, sw_t, r, Addend{}, M, N, K, G, y, y_dtype, stream,
                             0, 0, true);
 }
 
@@ -725,5 +768,5 @@ extern "C" int dq_gemm_w4a4_int4_ar_residual(const int8_t* codes, const float* s
   const int total_groups = K / kGroup;
   const int split = gemv_pick_split((N + kBN - 1) / kBN, total_groups, tok, st->sm_count);
   return launch_gemv_int4(codes, sx, w_packed, sw_t, r, M, N, K, y, y_dtype, tok, split,
-                          static_cast<cudaStream_t>(stream), st, ctx, residual);
+                          static_cast<cudaStream_t>(stream), st, ctx, Addend{residual, N});
 }

@@ -26,11 +26,13 @@ cudaError_t run_out0(int tn, const Launch& l);
 cudaError_t run_out1(int tn, const Launch& l);
 cudaError_t run_out2(int tn, const Launch& l);
 cudaError_t run_out3(int tn, const Launch& l);
+cudaError_t run_out5(int tn, const Launch& l);
 cudaError_t run_scatter(const Launch& l);
 cudaError_t init_out0();
 cudaError_t init_out1();
 cudaError_t init_out2();
 cudaError_t init_out3();
+cudaError_t init_out5();
 
 // Four two's-complement nibbles (bits 0-15 of sel) -> four E4M3 bytes of the same integers.
 // Non-negative codes 0..7: 00 38 40 44 48 4A 4C 4E; negative codes -8..-1: D0 CE CC CA C8 C4 C0 B8.
@@ -133,6 +135,7 @@ int init_gemm_int4_f8_kernels() {
   if (e == cudaSuccess) e = f8::init_out1();
   if (e == cudaSuccess) e = f8::init_out2();
   if (e == cudaSuccess) e = f8::init_out3();
+  if (e == cudaSuccess) e = f8::init_out5();
   if (e != cudaSuccess)
     return set_error(DQ_ERR_CUDA, "cudaFuncSetAttribute(gemm_w4a4_e4m3) failed: %s", cudaGetErrorString(e));
   return DQ_OK;
@@ -140,17 +143,17 @@ int init_gemm_int4_f8_kernels() {
 
 // w8 / x8: E4M3 bytes, row-major [N, K] / [M, K]
 static int launch_gemm_int4_e4m3_impl(const uint8_t* x8, const float* sx, const uint8_t* w8, const void* sw_t,
-                                      const float* r, int M, int N, int K, void* y, int y_dtype, const void* residual,
+                                      const float* r, int M, int N, int K, void* y, int y_dtype, Addend add,
                                       cudaStream_t stream, DeviceState* st, const f8::ScatterDst* scatter) {
-  f8::Launch l;
-  memset(&l, 0, sizeof(l));
+  f8::Launch l = {};
   // bf16 output (optionally with a residual) and fp32 output without one leave through tiled bulk stores (16-byte
   // aligned rows); anything else is stored directly
   const bool yb = y_dtype == DQ_DTYPE_BF16;
   int out = 0;
   if (scatter != nullptr) out = 4;
-  else if (yb && N % 8 == 0 && aligned(y, 16) && (residual == nullptr || aligned(residual, 16))) out = residual != nullptr ? 3 : 1;
-  else if (!yb && residual == nullptr && N % 4 == 0 && aligned(y, 16)) out = 2;
+  else if (yb && N % 8 == 0 && aligned(y, 16) && (add.ld == 0 || aligned(add.p, 16)))
+    out = add.p == nullptr ? 1 : add.ld == 0 ? 5 : 3;
+  else if (!yb && add.p == nullptr && N % 4 == 0 && aligned(y, 16)) out = 2;
   l.row_pairs = (N + 2 * f8::kBN - 1) / (2 * f8::kBN);
   const int pairs = st->sm_count / 2;
   const int tn = out == 4 ? 256 : f8::pick_tile(M, l.row_pairs, K / kGroup, pairs, out == 0);
@@ -160,10 +163,10 @@ static int launch_gemm_int4_e4m3_impl(const uint8_t* x8, const float* sx, const 
   rc = make_tmap_2d_u8(&l.tm_x, x8, static_cast<uint64_t>(K), static_cast<uint64_t>(M), static_cast<uint64_t>(K), 128,
                        static_cast<uint32_t>(tn / 2), CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc != DQ_OK) return rc;
-  if (out == 1 || out == 3) {
+  if (out == 1 || out == 3 || out == 5) {
     rc = make_tmap_2d_out(&l.tm_y, y, 2, static_cast<uint64_t>(N), static_cast<uint64_t>(M), f8::kBN, tn);
     if (rc == DQ_OK && out == 3)
-      rc = make_tmap_2d_out(&l.tm_res, residual, 2, static_cast<uint64_t>(N), static_cast<uint64_t>(M), f8::kBN, tn);
+      rc = make_tmap_2d_out(&l.tm_res, add.p, 2, static_cast<uint64_t>(N), static_cast<uint64_t>(M), f8::kBN, tn);
   } else if (out == 2) {
     rc = make_tmap_2d_out(&l.tm_y, y, 4, static_cast<uint64_t>(N), static_cast<uint64_t>(M), f8::kBN, tn / 2);
   }
@@ -182,7 +185,7 @@ static int launch_gemm_int4_e4m3_impl(const uint8_t* x8, const float* sx, const 
   l.sx = sx;
   l.y = y;
   l.y_bf16 = yb ? 1 : 0;
-  l.residual = residual;
+  l.add = add;
   l.M = M;
   l.N = N;
   l.K = K;
@@ -190,6 +193,7 @@ static int launch_gemm_int4_e4m3_impl(const uint8_t* x8, const float* sx, const 
   l.stream = stream;
   if (scatter != nullptr) l.sc = *scatter;
   const cudaError_t e = out == 4   ? f8::run_scatter(l)
+                        : out == 5 ? f8::run_out5(tn, l)
                         : out == 3 ? f8::run_out3(tn, l)
                         : out == 2 ? f8::run_out2(tn, l)
                         : out == 1 ? f8::run_out1(tn, l)
@@ -199,9 +203,9 @@ static int launch_gemm_int4_e4m3_impl(const uint8_t* x8, const float* sx, const 
 }
 
 int launch_gemm_int4_e4m3(const uint8_t* x8, const float* sx, const uint8_t* w8, const void* sw_t, const float* r,
-                          int M, int N, int K, void* y, int y_dtype, const void* residual, cudaStream_t stream,
+                          int M, int N, int K, void* y, int y_dtype, Addend add, cudaStream_t stream,
                           DeviceState* st) {
-  return launch_gemm_int4_e4m3_impl(x8, sx, w8, sw_t, r, M, N, K, y, y_dtype, residual, stream, st, nullptr);
+  return launch_gemm_int4_e4m3_impl(x8, sx, w8, sw_t, r, M, N, K, y, y_dtype, add, stream, st, nullptr);
 }
 
 }  // namespace dq
@@ -234,7 +238,7 @@ extern "C" int dq_gemm_w4a4_int4_e4m3_scatter(const uint8_t* x8, const float* sx
   sc.rank = ctx->rank;
   sc.tq = static_cast<int>(ctx->tokens_per_rank);
   sc.rot = static_cast<int>(((ctx->rank + 1) % ctx->world) * (ctx->tokens_per_rank / 256));
-  return launch_gemm_int4_e4m3_impl(x8, sx, w8, sw_t, r, M, N, K, nullptr, DQ_DTYPE_BF16, nullptr,
+  return launch_gemm_int4_e4m3_impl(x8, sx, w8, sw_t, r, M, N, K, nullptr, DQ_DTYPE_BF16, Addend{},
                                     static_cast<cudaStream_t>(stream), st, &sc);
 }
 
@@ -279,6 +283,6 @@ extern "C" int dq_gemm_w4a4_int4_e4m3(const uint8_t* x8, const float* sx, const 
   DQ_REQUIRE(M >= 1 && N >= 1 && K >= kGroup && K % kGroup == 0, DQ_ERR_SHAPE, "bad shape M=%d N=%d K=%d", M, N, K);
   DQ_REQUIRE(y_dtype == DQ_DTYPE_F32 || y_dtype == DQ_DTYPE_BF16, DQ_ERR_UNSUPPORTED, "unknown y_dtype %d", y_dtype);
   DQ_REQUIRE(aligned(x8, 16) && aligned(w8, 16), DQ_ERR_ALIGN, "x8 and w8 must be 16-byte aligned");
-  return launch_gemm_int4_e4m3(x8, sx, w8, sw_t, r, M, N, K, y, y_dtype, residual,
+  return launch_gemm_int4_e4m3(x8, sx, w8, sw_t, r, M, N, K, y, y_dtype, Addend{residual, N},
                                static_cast<cudaStream_t>(stream), st);
 }

@@ -94,8 +94,8 @@ struct ScatterDst {
   int rank, tq, rot;  // rot: token tiles are visited starting at tile `rot`, so that the ranks start on different owners
 };
 
-// OUT: how the output tile leaves - 0 direct stores (any shape, fp32 or bf16, optional residual),
-// 1 bf16 through shared memory and one tiled bulk store, 3 the same with the residual added, 2 fp32
+// OUT: how the output tile leaves - 0 direct stores (any shape, fp32 or bf16, optional residual or bias),
+// 1 bf16 through shared memory and one tiled bulk store, 3 the same with the residual added, 5 with a bias, 2 fp32
 // through shared memory in two halves, 4 bf16 through shared memory and then 16-byte stores into the partial
 // buffer of the rank that owns the tile's tokens (peer memory; tensor-parallel prompt pass).  A template
 // parameter: with all three epilogues in one kernel the K loop's code ran 20-25 % slower.
@@ -105,10 +105,10 @@ gemm_w4a4_e4m3_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
                       const __grid_constant__ CUtensorMap tm_y, const __grid_constant__ CUtensorMap tm_res,
                       const __half* __restrict__ sw_t, const float* __restrict__ r,
                       const float* __restrict__ sx, void* __restrict__ y, int y_bf16,
-                      const void* __restrict__ residual, int M, int N, int K, int row_pairs, int tok_tiles,
+                      const Addend add, int M, int N, int K, int row_pairs, int tok_tiles,
                       int tok_block, int* status, const __grid_constant__ ScatterDst sc) {
   using C = Cfg<TN>;
-  constexpr int bulk_out = (OUT == 3) ? 1 : OUT;  // non-zero: the tile is staged in shared memory
+  constexpr int bulk_out = (OUT == 3 || OUT == 5) ? 1 : OUT;  // non-zero: the tile is staged in shared memory
   constexpr int kTN = TN, kCPW = C::kCPW, kStages = C::kStages, kAccs = C::kAccs;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kOffBar);
@@ -298,7 +298,7 @@ gemm_w4a4_e4m3_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
           const uint4 v16 = *reinterpret_cast<const uint4*>(out_sm + tok * kBN + (lane & 15) * 8);
           *reinterpret_cast<uint4*>(base + static_cast<size_t>(tok) * N + (lane & 15) * 8) = v16;
         }
-      } else if constexpr (OUT == 1 || OUT == 3) {
+      } else if constexpr (OUT == 1 || OUT == 3 || OUT == 5) {
         // Y tile -> shared memory as [token][row] bf16 (a warp's 32 rows of one token are 64
         // contiguous bytes), then one tiled bulk store; rows past N and tokens past M are clipped
         // by the copy.  With a residual, its tile was copied into the same buffer during the K loop.  Two-byte global stores from here would cost more than two groups' UMMAs.
@@ -310,7 +310,10 @@ gemm_w4a4_e4m3_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
         const float rn = (r != nullptr && n < N) ? r[n] : 1.f;
         const float4* sx4 = reinterpret_cast<const float4*>(sx_sm + (it & 1) * kTN + h * kCPW);
         unsigned short* dst = out_sm + (h * kCPW) * kBN + q * 32 + lane;
-        // bf16(linear) [+ residual, rounded again]: what a bf16 "x = x + linear(h)" computes
+        // bf16(linear) [+ residual or bias, rounded again]: what a bf16 "x = x + linear(h)" computes
+        float bias = 0.f;
+        if (OUT == 5 && n < N)
+          bias = __uint_as_float(static_cast<uint32_t>(reinterpret_cast<const unsigned short*>(add.p)[n]) << 16);
         auto put = [&](int j, float val) {
           unsigned short bits = __bfloat16_as_ushort(__float2bfloat16_rn(val));
           if (bulk_res) {
@@ -318,6 +321,9 @@ gemm_w4a4_e4m3_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
             const float res = __uint_as_float(static_cast<uint32_t>(dst[j * kBN]) << 16);
             bits = __bfloat16_as_ushort(__float2bfloat16_rn(__fadd_rn(lin, res)));
           }
+          if (OUT == 5)
+            bits = __bfloat16_as_ushort(
+                __float2bfloat16_rn(__fadd_rn(__uint_as_float(static_cast<uint32_t>(bits) << 16), bias)));
           dst[j * kBN] = bits;
         };
 #pragma unroll
@@ -383,30 +389,9 @@ gemm_w4a4_e4m3_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
       } else if (n < N) {  // OUT == 0
         const float rn = (r != nullptr) ? r[n] : 1.f;
         const int m0 = t0 + h * kCPW;
-        const int cnt = (M - m0 < kCPW) ? (M - m0) : kCPW;
-        const float* sxp = sx + m0;
-        if (residual != nullptr) {
-          size_t idx = static_cast<size_t>(m0) * N + n;
 #pragma unroll
-          for (int j = 0; j < kCPW; ++j) {
-            if (j < cnt) store_y(y, residual, y_bf16, idx, run[j] * (rn * __ldg(sxp + j)));
-            idx += N;
-          }
-        } else if (y_bf16) {
-          __nv_bfloat16* yp = reinterpret_cast<__nv_bfloat16*>(y) + static_cast<size_t>(m0) * N + n;
-#pragma unroll
-          for (int j = 0; j < kCPW; ++j) {
-            if (j < cnt) *yp = __float2bfloat16_rn(run[j] * (rn * __ldg(sxp + j)));
-            yp += N;
-          }
-        } else {
-          float* yp = reinterpret_cast<float*>(y) + static_cast<size_t>(m0) * N + n;
-#pragma unroll
-          for (int j = 0; j < kCPW; ++j) {
-            if (j < cnt) *yp = run[j] * (rn * __ldg(sxp + j));
-            yp += N;
-          }
-        }
+        for (int j = 0; j < kCPW; ++j)
+          if (m0 + j < M) store_y(y, add, y_bf16, m0 + j, n, N, run[j] * (rn * __ldg(sx + m0 + j)));
       }
     }
     if constexpr (OUT == 4) __threadfence_system();  // this thread's stores to peers are performed before the kernel ends
@@ -477,7 +462,7 @@ struct Launch {
   const float *r, *sx;
   void* y;
   int y_bf16;
-  const void* residual;
+  Addend add;
   int M, N, K, row_pairs, tok_tiles, tok_block;
   int* status;
   ScatterDst sc;
@@ -487,7 +472,7 @@ struct Launch {
 template <int TN, int OUT>
 cudaError_t run(const Launch& l) {
   return launch_pdl(gemm_w4a4_e4m3_kernel<TN, OUT>, dim3(l.ctas), dim3(kThreads), Cfg<TN>::kSmemBytes, l.stream, l.tm_w,
-                    l.tm_x, l.tm_y, l.tm_res, l.sw_t, l.r, l.sx, l.y, l.y_bf16, l.residual, l.M, l.N, l.K, l.row_pairs,
+                    l.tm_x, l.tm_y, l.tm_res, l.sw_t, l.r, l.sx, l.y, l.y_bf16, l.add, l.M, l.N, l.K, l.row_pairs,
                     l.tok_tiles, l.tok_block, l.status, l.sc);
 }
 template <int TN, int OUT>

@@ -137,7 +137,7 @@ gemm_w4a4_int4_tm_kernel(const uint8_t* __restrict__ w_packed,
                          const __grid_constant__ CUtensorMap tm_x,
                          const __half* __restrict__ sw_t, const float* __restrict__ r,
                          const float* __restrict__ sx, void* __restrict__ y, int y_bf16,
-                         const void* __restrict__ residual,
+                         const Addend add,
                          int32_t* __restrict__ acc_dump, int M, int N, int K,
                          int groups_per_split, int split_k, int w_stream_once, int* status) {
   using C = Cfg<TN>;
@@ -391,12 +391,10 @@ gemm_w4a4_int4_tm_kernel(const uint8_t* __restrict__ w_packed,
             if constexpr (GS) return 1.f;
             return __ldg(sxp + j);
           };
-          if (residual != nullptr) {
-            size_t idx = static_cast<size_t>(m0) * N + n;
+          if (add.p != nullptr) {
 #pragma unroll
             for (int j = 0; j < C::CPW; ++j) {
-              if (j < cnt) store_y(y, residual, y_bf16, idx, run[j] * (rn * tok_scale(j)));
-              idx += N;
+              if (j < cnt) store_y(y, add, y_bf16, m0 + j, n, N, run[j] * (rn * tok_scale(j)));
             }
           } else if (y_bf16) {
             __nv_bfloat16* yp = reinterpret_cast<__nv_bfloat16*>(y) + static_cast<size_t>(m0) * N + n;
@@ -533,7 +531,7 @@ gemm_w4a4_int4_tm_kernel(const uint8_t* __restrict__ w_packed,
             const int n = n0 + c4 * 4 + u;
             if (n < N) {
               const float rn = (r != nullptr) ? r[n] : 1.f;
-              store_y(y, residual, y_bf16, static_cast<size_t>(m) * N + n, vals[u] * (rn * sm));
+              store_y(y, add, y_bf16, m, n, N, vals[u] * (rn * sm));
             }
           }
         }
@@ -568,7 +566,7 @@ static int set_attr() {
 template <int TN, int MODE>
 static int launch(const int8_t* codes, const float* sx, const uint8_t* w_packed, const __half* sw_t,
                   const float* r, int M, int N, int K, void* y, int y_dtype, int32_t* acc_dump,
-                  int split, cudaStream_t stream, DeviceState* st, const void* residual) {
+                  int split, cudaStream_t stream, DeviceState* st, Addend add) {
   CUtensorMap tm_x;
   int rc = make_tmap_x_groups(&tm_x, codes, K, M, TN, kStepGroups);
   if (rc != DQ_OK) return rc;
@@ -591,7 +589,7 @@ static int launch(const int8_t* codes, const float* sx, const uint8_t* w_packed,
   cfg.numAttrs = 2;
   const int w_stream_once = (tok_tiles == 1) ? 1 : 0;
   cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_w4a4_int4_tm_kernel<TN, MODE>, w_packed, tm_x, sw_t,
-                                     r, sx, y, y_dtype == DQ_DTYPE_BF16 ? 1 : 0, residual, acc_dump, M, N, K,
+                                     r, sx, y, y_dtype == DQ_DTYPE_BF16 ? 1 : 0, add, acc_dump, M, N, K,
                                      gps, split, w_stream_once, st->status_dev);
   if (e != cudaSuccess)
     return set_error(DQ_ERR_CUDA, "gemm_w4a4_int4 (tm) launch failed (TN=%d split=%d): %s", TN,
@@ -620,26 +618,26 @@ int init_gemm_int4_tm_kernels() {
 int launch_gemm_int4_tm(const int8_t* codes, const float* sx, const uint8_t* w_packed,
                         const void* sw_t, const float* r, int M, int N, int K, void* y, int y_dtype,
                         int32_t* acc_dump, int tn, int split, cudaStream_t s, DeviceState* st,
-                        const void* residual, bool grouped_sx) {
+                        Addend add, bool grouped_sx) {
   const __half* swp = static_cast<const __half*>(sw_t);
   if (grouped_sx && acc_dump == nullptr) {
     switch (tn) {
-      case 16: return tm::launch<16, 2>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, nullptr, split, s, st, residual);
-      case 32: return tm::launch<32, 2>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, nullptr, split, s, st, residual);
-      case 64: return tm::launch<64, 2>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, nullptr, split, s, st, residual);
-      default: return tm::launch<128, 2>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, nullptr, split, s, st, residual);
+      case 16: return tm::launch<16, 2>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, nullptr, split, s, st, add);
+      case 32: return tm::launch<32, 2>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, nullptr, split, s, st, add);
+      case 64: return tm::launch<64, 2>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, nullptr, split, s, st, add);
+      default: return tm::launch<128, 2>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, nullptr, split, s, st, add);
     }
   }
   if (acc_dump != nullptr) {
     if (tn == 16)
-      return tm::launch<16, 1>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, acc_dump, 1, s, st, residual);
-    return tm::launch<128, 1>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, acc_dump, 1, s, st, residual);
+      return tm::launch<16, 1>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, acc_dump, 1, s, st, add);
+    return tm::launch<128, 1>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, acc_dump, 1, s, st, add);
   }
   switch (tn) {
-    case 16: return tm::launch<16, 0>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, nullptr, split, s, st, residual);
-    case 32: return tm::launch<32, 0>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, nullptr, split, s, st, residual);
-    case 64: return tm::launch<64, 0>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, nullptr, split, s, st, residual);
-    default: return tm::launch<128, 0>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, nullptr, split, s, st, residual);
+    case 16: return tm::launch<16, 0>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, nullptr, split, s, st, add);
+    case 32: return tm::launch<32, 0>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, nullptr, split, s, st, add);
+    case 64: return tm::launch<64, 0>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, nullptr, split, s, st, add);
+    default: return tm::launch<128, 0>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, nullptr, split, s, st, add);
   }
 }
 

@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(kVThreads, VCfg<NT>::kMinCtas)
 gemv_w4a4_int4_kernel(const uint8_t* __restrict__ w_packed,
                       const __grid_constant__ CUtensorMap tm_x,
                       const float* __restrict__ r, const float* __restrict__ sx,
-                      void* __restrict__ y, int y_bf16, const void* __restrict__ residual, int M, int N,
+                      void* __restrict__ y, int y_bf16, const Addend add, int M, int N,
                       int K, int groups_per_split, int split_k, int stages, int* status, const ArDev ar) {
   using C = VCfg<NT>;
   extern __shared__ uint8_t smem_raw[];
@@ -310,7 +310,7 @@ gemv_w4a4_int4_kernel(const uint8_t* __restrict__ w_packed,
             for (int e = 0; e < 2; ++e) {
               const int m = nb * 8 + 2 * t + e;
               if (m < M) {
-                store_y(y, residual, y_bf16, static_cast<size_t>(m) * N + n, run[nb][2 * hrow + e] * (GS ? rn : rn * sx[m]));
+                store_y(y, add, y_bf16, m, n, N, run[nb][2 * hrow + e] * (GS ? rn : rn * sx[m]));
               }
             }
         }
@@ -371,7 +371,7 @@ gemv_w4a4_int4_kernel(const uint8_t* __restrict__ w_packed,
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
               const int n = n0 + c4 * 4 + u;
-              if (n < N) store_y(y, residual, y_bf16, static_cast<size_t>(m) * N + n, vals[u]);
+              if (n < N) store_y(y, add, y_bf16, m, n, N, vals[u]);
             }
           }
         }
@@ -410,7 +410,7 @@ gemv_w4a4_int4_kernel(const uint8_t* __restrict__ w_packed,
               }
               const float vals[4] = {acc.x, acc.y, acc.z, acc.w};
 #pragma unroll
-              for (int u = 0; u < 4; ++u) store_y(y, residual, y_bf16, static_cast<size_t>(m) * N + nb + u, vals[u]);
+              for (int u = 0; u < 4; ++u) store_y(y, add, y_bf16, m, nb + u, N, vals[u]);
             }
           }
         }
@@ -459,7 +459,7 @@ template <int NT, bool GS>
 static int launch_gemv_t(const int8_t* codes, const float* sx, const uint8_t* w_packed,
                          const __half* sw_t, const float* r, int M, int N, int K, void* y,
                          int y_dtype, int split, cudaStream_t stream, DeviceState* st,
-                         const ArDev& ar, const void* residual) {
+                         const ArDev& ar, Addend add) {
   using C = VCfg<NT>;
   CUtensorMap tm_x;
   int rc = make_tmap_x_groups(&tm_x, codes, K, M, C::kXRows, kVGS);
@@ -494,7 +494,7 @@ static int launch_gemv_t(const int8_t* codes, const float* sx, const uint8_t* w_
   cfg.attrs = attr;
   cfg.numAttrs = 2;
   cudaError_t e = cudaLaunchKernelEx(&cfg, gemv_w4a4_int4_kernel<NT, GS>, w_packed, tm_x, r, sx, y,
-                                     y_dtype == DQ_DTYPE_BF16 ? 1 : 0, residual, M, N, K, gps, split,
+                                     y_dtype == DQ_DTYPE_BF16 ? 1 : 0, add, M, N, K, gps, split,
                                      stages, st->status_dev, ar);
   if (e != cudaSuccess)
     return set_error(DQ_ERR_CUDA, "gemv_w4a4_int4 launch failed (tokens=%d split=%d): %s", C::TOK,
@@ -506,7 +506,7 @@ static int launch_gemv_t(const int8_t* codes, const float* sx, const uint8_t* w_
 int launch_gemv_int4(const int8_t* codes, const float* sx, const uint8_t* w_packed,
                      const void* sw_t, const float* r, int M, int N, int K, void* y, int y_dtype,
                      int tok, int split, cudaStream_t stream, DeviceState* st,
-                     const dq_allreduce_ctx* ctx, const void* residual, bool grouped_sx) {
+                     const dq_allreduce_ctx* ctx, Addend add, bool grouped_sx) {
   const __half* swp = static_cast<const __half*>(sw_t);
   ArDev ar = {};
   ar.world = 1;
@@ -537,13 +537,13 @@ int launch_gemv_int4(const int8_t* codes, const float* sx, const uint8_t* w_pack
   if (tok != 8 && tok != 16 && tok != 32)
     return set_error(DQ_ERR_SHAPE, "register-path token capacity must be 8/16/32 (got %d)", tok);
   if (grouped_sx) {
-    rc = (tok == 8) ? launch_gemv_t<1, true>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, split, stream, st, ar, residual)
-       : (tok == 16) ? launch_gemv_t<2, true>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, split, stream, st, ar, residual)
-                     : launch_gemv_t<4, true>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, split, stream, st, ar, residual);
+    rc = (tok == 8) ? launch_gemv_t<1, true>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, split, stream, st, ar, add)
+       : (tok == 16) ? launch_gemv_t<2, true>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, split, stream, st, ar, add)
+                     : launch_gemv_t<4, true>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, split, stream, st, ar, add);
   } else {
-    rc = (tok == 8) ? launch_gemv_t<1, false>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, split, stream, st, ar, residual)
-       : (tok == 16) ? launch_gemv_t<2, false>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, split, stream, st, ar, residual)
-                     : launch_gemv_t<4, false>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, split, stream, st, ar, residual);
+    rc = (tok == 8) ? launch_gemv_t<1, false>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, split, stream, st, ar, add)
+       : (tok == 16) ? launch_gemv_t<2, false>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, split, stream, st, ar, add)
+                     : launch_gemv_t<4, false>(codes, sx, w_packed, swp, r, M, N, K, y, y_dtype, split, stream, st, ar, add);
   }
   if (rc == DQ_OK && ar.world > 1) {
     ar_bump_kernel<<<1, 1, 0, stream>>>(static_cast<uint32_t*>(ctx->seq));

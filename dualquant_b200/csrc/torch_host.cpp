@@ -13,6 +13,7 @@
 #include <Python.h>
 
 #include <ATen/core/Tensor.h>
+#include <ATen/core/grad_mode.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/ops/add.h>
 #include <c10/cuda/CUDAFunctions.h>
@@ -34,7 +35,7 @@ namespace {
 #define DQ_FUNCTIONS(X)                                                                              \
   X(dq_quant_act_int4) X(dq_quant_act_int4_f32) X(dq_quant_act_int4_gated) X(dq_quant_act_int4_rmsnorm) \
   X(dq_gemm_w4a4_int4_ex) X(dq_gemm_w4a4_int4_residual) X(dq_gemm_w4a4_int4_e4m3)                      \
-  X(dq_linear_w4a4_int4) X(dq_linear_w4a4_int4_scratch_bytes)                                         \
+  X(dq_linear_w4a4_int4) X(dq_linear_w4a4_int4_bias) X(dq_linear_w4a4_int4_scratch_bytes)                                         \
   X(dq_linear_w4a4_int4_prefill_scratch_bytes) X(dq_linear_a16w4) X(dq_linear_a16w4_scratch_bytes)     \
   X(dq_quant_fp4_atoms) X(dq_fp4_sf_atoms_bytes) X(dq_gemm_w4a4_fp4_tiled)
 #define DQ_DECLARE(name) decltype(&::name) name = nullptr;
@@ -395,21 +396,18 @@ int64_t int4_scratch_bytes(const uint8_t* w8, int M, int N, int K) {
 }
 // Activation quantiser + GEMM of one linear: with the weight's byte form on the FP8 path, else as the library chooses.
 void linear_int4(const void* x, int64_t ldx, const float* a, const dq_hadamard_desc* had, const PackedInt4& w,
-                 const uint8_t* w8, const float* r, int M, const at::Tensor& out, int mode, const at::Tensor& scratch,
-                 int idx) {
+                 const uint8_t* w8, const float* r, const void* bias, int M, const at::Tensor& out, int mode,
+                 const at::Tensor& scratch, int idx) {
   void* stream = stream_of(idx);
-  if (w8 == nullptr) {
+  const size_t bytes = static_cast<size_t>(scratch.numel());
+  if (w8 == nullptr && bias == nullptr)
     check(abi.dq_linear_w4a4_int4(x, ldx, a, had, w.w_packed, w.sw_t, r, M, w.N, w.K, w.group, out.data_ptr(),
-                                  y_dtype_of(out), mode, scratch.data_ptr(), static_cast<size_t>(scratch.numel()), stream),
+                                  y_dtype_of(out), mode, scratch.data_ptr(), bytes, stream),
           "dq_linear_w4a4_int4");
-    return;
-  }
-  int8_t* codes = static_cast<int8_t*>(scratch.data_ptr());
-  float* sx = reinterpret_cast<float*>(codes + (static_cast<int64_t>(M) * w.K + 255) / 256 * 256);
-  check(abi.dq_quant_act_int4(x, ldx, a, had, M, w.K, codes, sx, mode | DQ_CODES_E4M3, stream), "dq_quant_act_int4");
-  check(abi.dq_gemm_w4a4_int4_e4m3(reinterpret_cast<const uint8_t*>(codes), sx, w8, w.sw_t, r, M, w.N, w.K, w.group,
-                                   out.data_ptr(), y_dtype_of(out), nullptr, stream),
-        "dq_gemm_w4a4_int4_e4m3");
+  else
+    check(abi.dq_linear_w4a4_int4_bias(x, ldx, a, had, w.w_packed, w8, w.sw_t, r, bias, M, w.N, w.K, w.group,
+                                       out.data_ptr(), y_dtype_of(out), mode, scratch.data_ptr(), bytes, stream),
+          "dq_linear_w4a4_int4_bias");
 }
 
 // linear_w4a4_int4(x, a, had, pw, r, out_dtype, scale_mode, scratch, out) -> out
@@ -440,7 +438,7 @@ PyObject* linear_w4a4_int4(PyObject*, PyObject* const* v, Py_ssize_t n) {
     at::Tensor out = output(v[8], Py_None, v[5], M, w.N, idx);
     const dq_hadamard_desc d = hadamard(v[2]);
     linear_int4(x.data_ptr(), row_stride(x), static_cast<const float*>(ptr_or_null(v[1], "a")), desc(d), w, w8,
-                static_cast<const float*>(ptr_or_null(v[4], "r")), M, out, static_cast<int>(as_long(v[6])), scratch, idx);
+                static_cast<const float*>(ptr_or_null(v[4], "r")), nullptr, M, out, static_cast<int>(as_long(v[6])), scratch, idx);
     return wrap(std::move(out));
   });
 }
@@ -677,8 +675,18 @@ PyObject* perm_forward(PyObject*, PyObject* const* v, Py_ssize_t n) {
     c10::SmallVector<int64_t, 5> sizes(x.sizes().begin(), x.sizes().end());
     sizes.back() = N;
     at::Tensor out = empty(sizes, p->out_dtype, idx);
+    // a bias of the output's type is added in the GEMM's epilogue, any other (or one that wants a gradient) by torch
+    const void* bias_ptr = nullptr;
+    if (p->kind == PLAN_INT4 && bias != Py_None) {
+      const at::Tensor& b = tensor(bias, "bias");
+      if (b.scalar_type() == p->out_dtype && b.dim() == 1 && b.is_contiguous() && b.is_cuda() &&
+          b.get_device() == p->device && !(b.requires_grad() && at::GradMode::is_enabled())) {
+        bias_ptr = b.data_ptr();
+        bias = Py_None;
+      }
+    }
     if (p->kind == PLAN_INT4) {
-      linear_int4(x.data_ptr(), ldx, a, desc(p->had), p->w4, w8, nullptr, M, out, p->scale_mode, *p->scratch, idx);
+      linear_int4(x.data_ptr(), ldx, a, desc(p->had), p->w4, w8, nullptr, bias_ptr, M, out, p->scale_mode, *p->scratch, idx);
     } else if (p->kind == PLAN_FP4) {
       linear_fp4(x.data_ptr(), false, K, M, a, p->w_fp4, nullptr, out, *p->scratch, idx);
     } else {

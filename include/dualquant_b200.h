@@ -486,6 +486,19 @@ DQ_API int dq_linear_w4a4_int4(const void* x_bf16, int64_t ldx, const float* a,
                         int scale_fp16, void* scratch, size_t scratch_bytes, void* stream);
 
 /*
+ * The same linear with what a layer adds or keeps (PermLinear.forward of a layer with a bias,
+ * activations/perm_linear.py:136-141 into F.linear):
+ *   bias [N] of y's element type or null: for bf16 added to the rounded result and rounded again, as "linear(x) + bias"
+ *   w8   the weight's byte form from dq_expand_w_int4_e4m3, or null: with it the call runs on the FP8-path GEMM whatever
+ *        the batch size, and expands nothing
+ * scratch: dq_linear_w4a4_int4_scratch_bytes(M,N,K) bytes.
+ */
+DQ_API int dq_linear_w4a4_int4_bias(const void* x_bf16, int64_t ldx, const float* a, const dq_hadamard_desc* had,
+                                    const uint8_t* w_packed, const uint8_t* w8, const void* sw_t, const float* r,
+                                    const void* bias, int M, int N, int K, int G, void* y, int y_dtype, int scale_fp16,
+                                    void* scratch, size_t scratch_bytes, void* stream);
+
+/*
  * A16W4: 16-bit activations against the int4 weight artefact - the reference's fused-beta kernel
  * (vendor/dualscale_kernel_benchmark/fused_dual_scale_kernel.py:55-149, wrapper :220-262) and what
  * PermLinear computes when its activation cast is switched off (activations/perm_linear.py:108-141

@@ -438,3 +438,18 @@ def test_quant_act_many_rows_bit_exact(M, K):
     q, s, _ = O.quant_act_int4(x, a, None, scale_fp16=True)
     assert torch.equal(codes.cpu(), q)
     assert torch.equal(sx.cpu(), s)
+
+
+@pytest.mark.parametrize("M", [17, 33, 64, 65, 100, 129, 200, 255])
+@pytest.mark.parametrize("N,K", [(96, 256), (4608, 3584), (4104, 1152), (5000, 128)])
+def test_chosen_tile_and_split_against_the_unsplit_kernel(M, N, K):
+    """Whatever token tile and split the library picks for a medium batch, the result equals the unsplit kernel's up
+    to the order of fp32 sums, with a residual and with a bias added in the epilogue."""
+    g = torch.Generator(device=DEV).manual_seed(M * 7 + N)
+    pw = ops.pack_w_int4(*ops.quant_w_int4((torch.randn(N, K, generator=g, device=DEV) * 0.02).to(torch.bfloat16)))
+    codes, sx = ops.quant_act_int4(torch.randn(M, K, generator=g, device=DEV).to(torch.bfloat16))
+    ref = ops.gemm_w4a4_int4(codes, sx, pw, token_tile=1128, split_k=1)
+    res = torch.randn(M, N, generator=g, device=DEV)
+    for y, want in ((ops.gemm_w4a4_int4(codes, sx, pw), ref), (ops.gemm_w4a4_int4(codes, sx, pw, residual=res), ref + res)):
+        assert ((y - want).abs().max() / want.abs().max()).item() < 1e-6
+    _lib.device_status(0)

@@ -237,7 +237,7 @@ def test_native_forward_equals_the_python_forward_and_follows_changes(name):
     if name == "off":
         pl.set_act_quant_enabled(False)
     pl._packed_fp4 is None and name in ("mxfp4", "nvfp4") and pl.pack_fp4(pl._fp4_fmt(), force=True)
-    for shape in ((1, K), (2, 3, K), (1, 40, K), (1100, K)):
+    for shape in ((1, K), (2, 3, K), (1, 40, K), (100, K), (300, K), (1100, K)):  # every GEMM kernel's bias
         x = torch.randn(*shape, device=DEV).to(torch.bfloat16)
         ref = pl._forward(x)
         assert pl._plan is not None
