@@ -114,7 +114,7 @@ int init_gemm_int4_f8_kernels();
 int init_gemm_fp4_persist_kernels();
 int launch_gemm_fp4_persist(const uint8_t* x_codes, const uint8_t* x_sf_atoms, const float* x_scale,
                             const uint8_t* w_codes, const uint8_t* w_sf_atoms, const float* w_scale, const float* r,
-                            int M, int N, int K, int nvfp4, void* y, int y_dtype, int row_tiles, cudaStream_t stream,
+                            const void* bias, int M, int N, int K, int nvfp4, void* y, int y_dtype, int row_tiles, cudaStream_t stream,
                             DeviceState* st);
 int launch_gemm_int4_e4m3(const uint8_t* x8, const float* sx, const uint8_t* w8, const void* sw_t, const float* r,
                           int M, int N, int K, void* y, int y_dtype, Addend add, cudaStream_t stream,
@@ -134,6 +134,8 @@ int launch_gemm_int4_tm(const int8_t* codes, const float* sx, const uint8_t* w_p
 // dq_gemm_w4a4_int4 with a residual or bias.
 int gemm_w4a4_int4_addend(const int8_t* codes, const float* sx, const uint8_t* w_packed, const void* sw_t, const float* r,
                           Addend add, int M, int N, int K, int G, void* y, int y_dtype, void* stream);
+int quant_fp4_activations(const void* x, int x_is_f32, int64_t ldx, const float* a, int M, int K, int fmt, uint8_t* codes,
+                          uint8_t* sf_atoms, float* row_scale, cudaStream_t s);
 int gemv_pick_split(int tiles, int total_groups, int tok, int sm_count);
 int launch_gemv_int4(const int8_t* codes, const float* sx, const uint8_t* w_packed,
                      const void* sw_t, const float* r, int M, int N, int K, void* y, int y_dtype,

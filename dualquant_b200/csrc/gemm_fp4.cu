@@ -66,7 +66,7 @@ gemm_fp4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                 const __grid_constant__ CUtensorMap tm_y, int bulk_store,
                 const uint8_t* __restrict__ sfw, const uint8_t* __restrict__ sfx,
                 const float* __restrict__ r, const float* __restrict__ w_scale,
-                const float* __restrict__ x_scale, void* __restrict__ y, int y_bf16, int M, int N,
+                const float* __restrict__ x_scale, const void* __restrict__ bias, void* __restrict__ y, int y_bf16, int M, int N,
                 int K, int stages_per_split, int split_k, int tok_fast, int row_tile0, int* status) {
   using C = FCfg<NT>;
   constexpr int kFStages = C::kStages;
@@ -114,6 +114,7 @@ gemm_fp4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     tma_prefetch_desc(&tm_x);
     if (bulk_store) tma_prefetch_desc(&tm_y);
   }
+  grid_dep_launch_dependents();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -121,6 +122,8 @@ gemm_fp4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
+    // The ring is filled with weights and their scale factors first; the activation operands come from the kernel
+    // before this one (programmatic dependent launch).
     const uint64_t pol = l2_policy_evict_last();
     const uint8_t* sfw_tile = sfw + (static_cast<size_t>(n0 / kFBN) * total_st + st_begin) * kSfBytes;
     const uint8_t* sfx_tile = sfx + (static_cast<size_t>(t0 / kFTN) * total_st + st_begin) * kSfBytes;
@@ -128,15 +131,23 @@ gemm_fp4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     // Only lane 0 works; the other lanes go straight to the end of the role (32 lanes polling a
     // barrier cost issue slots and barrier-unit bandwidth that the other warps need).
     if (lane == 0) {
-      for (int i = 0; i < nst; ++i) {
-        const int s = i % kFStages;
-        if (!mbar_wait(&empty[s], ((i / kFStages) & 1) ^ 1, abort_flag, FSITE_TMA)) break;
+      auto load_w = [&](int i, int s) {
         // the activation box is the CTA's whole token tile (rows past M arrive as zeros and count)
         mbar_expect_tx(&full[s], kFTileBytes + C::kBTileBytes + (1 + nblk) * kSfBytes);
         tma_load_2d(smem + C::kOffA + s * kFTileBytes, &tm_w, (st_begin + i) * 128, n0, &full[s], pol);
-        tma_load_2d(smem + C::kOffB + s * C::kBTileBytes, &tm_x, (st_begin + i) * 128, t0, &full[s], pol);
         bulk_load_1d(smem + C::kOffSFA + s * 2048, sfw_tile + static_cast<size_t>(i) * kSfBytes,
                      kSfBytes, &full[s], pol);
+      };
+      const int ahead = nst < kFStages ? nst : kFStages;
+      for (int i = 0; i < ahead; ++i) load_w(i, i);
+      grid_dep_wait();
+      for (int i = 0; i < nst; ++i) {
+        const int s = i % kFStages;
+        if (i >= ahead) {
+          if (!mbar_wait(&empty[s], ((i / kFStages) & 1) ^ 1, abort_flag, FSITE_TMA)) break;
+          load_w(i, s);
+        }
+        tma_load_2d(smem + C::kOffB + s * C::kBTileBytes, &tm_x, (st_begin + i) * 128, t0, &full[s], pol);
         for (int b = 0; b < nblk; ++b)
           bulk_load_1d(smem + C::kOffSFB + (s * C::kSfBlocks + b) * 2048,
                        sfx_tile + b * sfx_block + static_cast<size_t>(i) * kSfBytes, kSfBytes, &full[s], pol);
@@ -209,6 +220,7 @@ gemm_fp4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
   // other role, and - when the output goes through bulk stores - the producer, issuer and copier
   // warps once their loops are over (four warps alone are too few to hide the latency of their own
   // instruction chains).  The teams take alternate 32-token chunks.
+  grid_dep_wait();  // the token scales come from the kernel before this one; so does what last used y
   const int team = (warp >= 2 && warp < 6) ? 0 : 1;
   const int nteams = (split_k == 1 && bulk_store) ? 2 : 1;
   if (team < nteams) {
@@ -225,6 +237,7 @@ gemm_fp4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
       rn = (r != nullptr) ? r[n] : 1.f;
       if (w_scale != nullptr) rn *= *w_scale;
     }
+    const float bias_n = n < N ? bias_value(bias, y_bf16, n) : 0.f;
 #pragma unroll 1
     for (int c0 = team * 32; c0 < col_end; c0 += 32 * nteams) {
       uint32_t v[32];
@@ -248,9 +261,9 @@ gemm_fp4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
           const float tx = (x_scale != nullptr && m < M) ? x_scale[m] : 1.f;
           const float val = __uint_as_float(v[j]) * (rn * tx);
           if (y_bf16)
-            reinterpret_cast<__nv_bfloat16*>(buf)[j * kFBN + q * 32 + lane] = __float2bfloat16_rn(val);
+            reinterpret_cast<__nv_bfloat16*>(buf)[j * kFBN + q * 32 + lane] = bf16_with_bias(val, bias, bias_n);
           else
-            reinterpret_cast<float*>(buf)[j * kFBN + q * 32 + lane] = val;
+            reinterpret_cast<float*>(buf)[j * kFBN + q * 32 + lane] = bias != nullptr ? __fadd_rn(val, bias_n) : val;
         }
         fence_proxy_async_smem();  // generic-proxy writes before the async-proxy read of the store
         if (team == 0)  // the four warps of the team
@@ -270,9 +283,9 @@ gemm_fp4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
               const float tx = (x_scale != nullptr) ? x_scale[m] : 1.f;
               const float val = __uint_as_float(v[j]) * (rn * tx);
               if (y_bf16)
-                reinterpret_cast<__nv_bfloat16*>(y)[static_cast<size_t>(m) * N + n] = __float2bfloat16_rn(val);
+                reinterpret_cast<__nv_bfloat16*>(y)[static_cast<size_t>(m) * N + n] = bf16_with_bias(val, bias, bias_n);
               else
-                reinterpret_cast<float*>(y)[static_cast<size_t>(m) * N + n] = val;
+                reinterpret_cast<float*>(y)[static_cast<size_t>(m) * N + n] = bias != nullptr ? __fadd_rn(val, bias_n) : val;
             }
           }
         }
@@ -314,11 +327,11 @@ gemm_fp4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
           const int nn = n0 + c4 * 4 + u;
           if (nn < N) {
             const float rr = ((r != nullptr) ? r[nn] : 1.f) * ws;
-            const float val = vals[u] * (rr * tx);
+            const float val = vals[u] * (rr * tx), bias_n = bias_value(bias, y_bf16, nn);
             if (y_bf16)
-              reinterpret_cast<__nv_bfloat16*>(y)[static_cast<size_t>(m) * N + nn] = __float2bfloat16_rn(val);
+              reinterpret_cast<__nv_bfloat16*>(y)[static_cast<size_t>(m) * N + nn] = bf16_with_bias(val, bias, bias_n);
             else
-              reinterpret_cast<float*>(y)[static_cast<size_t>(m) * N + nn] = val;
+              reinterpret_cast<float*>(y)[static_cast<size_t>(m) * N + nn] = bias != nullptr ? __fadd_rn(val, bias_n) : val;
           }
         }
       }
@@ -409,11 +422,9 @@ extern "C" int dq_gemm_w4a4_fp4(const uint8_t* x_codes, const uint8_t* x_sf_atom
                                 fmt, y, y_dtype, 0, stream);  // 0: the library picks the token tile
 }
 
-extern "C" int dq_gemm_w4a4_fp4_tiled(const uint8_t* x_codes, const uint8_t* x_sf_atoms,
-                                      const float* x_scale, const uint8_t* w_codes,
-                                      const uint8_t* w_sf_atoms, const float* w_scale,
-                                      const float* r, int M, int N, int K, int fmt, void* y,
-                                      int y_dtype, int token_tile, void* stream) {
+static int gemm_fp4(const uint8_t* x_codes, const uint8_t* x_sf_atoms, const float* x_scale, const uint8_t* w_codes,
+                    const uint8_t* w_sf_atoms, const float* w_scale, const float* r, const void* bias, int M, int N, int K,
+                    int fmt, void* y, int y_dtype, int token_tile, void* stream) {
   DeviceState* st = current_state();
   if (st == nullptr) return DQ_ERR_NOT_INIT;
   if (M == 0) return DQ_OK;
@@ -446,7 +457,7 @@ extern "C" int dq_gemm_w4a4_fp4_tiled(const uint8_t* x_codes, const uint8_t* x_s
       else if (tiles256 >= st->sm_count && K >= 8192)  // long K loops only: a second launch costs ~10 us
         rt_p = static_cast<int>((tiles256 / st->sm_count) * st->sm_count / tok256);
       if (rt_p > 0) {
-        int rc0 = launch_gemm_fp4_persist(x_codes, x_sf_atoms, x_scale, w_codes, w_sf_atoms, w_scale, r, M, N, K,
+        int rc0 = launch_gemm_fp4_persist(x_codes, x_sf_atoms, x_scale, w_codes, w_sf_atoms, w_scale, r, bias, M, N, K,
                                           fmt == DQ_FP4_NVFP4 ? 1 : 0, y, y_dtype, rt_p,
                                           static_cast<cudaStream_t>(stream), st);
         if (rc0 != DQ_OK || rt_p == rt_all) return rc0;
@@ -494,22 +505,60 @@ extern "C" int dq_gemm_w4a4_fp4_tiled(const uint8_t* x_codes, const uint8_t* x_s
   cfg.blockDim = dim3(kFThreads, 1, 1);
   cfg.dynamicSmemBytes = (nt == 2) ? FCfg<2>::kSmemBytes : (nt == 1) ? FCfg<1>::kSmemBytes : FCfg<0>::kSmemBytes;
   cfg.stream = static_cast<cudaStream_t>(stream);
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 1;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = split;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   const int bf = y_dtype == DQ_DTYPE_BF16 ? 1 : 0;
   cudaError_t e;
   auto kern = (fmt == DQ_FP4_NVFP4)
                   ? (nt == 2 ? gemm_fp4_kernel<1, 2> : nt == 1 ? gemm_fp4_kernel<1, 1> : gemm_fp4_kernel<1, 0>)
                   : (nt == 2 ? gemm_fp4_kernel<0, 2> : nt == 1 ? gemm_fp4_kernel<0, 1> : gemm_fp4_kernel<0, 0>);
-  e = cudaLaunchKernelEx(&cfg, kern, tm_w, tm_x, tm_y, bulk_store, w_sf_atoms, x_sf_atoms, r, w_scale, x_scale, y, bf, M, N,
+  e = cudaLaunchKernelEx(&cfg, kern, tm_w, tm_x, tm_y, bulk_store, w_sf_atoms, x_sf_atoms, r, w_scale, x_scale, bias, y, bf, M, N,
                          K, sps, split, tok_fast, row_tile0, st->status_dev);
   if (e != cudaSuccess)
     return set_error(DQ_ERR_CUDA, "gemm_fp4 launch failed (split=%d): %s", split, cudaGetErrorString(e));
   DQ_CHECK_CUDA(cudaGetLastError());
   return DQ_OK;
+}
+
+extern "C" int dq_gemm_w4a4_fp4_tiled(const uint8_t* x_codes, const uint8_t* x_sf_atoms,
+                                      const float* x_scale, const uint8_t* w_codes,
+                                      const uint8_t* w_sf_atoms, const float* w_scale,
+                                      const float* r, int M, int N, int K, int fmt, void* y,
+                                      int y_dtype, int token_tile, void* stream) {
+  return gemm_fp4(x_codes, x_sf_atoms, x_scale, w_codes, w_sf_atoms, w_scale, r, nullptr, M, N, K, fmt, y, y_dtype,
+                  token_tile, stream);
+}
+
+static size_t up256(size_t v) { return (v + 255) / 256 * 256; }
+
+extern "C" size_t dq_linear_w4a4_fp4_scratch_bytes(int M, int K, int fmt) {
+  if (M < 1 || K < 1) return 0;
+  return up256(static_cast<size_t>(M) * K / 2) + up256(dq_fp4_sf_atoms_bytes(M, K, fmt)) + up256(static_cast<size_t>(M) * 4);
+}
+
+extern "C" int dq_linear_w4a4_fp4(const void* x, int x_is_f32, int64_t ldx, const float* a, const uint8_t* w_codes,
+                                  const uint8_t* w_sf_atoms, const float* w_scale, const float* r, const void* bias, int M,
+                                  int N, int K, int fmt, void* y, int y_dtype, void* scratch, size_t scratch_bytes,
+                                  void* stream) {
+  if (current_state() == nullptr) return DQ_ERR_NOT_INIT;
+  if (M == 0) return DQ_OK;
+  DQ_REQUIRE(fmt == DQ_FP4_MXFP4 || fmt == DQ_FP4_NVFP4, DQ_ERR_UNSUPPORTED, "unknown FP4 format %d", fmt);
+  DQ_REQUIRE(scratch != nullptr && aligned(scratch, 256), DQ_ERR_ALIGN, "scratch must be non-null and 256-byte aligned");
+  DQ_REQUIRE(M >= 1 && K >= kFKStage && K % kFKStage == 0, DQ_ERR_SHAPE, "bad shape M=%d K=%d (K %% %d != 0)", M, K, kFKStage);
+  DQ_REQUIRE(scratch_bytes >= dq_linear_w4a4_fp4_scratch_bytes(M, K, fmt), DQ_ERR_WORKSPACE,
+             "scratch of %zu bytes is smaller than the %zu required", scratch_bytes, dq_linear_w4a4_fp4_scratch_bytes(M, K, fmt));
+  uint8_t* codes = static_cast<uint8_t*>(scratch);
+  uint8_t* sf = codes + up256(static_cast<size_t>(M) * K / 2);
+  float* row_scale =
+      fmt == DQ_FP4_NVFP4 ? reinterpret_cast<float*>(sf + up256(dq_fp4_sf_atoms_bytes(M, K, fmt))) : nullptr;
+  const int rc = quant_fp4_activations(x, x_is_f32, ldx, a, M, K, fmt, codes, sf, row_scale, static_cast<cudaStream_t>(stream));
+  if (rc != DQ_OK) return rc;
+  return gemm_fp4(codes, sf, row_scale, w_codes, w_sf_atoms, w_scale, r, bias, M, N, K, fmt, y, y_dtype, 0, stream);
 }

@@ -3,7 +3,20 @@
 #include "dq_common.h"
 #include "dq_ptx.cuh"
 
+#include <cuda_bf16.h>
+
 namespace dq {
+
+// Bias of output column n (of Y's element type), 0 without one; and the bf16 result of a linear with it: rounded, then
+// the sum rounded again, as "linear(x) + bias" computes.
+__device__ __forceinline__ float bias_value(const void* bias, int y_bf16, int n) {
+  if (bias == nullptr) return 0.f;
+  return y_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(bias)[n]) : static_cast<const float*>(bias)[n];
+}
+__device__ __forceinline__ __nv_bfloat16 bf16_with_bias(float val, const void* bias, float b) {
+  const __nv_bfloat16 y = __float2bfloat16_rn(val);
+  return bias == nullptr ? y : __float2bfloat16_rn(__fadd_rn(__bfloat162float(y), b));
+}
 
 constexpr int kFBN = 128;      // weight rows per CTA
 constexpr int kFTN = 128;      // tokens per scale-factor block

@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 gemm_fp4_persist_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
                         const __grid_constant__ CUtensorMap tm_y, const uint8_t* __restrict__ sfw,
                         const uint8_t* __restrict__ sfx, const float* __restrict__ r,
-                        const float* __restrict__ w_scale, const float* __restrict__ x_scale, int y_bf16, int M,
+                        const float* __restrict__ w_scale, const float* __restrict__ x_scale, const void* __restrict__ bias, int y_bf16, int M,
                         int N, int K, int row_tiles, int tok_tiles, int tok_block, int* status) {
   constexpr int kAtoms = NVFP4 ? 4 : 2;  // scale-factor atoms per operand block per stage
   constexpr uint32_t kSfBytes = kAtoms * 512;
@@ -232,6 +232,7 @@ gemm_fp4_persist_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_c
         rn = (r != nullptr) ? r[n] : 1.f;
         if (w_scale != nullptr) rn *= *w_scale;
       }
+      const float bias_n = n < N ? bias_value(bias, y_bf16, n) : 0.f;
       if (!mbar_wait(acc_full, it & 1, abort_flag, PSITE_EPI)) break;
       tc_fence_after();
       // all of this warp's columns (up to four chunks of 32) to registers, then the accumulator
@@ -262,9 +263,9 @@ gemm_fp4_persist_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_c
             const float tx = (x_scale != nullptr && m < M) ? __ldg(x_scale + m) : 1.f;
             const float val = __uint_as_float(v[k][j]) * (rn * tx);
             if (y_bf16)
-              reinterpret_cast<__nv_bfloat16*>(buf)[j * kFBN + q * 32 + lane] = __float2bfloat16_rn(val);
+              reinterpret_cast<__nv_bfloat16*>(buf)[j * kFBN + q * 32 + lane] = bf16_with_bias(val, bias, bias_n);
             else
-              reinterpret_cast<float*>(buf)[j * kFBN + q * 32 + lane] = val;
+              reinterpret_cast<float*>(buf)[j * kFBN + q * 32 + lane] = bias != nullptr ? __fadd_rn(val, bias_n) : val;
           }
           fence_proxy_async_smem();
           if (team == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -306,7 +307,7 @@ int init_gemm_fp4_persist_kernels() {
 // Processes row tiles [0, row_tiles) of the weight (the caller may give the rest to the one-tile kernel).
 int launch_gemm_fp4_persist(const uint8_t* x_codes, const uint8_t* x_sf_atoms, const float* x_scale,
                             const uint8_t* w_codes, const uint8_t* w_sf_atoms, const float* w_scale, const float* r,
-                            int M, int N, int K, int nvfp4, void* y, int y_dtype, int row_tiles, cudaStream_t stream,
+                            const void* bias, int M, int N, int K, int nvfp4, void* y, int y_dtype, int row_tiles, cudaStream_t stream,
                             DeviceState* st) {
   CUtensorMap tm_w, tm_x, tm_y;
   int rc = make_tmap_2d_u8(&tm_w, w_codes, static_cast<uint64_t>(K) / 2, N, static_cast<uint64_t>(K) / 2, 128, kFBN,
@@ -329,11 +330,11 @@ int launch_gemm_fp4_persist(const uint8_t* x_codes, const uint8_t* x_sf_atoms, c
   cudaError_t e;
   if (nvfp4)
     e = launch_pdl(fp4p::gemm_fp4_persist_kernel<1>, dim3(grid), dim3(fp4p::kThreads), fp4p::kSmemBytes, stream, tm_w,
-                   tm_x, tm_y, w_sf_atoms, x_sf_atoms, r, w_scale, x_scale, bf, M, N, K, row_tiles, tok_tiles,
+                   tm_x, tm_y, w_sf_atoms, x_sf_atoms, r, w_scale, x_scale, bias, bf, M, N, K, row_tiles, tok_tiles,
                    tok_block, st->status_dev);
   else
     e = launch_pdl(fp4p::gemm_fp4_persist_kernel<0>, dim3(grid), dim3(fp4p::kThreads), fp4p::kSmemBytes, stream, tm_w,
-                   tm_x, tm_y, w_sf_atoms, x_sf_atoms, r, w_scale, x_scale, bf, M, N, K, row_tiles, tok_tiles,
+                   tm_x, tm_y, w_sf_atoms, x_sf_atoms, r, w_scale, x_scale, bias, bf, M, N, K, row_tiles, tok_tiles,
                    tok_block, st->status_dev);
   if (e != cudaSuccess) return set_error(DQ_ERR_CUDA, "gemm_fp4_persist launch failed: %s", cudaGetErrorString(e));
   return DQ_OK;

@@ -11,6 +11,7 @@
 // in registers, 8 consecutive elements per thread; a block spans 2 (NVFP4) or 4 (MXFP4) lanes.
 // HBM-bound: 2 bytes in, 0.5 byte + scale out per element.
 #include "dq_common.h"
+#include "dq_ptx.cuh"
 
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -18,21 +19,37 @@
 namespace dq {
 
 enum { FP4_MODE_CODES = 0, FP4_MODE_FAKE = 1 };
-// the streaming kernel (several small CTAs per SM) takes over from the row-in-registers kernel
-constexpr int kFp4StreamMinRows = 512;  // rows: enough CTAs to fill the SMs several times
-constexpr int kFp4StreamMinVec = 1024;  // MXFP4: vectors of 8 per row (K >= 8192); shorter rows are as fast in registers
-constexpr int kFp4StreamMinVecNv = 256;  // NVFP4 (two phases per row): from K = 2048 (6-10 % at K = 3584-4096)
+constexpr int kFp4ManyRows = 512;  // from here on the chip is full of rows: fewer threads per row, more rows per SM
 
-__device__ __forceinline__ uint32_t e2m1x2(float lo, float hi) {
-  uint16_t out;
+// Eight values -> eight E2M1 codes in one word, the first in the lowest nibble.
+__device__ __forceinline__ uint32_t e2m1x8(const float* v) {
+  uint32_t out;
   asm("{\n"
-      ".reg .b8 t;\n"
-      "cvt.rn.satfinite.e2m1x2.f32 t, %1, %2;\n"
-      "cvt.u16.u8 %0, t;\n"
+      ".reg .b8 t0, t1, t2, t3;\n"
+      "cvt.rn.satfinite.e2m1x2.f32 t0, %2, %1;\n"
+      "cvt.rn.satfinite.e2m1x2.f32 t1, %4, %3;\n"
+      "cvt.rn.satfinite.e2m1x2.f32 t2, %6, %5;\n"
+      "cvt.rn.satfinite.e2m1x2.f32 t3, %8, %7;\n"
+      "mov.b32 %0, {t0, t1, t2, t3};\n"
       "}\n"
-      : "=h"(out)
-      : "f"(hi), "f"(lo));
-  return out;  // high nibble = hi, low nibble = lo
+      : "=r"(out)
+      : "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]));
+  return out;
+}
+// The eight values times f, two per instruction.
+__device__ __forceinline__ void mul8(const float* v, float f, float* out) {
+#pragma unroll
+  for (int k = 0; k < 8; k += 2) {
+    const float2 t = __fmul2_rn(make_float2(v[k], v[k + 1]), make_float2(f, f));
+    out[k] = t.x;
+    out[k + 1] = t.y;
+  }
+}
+// 1 / x to one unit in the last place, subnormals flushed
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
 }
 
 __device__ __forceinline__ float e2m1_value(uint32_t code) {
@@ -49,11 +66,20 @@ __device__ __forceinline__ uint32_t e4m3_byte_of(float v) {
   return out & 0xFFu;  // second operand lands in the low byte
 }
 
-__device__ __forceinline__ float e4m3_value(uint32_t byte) {
-  // unsigned use only (scales are non-negative): 4 exponent bits (bias 7), 3 mantissa bits
-  const uint32_t e = (byte >> 3) & 0xF, m = byte & 7;
-  if (e == 0) return static_cast<float>(m) * 0.001953125f;  // m * 2^-9
-  return __uint_as_float(((e + 120u) << 23) | (m << 20));
+// Scale bytes of an NVFP4 block: want = bmax / 6 / ts, clamped to the normal range of E4M3 [2^-6, 448] before the cast, as
+// the reference's scale quantiser does (scale_formats.py:39-45): an all-zero or tiny block gets the scale 2^-6.  The
+// quotient is estimated with a product (inv6ts = 1 / 6 / ts, within 2^-21); where both ends of that interval convert to
+// the same byte, so does the quotient, and the two IEEE divisions are left to the blocks on a rounding boundary.
+__device__ __forceinline__ uint32_t nvfp4_scale_byte(float bmax, float ts, float inv6ts) {
+  const float w = __fmul_rn(bmax, inv6ts);
+  const float lo = fmaxf(fminf(__fmul_rn(w, 0.99999904632568359375f), 448.0f), 0.015625f);  // 1 - 2^-20
+  const float hi = fmaxf(fminf(__fmul_rn(w, 1.00000095367431640625f), 448.0f), 0.015625f);  // 1 + 2^-20
+  unsigned short two;
+  asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(two) : "f"(hi), "f"(lo));
+  const uint32_t b = two & 0xFFu;
+  if (b == static_cast<uint32_t>(two >> 8) && inv6ts >= 1e-30f && inv6ts <= 1e30f) return b;
+  const float want = __fdiv_rn(__fdiv_rn(bmax, 6.0f), ts);
+  return e4m3_byte_of(fmaxf(fminf(want, 448.0f), 0.015625f));
 }
 
 __device__ __forceinline__ void fp4_load8(const __nv_bfloat16* p, float* v) {
@@ -75,13 +101,13 @@ __device__ __forceinline__ void fp4_load8(const float* p, float* v) {
 // One vector of 8 consecutive elements (already scaled by the column scale) whose block absmax is
 // known: block scale, element codes, stores.  sf_off = where this vector's block scale byte goes
 // (used by the first vector of a block only).
-__device__ __forceinline__ void fp4_emit_vector(const float* v, float bmax, float ts, int fmt, int mode,
+__device__ __forceinline__ void fp4_emit_vector(const float* v, float bmax, float ts, float inv6ts, int fmt, int mode,
                                                 int row, int K, int idx, int blk, int64_t sf_off,
                                                 uint8_t* __restrict__ codes, uint8_t* __restrict__ sf,
                                                 float* __restrict__ out) {
     float q[8];
     float deq_scale;
-    uint32_t sf_byte;
+    uint32_t sf_byte, packed;
     if (fmt == DQ_FP4_MXFP4) {
       int e = -127;
       if (bmax != 0.f) {
@@ -89,58 +115,37 @@ __device__ __forceinline__ void fp4_emit_vector(const float* v, float bmax, floa
         e = max(-127, min(127, e));
       }
       sf_byte = static_cast<uint32_t>(e + 127);
-      // 2^-e is representable (as a subnormal at the far end), so one multiplication rounds
-      // exactly like scalbnf(v, -e) would
-      const float down = scalbnf(1.0f, -e);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) q[k] = __fmul_rn(v[k], down);
-      deq_scale = scalbnf(1.0f, e);
+      // 2^-e and 2^e by their bits (subnormal at the far end): one multiplication rounds exactly like scalbnf(v, -e)
+      const float down = __uint_as_float(e == 127 ? 0x00400000u : static_cast<uint32_t>(127 - e) << 23);
+      deq_scale = __uint_as_float(e == -127 ? 0x00400000u : static_cast<uint32_t>(127 + e) << 23);
+      mul8(v, down, q);
+      packed = e2m1x8(q);
     } else {
-      const float want = __fdiv_rn(__fdiv_rn(bmax, 6.0f), ts);
-      // clamped to the normal range of E4M3 [2^-6, 448] before the cast, as the reference's scale
-      // quantiser does (scale_formats.py:39-45): an all-zero or tiny block gets the scale 2^-6
-      sf_byte = e4m3_byte_of(fmaxf(fminf(want, 448.0f), 0.015625f));
-      const float bs = e4m3_value(sf_byte);
+      sf_byte = nvfp4_scale_byte(bmax, ts, inv6ts);
+      const float bs = __uint_as_float((sf_byte << 20) + (120u << 23));  // a normal E4M3 number, by its bits
       const float denom = __fmul_rn(ts, bs);
       deq_scale = denom;
       if (mode == FP4_MODE_FAKE) deq_scale = bs;  // applied as (q * bs) * ts below
       if (denom == 0.f) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) q[k] = 0.f;
+        packed = 0;
       } else {
-        // v / denom rounded to E2M1 without eight IEEE divisions: t = v * (1 / denom) is within
-        // 2^-22 |t| of the quotient; if t (1 - 2^-21) and t (1 + 2^-21) convert to the same codes,
-        // so does everything between them, the correctly rounded quotient included.  Otherwise
-        // (an element sits on a rounding boundary, or t is not finite) the thread takes the exact
-        // divisions, in a branch of its own.
-        const float inv = __fdiv_rn(1.0f, denom);
-        float lo[8], hi[8];
-        bool exact = false;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const float t = __fmul_rn(v[k], inv);
-          exact |= !(fabsf(t) <= 1e30f);
-          lo[k] = __fmul_rn(t, 0.99999952316284179688f);  // 1 - 2^-21
-          hi[k] = __fmul_rn(t, 1.00000047683715820312f);  // 1 + 2^-21
-        }
-        uint32_t plo = 0, phi = 0;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          plo |= e2m1x2(lo[2 * k], lo[2 * k + 1]) << (8 * k);
-          phi |= e2m1x2(hi[2 * k], hi[2 * k + 1]) << (8 * k);
-        }
-        if (exact || plo != phi) {
+        // v / denom rounded to E2M1 without eight IEEE divisions: t = v * rcp(denom) is within 2^-21.4 |t| of the
+        // quotient; if t (1 - 2^-20) and t (1 + 2^-20) convert to the same codes, so does everything between them, the
+        // correctly rounded quotient included.  Otherwise (an element sits on a rounding boundary, or the reciprocal
+        // left its range) the thread takes the exact divisions, in a branch of its own.
+        const float inv = rcp_approx(denom);
+        float t[8], lo[8], hi[8];
+        mul8(v, inv, t);
+        mul8(t, 0.99999904632568359375f, lo);  // 1 - 2^-20
+        mul8(t, 1.00000095367431640625f, hi);  // 1 + 2^-20
+        packed = e2m1x8(lo);
+        if (packed != e2m1x8(hi) || !(inv >= 1e-30f && inv <= 1e30f && __fmul_rn(bmax, inv) <= 1e30f)) {
 #pragma unroll
           for (int k = 0; k < 8; ++k) q[k] = __fdiv_rn(v[k], denom);
-        } else {
-#pragma unroll
-          for (int k = 0; k < 8; ++k) q[k] = lo[k];
+          packed = e2m1x8(q);
         }
       }
     }
-    uint32_t packed = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) packed |= e2m1x2(q[2 * k], q[2 * k + 1]) << (8 * k);
     if (mode == FP4_MODE_CODES) {
       *reinterpret_cast<uint32_t*>(codes + static_cast<int64_t>(row) * (K / 2) + idx / 2) = packed;
       if ((idx % blk) == 0) sf[sf_off] = static_cast<uint8_t>(sf_byte);
@@ -157,64 +162,104 @@ __device__ __forceinline__ void fp4_emit_vector(const float* v, float bmax, floa
     }
 }
 
-template <int THREADS, int VPT, typename XT>
-__global__ void __launch_bounds__(THREADS)
+// Eight input elements as loaded (bf16: one 16-byte vector; fp32: two).
+template <typename XT>
+struct Fp4Raw;
+template <>
+struct Fp4Raw<__nv_bfloat16> {
+  uint4 r;
+  __device__ __forceinline__ void load(const __nv_bfloat16* p) { r = *reinterpret_cast<const uint4*>(p); }
+  __device__ __forceinline__ void expand(float* v) const {
+    const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      v[2 * i] = __uint_as_float(w[i] << 16);
+      v[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+    }
+  }
+};
+template <>
+struct Fp4Raw<float> {
+  float v8[8];
+  __device__ __forceinline__ void load(const float* p) { fp4_load8(p, v8); }
+  __device__ __forceinline__ void expand(float* v) const {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = v8[i];
+  }
+};
+
+// One CTA per row, the row in registers in its input width: all of a row's loads are in flight at once, and it is read
+// from memory once although NVFP4 needs the row's absmax before its first block scale.  The column scale is applied
+// again in the second pass (from L1).  PER_SM CTAs' worth of registers.
+template <int THREADS, int VPT, int PER_SM, typename XT>
+__global__ void __launch_bounds__(THREADS, PER_SM)
 quant_fp4_kernel(const XT* __restrict__ x, int64_t ldx, const float* __restrict__ a, int K, int fmt,
                  const float* __restrict__ tensor_scale, uint8_t* __restrict__ codes,
                  uint8_t* __restrict__ sf, float* __restrict__ row_scale, float* __restrict__ out,
-                 int mode, int M, int sf_atoms) {
+                 int mode, int M, int sf_atoms, int activations) {
   // THREADS bounds the launch; the CTA may be smaller (a multiple of 32): vectors are dealt out
   // with the launched size as the stride, so that a row of K/8 vectors leaves few idle slots.
   __shared__ float red[THREADS / 32];
+  // x comes from the kernel before this one.  As the first half of a linear (activations = 1) the GEMM behind it may
+  // start at once and fetch its weights; a stand-alone call may be making those weights.
+  if (activations) grid_dep_launch_dependents();
+  grid_dep_wait();
   const int nthreads = static_cast<int>(blockDim.x);
   const int row = blockIdx.x;
   // sf_atoms: the scale bytes go straight into the order the GEMM streams,
   // [row tile of 128][k / (4 blocks)][(r % 32) * 16 + (r / 32) * 4 + block % 4]; the grid then
   // covers the rows up to the next multiple of 128 and the CTAs past M write zero scales.
-  const int blk_sz = (fmt == DQ_FP4_MXFP4) ? 32 : 16;
-  const int nsf = K / blk_sz;
-  auto sf_offset = [&](int ksf) -> int64_t {
-    if (!sf_atoms) return static_cast<int64_t>(row) * nsf + ksf;
-    const int rr = row & 127;
-    return (static_cast<int64_t>(row >> 7) * (nsf >> 2) + (ksf >> 2)) * 512 + (rr & 31) * 16 +
-           (rr >> 5) * 4 + (ksf & 3);
-  };
+  const int lg_blk = (fmt == DQ_FP4_MXFP4) ? 5 : 4;
+  const int nsf = K >> lg_blk;
+  const int rr = row & 127;
+  uint8_t* sf_row = sf + (sf_atoms ? static_cast<int64_t>(row >> 7) * (nsf >> 2) * 512 + (rr & 31) * 16 + (rr >> 5) * 4
+                                   : static_cast<int64_t>(row) * nsf);
+  auto sf_offset = [&](int ksf) -> int64_t { return sf_atoms ? (ksf >> 2) * 512 + (ksf & 3) : ksf; };
   if (row >= M) {
-    for (int ksf = threadIdx.x; ksf < nsf; ksf += nthreads) sf[sf_offset(ksf)] = 0;
+    for (int ksf = threadIdx.x; ksf < nsf; ksf += nthreads) sf_row[sf_offset(ksf)] = 0;
     return;
   }
   const XT* xr = x + static_cast<int64_t>(row) * ldx;
-  float v[VPT][8];
-  float bmax[VPT];
-  float rmax = 0.f;
+  Fp4Raw<XT> raw[VPT];
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int idx = (i * nthreads + threadIdx.x) * 8;
-    bmax[i] = 0.f;
-    if (idx < K) {
-      fp4_load8(xr + idx, v[i]);
-      if (a != nullptr) {
-        float av[8];
-        fp4_load8(a + idx, av);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) v[i][e] = __fmul_rn(v[i][e], av[e]);
-      }
-#pragma unroll
-      for (int e = 0; e < 8; ++e) bmax[i] = fmaxf(bmax[i], fabsf(v[i][e]));
-    } else {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) v[i][e] = 0.f;
-    }
-    // block absmax: 16 elements = 2 adjacent lanes, 32 elements = 4 adjacent lanes
-    bmax[i] = fmaxf(bmax[i], __shfl_xor_sync(0xffffffffu, bmax[i], 1));
-    if (fmt == DQ_FP4_MXFP4) bmax[i] = fmaxf(bmax[i], __shfl_xor_sync(0xffffffffu, bmax[i], 2));
-    rmax = fmaxf(rmax, bmax[i]);
+    if (idx < K) raw[i].load(xr + idx);
   }
-  float ts = 1.f;
+  auto scaled = [&](int i, int idx, float* v) {
+    raw[i].expand(v);
+    if (a != nullptr) {
+      float av[8];
+      fp4_load8(a + idx, av);
+#pragma unroll
+      for (int e = 0; e < 8; e += 2) {
+        const float2 t = __fmul2_rn(make_float2(v[e], v[e + 1]), make_float2(av[e], av[e + 1]));
+        v[e] = t.x;
+        v[e + 1] = t.y;
+      }
+    }
+  };
+  auto absmax8 = [&](const float* v) -> float {
+    float m = fabsf(v[0]);
+#pragma unroll
+    for (int e = 1; e < 8; ++e) m = fmaxf(m, fabsf(v[e]));
+    return m;
+  };
+  float ts = 1.f, inv6ts = 1.f;
   if (fmt == DQ_FP4_NVFP4) {
     if (tensor_scale != nullptr) {
       ts = *tensor_scale;
     } else {
+      float rmax = 0.f;
+#pragma unroll
+      for (int i = 0; i < VPT; ++i) {
+        const int idx = (i * nthreads + threadIdx.x) * 8;
+        if (idx < K) {
+          float v[8];
+          scaled(i, idx, v);
+          rmax = fmaxf(rmax, absmax8(v));
+        }
+      }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
       if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = rmax;
@@ -224,98 +269,21 @@ quant_fp4_kernel(const XT* __restrict__ x, int64_t ldx, const float* __restrict_
       ts = (m == 0.f) ? 1.f : __fdiv_rn(m, 2688.0f);
     }
     if (threadIdx.x == 0 && row_scale != nullptr) row_scale[row] = ts;
+    inv6ts = __fmul_rn(rcp_approx(ts), 0.16666667163372039794921875f);
   }
-  const int blk = (fmt == DQ_FP4_MXFP4) ? 32 : 16;
 #pragma unroll
-  for (int i = 0; i < VPT; ++i) {
+  for (int i = 0; i < VPT; ++i) {  // every lane runs every vector: the shuffles need the warp
     const int idx = (i * nthreads + threadIdx.x) * 8;
-    if (idx >= K) continue;
-    fp4_emit_vector(v[i], bmax[i], ts, fmt, mode, row, K, idx, blk, sf_offset(idx / blk), codes, sf, out);
-  }
-}
-
-// The same quantiser for many long rows: a CTA of 256 threads walks its row in steps of 256
-// vectors instead of holding it in registers, so that several CTAs share an SM and one row's loads
-// overlap another row's arithmetic (the register version runs one 800-thread CTA per SM at
-// K = 18944).  NVFP4 without a given tensor scale needs the row's absmax first: a first pass over
-// the row, which the second pass then finds in L2.  Same per-vector arithmetic (fp4_emit_vector),
-// same results.
-template <typename XT>
-__global__ void __launch_bounds__(256, 6)  // 39 registers: six CTAs per SM (four measured 12 % slower)
-quant_fp4_stream_kernel(const XT* __restrict__ x, int64_t ldx, const float* __restrict__ a, int K, int fmt,
-                        const float* __restrict__ tensor_scale, uint8_t* __restrict__ codes,
-                        uint8_t* __restrict__ sf, float* __restrict__ row_scale, float* __restrict__ out,
-                        int mode, int M, int sf_atoms) {
-  constexpr int T = 256;
-  __shared__ float red[T / 32];
-  const int row = blockIdx.x;
-  const int blk = (fmt == DQ_FP4_MXFP4) ? 32 : 16;
-  const int nsf = K / blk;
-  auto sf_offset = [&](int ksf) -> int64_t {
-    if (!sf_atoms) return static_cast<int64_t>(row) * nsf + ksf;
-    const int rr = row & 127;
-    return (static_cast<int64_t>(row >> 7) * (nsf >> 2) + (ksf >> 2)) * 512 + (rr & 31) * 16 +
-           (rr >> 5) * 4 + (ksf & 3);
-  };
-  if (row >= M) {
-    for (int ksf = threadIdx.x; ksf < nsf; ksf += T) sf[sf_offset(ksf)] = 0;
-    return;
-  }
-  const XT* xr = x + static_cast<int64_t>(row) * ldx;
-  const int nvec = K / 8;
-  const int iters = (nvec + T - 1) / T;
-  auto load_scaled = [&](int idx, float* v) {
-    fp4_load8(xr + idx, v);
-    if (a != nullptr) {
-      float av[8];
-      fp4_load8(a + idx, av);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) v[e] = __fmul_rn(v[e], av[e]);
-    }
-  };
-  float ts = 1.f;
-  if (fmt == DQ_FP4_NVFP4) {
-    if (tensor_scale != nullptr) {
-      ts = *tensor_scale;
-    } else {
-      float rmax = 0.f;
-      for (int it = 0; it < iters; ++it) {
-        const int idx = (it * T + threadIdx.x) * 8;
-        if (idx < K) {
-          float v[8];
-          load_scaled(idx, v);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) rmax = fmaxf(rmax, fabsf(v[e]));
-        }
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
-      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = rmax;
-      __syncthreads();
-      float m = red[0];
-#pragma unroll
-      for (int i = 1; i < T / 32; ++i) m = fmaxf(m, red[i]);
-      ts = (m == 0.f) ? 1.f : __fdiv_rn(m, 2688.0f);
-    }
-    if (threadIdx.x == 0 && row_scale != nullptr) row_scale[row] = ts;
-  }
-  for (int it = 0; it < iters; ++it) {  // every lane runs every iteration: the shuffles need the warp
-    const int idx = (it * T + threadIdx.x) * 8;
-    float v[8];
-    float bmax = 0.f;
+    float v[8], bmax = 0.f;
     if (idx < K) {
-      load_scaled(idx, v);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) bmax = fmaxf(bmax, fabsf(v[e]));
-    } else {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) v[e] = 0.f;
+      scaled(i, idx, v);
+      bmax = absmax8(v);
     }
     // block absmax: 16 elements = 2 adjacent lanes, 32 elements = 4 adjacent lanes
     bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, 1));
     if (fmt == DQ_FP4_MXFP4) bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, 2));
     if (idx < K)
-      fp4_emit_vector(v, bmax, ts, fmt, mode, row, K, idx, blk, sf_offset(idx / blk), codes, sf, out);
+      fp4_emit_vector(v, bmax, ts, inv6ts, fmt, mode, row, K, idx, 1 << lg_blk, sf_offset(idx >> lg_blk), codes, sf_row, out);
   }
 }
 
@@ -338,7 +306,7 @@ __global__ void nvfp4_scale_finalize_kernel(float* scale) {
 template <typename XT>
 static int launch_fp4(const XT* x, int64_t ldx, const float* a, int M, int K, int fmt,
                       const float* tensor_scale, uint8_t* codes, uint8_t* sf, float* row_scale,
-                      float* out, int mode, cudaStream_t stream, int sf_atoms = 0) {
+                      float* out, int mode, cudaStream_t stream, int sf_atoms = 0, int activations = 0) {
   DQ_REQUIRE(fmt == DQ_FP4_MXFP4 || fmt == DQ_FP4_NVFP4, DQ_ERR_UNSUPPORTED, "unknown FP4 format %d", fmt);
   DQ_REQUIRE(x != nullptr, DQ_ERR_NULL, "x is null");
   const int blk = (fmt == DQ_FP4_MXFP4) ? 32 : 16;
@@ -353,27 +321,38 @@ static int launch_fp4(const XT* x, int64_t ldx, const float* a, int M, int K, in
              "scale factors in GEMM order need K %% %d == 0 (K=%d)", 4 * blk, K);
   const int vec = K / 8;
   const int rows = sf_atoms ? (M + 127) / 128 * 128 : M;
-  // T bounds the CTA, V = vectors of 8 per thread; the CTA launched is the smallest multiple of
-  // 32 threads that covers the row with V vectors each.
-#define DQ_FP4_LAUNCH(T, V)                                                                        \
-  quant_fp4_kernel<T, V, XT><<<rows, ((vec + (V) - 1) / (V) + 31) / 32 * 32, 0, stream>>>(        \
-      x, ldx, a, K, fmt, tensor_scale, codes, sf, row_scale, out, mode, M, sf_atoms)
-  // (four vectors per thread in smaller CTAs for many rows measured no faster: 126 vs 107 us at
-  // M = 4096, K = 18944)
-  if (M >= kFp4StreamMinRows && vec >= (fmt == DQ_FP4_NVFP4 ? kFp4StreamMinVecNv : kFp4StreamMinVec)) {
-    quant_fp4_stream_kernel<XT><<<rows, 256, 0, stream>>>(x, ldx, a, K, fmt, tensor_scale, codes, sf,
-                                                          row_scale, out, mode, M, sf_atoms);
-  } else if (vec <= 128) DQ_FP4_LAUNCH(128, 1);
-  else if (vec <= 256) DQ_FP4_LAUNCH(256, 1);
-  else if (vec <= 512) DQ_FP4_LAUNCH(512, 1);
-  else if (vec <= 1024) DQ_FP4_LAUNCH(512, 2);
-  else if (vec <= 1536) DQ_FP4_LAUNCH(512, 3);
-  else if (vec <= 2048) DQ_FP4_LAUNCH(512, 4);
-  else if (vec <= 3072) DQ_FP4_LAUNCH(1024, 3);
-  else DQ_FP4_LAUNCH(1024, 4);
+  // T bounds the CTA, V = vectors of 8 per thread, P = CTAs per SM the registers are limited for; the CTA launched is the
+  // smallest multiple of 32 threads that covers the row with V vectors each.  Few rows: many threads per row, one or two
+  // vectors each, because latency counts.  Many rows: eight (fp32: four) vectors per thread, so that an SM holds three
+  // rows of 18944 and has their 110 KB in flight.
+#define DQ_FP4_LAUNCH(T, V, P)                                                                                           \
+  DQ_CHECK_CUDA(launch_pdl(quant_fp4_kernel<T, V, P, XT>, dim3(rows), dim3(((vec + (V) - 1) / (V) + 31) / 32 * 32), 0,   \
+                           stream, x, ldx, a, K, fmt, tensor_scale, codes, sf, row_scale, out, mode, M, sf_atoms, activations))
+  constexpr int kMany = sizeof(XT) == 2 ? 8 : 4;
+  if (M >= kFp4ManyRows && vec > 256) {
+    if (vec <= 128 * kMany) DQ_FP4_LAUNCH(128, kMany, 7);
+    else if (vec <= 320 * kMany) DQ_FP4_LAUNCH(320, kMany, 3);
+    else if (vec <= 512 * kMany) DQ_FP4_LAUNCH(512, kMany, 2);
+    else DQ_FP4_LAUNCH(1024, kMany, 1);
+  } else if (vec <= 128) DQ_FP4_LAUNCH(128, 1, 1);
+  else if (vec <= 256) DQ_FP4_LAUNCH(256, 1, 1);
+  else if (vec <= 512) DQ_FP4_LAUNCH(512, 1, 1);
+  else if (vec <= 1024) DQ_FP4_LAUNCH(512, 2, 1);
+  else if (vec <= 2048) DQ_FP4_LAUNCH(1024, 2, 1);
+  else DQ_FP4_LAUNCH(1024, 4, 1);
 #undef DQ_FP4_LAUNCH
   DQ_CHECK_CUDA(cudaGetLastError());
   return DQ_OK;
+}
+
+// The activation half of a linear: dq_quant_fp4_atoms whose GEMM may start early.
+int quant_fp4_activations(const void* x, int x_is_f32, int64_t ldx, const float* a, int M, int K, int fmt, uint8_t* codes,
+                          uint8_t* sf_atoms, float* row_scale, cudaStream_t s) {
+  if (x_is_f32)
+    return launch_fp4(static_cast<const float*>(x), ldx, a, M, K, fmt, static_cast<const float*>(nullptr), codes, sf_atoms,
+                      row_scale, nullptr, FP4_MODE_CODES, s, 1, 1);
+  return launch_fp4(static_cast<const __nv_bfloat16*>(x), ldx, a, M, K, fmt, static_cast<const float*>(nullptr), codes,
+                    sf_atoms, row_scale, nullptr, FP4_MODE_CODES, s, 1, 1);
 }
 
 }  // namespace dq

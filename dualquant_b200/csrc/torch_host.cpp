@@ -37,7 +37,7 @@ namespace {
   X(dq_gemm_w4a4_int4_ex) X(dq_gemm_w4a4_int4_residual) X(dq_gemm_w4a4_int4_e4m3)                      \
   X(dq_linear_w4a4_int4) X(dq_linear_w4a4_int4_bias) X(dq_linear_w4a4_int4_scratch_bytes)                                         \
   X(dq_linear_w4a4_int4_prefill_scratch_bytes) X(dq_linear_a16w4) X(dq_linear_a16w4_scratch_bytes)     \
-  X(dq_quant_fp4_atoms) X(dq_fp4_sf_atoms_bytes) X(dq_gemm_w4a4_fp4_tiled)
+  X(dq_linear_w4a4_fp4) X(dq_linear_w4a4_fp4_scratch_bytes)
 #define DQ_DECLARE(name) decltype(&::name) name = nullptr;
 struct Abi {
   DQ_FUNCTIONS(DQ_DECLARE)
@@ -471,34 +471,15 @@ PyObject* linear_a16w4(PyObject*, PyObject* const* v, Py_ssize_t n) {
   });
 }
 
-// Activations [M, K] -> FP4 operands in one block of scratch: packed codes, scale atoms, row scales (NVFP4).
-struct Fp4Operands {
-  uint8_t *codes, *sf;
-  float* row_scale;
-};
-int64_t round_up_256(int64_t v) { return (v + 255) / 256 * 256; }
-int64_t fp4_scratch_bytes(int64_t M, int64_t K, int fmt) {
-  return round_up_256(M * K / 2) +
-         round_up_256(static_cast<int64_t>(abi.dq_fp4_sf_atoms_bytes(static_cast<int>(M), static_cast<int>(K), fmt))) +
-         round_up_256(M * 4) + 256;
+int64_t fp4_scratch_bytes(int M, int K, int fmt) {
+  return std::max<int64_t>(static_cast<int64_t>(abi.dq_linear_w4a4_fp4_scratch_bytes(M, K, fmt)), 256);
 }
-at::Tensor linear_fp4(const void* x, bool f32, int64_t ldx, int M, const float* a, const PackedFp4& w, const float* r,
-                      at::Tensor out, const at::Tensor& scratch, int idx) {
-  const int K = w.K;
-  uint8_t* base = static_cast<uint8_t*>(scratch.data_ptr());
-  Fp4Operands o;
-  o.codes = base;
-  o.sf = base + round_up_256(static_cast<int64_t>(M) * K / 2);
-  o.row_scale = w.fmt == DQ_FP4_NVFP4
-                    ? reinterpret_cast<float*>(o.sf + round_up_256(static_cast<int64_t>(abi.dq_fp4_sf_atoms_bytes(M, K, w.fmt))))
-                    : nullptr;
-  void* s = stream_of(idx);
-  check(abi.dq_quant_fp4_atoms(x, f32 ? 1 : 0, ldx, a, M, K, w.fmt, nullptr, o.codes, o.sf, o.row_scale, s),
-        "dq_quant_fp4_atoms");
-  check(abi.dq_gemm_w4a4_fp4_tiled(o.codes, o.sf, o.row_scale, w.codes, w.sf_atoms, w.tensor_scale, r, M, w.N, K, w.fmt,
-                                   out.data_ptr(), y_dtype_of(out), 0, s),
-        "dq_gemm_w4a4_fp4_tiled");
-  return out;
+void linear_fp4(const void* x, bool f32, int64_t ldx, int M, const float* a, const PackedFp4& w, const float* r,
+                const void* bias, const at::Tensor& out, const at::Tensor& scratch, int idx) {
+  check(abi.dq_linear_w4a4_fp4(x, f32 ? 1 : 0, ldx, a, w.codes, w.sf_atoms, w.tensor_scale, r, bias, M, w.N, w.K, w.fmt,
+                               out.data_ptr(), y_dtype_of(out), scratch.data_ptr(), static_cast<size_t>(scratch.numel()),
+                               stream_of(idx)),
+        "dq_linear_w4a4_fp4");
 }
 
 // linear_w4a4_fp4(x, a, pw, r, out_dtype) -> out
@@ -519,8 +500,9 @@ PyObject* linear_w4a4_fp4(PyObject*, PyObject* const* v, Py_ssize_t n) {
     }
     const at::Tensor scratch = empty({fp4_scratch_bytes(M, w.K, w.fmt)}, at::kByte, idx);
     at::Tensor out = empty({M, w.N}, dtype_arg(v[4]), idx);
-    return wrap(linear_fp4(x.data_ptr(), f32, w.K, M, static_cast<const float*>(ptr_or_null(v[1], "a")), w,
-                           static_cast<const float*>(ptr_or_null(v[3], "r")), std::move(out), scratch, idx));
+    linear_fp4(x.data_ptr(), f32, w.K, M, static_cast<const float*>(ptr_or_null(v[1], "a")), w,
+               static_cast<const float*>(ptr_or_null(v[3], "r")), nullptr, out, scratch, idx);
+    return wrap(std::move(out));
   });
 }
 
@@ -677,7 +659,7 @@ PyObject* perm_forward(PyObject*, PyObject* const* v, Py_ssize_t n) {
     at::Tensor out = empty(sizes, p->out_dtype, idx);
     // a bias of the output's type is added in the GEMM's epilogue, any other (or one that wants a gradient) by torch
     const void* bias_ptr = nullptr;
-    if (p->kind == PLAN_INT4 && bias != Py_None) {
+    if (p->kind != PLAN_A16 && bias != Py_None) {
       const at::Tensor& b = tensor(bias, "bias");
       if (b.scalar_type() == p->out_dtype && b.dim() == 1 && b.is_contiguous() && b.is_cuda() &&
           b.get_device() == p->device && !(b.requires_grad() && at::GradMode::is_enabled())) {
@@ -688,7 +670,7 @@ PyObject* perm_forward(PyObject*, PyObject* const* v, Py_ssize_t n) {
     if (p->kind == PLAN_INT4) {
       linear_int4(x.data_ptr(), ldx, a, desc(p->had), p->w4, w8, nullptr, bias_ptr, M, out, p->scale_mode, *p->scratch, idx);
     } else if (p->kind == PLAN_FP4) {
-      linear_fp4(x.data_ptr(), false, K, M, a, p->w_fp4, nullptr, out, *p->scratch, idx);
+      linear_fp4(x.data_ptr(), false, K, M, a, p->w_fp4, nullptr, bias_ptr, out, *p->scratch, idx);
     } else {
       check(abi.dq_linear_a16w4(x.data_ptr(), ldx, a, p->w4.w_packed, nullptr, M, N, K, p->w4.group, out.data_ptr(),
                                 y_dtype_of(out), p->scratch->data_ptr(), static_cast<size_t>(p->scratch->numel()),

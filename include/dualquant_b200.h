@@ -297,6 +297,18 @@ DQ_API int dq_gemm_w4a4_fp4_tiled(const uint8_t* x_codes, const uint8_t* x_sf_at
                                   int M, int N, int K, int fmt, void* y, int y_dtype,
                                   int token_tile, void* stream);
 
+/*
+ * One call for a PermLinear.forward on mxfp4 / nvfp4 activations and weights (activations/perm_linear.py:136-141):
+ * quantise x [M,K] (bf16 or fp32, optional column scale a; NVFP4 with one second-level scale per token) into scratch,
+ * then the GEMM; bias [N] of y's element type or null (bf16: added to the rounded result and rounded again).  Other
+ * operands as in dq_gemm_w4a4_fp4.  scratch: dq_linear_w4a4_fp4_scratch_bytes(M,K,fmt) bytes, 256-byte aligned.
+ */
+DQ_API size_t dq_linear_w4a4_fp4_scratch_bytes(int M, int K, int fmt);
+DQ_API int dq_linear_w4a4_fp4(const void* x, int x_is_f32, int64_t ldx, const float* a, const uint8_t* w_codes,
+                              const uint8_t* w_sf_atoms, const float* w_scale, const float* r, const void* bias, int M,
+                              int N, int K, int fmt, void* y, int y_dtype, void* scratch, size_t scratch_bytes,
+                              void* stream);
+
 /* ---- int4 dual-scale GEMM ------------------------------------------------------------------ */
 
 /* Scratch bytes dq_gemm_w4a4_int4 needs for (M,N,K); may be 0. */
