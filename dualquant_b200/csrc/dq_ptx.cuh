@@ -314,6 +314,30 @@ __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// Registers -> TMEM, the same lane assignment, 32 consecutive 32-bit columns.
+__device__ __forceinline__ void tmem_st_x32(uint32_t taddr, const uint32_t* v) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
+      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+      "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]),
+      "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]),
+      "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]),
+      "r"(v[30]), "r"(v[31])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() {
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+// One lane of a converged warp: with the branch on this predicate (not on the lane number) the compiler keeps what the
+// warp computes alike in uniform registers, where the tcgen05 instructions want their operands.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t pred;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xFFFFFFFF;\nselp.b32 %0, 1, 0, p;\n}\n" : "=r"(pred));
+  return pred != 0;
+}
+
 // ---------------------------------------------------------------------------------------
 // CTA pairs (tcgen05 cta_group::2): two CTAs of a cluster work on one 256-row tile.  Every CTA keeps its own 128
 // rows of A and of the accumulator and one half of B; one thread of the even-ranked CTA issues for both.
@@ -330,11 +354,12 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 // Completes `bar` (same offset in both CTAs of the pair) in both once all UMMAs issued so far by this thread have finished.
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+// first: cluster rank of the pair's even CTA.
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint32_t first = 0) {
   asm volatile(
       "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
           smem_u32(bar)),
-      "h"(static_cast<unsigned short>(3))
+      "h"(static_cast<unsigned short>(3u << first))
       : "memory");
 }
 // Tile of this GPU's memory into the issuing CTA's shared memory; the bytes are counted on `bar_addr`, a barrier of

@@ -5,35 +5,31 @@
 // the computation of the reference's fused-beta Triton kernel
 // (vendor/dualscale_kernel_benchmark/fused_dual_scale_kernel.py:55-149: beta multiplied into the
 // activation tile on its way in, nibbles de-quantised with the group scale, floating-point dot
-// product) on the tensor cores of this GPU: tcgen05.mma kind::f16 with fp16 operands and ONE fp32
-// accumulator in tensor memory over the whole K (the group scale is folded into the fp16 weight,
+// product) on the tensor cores of this GPU: tcgen05.mma kind::f16 with fp16 operands and fp32
+// accumulators in tensor memory over the whole K (the group scale is folded into the fp16 weight,
 // so nothing has to be drained per group).  fp16 rather than bf16 operands: with 8-bit mantissas
 // the reference's own acceptance check (mean relative error below 1 % against the fp32 formulation,
 // fused_dual_scale_kernel.py:269-308) fails at 1.4-5.7 %, with 11-bit mantissas it passes at
 // 0.25-0.4 %; the group scales are fp16 already, so code * scale is one exactly rounded product.
 // Activations beyond the fp16 range saturate at +-65504.
 //
-// Orientation as in the int4 kernels: the CTA's 128 weight rows are the UMMA M dimension, the token
-// tile TN is UMMA N.  Per weight group (128 k, one pipeline step):
-//   producer warp   one bulk copy of the packed tile (8 KB codes + 256 B fp16 scales) and two tiled
-//                   copies of the activation tile (TN x 64 fp16 each, 128-byte swizzle);
-//   16 unpack warps thread (row, k chunk) expands 16 bytes of nibbles into 32 fp16 = code * scale and
-//                   writes them as four 16-byte pieces into the 128B-swizzled K-major operand tile.
-//                   A nibble pair becomes half2 by bit tricks: (w >> s) & 0x000F000F picks two
-//                   two's-complement nibbles, ^ 0x64086408 turns them into the fp16 numbers
-//                   1032 + code, a packed subtract gives code exactly and a packed multiply by the
-//                   fp16 group scale the weight;
-//   issuing warp    eight tcgen05.mma (K = 16) per group, tcgen05.commit frees the operand buffers.
-// After the last group the first four unpack warps read the accumulator (one weight row per
-// thread), multiply by r[n] and store bf16 or fp32.  Every wait is bounded.
-//
-// Bound (ncu at gate+up, M = 4096: tensor pipe 31 % active, issue slots 45 %): the shared-memory port.
-// Per 128 x 128 x 128 block the tensor core reads 64 KB of operands (a 128 x 128 tile saturates the
-// port on its own: 8 KB per 68-cycle UMMA), the unpack warps write 32 KB and read 8 KB, the copy
-// engine writes 40 KB - 144 KB against the ~69 KB the port moves in the block's 542 UMMA cycles.  Tried
-// and not kept: a second issuing warp with its own accumulator (slower: one activation stage less).
-// The next step is the weight operand through tensor memory (tcgen05.st by the unpack warps, as
-// the int4 kernel for small token tiles does), which takes 64 KB per block off the port.
+// Tile: 256 weight rows x TN tokens on a pair of CTAs (tcgen05 cta_group::2); a CTA holds 128 of the rows and half of
+// the tokens' activations.  The weight operand goes to the tensor core from TENSOR MEMORY: eight unpack warps read the
+// packed tile (8 KB codes + 256 B scales per group of 128 k), expand the nibbles of their row to fp16 code * scale and
+// store them with tcgen05.st (lane = weight row, column = two k).  Shared memory then carries only the packed tile and
+// the activations: 80 KB per group of a 256-token tile, in 1024 cycles of UMMAs.  (A single-CTA 128 x 128 tile with the
+// expanded weights in shared memory moved 144 KB in 512 and was bound by that port: 4096 -> 28672 at 512 tokens 191 us.)
+//   warps 0-7    unpack: warp w owns TMEM lanes 32 (w & 3) .. and k 64 (w >> 2) .. of a group.  A nibble pair becomes
+//                half2 by bit tricks: (w >> s) & 0x000F000F picks two two's-complement nibbles, ^ 0x64086408 turns them
+//                into the fp16 numbers 1032 + code, a packed subtract gives code exactly, a packed multiply by the fp16
+//                group scale the weight.  The nibbles picked together are k and k + 2; the pre-pass below writes the
+//                activations in that order, so nothing has to be shuffled here.
+//   warps 8-11   epilogue: accumulator -> registers -> shared memory (32 tokens at a time) -> bulk store
+//   warp 12      producer: one bulk copy and two tiled copies per group
+//   warps 13-14  UMMA issue (of the even CTA, for both); tiles of up to 64 tokens: two warps take alternate groups into
+//                an accumulator each, because issuing a group takes one warp longer than executing it
+// Persistent CTAs; where the tiles leave the chip idle (decode batches) K is split over the pairs of a larger cluster
+// instead, and the partial tiles are summed in rank order through distributed shared memory.  Every wait is bounded.
 //
 // The activation scale and the conversion to fp16 run as a small separate pass
 // (xs = fp16(x * a), caller scratch) so that the GEMM can stage activations with TMA.
@@ -46,33 +42,35 @@
 namespace dq {
 namespace a16 {
 
-constexpr int kBN = 128;                 // weight rows per CTA (UMMA M)
-constexpr int kUnpackWarps = 16;  // four threads per weight row: two resident warps per scheduler hid too little latency
-constexpr int kProducerWarp = kUnpackWarps;
-constexpr int kIssuerWarp = kUnpackWarps + 1;
-constexpr int kThreads = (kUnpackWarps + 2) * 32;
-constexpr int kWTile = kBN * kGroup * 2;  // fp16 weight tile of one group: 32 KB (two 16 KB atoms)
-constexpr int kAtom = kBN * 128;          // 128 rows x 128 B
+constexpr int kBN = 128;                 // weight rows per CTA; a pair works on 256
+constexpr int kUnpackWarps = 8, kEpiWarps = 4, kProducerWarp = 12, kIssuerWarp = 13;
+constexpr int kThreads = 512;
+constexpr int kACols = 64;               // TMEM columns of one expanded group: 128 fp16
+constexpr int kOutChunk = 32 * kBN * 4;  // 32 tokens x 128 rows of fp32 (bf16 uses half)
 
 enum { ASITE_TMA = 51, ASITE_UNPACK = 52, ASITE_MMA = 53, ASITE_EPI = 54, ASITE_ALIGN = 55 };
 
 template <int TN>
 struct Cfg {
-  static constexpr int NB = 2;                      // unpacked weight buffers
-  static constexpr int SP = 4;                      // packed-tile stages
-  static constexpr int SX = (TN <= 64) ? 4 : 3;     // activation stages
-  static constexpr int kXStage = TN * kGroup * 2;   // TN x 128 fp16 = two atoms of TN x 128 B
-  static constexpr int kXAtom = TN * 128;
-  static constexpr int kOffW = 0;
-  static constexpr int kOffX = kOffW + NB * kWTile;
-  static constexpr int kOffP = kOffX + SX * kXStage;
-  static constexpr int kPStage = (kTileBytes + 127) / 128 * 128;
-  static constexpr int kOffBar = kOffP + SP * kPStage;
-  static constexpr int kNumBars = 2 * SP + 2 * NB + 2 * SX + 1;
-  static constexpr int kSmemBytes = kOffBar + kNumBars * 8 + 32;
-  static constexpr int kTmemCols = (TN <= 32) ? 32 : (TN <= 64) ? 64 : 128;
-  static_assert(kSmemBytes + 1024 <= 227 * 1024, "shared memory");
-  static_assert(kOffX % 1024 == 0 && kXStage % 1024 == 0 && kXAtom % 1024 == 0, "swizzle atoms on 1 KB boundaries");
+  static constexpr int kIssuers = (TN <= 64) ? 2 : 1;           // accumulators per tile
+  static constexpr int kAccTiles = (TN <= 192) ? 2 : 1;         // tiles whose accumulators fit
+  static constexpr int kAccCols = TN * kIssuers * kAccTiles;
+  static constexpr int NA = (512 - kAccCols) / kACols < 4 ? (512 - kAccCols) / kACols : 4;  // expanded groups
+  static constexpr int kXAtom = TN / 2 * 128;                   // this CTA's tokens x 64 k
+  static constexpr int kXStage = 2 * kXAtom;
+  static constexpr int SP = 6;                                  // packed-tile stages
+  static constexpr int kFixed = SP * kTileBytes + 2 * kOutChunk + 512;
+  static constexpr int kFit = (227 * 1024 - kFixed) / kXStage;
+  static constexpr int SX = kFit < 8 ? kFit : 8;                // activation stages
+  static constexpr int kOffX = 0;
+  static constexpr int kOffOut = SX * kXStage;
+  static constexpr int kOffP = kOffOut + 2 * kOutChunk;
+  static constexpr int kOffBar = kOffP + SP * kTileBytes;
+  static constexpr int kNumBars = 2 * SP + 2 * SX + 2 * NA + 2 * kAccTiles;
+  static constexpr int kSmemBytes = kOffBar + kNumBars * 8 + 16;
+  static_assert(kSmemBytes <= 227 * 1024 && SX >= 3 && NA >= 2, "rings");
+  static_assert(kXAtom % 1024 == 0, "swizzle atoms on 1 KB boundaries");
+  static_assert(TN > 64 || TN * kBN * 4 <= kOffP, "split-K exchange tile");
 };
 
 // Instruction descriptor, kind::f16: fp16 A and B (both K-major), fp32 accumulator.
@@ -82,15 +80,16 @@ __host__ __device__ constexpr uint32_t idesc_f16(int m, int n) {
   return (1u << 4) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
 }
 
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                         uint32_t accumulate) {
+// D[tmem of both CTAs] (+)= A[tmem of both] * B[smem of both]
+__device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                              uint32_t accumulate) {
   asm volatile(
       "{\n"
       ".reg .pred p;\n"
       "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n"
       "}\n" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 
@@ -104,182 +103,299 @@ __device__ __forceinline__ uint32_t nib2_to_f16x2(uint32_t t, __half2 s2) {
   return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-// Eight consecutive k of one row: the low (HI = 0) or high (HI = 1) nibbles of packed words wa, wb.
-template <int HI>
-__device__ __forceinline__ uint4 expand8(uint32_t wa, uint32_t wb, __half2 s2) {
-  // byte b of a word: nibble of k = 4j + b (low) or 16 + 4j + b (high).  (w >> s) & 0x000F000F
-  // picks bytes 0 and 2, (w >> (s + 8)) bytes 1 and 3.
-  const uint32_t a02 = nib2_to_f16x2(wa >> (4 * HI), s2), a13 = nib2_to_f16x2(wa >> (4 * HI + 8), s2);
-  const uint32_t b02 = nib2_to_f16x2(wb >> (4 * HI), s2), b13 = nib2_to_f16x2(wb >> (4 * HI + 8), s2);
-  uint4 o;
-  o.x = __byte_perm(a02, a13, 0x5410);  // (k0, k1)
-  o.y = __byte_perm(a02, a13, 0x7632);  // (k2, k3)
-  o.z = __byte_perm(b02, b13, 0x5410);
-  o.w = __byte_perm(b02, b13, 0x7632);
-  return o;
-}
-
 template <int TN>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_a16w4_kernel(const uint8_t* __restrict__ w_packed, const __grid_constant__ CUtensorMap tm_x,
-                  const float* __restrict__ r, void* __restrict__ y, int y_bf16, int M, int N, int K,
-                  int* status) {
+                  const __grid_constant__ CUtensorMap tm_y, int bulk_store, const float* __restrict__ r,
+                  void* __restrict__ y, int y_bf16, int M, int N, int K, int row_pairs, int tok_tiles, int tok_block,
+                  int split, int groups_per_split, int* status) {
   using C = Cfg<TN>;
+  constexpr int kIssuers = C::kIssuers;
   extern __shared__ __align__(1024) uint8_t smem[];
-  if ((smem_u32(smem) & 1023u) != 0) {
-    if (threadIdx.x == 0) atomicCAS(status, 0, ASITE_ALIGN);
-    return;
-  }
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kOffBar);
-  uint64_t* full_p = bars;
+  uint64_t* full_p = reinterpret_cast<uint64_t*>(smem + C::kOffBar);
   uint64_t* empty_p = full_p + C::SP;
-  uint64_t* w_ready = empty_p + C::SP;
-  uint64_t* w_free = w_ready + C::NB;
-  uint64_t* full_x = w_free + C::NB;
+  uint64_t* full_x = empty_p + C::SP;      // (even CTA) both CTAs' activations of a group have landed
   uint64_t* empty_x = full_x + C::SX;
-  uint64_t* acc_done = empty_x + C::SX;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 1);
+  uint64_t* a_full = empty_x + C::SX;      // (even CTA) both CTAs' weights of a group are expanded
+  uint64_t* a_free = a_full + C::NA;
+  uint64_t* acc_full = a_free + C::NA;
+  uint64_t* acc_empty = acc_full + C::kAccTiles;  // (even CTA)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + C::kAccTiles);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int lane = tid & 31;
-  const int ng = K / kGroup;
-  const int n0 = blockIdx.x * kBN;
-  const int t0 = blockIdx.y * TN;
+  const uint32_t crank = cluster_ctarank();
+  const uint32_t even = crank & ~1u;                 // the pair's even CTA
+  const int rank = static_cast<int>(crank & 1u);
+  const int total_groups = K / kGroup;
+  // split == 1: persistent pairs over the tiles; else one tile per cluster, pair s of it takes a slice of K
+  const int pair = split == 1 ? static_cast<int>(blockIdx.x) >> 1 : static_cast<int>(blockIdx.x) / (2 * split);
+  const int pairs = split == 1 ? static_cast<int>(gridDim.x) >> 1 : static_cast<int>(gridDim.x) / (2 * split);
+  const int g_begin = split == 1 ? 0 : static_cast<int>(crank >> 1) * groups_per_split;
+  int ng = total_groups - g_begin;
+  if (ng > groups_per_split) ng = groups_per_split;
+  if (ng < 0) ng = 0;
+  const int row_tiles = (N + kBN - 1) / kBN;
+  const int total_tiles = row_pairs * tok_tiles;
+  const int my_tiles = (total_tiles - pair + pairs - 1) / pairs;
+  // token tiles in blocks whose activations stay in L2 while every row pair passes over them, tokens fastest
+  const int full_block = tok_block * row_pairs;
+  auto tile_of = [&](int it, int& row, int& tok) {
+    const int t = pair + it * pairs;
+    const int b = t / full_block, rem = t - b * full_block;
+    const int width = (tok_tiles - b * tok_block < tok_block) ? (tok_tiles - b * tok_block) : tok_block;
+    const int rp = rem / width;
+    tok = b * tok_block + (rem - rp * width);
+    row = 2 * rp + rank;
+  };
 
   if (tid == 0) {
     for (int i = 0; i < C::SP; ++i) { mbar_init(&full_p[i], 1); mbar_init(&empty_p[i], kUnpackWarps); }
-    for (int i = 0; i < C::NB; ++i) { mbar_init(&w_ready[i], kUnpackWarps); mbar_init(&w_free[i], 1); }
     for (int i = 0; i < C::SX; ++i) { mbar_init(&full_x[i], 1); mbar_init(&empty_x[i], 1); }
-    mbar_init(acc_done, 1);
-    *abort_flag = 0;
+    for (int i = 0; i < C::NA; ++i) { mbar_init(&a_full[i], 2 * kUnpackWarps); mbar_init(&a_free[i], 1); }
+    for (int i = 0; i < C::kAccTiles; ++i) { mbar_init(&acc_full[i], kIssuers); mbar_init(&acc_empty[i], 2 * kEpiWarps); }
+    *abort_flag = (smem_u32(smem) & 1023u) != 0 ? ASITE_ALIGN : 0;  // the swizzle needs 1 KB boundaries: nothing runs then
     fence_mbar_init();
   }
   if (warp == kIssuerWarp) {
-    tmem_alloc(tmem_slot, C::kTmemCols);
-    tmem_relinquish();
+    tmem_alloc_pair(tmem_slot, 512);
+    tmem_relinquish_pair();
   }
-  if (warp == kProducerWarp && lane == 0) tma_prefetch_desc(&tm_x);
+  if (warp == kProducerWarp && lane == 0) {
+    tma_prefetch_desc(&tm_x);
+    if (bulk_store) tma_prefetch_desc(&tm_y);
+  }
   grid_dep_launch_dependents();
   tc_fence_before();
   __syncthreads();
+  cluster_sync_all();  // the peers' barriers are initialised before anything arrives on them
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  const uint32_t a_base = tmem_base + C::kAccCols;
+  const bool live = *abort_flag == 0;
 
-  if (warp == kProducerWarp) {
-    // ------------------------------------------------------------------ producer
-    if (lane == 0) {
-      const uint64_t pol_w = (gridDim.y == 1) ? l2_policy_evict_first() : l2_policy_evict_last();
-      const uint64_t pol_x = l2_policy_evict_last();
-      const uint8_t* w_src = w_packed + static_cast<size_t>(blockIdx.x) * ng * kTileBytes;
-      // The weights do not depend on the kernel before this one, the activations may: the first
-      // weight tiles go out before the dependency wait.
-      const int pre = (ng < C::SP) ? ng : C::SP;
-      for (int i = 0; i < pre; ++i) {
-        mbar_expect_tx(&full_p[i], kTileBytes);
-        bulk_load_1d(smem + C::kOffP + i * C::kPStage, w_src + static_cast<size_t>(i) * kTileBytes, kTileBytes,
-                     &full_p[i], pol_w);
-      }
-      grid_dep_wait();
-      for (int i = 0; i < ng; ++i) {
-        const int sp = i % C::SP, sx = i % C::SX;
-        if (i >= pre) {
-          if (!mbar_wait(&empty_p[sp], ((i / C::SP) & 1) ^ 1, abort_flag, ASITE_TMA)) break;
-          mbar_expect_tx(&full_p[sp], kTileBytes);
-          bulk_load_1d(smem + C::kOffP + sp * C::kPStage, w_src + static_cast<size_t>(i) * kTileBytes,
-                       kTileBytes, &full_p[sp], pol_w);
-        }
-        if (!mbar_wait(&empty_x[sx], ((i / C::SX) & 1) ^ 1, abort_flag, ASITE_TMA)) break;
-        mbar_expect_tx(&full_x[sx], C::kXStage);
-        uint8_t* xs = smem + C::kOffX + sx * C::kXStage;
-        tma_load_2d(xs, &tm_x, i * 256, t0, &full_x[sx], pol_x);                    // k 0..63 of the group
-        tma_load_2d(xs + C::kXAtom, &tm_x, i * 256 + 128, t0, &full_x[sx], pol_x);  // k 64..127
-      }
-    }
-  } else if (warp == kIssuerWarp) {
-    // ------------------------------------------------------------------ UMMA issue
-    if (lane == 0) {
-      const uint32_t idesc = idesc_f16(kBN, TN);
-      for (int i = 0; i < ng; ++i) {
-        const int b = i % C::NB, sx = i % C::SX;
-        if (!mbar_wait(&w_ready[b], (i / C::NB) & 1, abort_flag, ASITE_MMA)) break;
-        if (!mbar_wait(&full_x[sx], (i / C::SX) & 1, abort_flag, ASITE_MMA)) break;
-        tc_fence_after();
-        const uint32_t wbase = smem_u32(smem + C::kOffW + b * kWTile);
-        const uint32_t xbase = smem_u32(smem + C::kOffX + sx * C::kXStage);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {  // eight K = 16 steps: 32 bytes along K inside an atom
-          const uint64_t da = umma_desc_k_sw128(wbase + (j >> 2) * kAtom) + 2 * (j & 3);
-          const uint64_t db = umma_desc_k_sw128(xbase + (j >> 2) * C::kXAtom) + 2 * (j & 3);
-          umma_f16(tmem_base, da, db, idesc, (i | j) ? 1u : 0u);
-        }
-        umma_commit(&w_free[b]);
-        umma_commit(&empty_x[sx]);
-      }
-      umma_commit(acc_done);
-    }
-  } else {
-    // ------------------------------------------------------------------ unpack warps
-    const int row = tid & 127;
-    const int ch = tid >> 7;    // k chunk (32 k) of the group this thread expands: 0..3
-    const int swz = row & 7;
-    bool ok = true;
-    for (int i = 0; i < ng && ok; ++i) {
-      const int sp = i % C::SP, b = i % C::NB;
-      if (!mbar_wait(&full_p[sp], (i / C::SP) & 1, abort_flag, ASITE_UNPACK)) { ok = false; break; }
-      if (!mbar_wait(&w_free[b], ((i / C::NB) & 1) ^ 1, abort_flag, ASITE_UNPACK)) { ok = false; break; }
-      const uint8_t* tile = smem + C::kOffP + sp * C::kPStage;
-      const __half sc = reinterpret_cast<const __half*>(tile + kTileCodeBytes)[row];
-      const __half2 s2 = __half2half2(sc);
-      // chunks 0, 1 -> atom 0 (k 0..63), chunks 2, 3 -> atom 1; inside the atom 16-byte pieces c0..c0+3
-      uint8_t* dst = smem + C::kOffW + b * kWTile + (ch >> 1) * kAtom + row * 128;
-      const int c0 = (ch & 1) * 4;
-      const int pos = ch ^ ((row >> 1) & 3);           // the chunk's position in the packed row
-      const uint4 w = *reinterpret_cast<const uint4*>(tile + row * 64 + pos * 16);
-      // the chunk's 32 k as four 16-byte pieces: k 0-7, 8-15 (low nibbles of words 0,1 / 2,3),
-      // 16-23, 24-31 (high nibbles)
-      *reinterpret_cast<uint4*>(dst + (((c0 + 0) ^ swz) << 4)) = expand8<0>(w.x, w.y, s2);
-      *reinterpret_cast<uint4*>(dst + (((c0 + 1) ^ swz) << 4)) = expand8<0>(w.z, w.w, s2);
-      *reinterpret_cast<uint4*>(dst + (((c0 + 2) ^ swz) << 4)) = expand8<1>(w.x, w.y, s2);
-      *reinterpret_cast<uint4*>(dst + (((c0 + 3) ^ swz) << 4)) = expand8<1>(w.z, w.w, s2);
-      fence_proxy_async_smem();  // generic-proxy stores before the tensor core's reads
+  if (warp < kUnpackWarps) {
+    // ------------------------------------------------------------------ unpack
+    const int q = warp & 3, h = warp >> 2;
+    const int row = q * 32 + lane;
+    const uint32_t t_lane = a_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(h * 32);
+    const uint32_t a_full_addr = dsmem_map(smem_u32(a_full), even);
+    const int total = live ? my_tiles * ng : 0;
+    // chunk positions inside the packed row are swizzled by (row >> 1) & 3
+    const int at0 = row * 64 + (((2 * h) ^ ((row >> 1) & 3)) << 4), at1 = row * 64 + (((2 * h + 1) ^ ((row >> 1) & 3)) << 4);
+    for (int gi = 0; gi < total; ++gi) {
+      const int sp = gi % C::SP, ab = gi % C::NA;
+      if (!mbar_wait(&full_p[sp], (gi / C::SP) & 1, abort_flag, ASITE_UNPACK)) break;
+      const uint8_t* tile = smem + C::kOffP + sp * kTileBytes;
+      const uint4 w0 = *reinterpret_cast<const uint4*>(tile + at0), w1 = *reinterpret_cast<const uint4*>(tile + at1);
+      const __half2 s2 = __half2half2(reinterpret_cast<const __half*>(tile + kTileCodeBytes)[row]);
       __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(&w_ready[b]);
-        mbar_arrive(&empty_p[sp]);
-      }
-    }
-    // ------------------------------------------------------------------ epilogue (warps 0-3)
-    if (warp < 4 && ok) {
-      if (mbar_wait_relaxed(acc_done, 0, abort_flag, ASITE_EPI)) {
-        tc_fence_after();
-        const int n = n0 + warp * 32 + lane;  // warp w reads TMEM lanes 32 w .. 32 w + 31
-        const float rn = (n < N && r != nullptr) ? r[n] : 1.f;
-#pragma unroll 1
-        for (int c0 = 0; c0 < TN; c0 += 16) {
-          uint32_t v[16];
-          tmem_ld_x16(tmem_base + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(c0), v);
-          tmem_ld_wait();
-          if (n < N) {
+      if (lane == 0) mbar_arrive(&empty_p[sp]);
+      uint32_t v[32];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const int m = t0 + c0 + j;
-              if (m < M) store_y(y, Addend{}, y_bf16, m, n, N, __uint_as_float(v[j]) * rn);
-            }
+      for (int c = 0; c < 2; ++c) {
+        const uint4 w = c ? w1 : w0;
+        const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          // low nibbles: k = 4 j + {0, 2}, {1, 3} of the chunk's first half; high nibbles: of its second
+          v[16 * c + 2 * j] = nib2_to_f16x2(ww[j], s2);
+          v[16 * c + 2 * j + 1] = nib2_to_f16x2(ww[j] >> 8, s2);
+          v[16 * c + 8 + 2 * j] = nib2_to_f16x2(ww[j] >> 4, s2);
+          v[16 * c + 8 + 2 * j + 1] = nib2_to_f16x2(ww[j] >> 12, s2);
+        }
+      }
+      if (!mbar_wait(&a_free[ab], ((gi / C::NA) & 1) ^ 1, abort_flag, ASITE_UNPACK)) break;
+      tc_fence_after();
+      tmem_st_x32(t_lane + static_cast<uint32_t>(ab * kACols), v);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(a_full_addr + static_cast<uint32_t>(ab) * 8u);
+    }
+  } else if (warp < kProducerWarp) {
+    // ------------------------------------------------------------------ epilogue
+    const int q = warp & 3;
+    const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
+    const uint32_t acc_empty_addr = dsmem_map(smem_u32(acc_empty), even);
+    const bool leader = warp == kUnpackWarps && lane == 0;
+    const bool second = kIssuers == 2 && ng > 1;  // the second issuer had groups to add up
+    int chunk_no = 0;
+    grid_dep_wait();  // what last used y may still be running
+    for (int it = 0; it < my_tiles && live; ++it) {
+      int row_tile, tok_tile;
+      tile_of(it, row_tile, tok_tile);
+      const int n = row_tile * kBN + q * 32 + lane, t0 = tok_tile * TN;
+      const int cols = M - t0 < TN ? (M - t0 + 31) & ~31 : TN;
+      const float rn = (n < N && r != nullptr) ? r[n] : 1.f;
+      const int set = it % C::kAccTiles;
+      if (TN <= 64 ? !mbar_wait(&acc_full[set], (it / C::kAccTiles) & 1, abort_flag, ASITE_EPI)
+                   : !mbar_wait_relaxed(&acc_full[set], (it / C::kAccTiles) & 1, abort_flag, ASITE_EPI))
+        break;
+      tc_fence_after();
+#pragma unroll 1
+      for (int c0 = 0; c0 < cols; c0 += 32) {
+        float v[32];
+        {
+          uint32_t u[32];
+          const uint32_t at = t_lane + static_cast<uint32_t>(set * kIssuers * TN + c0);
+          tmem_ld_x32(at, u);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = ng > 0 ? __uint_as_float(u[j]) : 0.f;
+          if (second) {
+            tmem_ld_x32(at + TN, u);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] += __uint_as_float(u[j]);
           }
         }
+        if (c0 + 32 >= cols) {  // the accumulator goes back before its last columns are stored
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(acc_empty_addr + static_cast<uint32_t>(set) * 8u);
+        }
+        if (split > 1) {
+          // partial tile -> this CTA's exchange buffer [token][row] over the idle activation ring
+          float* red = reinterpret_cast<float*>(smem);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) red[(c0 + j) * kBN + q * 32 + lane] = v[j];
+        } else if (bulk_store) {
+          uint8_t* buf = smem + C::kOffOut + (chunk_no & 1) * kOutChunk;
+          ++chunk_no;
+          // at most one store is outstanding, so the buffer of the chunk before the last has been read
+          if (leader) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+          asm volatile("bar.sync 1, 128;" ::: "memory");
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            if (y_bf16)
+              reinterpret_cast<__nv_bfloat16*>(buf)[j * kBN + q * 32 + lane] = __float2bfloat16_rn(v[j] * rn);
+            else
+              reinterpret_cast<float*>(buf)[j * kBN + q * 32 + lane] = v[j] * rn;
+          }
+          fence_proxy_async_smem();
+          asm volatile("bar.sync 1, 128;" ::: "memory");
+          if (leader) {
+            if (row_tile < row_tiles) tma_store_2d(&tm_y, buf, row_tile * kBN, t0 + c0);
+            bulk_commit_group();
+          }
+        } else if (n < N) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            if (t0 + c0 + j < M) store_y(y, Addend{}, y_bf16, t0 + c0 + j, n, N, v[j] * rn);
+        }
       }
     }
+    if (leader) bulk_wait_group_read0();
+  } else if (warp == kProducerWarp) {
+    // ------------------------------------------------------------------ producer (both CTAs)
+    if (lane == 0 && live) {
+      const uint64_t pol_w = tok_tiles == 1 ? l2_policy_evict_first() : l2_policy_evict_last();
+      const uint64_t pol_x = l2_policy_evict_last();
+      const uint32_t full_x_addr = dsmem_map(smem_u32(full_x), even);
+      const int total = my_tiles * ng;
+      auto load_w = [&](int gi) {
+        int row_tile, tok_tile;
+        tile_of(gi / ng, row_tile, tok_tile);
+        if (row_tile >= row_tiles) row_tile = row_tiles - 1;  // computed and not stored
+        mbar_expect_tx(&full_p[gi % C::SP], kTileBytes);
+        bulk_load_1d(smem + C::kOffP + (gi % C::SP) * kTileBytes,
+                     w_packed + (static_cast<size_t>(row_tile) * total_groups + g_begin + gi % ng) * kTileBytes, kTileBytes,
+                     &full_p[gi % C::SP], pol_w);
+      };
+      // The weights do not depend on the kernel before this one, the activations do: the packed ring is filled first.
+      const int pre = total < C::SP ? total : C::SP;
+      for (int gi = 0; gi < pre; ++gi) load_w(gi);
+      grid_dep_wait();
+      for (int gi = 0; gi < total; ++gi) {
+        const int sx = gi % C::SX;
+        int row_tile, tok_tile;
+        tile_of(gi / ng, row_tile, tok_tile);
+        const int t0 = tok_tile * TN + rank * (TN / 2), kx = (g_begin + gi % ng) * 256;
+        if (!mbar_wait(&empty_x[sx], ((gi / C::SX) & 1) ^ 1, abort_flag, ASITE_TMA)) break;
+        if (rank == 0) mbar_expect_tx(&full_x[sx], 2 * C::kXStage);
+        uint8_t* xs = smem + C::kOffX + sx * C::kXStage;
+        tma_load_2d_pair(xs, &tm_x, kx, t0, full_x_addr + static_cast<uint32_t>(sx) * 8u, pol_x);
+        tma_load_2d_pair(xs + C::kXAtom, &tm_x, kx + 128, t0, full_x_addr + static_cast<uint32_t>(sx) * 8u, pol_x);
+        if (gi + C::SP < total) {
+          if (!mbar_wait(&empty_p[gi % C::SP], (gi / C::SP) & 1, abort_flag, ASITE_TMA)) break;
+          load_w(gi + C::SP);
+        }
+      }
+    }
+  } else if (warp < kIssuerWarp + kIssuers && rank == 0 && live) {
+    // ------------------------------------------------------------------ UMMA issue, for both CTAs (whole warp, one lane acts)
+    constexpr uint32_t idesc = idesc_f16(2 * kBN, TN);
+    const int mine = warp - kIssuerWarp;
+    bool ok = true;
+    for (int it = 0; it < my_tiles && ok; ++it) {
+      const int set = it % C::kAccTiles;
+      const uint32_t d_tmem = tmem_base + static_cast<uint32_t>((set * kIssuers + mine) * TN);
+      ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[set], ((it / C::kAccTiles) & 1) ^ 1, abort_flag, ASITE_MMA));
+      for (int i = mine; i < ng && ok; i += kIssuers) {
+        const int gi = it * ng + i, ab = gi % C::NA, sx = gi % C::SX;
+        ok = mbar_wait(&full_x[sx], (gi / C::SX) & 1, abort_flag, ASITE_MMA) &&
+             mbar_wait(&a_full[ab], (gi / C::NA) & 1, abort_flag, ASITE_MMA);
+        ok = __all_sync(0xffffffffu, ok);  // the warp leaves the loop together
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
+          const uint64_t db = umma_desc_k_sw128(smem_u32(smem + C::kOffX + sx * C::kXStage));
+          const uint32_t at = a_base + static_cast<uint32_t>(ab * kACols);
+#pragma unroll
+          for (int j = 0; j < 8; ++j)  // eight K = 16 steps: 8 columns of A, 32 bytes along K of B inside an atom
+            umma_f16_pair(d_tmem, at + 8 * j, db + (j >> 2) * (C::kXAtom >> 4) + 2 * (j & 3), idesc,
+                          (i != mine || j > 0) ? 1u : 0u);
+          umma_commit_pair(&a_free[ab], even);
+          umma_commit_pair(&empty_x[sx], even);
+        }
+        __syncwarp();
+      }
+      if (ok && elect_one()) umma_commit_pair(&acc_full[set], even);
+      __syncwarp();
+    }
   }
+
+  __syncwarp();
+  // ---------------------------------------------------------------------- split-K reduction
+  if (split > 1) {
+    cluster_sync_all();
+    const int si = static_cast<int>(crank >> 1);
+    int row_tile, tok_tile;
+    tile_of(0, row_tile, tok_tile);
+    const int t0 = tok_tile * TN, c4 = lane;
+    const uint32_t red_base = smem_u32(smem);
+    for (int tl = si + split * warp; tl < TN && t0 + tl < M; tl += split * (kThreads / 32)) {
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      const uint32_t off = static_cast<uint32_t>((tl * kBN + c4 * 4) * 4);
+      for (int p = 0; p < split; ++p) {
+        const float4 v = dsmem_ld_f4(dsmem_map(red_base + off, static_cast<uint32_t>(2 * p + rank)));
+        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+      }
+      const float vals[4] = {acc.x, acc.y, acc.z, acc.w};
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int n = row_tile * kBN + c4 * 4 + u;
+        if (n < N) store_y(y, Addend{}, y_bf16, t0 + tl, n, N, vals[u] * (r != nullptr ? r[n] : 1.f));
+      }
+    }
+    __syncwarp();
+  }
+  // The CTAs leave together: until here a peer may read this CTA's operands or exchange tile and arrive on its barriers.
   tc_fence_before();
   __syncthreads();
-  tc_fence_after();
-  if (warp == kIssuerWarp) tmem_dealloc(tmem_base, C::kTmemCols);
+  cluster_sync_all();
+  if (warp == kIssuerWarp) {
+    tc_fence_after();
+    tmem_dealloc_pair(tmem_base, 512);
+  }
   if (tid == 0 && *abort_flag != 0) atomicCAS(status, 0, *abort_flag);
 }
 
-// xs[m, k] = fp16(float(x[m, k]) * a[k]) (a may be null), saturating at the fp16 range
+// xs[m, k] = fp16(float(x[m, k]) * a[k]) (a may be null), saturating at the fp16 range; inside every four k the order is
+// 0, 2, 1, 3 (see the unpack warps)
 __global__ void __launch_bounds__(256) scale_cols_f16_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx,
                                                              const float* __restrict__ a, int M, int K,
                                                              __half* __restrict__ xs) {
@@ -299,12 +415,17 @@ __global__ void __launch_bounds__(256) scale_cols_f16_kernel(const __nv_bfloat16
       av[4] = a1.x; av[5] = a1.y; av[6] = a1.z; av[7] = a1.w;
     }
     const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      v[2 * i] = fminf(fmaxf(__fmul_rn(__uint_as_float(w[i] << 16), av[2 * i]), -65504.f), 65504.f);
+      v[2 * i + 1] = fminf(fmaxf(__fmul_rn(__uint_as_float(w[i] & 0xFFFF0000u), av[2 * i + 1]), -65504.f), 65504.f);
+    }
     uint32_t o[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const float lo = fminf(fmaxf(__fmul_rn(__uint_as_float(w[i] << 16), av[2 * i]), -65504.f), 65504.f);
-      const float hi = fminf(fmaxf(__fmul_rn(__uint_as_float(w[i] & 0xFFFF0000u), av[2 * i + 1]), -65504.f), 65504.f);
-      const __half2 p = __floats2half2_rn(lo, hi);
+      const int k = 4 * (i >> 1) + (i & 1);  // (0, 2), (1, 3), (4, 6), (5, 7)
+      const __half2 p = __floats2half2_rn(v[k], v[k + 2]);
       o[i] = *reinterpret_cast<const uint32_t*>(&p);
     }
     *reinterpret_cast<uint4*>(xs + static_cast<int64_t>(m) * K + kv * 8) = make_uint4(o[0], o[1], o[2], o[3]);
@@ -312,18 +433,73 @@ __global__ void __launch_bounds__(256) scale_cols_f16_kernel(const __nv_bfloat16
 }
 
 template <int TN>
-static int launch(const void* xs, int64_t ld_elems, const uint8_t* w_packed, const float* r, int M, int N,
-                  int K, void* y, int y_dtype, cudaStream_t stream, DeviceState* st) {
-  CUtensorMap tm_x;
-  int rc = make_tmap_2d_u8(&tm_x, xs, static_cast<uint64_t>(K) * 2, M, static_cast<uint64_t>(ld_elems) * 2, 128, TN,
+static int launch(const void* xs, const uint8_t* w_packed, const float* r, int M, int N, int K, void* y, int y_dtype,
+                  int split, cudaStream_t stream, DeviceState* st) {
+  CUtensorMap tm_x, tm_y;
+  int rc = make_tmap_2d_u8(&tm_x, xs, static_cast<uint64_t>(K) * 2, M, static_cast<uint64_t>(K) * 2, 128, TN / 2,
                            CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc != DQ_OK) return rc;
-  const dim3 grid((N + kBN - 1) / kBN, (M + TN - 1) / TN, 1);
-  cudaError_t e = launch_pdl(gemm_a16w4_kernel<TN>, grid, dim3(kThreads), Cfg<TN>::kSmemBytes, stream, w_packed,
-                             tm_x, r, y, y_dtype == DQ_DTYPE_BF16 ? 1 : 0, M, N, K, st->status_dev);
+  const int esz = y_dtype == DQ_DTYPE_BF16 ? 2 : 4;
+  const int bulk = split == 1 && (static_cast<size_t>(N) * esz) % 16 == 0 && aligned(y, 16) ? 1 : 0;
+  tm_y = tm_x;  // a valid map is passed either way
+  if (bulk) {
+    rc = make_tmap_2d_out(&tm_y, y, esz, static_cast<uint64_t>(N), static_cast<uint64_t>(M), kBN, 32);
+    if (rc != DQ_OK) return rc;
+  }
+  const int row_pairs = (N + 2 * kBN - 1) / (2 * kBN), tok_tiles = (M + TN - 1) / TN;
+  const int tiles = row_pairs * tok_tiles, pairs = st->sm_count / 2;
+  const int ng = K / kGroup, gps = (ng + split - 1) / split;
+  int tok_block = static_cast<int>((40ll << 20) / (static_cast<int64_t>(TN) * K * 2));
+  if (tok_block < 1) tok_block = 1;
+  if (tok_block > tok_tiles) tok_block = tok_tiles;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * (split > 1 ? tiles * split : (tiles < pairs ? tiles : pairs)), 1, 1);
+  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.dynamicSmemBytes = Cfg<TN>::kSmemBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2 * split;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_a16w4_kernel<TN>, w_packed, tm_x, tm_y, bulk, r, y,
+                                           y_dtype == DQ_DTYPE_BF16 ? 1 : 0, M, N, K, row_pairs, tok_tiles, tok_block,
+                                           split, gps, st->status_dev);
   if (e != cudaSuccess)
-    return set_error(DQ_ERR_CUDA, "gemm_a16w4 launch failed (TN=%d): %s", TN, cudaGetErrorString(e));
+    return set_error(DQ_ERR_CUDA, "gemm_a16w4 launch failed (TN=%d split=%d): %s", TN, split, cudaGetErrorString(e));
   return DQ_OK;
+}
+
+// Token tile and split of K: the cheapest in rounds of one tile per CTA pair.
+struct Shape {
+  int tn, split;
+};
+static Shape pick_shape(int M, int row_pairs, int ng, int sm_count) {
+  static const struct { int tn; float group_us; } kTiles[] = {{256, 0.62f}, {192, 0.55f}, {128, 0.45f}, {64, 0.30f}, {32, 0.28f}};
+  const int forced = tuning(DQ_TUNE_A16_TILE);
+  Shape best = {256, 1};
+  float best_cost = 1e30f;
+  for (const auto& t : kTiles) {
+    if (forced != 0 && forced % 1000 != t.tn) continue;
+    const int tiles = row_pairs * ((M + t.tn - 1) / t.tn);
+    for (int split = 1; split <= (t.tn <= 64 ? 4 : 1); split *= 2) {
+      if (split > 1 && ng / split < 2) break;
+      if (forced >= 1000 && forced / 1000 != split) continue;
+      // a cluster needs its CTAs in one GPC, which leaves about a tenth of the SMs unused
+      const int fit = split == 1 ? sm_count / 2 : sm_count * 9 / 10 / (2 * split);
+      const int rounds = (tiles + fit - 1) / fit;
+      const float cost = rounds * ((ng + split - 1) / split * t.group_us + 1.0f + (split > 1 ? 1.0f : 0.0f));
+      if (cost < best_cost) {
+        best_cost = cost;
+        best = {t.tn, split};
+      }
+    }
+  }
+  return best;
 }
 
 }  // namespace a16
@@ -331,9 +507,12 @@ static int launch(const void* xs, int64_t ld_elems, const uint8_t* w_packed, con
 int init_gemm_a16w4_kernels() {
   cudaError_t e = cudaFuncSetAttribute(a16::gemm_a16w4_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        a16::Cfg<32>::kSmemBytes);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(a16::gemm_a16w4_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             a16::Cfg<128>::kSmemBytes);
+#define DQ_A16_ATTR(TN)                                                                                     \
+  if (e == cudaSuccess)                                                                                     \
+    e = cudaFuncSetAttribute(a16::gemm_a16w4_kernel<TN>, cudaFuncAttributeMaxDynamicSharedMemorySize,       \
+                             a16::Cfg<TN>::kSmemBytes);
+  DQ_A16_ATTR(64) DQ_A16_ATTR(128) DQ_A16_ATTR(192) DQ_A16_ATTR(256)
+#undef DQ_A16_ATTR
   if (e != cudaSuccess)
     return set_error(DQ_ERR_CUDA, "cudaFuncSetAttribute(gemm_a16w4) failed: %s", cudaGetErrorString(e));
   return DQ_OK;
@@ -373,8 +552,12 @@ extern "C" int dq_linear_a16w4(const void* x_bf16, int64_t ldx, const float* a, 
   DQ_CHECK_CUDA(launch_pdl(a16::scale_cols_f16_kernel, dim3(blocks), dim3(256), 0, s,
                            static_cast<const __nv_bfloat16*>(x_bf16), ldx, a, M, K,
                            static_cast<__half*>(scratch)));
-  const void* xs = scratch;
-  const int64_t ld = K;
-  if (M <= 32) return a16::launch<32>(xs, ld, w_packed, r, M, N, K, y, y_dtype, s, st);
-  return a16::launch<128>(xs, ld, w_packed, r, M, N, K, y, y_dtype, s, st);
+  const a16::Shape shape = a16::pick_shape(M, (N + 2 * a16::kBN - 1) / (2 * a16::kBN), K / kGroup, st->sm_count);
+  switch (shape.tn) {
+    case 32: return a16::launch<32>(scratch, w_packed, r, M, N, K, y, y_dtype, shape.split, s, st);
+    case 64: return a16::launch<64>(scratch, w_packed, r, M, N, K, y, y_dtype, shape.split, s, st);
+    case 128: return a16::launch<128>(scratch, w_packed, r, M, N, K, y, y_dtype, shape.split, s, st);
+    case 192: return a16::launch<192>(scratch, w_packed, r, M, N, K, y, y_dtype, shape.split, s, st);
+    default: return a16::launch<256>(scratch, w_packed, r, M, N, K, y, y_dtype, shape.split, s, st);
+  }
 }
