@@ -17,16 +17,19 @@
 // the tokens' activations.  The weight operand goes to the tensor core from TENSOR MEMORY: eight unpack warps read the
 // packed tile (8 KB codes + 256 B scales per group of 128 k), expand the nibbles of their row to fp16 code * scale and
 // store them with tcgen05.st (lane = weight row, column = two k).  Shared memory then carries only the packed tile and
-// the activations: 80 KB per group of a 256-token tile, in 1024 cycles of UMMAs.  (A single-CTA 128 x 128 tile with the
-// expanded weights in shared memory moved 144 KB in 512 and was bound by that port: 4096 -> 28672 at 512 tokens 191 us.)
-//   warps 0-7    unpack: warp w owns TMEM lanes 32 (w & 3) .. and k 64 (w >> 2) .. of a group.  A nibble pair becomes
-//                half2 by bit tricks: (w >> s) & 0x000F000F picks two two's-complement nibbles, ^ 0x64086408 turns them
-//                into the fp16 numbers 1032 + code, a packed subtract gives code exactly, a packed multiply by the fp16
-//                group scale the weight.  The nibbles picked together are k and k + 2; the pre-pass below writes the
-//                activations in that order, so nothing has to be shuffled here.
-//   warps 8-11   epilogue: accumulator -> registers -> shared memory (32 tokens at a time) -> bulk store
-//   warp 12      producer: one bulk copy and two tiled copies per group
-//   warps 13-14  UMMA issue (of the even CTA, for both); tiles of up to 64 tokens: two warps take alternate groups into
+// the activations: 80 KB per group of a 256-token tile, in 1024 cycles of UMMAs.  4096 -> 28672: 16 tokens 25 us, 512 tokens 92, 8192 tokens 1212
+// (1.6 PFLOPS).  (A single-CTA 128 x 128 tile with the
+// expanded weights in shared memory moved 144 KB in 512 and was bound by that port: 50, 209, 2820 us.)
+//   warps 0-15   unpack, two sets of eight that take groups in turn: warp w owns TMEM lanes 32 (w & 3) .. and
+//                k 64 ((w >> 2) & 1) .. of a group.  A nibble pair becomes half2 by bit tricks: (w >> s) & 0x000F000F
+//                picks two two's-complement nibbles, ^ 0x64086408 turns them into the fp16 numbers 1032 + code, a packed
+//                subtract gives code exactly, a packed multiply by the fp16 group scale the weight.  The nibbles picked
+//                together are k and k + 2; the pre-pass below writes the activations in that order, so nothing has to be
+//                shuffled here.
+//   warps 16-19  epilogue: accumulator -> registers -> shared memory (32 tokens at a time) -> bulk store
+//   warps 20, 23 producers: two tiled copies of activations, one bulk copy of packed weights per group.  (One producer
+//                for both, with the tile and ring positions divided out of a group counter, took 0.9 us per group.)
+//   warps 21-22  UMMA issue (of the even CTA, for both); tiles of up to 64 tokens: two warps take alternate groups into
 //                an accumulator each, because issuing a group takes one warp longer than executing it
 // Persistent CTAs; where the tiles leave the chip idle (decode batches) K is split over the pairs of a larger cluster
 // instead, and the partial tiles are summed in rank order through distributed shared memory.  Every wait is bounded.
@@ -43,8 +46,10 @@ namespace dq {
 namespace a16 {
 
 constexpr int kBN = 128;                 // weight rows per CTA; a pair works on 256
-constexpr int kUnpackWarps = 8, kEpiWarps = 4, kProducerWarp = 12, kIssuerWarp = 13;
-constexpr int kThreads = 512;
+constexpr int kSets = 2;  // sets of eight unpack warps, taking groups in turn: one set needs 0.42 us for a group, two 0.33
+constexpr int kUnpackWarps = 8, kEpiWarp = kSets * 8, kEpiWarps = 4, kProducerWarp = kEpiWarp + 4, kIssuerWarp = kEpiWarp + 5,
+              kWeightWarp = kEpiWarp + 7;
+constexpr int kThreads = (kEpiWarp + 8) * 32;
 constexpr int kACols = 64;               // TMEM columns of one expanded group: 128 fp16
 constexpr int kOutChunk = 32 * kBN * 4;  // 32 tokens x 128 rows of fp32 (bf16 uses half)
 
@@ -176,16 +181,16 @@ gemm_a16w4_kernel(const uint8_t* __restrict__ w_packed, const __grid_constant__ 
   const uint32_t a_base = tmem_base + C::kAccCols;
   const bool live = *abort_flag == 0;
 
-  if (warp < kUnpackWarps) {
+  if (warp < kEpiWarp) {
     // ------------------------------------------------------------------ unpack
-    const int q = warp & 3, h = warp >> 2;
+    const int q = warp & 3, h = (warp >> 2) & 1;
     const int row = q * 32 + lane;
     const uint32_t t_lane = a_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(h * 32);
     const uint32_t a_full_addr = dsmem_map(smem_u32(a_full), even);
     const int total = live ? my_tiles * ng : 0;
     // chunk positions inside the packed row are swizzled by (row >> 1) & 3
     const int at0 = row * 64 + (((2 * h) ^ ((row >> 1) & 3)) << 4), at1 = row * 64 + (((2 * h + 1) ^ ((row >> 1) & 3)) << 4);
-    for (int gi = 0; gi < total; ++gi) {
+    for (int gi = warp >> 3; gi < total; gi += kSets) {
       const int sp = gi % C::SP, ab = gi % C::NA;
       if (!mbar_wait(&full_p[sp], (gi / C::SP) & 1, abort_flag, ASITE_UNPACK)) break;
       const uint8_t* tile = smem + C::kOffP + sp * kTileBytes;
@@ -220,7 +225,7 @@ gemm_a16w4_kernel(const uint8_t* __restrict__ w_packed, const __grid_constant__ 
     const int q = warp & 3;
     const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
     const uint32_t acc_empty_addr = dsmem_map(smem_u32(acc_empty), even);
-    const bool leader = warp == kUnpackWarps && lane == 0;
+    const bool leader = warp == kEpiWarp && lane == 0;
     const bool second = kIssuers == 2 && ng > 1;  // the second issuer had groups to add up
     int chunk_no = 0;
     grid_dep_wait();  // what last used y may still be running
@@ -246,10 +251,14 @@ gemm_a16w4_kernel(const uint8_t* __restrict__ w_packed, const __grid_constant__ 
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = ng > 0 ? __uint_as_float(u[j]) : 0.f;
           if (second) {
-            tmem_ld_x32(at + TN, u);
-            tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] += __uint_as_float(u[j]);
+            for (int b = 0; b < 32; b += 16) {
+              uint32_t u2[16];
+              tmem_ld_x16(at + TN + b, u2);
+              tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < 16; ++j) v[b + j] += __uint_as_float(u2[j]);
+            }
           }
         }
         if (c0 + 32 >= cols) {  // the accumulator goes back before its last columns are stored
@@ -290,38 +299,47 @@ gemm_a16w4_kernel(const uint8_t* __restrict__ w_packed, const __grid_constant__ 
     }
     if (leader) bulk_wait_group_read0();
   } else if (warp == kProducerWarp) {
-    // ------------------------------------------------------------------ producer (both CTAs)
+    // ------------------------------------------------------------------ activations (both CTAs)
     if (lane == 0 && live) {
-      const uint64_t pol_w = tok_tiles == 1 ? l2_policy_evict_first() : l2_policy_evict_last();
       const uint64_t pol_x = l2_policy_evict_last();
       const uint32_t full_x_addr = dsmem_map(smem_u32(full_x), even);
-      const int total = my_tiles * ng;
-      auto load_w = [&](int gi) {
-        int row_tile, tok_tile;
-        tile_of(gi / ng, row_tile, tok_tile);
-        if (row_tile >= row_tiles) row_tile = row_tiles - 1;  // computed and not stored
-        mbar_expect_tx(&full_p[gi % C::SP], kTileBytes);
-        bulk_load_1d(smem + C::kOffP + (gi % C::SP) * kTileBytes,
-                     w_packed + (static_cast<size_t>(row_tile) * total_groups + g_begin + gi % ng) * kTileBytes, kTileBytes,
-                     &full_p[gi % C::SP], pol_w);
-      };
-      // The weights do not depend on the kernel before this one, the activations do: the packed ring is filled first.
-      const int pre = total < C::SP ? total : C::SP;
-      for (int gi = 0; gi < pre; ++gi) load_w(gi);
       grid_dep_wait();
-      for (int gi = 0; gi < total; ++gi) {
-        const int sx = gi % C::SX;
+      int sx = 0;
+      uint32_t ph = 1;
+      bool ok = true;
+      for (int it = 0; it < my_tiles && ok; ++it) {
         int row_tile, tok_tile;
-        tile_of(gi / ng, row_tile, tok_tile);
-        const int t0 = tok_tile * TN + rank * (TN / 2), kx = (g_begin + gi % ng) * 256;
-        if (!mbar_wait(&empty_x[sx], ((gi / C::SX) & 1) ^ 1, abort_flag, ASITE_TMA)) break;
-        if (rank == 0) mbar_expect_tx(&full_x[sx], 2 * C::kXStage);
-        uint8_t* xs = smem + C::kOffX + sx * C::kXStage;
-        tma_load_2d_pair(xs, &tm_x, kx, t0, full_x_addr + static_cast<uint32_t>(sx) * 8u, pol_x);
-        tma_load_2d_pair(xs + C::kXAtom, &tm_x, kx + 128, t0, full_x_addr + static_cast<uint32_t>(sx) * 8u, pol_x);
-        if (gi + C::SP < total) {
-          if (!mbar_wait(&empty_p[gi % C::SP], (gi / C::SP) & 1, abort_flag, ASITE_TMA)) break;
-          load_w(gi + C::SP);
+        tile_of(it, row_tile, tok_tile);
+        const int t0 = tok_tile * TN + rank * (TN / 2);
+        for (int i = 0; i < ng; ++i) {
+          if (!mbar_wait(&empty_x[sx], ph, abort_flag, ASITE_TMA)) { ok = false; break; }
+          if (rank == 0) mbar_expect_tx(&full_x[sx], 2 * C::kXStage);
+          uint8_t* xs = smem + C::kOffX + sx * C::kXStage;
+          const int kx = (g_begin + i) * 256;
+          tma_load_2d_pair(xs, &tm_x, kx, t0, full_x_addr + static_cast<uint32_t>(sx) * 8u, pol_x);
+          tma_load_2d_pair(xs + C::kXAtom, &tm_x, kx + 128, t0, full_x_addr + static_cast<uint32_t>(sx) * 8u, pol_x);
+          if (++sx == C::SX) { sx = 0; ph ^= 1u; }
+        }
+      }
+    }
+  } else if (warp == kWeightWarp) {
+    // ------------------------------------------------------------------ packed weights (both CTAs): they do not depend
+    // on the kernel before this one, so the ring fills while that one is still running
+    if (lane == 0 && live) {
+      const uint64_t pol_w = tok_tiles == 1 ? l2_policy_evict_first() : l2_policy_evict_last();
+      int sp = 0;
+      uint32_t ph = 1;
+      bool ok = true;
+      for (int it = 0; it < my_tiles && ok; ++it) {
+        int row_tile, tok_tile;
+        tile_of(it, row_tile, tok_tile);
+        if (row_tile >= row_tiles) row_tile = row_tiles - 1;  // computed and not stored
+        const uint8_t* src = w_packed + (static_cast<size_t>(row_tile) * total_groups + g_begin) * kTileBytes;
+        for (int i = 0; i < ng; ++i, src += kTileBytes) {
+          if (!mbar_wait(&empty_p[sp], ph, abort_flag, ASITE_TMA)) { ok = false; break; }
+          mbar_expect_tx(&full_p[sp], kTileBytes);
+          bulk_load_1d(smem + C::kOffP + sp * kTileBytes, src, kTileBytes, &full_p[sp], pol_w);
+          if (++sp == C::SP) { sp = 0; ph ^= 1u; }
         }
       }
     }
@@ -474,12 +492,14 @@ static int launch(const void* xs, const uint8_t* w_packed, const float* r, int M
   return DQ_OK;
 }
 
-// Token tile and split of K: the cheapest in rounds of one tile per CTA pair.
+// Token tile and split of K: the cheapest in rounds of one tile per CTA pair.  Group times measured on B200, the wide
+// tiles' in long runs at the power cap (a 256-token tile has one accumulator and waits for its drain once per tile; up to
+// 64 tokens a group costs what its nibbles cost to expand).
 struct Shape {
   int tn, split;
 };
 static Shape pick_shape(int M, int row_pairs, int ng, int sm_count) {
-  static const struct { int tn; float group_us; } kTiles[] = {{256, 0.62f}, {192, 0.55f}, {128, 0.45f}, {64, 0.30f}, {32, 0.28f}};
+  static const struct { int tn; float group_us; } kTiles[] = {{256, 0.82f}, {192, 0.60f}, {128, 0.45f}, {64, 0.335f}, {32, 0.33f}};
   const int forced = tuning(DQ_TUNE_A16_TILE);
   Shape best = {256, 1};
   float best_cost = 1e30f;
@@ -489,10 +509,10 @@ static Shape pick_shape(int M, int row_pairs, int ng, int sm_count) {
     for (int split = 1; split <= (t.tn <= 64 ? 4 : 1); split *= 2) {
       if (split > 1 && ng / split < 2) break;
       if (forced >= 1000 && forced / 1000 != split) continue;
-      // a cluster needs its CTAs in one GPC, which leaves about a tenth of the SMs unused
-      const int fit = split == 1 ? sm_count / 2 : sm_count * 9 / 10 / (2 * split);
+      // a cluster needs its CTAs in one GPC, which leaves some SMs unused: 33 clusters of four run together, 15 of eight
+      const int fit = split == 1 ? sm_count / 2 : sm_count * 17 / 20 / (2 * split);
       const int rounds = (tiles + fit - 1) / fit;
-      const float cost = rounds * ((ng + split - 1) / split * t.group_us + 1.0f + (split > 1 ? 1.0f : 0.0f));
+      const float cost = rounds * ((ng + split - 1) / split * t.group_us + (t.tn == 256 ? 2.0f : 1.0f) + (split > 1 ? 1.5f : 0.0f));
       if (cost < best_cost) {
         best_cost = cost;
         best = {t.tn, split};

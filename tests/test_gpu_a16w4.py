@@ -85,3 +85,25 @@ def test_perm_linear_without_activation_cast_runs_a16w4():
     ref = pl.layer(pl._quantise_act(x))  # the reference's formulation on the 16-bit weight
     err = ((y.float() - ref.float()).abs().max() / ref.float().abs().max()).item()
     assert err < 2e-2, err  # bf16 rounding of the output; the reference rounds x * a to bf16, this path to fp16
+
+
+@pytest.mark.parametrize("tile", [32, 2032, 4032, 64, 2064, 4064, 128, 192, 256])
+@pytest.mark.parametrize("M,N,K", [(1, 100, 128), (31, 136, 640), (64, 1000, 1152), (300, 4104, 256), (520, 384, 896)])
+def test_every_tile_and_split(tile, M, N, K):
+    """Each token tile and split of K of the CTA-pair kernel: ragged tokens and rows, an odd number of 128-row tiles,
+    fewer groups than the rings and than the split's CTAs, bulk and direct stores, both output types."""
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    qw, sw = ops.quant_w_int4((torch.randn(N, K, generator=g, device=DEV) * 0.02).to(torch.bfloat16))
+    pw = ops.pack_w_int4(qw, sw)
+    x = torch.randn(M, K, generator=g, device=DEV).to(torch.bfloat16)
+    a, r = torch.rand(K, generator=g, device=DEV) + 0.5, torch.rand(N, generator=g, device=DEV) + 0.5
+    ref = _restatement(x, a, qw, sw, r)
+    try:
+        _lib.set_tuning("a16_tile", tile if K // 128 >= 2 * (tile // 1000) else tile % 1000)
+        y = ops.linear_a16w4(x, a, pw, r, out_dtype=torch.float32)
+        yb = ops.linear_a16w4(x, a, pw, r)
+    finally:
+        _lib.set_tuning("a16_tile", 0)
+    _lib.device_status(0)
+    assert ((y.double() - ref).abs().max() / ref.abs().max()).item() < 1e-4
+    assert torch.equal(yb, y.to(torch.bfloat16))
