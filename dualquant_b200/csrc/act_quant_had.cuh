@@ -279,10 +279,13 @@ act_quant_had_fast_kernel(const XT* __restrict__ x, const XT* __restrict__ up, i
 // - load (+ SiLU * up), Walsh-Hadamard inside the segments, the S x S stage across them, absmax,
 // codes - are a serial chain.  Here four CTAs share a row: CTA c loads and transforms segments
 // [c S/4, (c+1) S/4), then computes the matrix stage for columns [c P/4, (c+1) P/4) of every
-// segment, reading the other CTAs' segments through distributed shared memory; the row absmax is
-// exchanged the same way.  Every sum is formed exactly as in the fast kernel (same Walsh-Hadamard
-// routine, j ascending fp32 FMAs with the factor's entry as coefficient), so scales and codes are
-// bit-identical.  Needs S % 4 == 0 and the factor in c_had_mat2.
+// segment; the row absmax is exchanged through distributed shared memory.  The columns of the other
+// CTAs' segments are copied over once, 16 bytes per load: read from there by every thread that needs
+// them, a value at a time, they were 448 warp-wide remote loads per CTA at some 20 cycles each.
+// Every sum is formed exactly as in the fast kernel (same Walsh-Hadamard routine, j ascending fp32
+// FMAs with the factor's entry as coefficient), so scales and codes are bit-identical.  The factor is
+// read from the caller's matrix, not from the constant bank: nothing has to be uploaded between the
+// kernels of a decode step.  Needs S % 4 == 0.
 constexpr int kHadClusterCtas = 4;
 constexpr int kHadClusterThreads = 512;
 constexpr int kHadClusterMaxRows = 64;
@@ -290,8 +293,9 @@ constexpr int kHadClusterMaxRows = 64;
 template <int R, typename XT>
 __global__ void __launch_bounds__(kHadClusterThreads, 1)
 act_quant_had_cluster_kernel(const XT* __restrict__ x, const XT* __restrict__ up, int64_t ldx,
-                             const float* __restrict__ a, int S, float had_scale, int8_t* __restrict__ codes,
-                             float* __restrict__ sx, float* __restrict__ out, int mode, int scale_fp16) {
+                             const float* __restrict__ a, int S, float had_scale, const float* __restrict__ had_mat,
+                             int8_t* __restrict__ codes, float* __restrict__ sx, float* __restrict__ out, int mode,
+                             int scale_fp16) {
   constexpr int P = 32 * R;                   // segment length
   constexpr int PC = P / kHadClusterCtas;     // columns of the matrix stage per CTA
   constexpr int G = kHadClusterThreads / PC;  // threads per column: output rows i = qi, qi + G, ...
@@ -301,7 +305,8 @@ act_quant_had_cluster_kernel(const XT* __restrict__ x, const XT* __restrict__ up
   const int SQ = S / kHadClusterCtas;         // segments per CTA
   const int K = S * P;
   float* seg = sm_row;                        // [SQ][P]: this CTA's segments (read by its peers)
-  float* outv = sm_row + SQ * P;              // [S][PC]: this CTA's slice of the transformed row
+  float* colv = sm_row + SQ * P;              // [S][PC]: this CTA's columns of all segments, then its slice of the result
+  float* coef = colv + S * PC;                // [S][32]: the factor, rows padded with zeros
   grid_dep_launch_dependents();
   grid_dep_wait();
   const int rank = static_cast<int>(cluster_ctarank());
@@ -324,35 +329,46 @@ act_quant_had_cluster_kernel(const XT* __restrict__ x, const XT* __restrict__ up
     *reinterpret_cast<float4*>(seg + idx) = make_float4(v[0], v[1], v[2], v[3]);
     *reinterpret_cast<float4*>(seg + idx + 4) = make_float4(v[4], v[5], v[6], v[7]);
   }
+  for (int i = tid; i < S * 32; i += kHadClusterThreads) {
+    const int j = i & 31;
+    coef[i] = j < S ? had_mat[(i >> 5) * S + j] : 0.f;
+  }
   __syncthreads();
-  for (int sgm = warp; sgm < SQ; sgm += kHadClusterThreads / 32) wht_segment_warp<R>(seg + sgm * P, lane);
-  cluster_sync_all();  // every CTA's segments are transformed and visible to its peers
+  for (int sgm = warp; sgm < SQ; sgm += kHadClusterThreads / 32) wht_segment_warp<R>(seg + sgm * P, lane, had_scale);
+  cluster_sync_all();  // every CTA's segments are transformed (and scaled) and visible to its peers
+  {
+    const uint32_t seg_addr = smem_u32(seg);
+    for (int u = tid; u < S * (PC / 4); u += kHadClusterThreads) {
+      const int j = u / (PC / 4), c4 = u - j * (PC / 4);
+      const int owner = j / SQ;
+      const uint32_t from = seg_addr + static_cast<uint32_t>(((j - owner * SQ) * P + rank * PC + c4 * 4) * 4);
+      *reinterpret_cast<float4*>(colv + j * PC + c4 * 4) = dsmem_ld_f4(dsmem_map(from, static_cast<uint32_t>(owner)));
+    }
+  }
+  __syncthreads();
 
   const int col = tid % PC, qi = tid / PC;
   float v[32];
-  {
-    const uint32_t seg_addr = smem_u32(seg);
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      v[j] = 0.f;
-      if (j < S) {
-        const int owner = j / SQ, local = j - owner * SQ;
-        const uint32_t addr = dsmem_map(seg_addr + static_cast<uint32_t>((local * P + rank * PC + col) * 4),
-                                        static_cast<uint32_t>(owner));
-        v[j] = __fmul_rn(dsmem_ld_f32(addr), had_scale);
-      }
-    }
-  }
+  for (int j = 0; j < 32; ++j) v[j] = j < S ? colv[j * PC + col] : 0.f;
+  __syncthreads();  // every thread holds its inputs before the first result replaces them
   float amax = 0.f;
   for (int i = qi; i < S; i += G) {  // i is the same for every lane of a warp
+    const float4* h4 = reinterpret_cast<const float4*>(coef + i * 32);
     float acc = 0.f;
 #pragma unroll
-    for (int j = 0; j < 32; ++j) acc = fmaf(c_had_mat2[i * 32 + j].x, v[j], acc);  // padding entries are zero
-    outv[i * PC + col] = acc;
+    for (int j = 0; j < 32; j += 4) {
+      const float4 h = h4[j >> 2];
+      acc = fmaf(h.x, v[j], acc);
+      acc = fmaf(h.y, v[j + 1], acc);
+      acc = fmaf(h.z, v[j + 2], acc);
+      acc = fmaf(h.w, v[j + 3], acc);
+    }
+    colv[i * PC + col] = acc;
     amax = fmaxf(amax, fabsf(acc));
   }
   float s = 1.f;
-  amax = block_max(amax, red, kHadClusterThreads / 32);  // (also orders the outv writes before their reads below)
+  amax = block_max(amax, red, kHadClusterThreads / 32);  // (also orders the colv writes before their reads below)
   if (tid < kHadClusterCtas)
     dsmem_store_f32(dsmem_map(smem_u32(&pmax[rank]), static_cast<uint32_t>(tid)), amax);
   cluster_sync_all();  // the four partial maxima have landed everywhere; no remote access after this point
@@ -369,7 +385,7 @@ act_quant_had_cluster_kernel(const XT* __restrict__ x, const XT* __restrict__ up
     const int i = u / (PC / 8), piece = u - i * (PC / 8);
     float e8[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) e8[e] = outv[i * PC + piece * 8 + e];
+    for (int e = 0; e < 8; ++e) e8[e] = colv[i * PC + piece * 8 + e];
     emit8(e8, s, mode, crow, orow, i * P + rank * PC + piece * 8, scale_fp16);
   }
 }
@@ -579,10 +595,6 @@ int launch_had_fast_t(const XT* x, const XT* up, int64_t ldx, const float* a, co
     HadPlan plan;
     if (plan_fast_hadamard(had, K, &plan)) {
       *taken = true;
-      if (plan.matrix) {
-        int rc2 = upload_had_matrix(had->had_mat, plan.S, stream);
-        if (rc2 != DQ_OK) return rc2;
-      }
       // across 2 ... 32 heads of 128 values, many rows: the register-only kernel
       if (had->kind == DQ_HAD_PARTIAL && had->had_dim == 128 && plan.S >= 2 && M >= kHeadsKernelMinRows &&
           up == nullptr && mode == MODE_CODES && codes != nullptr && (scale_fp16 & 0xFF) != 2) {
@@ -608,7 +620,7 @@ int launch_had_fast_t(const XT* x, const XT* up, int64_t ldx, const float* a, co
       // a handful of rows (decode): four CTAs per row
       if (plan.matrix && plan.inner && plan.S % kHadClusterCtas == 0 && M <= kHadClusterMaxRows && plan.R >= 4) {
         const int P = 32 * plan.R;
-        const size_t csmem = static_cast<size_t>(plan.S / kHadClusterCtas * P + plan.S * (P / kHadClusterCtas)) * 4;
+        const size_t csmem = static_cast<size_t>(plan.S / kHadClusterCtas * P + plan.S * (P / kHadClusterCtas) + plan.S * 32) * 4;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(kHadClusterCtas * M, 1, 1);
         cfg.blockDim = dim3(kHadClusterThreads, 1, 1);
@@ -625,7 +637,7 @@ int launch_had_fast_t(const XT* x, const XT* up, int64_t ldx, const float* a, co
         cfg.numAttrs = 2;
 #define DQ_HAD_CLUSTER(RR)                                                                                  \
   DQ_CHECK_CUDA(cudaLaunchKernelEx(&cfg, act_quant_had_cluster_kernel<RR, XT>, x, up, ldx, a, plan.S, had->scale, \
-                                   codes, sx, out, mode, scale_fp16))
+                                   had->had_mat, codes, sx, out, mode, scale_fp16))
         switch (plan.R) {
           case 4: DQ_HAD_CLUSTER(4); break;
           case 8: DQ_HAD_CLUSTER(8); break;
@@ -634,6 +646,10 @@ int launch_had_fast_t(const XT* x, const XT* up, int64_t ldx, const float* a, co
         }
 #undef DQ_HAD_CLUSTER
         return DQ_OK;
+      }
+      if (plan.matrix) {
+        int rc2 = upload_had_matrix(had->had_mat, plan.S, stream);
+        if (rc2 != DQ_OK) return rc2;
       }
       // many rows: smaller CTAs, several per SM (the row must leave room for three of them)
       const DeviceState* dst = current_state();
