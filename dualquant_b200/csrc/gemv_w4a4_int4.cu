@@ -28,7 +28,8 @@
 namespace dq {
 
 constexpr int kVBN = 128;       // weight rows per CTA
-constexpr int kVComputeWarps = 8;
+constexpr int kVSets = 1;  // warp sets that split the groups of a stage between them (1 or 2)
+constexpr int kVComputeWarps = 8 * kVSets;
 constexpr int kVThreads = (kVComputeWarps + 1) * 32;  // + 1 producer warp
 constexpr int kVGS = 2;         // weight groups per pipeline stage
 
@@ -48,7 +49,7 @@ struct VCfg {
   // the other CTAs expected on its SM, because throughput here is (bytes in flight) / (HBM latency).
   static constexpr int kMinStages = 2;
   static constexpr int kMaxStages = 10;
-  static constexpr int kMinCtas = (NT == 1) ? 3 : 2;
+  static constexpr int kMinCtas = (kVSets == 1) ? ((NT == 1) ? 4 : (NT == 2) ? 3 : 2) : ((NT <= 2) ? 2 : 1);
   static constexpr int kBarBytes = 2 * kMaxStages * 8 + 16;
   static_assert(TOK * kVBN * 4 <= kMinStages * kStage, "split-K exchange tile must fit in the ring");
   static constexpr int smem_bytes(int stages) { return stages * kStage + kBarBytes + 1024; }
@@ -184,7 +185,8 @@ gemv_w4a4_int4_kernel(const uint8_t* __restrict__ w_packed,
     // ------------------------------------------------------------------ compute warps
     const int g = lane >> 2;  // fragment row / token index inside an 8-block
     const int t = lane & 3;
-    const int row = warp * 16 + g;  // local weight row (and row + 8)
+    const int set = warp >> 3;      // which group of each stage this warp works on
+    const int row = (warp & 7) * 16 + g;  // local weight row (and row + 8)
     float run[NT][4];
 #pragma unroll
     for (int nb = 0; nb < NT; ++nb)
@@ -198,40 +200,33 @@ gemv_w4a4_int4_kernel(const uint8_t* __restrict__ w_packed,
       const uint8_t* st = smem + s * C::kStage;
       int cnt = ng - i * kVGS;
       if (cnt > kVGS) cnt = kVGS;
-      // The groups of a stage in two steps - all shared-memory reads, then the arithmetic in group order - so that
-      // a warp waits for shared memory once per stage and the MMA chains of the groups overlap.
-      uint4 wa[kVGS], wb[kVGS], xlo[kVGS][NT], xhi[kVGS][NT];
-      float s0[kVGS], s1[kVGS];
+      // with two warp sets, warps 0-7 take the first group of the stage and warps 8-15 the second
 #pragma unroll
-      for (int gi = 0; gi < kVGS; ++gi) {
-        if (gi < cnt) {
-          const uint8_t* tile = st + C::kOffW + gi * kTileBytes;
-          // k chunk t of rows `row` and `row + 8` (chunk positions are swizzled by (row >> 1) & 3,
-          // the same value for both rows)
-          const int tp = t ^ ((g >> 1) & 3);
-          wa[gi] = *reinterpret_cast<const uint4*>(tile + row * 64 + tp * 16);
-          wb[gi] = *reinterpret_cast<const uint4*>(tile + (row + 8) * 64 + tp * 16);
-          const __half* sc = reinterpret_cast<const __half*>(tile + kTileCodeBytes);
-          s0[gi] = __half2float(sc[row]) * 0.0625f;
-          s1[gi] = __half2float(sc[row + 8]) * 0.0625f;
-#pragma unroll
-          for (int nb = 0; nb < NT; ++nb) {
-            // activation codes: [group][token][128 B]; 16-byte chunk c of token row m sits at
-            // chunk position c ^ (m & 7) (128-byte swizzle); this lane needs chunks 2t and 2t + 1
-            const uint8_t* xr = st + C::kOffX + gi * C::kXGroupBytes + (nb * 8 + g) * kGroup;
-            xlo[gi][nb] = *reinterpret_cast<const uint4*>(xr + (((2 * t) ^ g) << 4));
-            xhi[gi][nb] = *reinterpret_cast<const uint4*>(xr + (((2 * t + 1) ^ g) << 4));
-          }
-        }
-      }
-#pragma unroll
-      for (int gi = 0; gi < kVGS; ++gi) {
+      for (int gi = set; gi < kVGS; gi += kVSets) {
         if (gi >= cnt) break;
+        const uint8_t* tile = st + C::kOffW + gi * kTileBytes;
+        // k chunk t of rows `row` and `row + 8` (chunk positions are swizzled by (row >> 1) & 3,
+        // the same value for both rows)
+        const int tp = t ^ ((g >> 1) & 3);
+        const uint4 wa = *reinterpret_cast<const uint4*>(tile + row * 64 + tp * 16);
+        const uint4 wb = *reinterpret_cast<const uint4*>(tile + (row + 8) * 64 + tp * 16);
+        const __half* sc = reinterpret_cast<const __half*>(tile + kTileCodeBytes);
+        const float s0 = __half2float(sc[row]) * 0.0625f;
+        const float s1 = __half2float(sc[row + 8]) * 0.0625f;
+        uint4 xlo[NT], xhi[NT];
+#pragma unroll
+        for (int nb = 0; nb < NT; ++nb) {
+          // activation codes: [group][token][128 B]; 16-byte chunk c of token row m sits at
+          // chunk position c ^ (m & 7) (128-byte swizzle); this lane needs chunks 2t and 2t + 1
+          const uint8_t* xr = st + C::kOffX + gi * C::kXGroupBytes + (nb * 8 + g) * kGroup;
+          xlo[nb] = *reinterpret_cast<const uint4*>(xr + (((2 * t) ^ g) << 4));
+          xhi[nb] = *reinterpret_cast<const uint4*>(xr + (((2 * t + 1) ^ g) << 4));
+        }
         // Word j of a lane's 16-byte chunk feeds MMA step j: low nibbles are
         // k = 32t + 4j + {0..3} of the group (fragment slots a0/a1), high nibbles
         // k = 32t + 16 + 4j + {0..3} (a2/a3).
-        const uint32_t wav[4] = {wa[gi].x, wa[gi].y, wa[gi].z, wa[gi].w};
-        const uint32_t wbv[4] = {wb[gi].x, wb[gi].y, wb[gi].z, wb[gi].w};
+        const uint32_t wav[4] = {wa.x, wa.y, wa.z, wa.w};
+        const uint32_t wbv[4] = {wb.x, wb.y, wb.z, wb.w};
         int c[NT][2][4];  // two partial accumulators per token block: dependent chains of 2 MMAs
 #pragma unroll
         for (int nb = 0; nb < NT; ++nb)
@@ -245,8 +240,8 @@ gemv_w4a4_int4_kernel(const uint8_t* __restrict__ w_packed,
           const uint32_t a3 = wbv[j] & 0xF0F0F0F0u;
 #pragma unroll
           for (int nb = 0; nb < NT; ++nb) {
-            const uint32_t b0 = (j == 0) ? xlo[gi][nb].x : (j == 1) ? xlo[gi][nb].y : (j == 2) ? xlo[gi][nb].z : xlo[gi][nb].w;
-            const uint32_t b1 = (j == 0) ? xhi[gi][nb].x : (j == 1) ? xhi[gi][nb].y : (j == 2) ? xhi[gi][nb].z : xhi[gi][nb].w;
+            const uint32_t b0 = (j == 0) ? xlo[nb].x : (j == 1) ? xlo[nb].y : (j == 2) ? xlo[nb].z : xlo[nb].w;
+            const uint32_t b1 = (j == 0) ? xhi[nb].x : (j == 1) ? xhi[nb].y : (j == 2) ? xhi[nb].z : xhi[nb].w;
             mma_s8_16x8x32(c[nb][j & 1], a0, a1, a2, a3, b0, b1);
           }
         }
@@ -259,10 +254,10 @@ gemv_w4a4_int4_kernel(const uint8_t* __restrict__ w_packed,
             xa = __ldg(sg + (m < M ? m : M - 1));
             xb = __ldg(sg + (m + 1 < M ? m + 1 : M - 1));
           }
-          run[nb][0] = fmaf(static_cast<float>(c[nb][0][0] + c[nb][1][0]), GS ? __fmul_rn(s0[gi], xa) : s0[gi], run[nb][0]);
-          run[nb][1] = fmaf(static_cast<float>(c[nb][0][1] + c[nb][1][1]), GS ? __fmul_rn(s0[gi], xb) : s0[gi], run[nb][1]);
-          run[nb][2] = fmaf(static_cast<float>(c[nb][0][2] + c[nb][1][2]), GS ? __fmul_rn(s1[gi], xa) : s1[gi], run[nb][2]);
-          run[nb][3] = fmaf(static_cast<float>(c[nb][0][3] + c[nb][1][3]), GS ? __fmul_rn(s1[gi], xb) : s1[gi], run[nb][3]);
+          run[nb][0] = fmaf(static_cast<float>(c[nb][0][0] + c[nb][1][0]), GS ? __fmul_rn(s0, xa) : s0, run[nb][0]);
+          run[nb][1] = fmaf(static_cast<float>(c[nb][0][1] + c[nb][1][1]), GS ? __fmul_rn(s0, xb) : s0, run[nb][1]);
+          run[nb][2] = fmaf(static_cast<float>(c[nb][0][2] + c[nb][1][2]), GS ? __fmul_rn(s1, xa) : s1, run[nb][2]);
+          run[nb][3] = fmaf(static_cast<float>(c[nb][0][3] + c[nb][1][3]), GS ? __fmul_rn(s1, xb) : s1, run[nb][3]);
         }
       }
       __syncwarp();
@@ -270,9 +265,40 @@ gemv_w4a4_int4_kernel(const uint8_t* __restrict__ w_packed,
       if (++s == stages) { s = 0; ph ^= 1u; }
     }
 
+    // Fold the second warp set's partial sums into the first through shared memory.  All compute
+    // warps are past their last stage at the first barrier, so the ring can be reused.
+    if constexpr (kVSets == 2) {
+      float* red = reinterpret_cast<float*>(smem);
+      asm volatile("bar.sync 1, 512;" ::: "memory");
+      if (set == 1) {
+#pragma unroll
+        for (int nb = 0; nb < NT; ++nb)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int m = nb * 8 + 2 * t + e;
+            red[m * kVBN + row] = run[nb][e];
+            red[m * kVBN + row + 8] = run[nb][2 + e];
+          }
+      }
+      asm volatile("bar.sync 1, 512;" ::: "memory");
+      if (set == 0) {
+#pragma unroll
+        for (int nb = 0; nb < NT; ++nb)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int m = nb * 8 + 2 * t + e;
+            run[nb][e] += red[m * kVBN + row];
+            run[nb][2 + e] += red[m * kVBN + row + 8];
+          }
+      }
+    }
     // accumulator fragment: c0/c1 = (row, tokens 2t, 2t+1), c2/c3 = (row + 8, same tokens)
-    if (split_k > 1 || ar.world > 1) asm volatile("bar.sync 1, 256;" ::: "memory");  // ring reused as exchange tile
-    if (split_k == 1 && ar.world <= 1) {
+    if constexpr (kVSets == 1) {
+      if (split_k > 1 || ar.world > 1) asm volatile("bar.sync 1, 256;" ::: "memory");  // ring reused as exchange tile
+    }
+    if (set == 1) {
+      // nothing left to do for the second set
+    } else if (split_k == 1 && ar.world <= 1) {
 #pragma unroll
       for (int hrow = 0; hrow < 2; ++hrow) {
         const int n = n0 + row + 8 * hrow;
