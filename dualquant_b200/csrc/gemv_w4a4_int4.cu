@@ -12,7 +12,7 @@
 //     well over 100 KB of weights in flight (throughput = bytes in flight / HBM latency);
 //   * eight compute warps, each owning 16 weight rows.  A lane reads its packed nibbles straight
 //     from the stage (two 16-byte loads), splits them in registers ((w << 4) & 0xF0.. and
-//     w & 0xF0.., i.e. 16 * code, the 1/16 folded into the group scale) and feeds
+//     w & 0xF0.., i.e. 16 * code, the 1/16 applied to the finished sums) and feeds
 //     mma.sync.m16n8k32.s8 with int32 accumulation per group - no second shared-memory pass,
 //     no cross-warp hand-off on the critical path.  The k order inside a group is permuted
 //     identically for weights and activations (a dot product does not care);
@@ -28,8 +28,7 @@
 namespace dq {
 
 constexpr int kVBN = 128;       // weight rows per CTA
-constexpr int kVSets = 1;  // warp sets that split the groups of a stage between them (1 or 2)
-constexpr int kVComputeWarps = 8 * kVSets;
+constexpr int kVComputeWarps = 8;
 constexpr int kVThreads = (kVComputeWarps + 1) * 32;  // + 1 producer warp
 constexpr int kVGS = 2;         // weight groups per pipeline stage
 
@@ -49,7 +48,7 @@ struct VCfg {
   // the other CTAs expected on its SM, because throughput here is (bytes in flight) / (HBM latency).
   static constexpr int kMinStages = 2;
   static constexpr int kMaxStages = 10;
-  static constexpr int kMinCtas = (kVSets == 1) ? ((NT == 1) ? 4 : (NT == 2) ? 3 : 2) : ((NT <= 2) ? 2 : 1);
+  static constexpr int kMinCtas = (NT == 1) ? 4 : (NT == 2) ? 3 : 2;
   static constexpr int kBarBytes = 2 * kMaxStages * 8 + 16;
   static_assert(TOK * kVBN * 4 <= kMinStages * kStage, "split-K exchange tile must fit in the ring");
   static constexpr int smem_bytes(int stages) { return stages * kStage + kBarBytes + 1024; }
@@ -99,6 +98,14 @@ __device__ __forceinline__ void mma_s8_16x8x32(int (&c)[4], uint32_t a0, uint32_
       "{%0,%1,%2,%3};"
       : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// the same with a zero C (no registers to clear)
+__device__ __forceinline__ void mma_s8_16x8x32_first(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                                     uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
 }
 
 // GS: one activation scale per (token, weight group) - sx is then [K / 128][M], group-major - instead
@@ -185,120 +192,98 @@ gemv_w4a4_int4_kernel(const uint8_t* __restrict__ w_packed,
     // ------------------------------------------------------------------ compute warps
     const int g = lane >> 2;  // fragment row / token index inside an 8-block
     const int t = lane & 3;
-    const int set = warp >> 3;      // which group of each stage this warp works on
-    const int row = (warp & 7) * 16 + g;  // local weight row (and row + 8)
+    const int row = warp * 16 + g;  // local weight row (and row + 8)
     float run[NT][4];
 #pragma unroll
     for (int nb = 0; nb < NT; ++nb)
 #pragma unroll
       for (int e = 0; e < 4; ++e) run[nb][e] = 0.f;
 
-    int s = 0;
-    uint32_t ph = 0;
+    // The loop is bound by this half, not by the weight stream: copies alone take 9.9 us where the whole kernel took
+    // 13.1 (8 tokens, 4096 -> 28672), 114 warp instructions a group.  So a lane's offsets inside a stage are formed once,
+    // the stage is an address that steps along the ring, the first MMAs of a group take a zero C instead of cleared
+    // registers, and the 1/16 of the codes (they come as 16 * code; the factor is exact) goes to the finished sums.
+    // Measured, us: 4096 -> 28672 13.1 -> 11.5 (8 tokens), 17.3 -> 15.4 (16); 14336 -> 4096 10.8 -> 10.0;
+    // 8960 -> 12000 16.2 -> 14.4.
+    const int tp = t ^ ((g >> 1) & 3);  // k chunk t of rows `row` and `row + 8`: swizzled position, the same for both
+    const uint32_t off_w = static_cast<uint32_t>(C::kOffW + row * 64 + tp * 16);
+    const uint32_t off_s = static_cast<uint32_t>(C::kOffW + kTileCodeBytes + row * 2);
+    // activation codes: [group][token][128 B]; 16-byte chunk c of token row m sits at chunk position c ^ (m & 7)
+    // (128-byte swizzle); this lane needs chunks 2t and 2t + 1
+    const uint32_t off_x0 = static_cast<uint32_t>(C::kOffX + g * kGroup + (((2 * t) ^ g) << 4));
+    const uint32_t off_x1 = static_cast<uint32_t>(C::kOffX + g * kGroup + (((2 * t + 1) ^ g) << 4));
+    auto group = [&](const uint8_t* st, int gi, int i) {
+      const uint4 wa = *reinterpret_cast<const uint4*>(st + off_w + gi * kTileBytes);
+      const uint4 wb = *reinterpret_cast<const uint4*>(st + off_w + gi * kTileBytes + 8 * 64);
+      const float s0 = __half2float(*reinterpret_cast<const __half*>(st + off_s + gi * kTileBytes));
+      const float s1 = __half2float(*reinterpret_cast<const __half*>(st + off_s + gi * kTileBytes + 16));
+      uint4 xlo[NT], xhi[NT];
+#pragma unroll
+      for (int nb = 0; nb < NT; ++nb) {
+        xlo[nb] = *reinterpret_cast<const uint4*>(st + off_x0 + gi * C::kXGroupBytes + nb * 8 * kGroup);
+        xhi[nb] = *reinterpret_cast<const uint4*>(st + off_x1 + gi * C::kXGroupBytes + nb * 8 * kGroup);
+      }
+      // Word j of a lane's 16-byte chunk feeds MMA step j: low nibbles are
+      // k = 32t + 4j + {0..3} of the group (fragment slots a0/a1), high nibbles
+      // k = 32t + 16 + 4j + {0..3} (a2/a3).
+      const uint32_t wav[4] = {wa.x, wa.y, wa.z, wa.w};
+      const uint32_t wbv[4] = {wb.x, wb.y, wb.z, wb.w};
+      int c[NT][2][4];  // two partial accumulators per token block: dependent chains of 2 MMAs
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t a0 = (wav[j] << 4) & 0xF0F0F0F0u;
+        const uint32_t a2 = wav[j] & 0xF0F0F0F0u;
+        const uint32_t a1 = (wbv[j] << 4) & 0xF0F0F0F0u;
+        const uint32_t a3 = wbv[j] & 0xF0F0F0F0u;
+#pragma unroll
+        for (int nb = 0; nb < NT; ++nb) {
+          const uint32_t b0 = (j == 0) ? xlo[nb].x : (j == 1) ? xlo[nb].y : (j == 2) ? xlo[nb].z : xlo[nb].w;
+          const uint32_t b1 = (j == 0) ? xhi[nb].x : (j == 1) ? xhi[nb].y : (j == 2) ? xhi[nb].z : xhi[nb].w;
+          if (j < 2) mma_s8_16x8x32_first(c[nb][j], a0, a1, a2, a3, b0, b1);
+          else mma_s8_16x8x32(c[nb][j & 1], a0, a1, a2, a3, b0, b1);
+        }
+      }
+#pragma unroll
+      for (int nb = 0; nb < NT; ++nb) {
+        float xa = 1.f, xb = 1.f;  // activation scales of tokens 2t, 2t + 1 of this block
+        if constexpr (GS) {
+          const float* sg = sx + static_cast<size_t>(g_begin + i * kVGS + gi) * M;
+          const int m = nb * 8 + 2 * t;
+          xa = __ldg(sg + (m < M ? m : M - 1));
+          xb = __ldg(sg + (m + 1 < M ? m + 1 : M - 1));
+        }
+        run[nb][0] = fmaf(static_cast<float>(c[nb][0][0] + c[nb][1][0]), GS ? __fmul_rn(s0, xa) : s0, run[nb][0]);
+        run[nb][1] = fmaf(static_cast<float>(c[nb][0][1] + c[nb][1][1]), GS ? __fmul_rn(s0, xb) : s0, run[nb][1]);
+        run[nb][2] = fmaf(static_cast<float>(c[nb][0][2] + c[nb][1][2]), GS ? __fmul_rn(s1, xa) : s1, run[nb][2]);
+        run[nb][3] = fmaf(static_cast<float>(c[nb][0][3] + c[nb][1][3]), GS ? __fmul_rn(s1, xb) : s1, run[nb][3]);
+      }
+    };
+    const uint32_t full_addr = smem_u32(full), full_end = full_addr + static_cast<uint32_t>(stages) * 8u;
+    uint32_t at = full_addr, ph = 0;
+    const uint8_t* st = smem;
     for (int i = 0; i < nst; ++i) {
-      if (!mbar_wait(&full[s], ph, abort_flag, VSITE_COMPUTE)) break;
-      const uint8_t* st = smem + s * C::kStage;
-      int cnt = ng - i * kVGS;
-      if (cnt > kVGS) cnt = kVGS;
-      // with two warp sets, warps 0-7 take the first group of the stage and warps 8-15 the second
-#pragma unroll
-      for (int gi = set; gi < kVGS; gi += kVSets) {
-        if (gi >= cnt) break;
-        const uint8_t* tile = st + C::kOffW + gi * kTileBytes;
-        // k chunk t of rows `row` and `row + 8` (chunk positions are swizzled by (row >> 1) & 3,
-        // the same value for both rows)
-        const int tp = t ^ ((g >> 1) & 3);
-        const uint4 wa = *reinterpret_cast<const uint4*>(tile + row * 64 + tp * 16);
-        const uint4 wb = *reinterpret_cast<const uint4*>(tile + (row + 8) * 64 + tp * 16);
-        const __half* sc = reinterpret_cast<const __half*>(tile + kTileCodeBytes);
-        const float s0 = __half2float(sc[row]) * 0.0625f;
-        const float s1 = __half2float(sc[row + 8]) * 0.0625f;
-        uint4 xlo[NT], xhi[NT];
-#pragma unroll
-        for (int nb = 0; nb < NT; ++nb) {
-          // activation codes: [group][token][128 B]; 16-byte chunk c of token row m sits at
-          // chunk position c ^ (m & 7) (128-byte swizzle); this lane needs chunks 2t and 2t + 1
-          const uint8_t* xr = st + C::kOffX + gi * C::kXGroupBytes + (nb * 8 + g) * kGroup;
-          xlo[nb] = *reinterpret_cast<const uint4*>(xr + (((2 * t) ^ g) << 4));
-          xhi[nb] = *reinterpret_cast<const uint4*>(xr + (((2 * t + 1) ^ g) << 4));
-        }
-        // Word j of a lane's 16-byte chunk feeds MMA step j: low nibbles are
-        // k = 32t + 4j + {0..3} of the group (fragment slots a0/a1), high nibbles
-        // k = 32t + 16 + 4j + {0..3} (a2/a3).
-        const uint32_t wav[4] = {wa.x, wa.y, wa.z, wa.w};
-        const uint32_t wbv[4] = {wb.x, wb.y, wb.z, wb.w};
-        int c[NT][2][4];  // two partial accumulators per token block: dependent chains of 2 MMAs
-#pragma unroll
-        for (int nb = 0; nb < NT; ++nb)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) { c[nb][0][e] = 0; c[nb][1][e] = 0; }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const uint32_t a0 = (wav[j] << 4) & 0xF0F0F0F0u;
-          const uint32_t a2 = wav[j] & 0xF0F0F0F0u;
-          const uint32_t a1 = (wbv[j] << 4) & 0xF0F0F0F0u;
-          const uint32_t a3 = wbv[j] & 0xF0F0F0F0u;
-#pragma unroll
-          for (int nb = 0; nb < NT; ++nb) {
-            const uint32_t b0 = (j == 0) ? xlo[nb].x : (j == 1) ? xlo[nb].y : (j == 2) ? xlo[nb].z : xlo[nb].w;
-            const uint32_t b1 = (j == 0) ? xhi[nb].x : (j == 1) ? xhi[nb].y : (j == 2) ? xhi[nb].z : xhi[nb].w;
-            mma_s8_16x8x32(c[nb][j & 1], a0, a1, a2, a3, b0, b1);
-          }
-        }
-#pragma unroll
-        for (int nb = 0; nb < NT; ++nb) {
-          float xa = 1.f, xb = 1.f;  // activation scales of tokens 2t, 2t + 1 of this block
-          if constexpr (GS) {
-            const float* sg = sx + static_cast<size_t>(g_begin + i * kVGS + gi) * M;
-            const int m = nb * 8 + 2 * t;
-            xa = __ldg(sg + (m < M ? m : M - 1));
-            xb = __ldg(sg + (m + 1 < M ? m + 1 : M - 1));
-          }
-          run[nb][0] = fmaf(static_cast<float>(c[nb][0][0] + c[nb][1][0]), GS ? __fmul_rn(s0, xa) : s0, run[nb][0]);
-          run[nb][1] = fmaf(static_cast<float>(c[nb][0][1] + c[nb][1][1]), GS ? __fmul_rn(s0, xb) : s0, run[nb][1]);
-          run[nb][2] = fmaf(static_cast<float>(c[nb][0][2] + c[nb][1][2]), GS ? __fmul_rn(s1, xa) : s1, run[nb][2]);
-          run[nb][3] = fmaf(static_cast<float>(c[nb][0][3] + c[nb][1][3]), GS ? __fmul_rn(s1, xb) : s1, run[nb][3]);
-        }
-      }
+      if (!mbar_wait_addr(at, ph, abort_flag, VSITE_COMPUTE)) break;
+      group(st, 0, i);
+      if (i * kVGS + 1 < ng) group(st, 1, i);  // (the last stage may hold one group)
       __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[s]);
-      if (++s == stages) { s = 0; ph ^= 1u; }
+      if (lane == 0)  // empty[s]: C::kMaxStages barriers behind full[s]
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(at + C::kMaxStages * 8u) : "memory");
+      at += 8;
+      st += C::kStage;
+      if (at == full_end) {
+        at = full_addr;
+        st = smem;
+        ph ^= 1u;
+      }
     }
+#pragma unroll
+    for (int nb = 0; nb < NT; ++nb)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) run[nb][e] *= 0.0625f;
 
-    // Fold the second warp set's partial sums into the first through shared memory.  All compute
-    // warps are past their last stage at the first barrier, so the ring can be reused.
-    if constexpr (kVSets == 2) {
-      float* red = reinterpret_cast<float*>(smem);
-      asm volatile("bar.sync 1, 512;" ::: "memory");
-      if (set == 1) {
-#pragma unroll
-        for (int nb = 0; nb < NT; ++nb)
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const int m = nb * 8 + 2 * t + e;
-            red[m * kVBN + row] = run[nb][e];
-            red[m * kVBN + row + 8] = run[nb][2 + e];
-          }
-      }
-      asm volatile("bar.sync 1, 512;" ::: "memory");
-      if (set == 0) {
-#pragma unroll
-        for (int nb = 0; nb < NT; ++nb)
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const int m = nb * 8 + 2 * t + e;
-            run[nb][e] += red[m * kVBN + row];
-            run[nb][2 + e] += red[m * kVBN + row + 8];
-          }
-      }
-    }
     // accumulator fragment: c0/c1 = (row, tokens 2t, 2t+1), c2/c3 = (row + 8, same tokens)
-    if constexpr (kVSets == 1) {
-      if (split_k > 1 || ar.world > 1) asm volatile("bar.sync 1, 256;" ::: "memory");  // ring reused as exchange tile
-    }
-    if (set == 1) {
-      // nothing left to do for the second set
-    } else if (split_k == 1 && ar.world <= 1) {
+    if (split_k > 1 || ar.world > 1) asm volatile("bar.sync 1, 256;" ::: "memory");  // ring reused as exchange tile
+    if (split_k == 1 && ar.world <= 1) {
 #pragma unroll
       for (int hrow = 0; hrow < 2; ++hrow) {
         const int n = n0 + row + 8 * hrow;
