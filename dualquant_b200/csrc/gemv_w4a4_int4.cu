@@ -432,11 +432,35 @@ int init_gemv_int4_kernels() {
   return DQ_OK;
 }
 
-// Smallest power-of-two split that gives roughly one CTA per SM (measured optimum on the
-// Llama-3.1-8B decode shapes: more splits cost more in cluster exchange than they win).
+// Clusters of 1, 2, 4 and 8 CTAs that fit with one CTA on each of 148 SMs (B200; a cluster stays inside one GPC).
+static int cluster_places(int split, int sm_count) {
+  return (split == 1 ? 148 : split == 2 ? 74 : split == 4 ? 33 : 15) * sm_count / 148;
+}
+
+// Weight groups that the busiest SM walks through, in tenths: two or three CTAs on an SM hide each other's latency, so a
+// group costs 1.3 where an SM has one CTA only; a split costs about four groups per CTA on the SM for the exchange.
+static int split_cost(int s, int tiles, int total_groups, int sm_count) {
+  const int per_sm = (tiles * s + sm_count - 1) / sm_count;
+  const int gps = (total_groups + s - 1) / s;
+  return gps * (per_sm == 1 ? 13 : 10 * per_sm) + (s > 1 ? 40 * per_sm : 0);
+}
+
+// The smallest power-of-two split that gives roughly one CTA per SM, unless the next one up or down costs less by a
+// tenth and by at least four groups (below that the order of two launches decides, not the split): a fuller last wave,
+// or two CTAs on an SM that hide each other's latency, pay for one more exchange once K is long.  A split is no
+// candidate where clusters would wait for a second wave, nor from 4 CTAs per SM on.
+// us, 16 tokens: 28672 -> 8192 33.6 -> 27.2, 8960 -> 12000 18.4 -> 15.8, 8192 -> 10240 16.9 -> 14.4,
+// 8192 -> 16746 20.7 -> 17.5, 5888 -> 9811 13.5 -> 11.8.
 int gemv_pick_split(int tiles, int total_groups, int tok, int sm_count) {
   int s = 1;
   while (s < 8 && tiles * s * 6 < sm_count * 5 && total_groups / (2 * s) >= 2 && 2 * s <= tok) s *= 2;
+  const int cost = split_cost(s, tiles, total_groups, sm_count);
+  for (int c = (s == 1 ? 2 : s / 2); c <= 2 * s; c = (c < s ? 2 * s : c * 2)) {
+    const int per_sm = (tiles * c + sm_count - 1) / sm_count;
+    if (c > 4 || c > tok || total_groups < 2 * c || per_sm > 3 || tiles > per_sm * cluster_places(c, sm_count)) continue;
+    const int cc = split_cost(c, tiles, total_groups, sm_count);
+    if (10 * cc <= 9 * cost && cc + 40 <= cost) return c;
+  }
   return s;
 }
 
@@ -453,7 +477,9 @@ static int launch_gemv_t(const int8_t* codes, const float* sx, const uint8_t* w_
   const int gps = (total_groups + split - 1) / split;
   const int tiles_n = (N + kVBN - 1) / kVBN;
   // stages: share the SM's shared memory between the CTAs expected to be co-resident
-  int per_sm = (tiles_n * split + st->sm_count - 1) / st->sm_count;
+  // (14336 -> 2048 in 16 clusters of 8, for which there are 15 places at one CTA per SM: 11.2 -> 7.2 us at 8 tokens)
+  const int places = cluster_places(split, st->sm_count);
+  int per_sm = (tiles_n + places - 1) / places;
   if (per_sm > C::kMinCtas) per_sm = C::kMinCtas;
   if (per_sm < 1) per_sm = 1;
   const int avail = (227 * 1024) / per_sm - 1024 - C::kBarBytes - 1024;

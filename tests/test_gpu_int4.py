@@ -453,3 +453,15 @@ def test_chosen_tile_and_split_against_the_unsplit_kernel(M, N, K):
     for y, want in ((ops.gemm_w4a4_int4(codes, sx, pw), ref), (ops.gemm_w4a4_int4(codes, sx, pw, residual=res), ref + res)):
         assert ((y - want).abs().max() / want.abs().max()).item() < 1e-6
     _lib.device_status(0)
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("N,K", [(2048, 14336), (8137, 9984), (9811, 5888), (16746, 8192), (100, 128), (1231, 1408)])
+def test_chosen_decode_split_against_the_unsplit_kernel(M, N, K):
+    """Whatever split of K the decode kernel gets, the result equals the unsplit kernel's up to the order of fp32 sums."""
+    g = torch.Generator(device=DEV).manual_seed(M * 7 + N)
+    pw = ops.pack_w_int4(*ops.quant_w_int4((torch.randn(N, K, generator=g, device=DEV) * 0.02).to(torch.bfloat16)))
+    codes, sx = ops.quant_act_int4(torch.randn(M, K, generator=g, device=DEV).to(torch.bfloat16))
+    ref = ops.gemm_w4a4_int4(codes, sx, pw, split_k=1)
+    assert ((ops.gemm_w4a4_int4(codes, sx, pw) - ref).abs().max() / ref.abs().max()).item() < 1e-6
+    _lib.device_status(0)
