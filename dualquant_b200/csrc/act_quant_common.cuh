@@ -33,12 +33,20 @@ __device__ __forceinline__ float block_max(float v, float* red, int nwarps) {
   return m;
 }
 
-__device__ __forceinline__ float block_sum(float v, float* red, int nwarps) {
+// for a `red` that nothing has read before in this kernel: one barrier
+__device__ __forceinline__ float block_max_once(float v, float* red, int nwarps) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  float m = red[0];
+  for (int i = 1; i < nwarps; ++i) m = fmaxf(m, red[i]);
+  return m;
+}
+__device__ __forceinline__ float block_sum_once(float v, float* red, int nwarps) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __syncthreads();  // red may still be read from a previous use
-  if (lane == 0) red[warp] = v;
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
   float m = red[0];
   for (int i = 1; i < nwarps; ++i) m += red[i];

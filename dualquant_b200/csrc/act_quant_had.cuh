@@ -391,102 +391,163 @@ act_quant_had_cluster_kernel(const XT* __restrict__ x, const XT* __restrict__ up
 }
 
 // ---------------------------------------------------------------------------------------------
-// the across-heads transform (o_proj input) for many rows: registers only
+// the across-heads transform (o_proj input): registers only
 // ---------------------------------------------------------------------------------------------
-// Row = S heads of 128 values, Walsh-Hadamard over the head index for each of the 128 lanes of a
-// head.  The one-CTA-per-row kernel above spends its time waiting (load, barrier, 128 busy threads,
-// barrier, store); here a lane owns eight adjacent columns of min(S, 16) heads and keeps them in
-// registers from the load to the codes: 16 lanes cover a row (32 for S = 32, where the halves of
-// the warp hold heads 0-15 and 16-31 and the last stage is one shuffle per value), nothing goes
-// through shared memory and no barrier is needed.  Same stage order and operand order as above.
-// Codes only (int8 or E4M3, fp32 or fp16 scale), no gate: everything is unrolled over the heads, and
-// with the other output modes and the SiLU gate expanded sixteen times the code outgrew the
-// instruction cache (measured: 2.4x slower than the kernel above at 32 heads).
-constexpr int kHeadsKernelThreads = 128;
-constexpr int kHeadsKernelMinRows = 64;
+// Row = S heads of 128 values, Walsh-Hadamard over the head index for each of the 128 lanes of a head.  A decode batch
+// is bound by the chain load -> stages -> absmax -> codes of one row, so a row gets as many threads as keep the chain
+// short: a thread owns two columns of at most eight heads (sixteen values), the head groups sit 8 (S = 32) or 16 (S = 16)
+// lanes apart, where the last stages are shuffles, and a row costs one barrier; up to four heads a row is one warp, four
+// columns to a lane, and costs none.  Many rows are bound by instruction issue: a CTA walks rows gridDim.x apart with
+// the activation scale in registers and the next row's loads in flight.  Same stage order and operand order as above.
+// Codes only (int8 or E4M3, fp32 or fp16 scale), no gate.
+// Against one lane for eight columns of sixteen heads (64 rows up; one CTA with two shared-memory passes below), us at
+// 32 heads: 8 rows 3.7 -> 2.6, 64 rows 9.0 -> 2.7, 1000 rows 10.7 -> 7.5, 16384 rows 150 -> 74 (2.7 TB/s).
+template <int S>
+struct HeadsRow {
+  static constexpr int kHeads = (S < 8) ? S : 8;          // heads per thread
+  static constexpr int kGroups = S / kHeads;              // head groups
+  static constexpr int kCols = (S <= 4) ? 4 : 2;          // columns per thread
+  static constexpr int kLanes = 32 / kGroups;             // column sets per warp
+  static constexpr int kWarps = 128 / (kLanes * kCols);   // warps per row
+  static constexpr int kRows = (S <= 4) ? 4 : 1;          // rows per CTA
+  static constexpr int kThreads = 32 * kWarps * kRows;
+  // CTAs per SM: 64 registers a thread hold eight heads of two columns, their scales and the next row
+  static constexpr int kCtas = (S == 2 ? 1280 : 1024) / kThreads;
+};
 
 template <int S, typename XT, bool E4M3>
-__global__ void __launch_bounds__(kHeadsKernelThreads)
-act_quant_had_heads_kernel(const XT* __restrict__ x, int64_t ldx, const float* __restrict__ a, int M,
-                           float had_scale, int8_t* __restrict__ codes, float* __restrict__ sx, int scale_fp16) {
-  constexpr int HL = (S < 16) ? S : 16;   // heads per lane
-  constexpr int L = (S == 32) ? 32 : 16;  // lanes per row
-  constexpr int K = S * 128;
+__global__ void __launch_bounds__(HeadsRow<S>::kThreads, HeadsRow<S>::kCtas)
+act_quant_had_heads_kernel(const XT* __restrict__ x, int64_t ldx, const float* __restrict__ a, int M, float had_scale,
+                           int8_t* __restrict__ codes, float* __restrict__ sx, int scale_fp16) {
+  using H = HeadsRow<S>;
+  constexpr int HL = H::kHeads, C = H::kCols, CL = H::kLanes;
+  __shared__ float red[2][H::kWarps];  // of alternate rows: one barrier per row
   grid_dep_launch_dependents();
   grid_dep_wait();
   const int lane = threadIdx.x & 31;
-  const int sub = lane & (L - 1);
-  const int64_t rr = (static_cast<int64_t>(blockIdx.x) * (kHeadsKernelThreads / 32) + (threadIdx.x >> 5)) * (32 / L) +
-                     lane / L;
-  const bool live = rr < M;  // lanes of a row past the end keep running (shuffles), but touch no memory
-  const int col = 8 * (sub & 15);
-  const int head0 = (S == 32 && sub >= 16) ? 16 : 0;
-  const XT* xr = x + (live ? rr : 0) * ldx;
-  float v[HL][8];
-#pragma unroll
-  for (int j = 0; j < HL; ++j) {
-    const int idx = (head0 + j) * 128 + col;
-    if (live) {
-      load8(xr + idx, v[j]);
-      if (a != nullptr) {
-        float av[8];
-        load8(a + idx, av);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) v[j][e] = __fmul_rn(v[j][e], av[e]);
-      }
-    } else {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) v[j][e] = 0.f;
-    }
-  }
-#pragma unroll
-  for (int h = 1; h < HL; h <<= 1) {
+  const int warp = (H::kRows > 1) ? 0 : threadIdx.x >> 5;  // warp of the row
+  const int row_in_cta = (H::kRows > 1) ? threadIdx.x >> 5 : 0;
+  const int at = (lane / CL) * HL * 128 + (warp * CL + (lane & (CL - 1))) * C;  // first head's columns
+  constexpr int kWords = C * sizeof(XT) / 4;
+  uint32_t raw[HL][kWords];
+  auto load = [&](int64_t row) {
 #pragma unroll
     for (int j = 0; j < HL; ++j) {
-      if ((j & h) == 0) {
+      const XT* p = x + row * ldx + at + j * 128;
+      if constexpr (kWords == 1) {
+        raw[j][0] = *reinterpret_cast<const uint32_t*>(p);
+      } else {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const float u = v[j][e], w = v[j + h][e];
-          v[j][e] = __fadd_rn(u, w);
-          v[j + h][e] = __fsub_rn(u, w);
+        for (int e = 0; e < kWords; e += 2) {
+          const uint2 w = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint32_t*>(p) + e);
+          raw[j][e] = w.x;
+          raw[j][e + 1] = w.y;
         }
       }
     }
-  }
-  if constexpr (S == 32) {  // heads j and j + 16 sit in lanes l and l + 16
-    const float sign = sub >= 16 ? -1.0f : 1.0f;  // a + b below, a - b above: other + sign * own, rounded once
+  };
+  const int64_t step = static_cast<int64_t>(gridDim.x) * H::kRows;
+  int64_t row = static_cast<int64_t>(blockIdx.x) * H::kRows + row_in_cta;
+  if (row < M) load(row);
+  float av[HL][C];
+  if (a != nullptr) {
 #pragma unroll
     for (int j = 0; j < HL; ++j) {
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const float other = __shfl_xor_sync(0xffffffffu, v[j][e], 16);
-        v[j][e] = __fmaf_rn(v[j][e], sign, other);
+      for (int e = 0; e < C; e += 2) {
+        const float2 w = *reinterpret_cast<const float2*>(a + at + j * 128 + e);
+        av[j][e] = w.x;
+        av[j][e + 1] = w.y;
       }
     }
   }
-  float amax = 0.f;
+  int buf = 0;
+  for (; row < M; row += step, buf ^= 1) {  // (a row's warps leave the loop together)
+    float v[HL][C];
 #pragma unroll
-  for (int j = 0; j < HL; ++j) {
+    for (int j = 0; j < HL; ++j) {
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      v[j][e] = __fmul_rn(v[j][e], had_scale);
-      amax = fmaxf(amax, fabsf(v[j][e]));
+      for (int e = 0; e < C; ++e) {
+        if constexpr (sizeof(XT) == 2)
+          v[j][e] = __uint_as_float((e & 1) ? raw[j][e / 2] & 0xFFFF0000u : raw[j][e / 2] << 16);
+        else
+          v[j][e] = __uint_as_float(raw[j][e]);
+      }
     }
-  }
+    if (row + step < M) load(row + step);
+    if (a != nullptr) {
 #pragma unroll
-  for (int o = L / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-  if (!live) return;
-  const float s = token_scale(amax, scale_fp16);
-  if (sub == 0 && sx != nullptr) sx[rr] = s;
-  const float inv_s = __fdiv_rn(1.0f, s);
-  int8_t* crow = codes + rr * K;
+      for (int j = 0; j < HL; ++j) {
 #pragma unroll
-  for (int j = 0; j < HL; ++j) {
-    float q[8];
-    quant_codes8(v[j], s, inv_s, q);
-    const uint32_t lo = E4M3 ? pack_codes4_e4m3(q[0], q[1], q[2], q[3]) : pack_codes4(q[0], q[1], q[2], q[3]);
-    const uint32_t hi = E4M3 ? pack_codes4_e4m3(q[4], q[5], q[6], q[7]) : pack_codes4(q[4], q[5], q[6], q[7]);
-    *reinterpret_cast<uint2*>(crow + (head0 + j) * 128 + col) = make_uint2(lo, hi);
+        for (int e = 0; e < C; ++e) v[j][e] = __fmul_rn(v[j][e], av[j][e]);
+      }
+    }
+#pragma unroll
+    for (int h = 1; h < HL; h <<= 1) {
+#pragma unroll
+      for (int j = 0; j < HL; ++j) {
+        if ((j & h) == 0) {
+#pragma unroll
+          for (int e = 0; e < C; ++e) {
+            const float u = v[j][e], w = v[j + h][e];
+            v[j][e] = __fadd_rn(u, w);
+            v[j + h][e] = __fsub_rn(u, w);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int o = CL; o < 32; o <<= 1) {  // heads HL * (o / CL) apart
+      const float sign = (lane & o) != 0 ? -1.0f : 1.0f;  // a + b below, a - b above: other + sign * own, rounded once
+#pragma unroll
+      for (int j = 0; j < HL; ++j) {
+#pragma unroll
+        for (int e = 0; e < C; ++e) {
+          const float other = __shfl_xor_sync(0xffffffffu, v[j][e], o);
+          v[j][e] = __fmaf_rn(v[j][e], sign, other);
+        }
+      }
+    }
+    float amax = 0.f;
+#pragma unroll
+    for (int j = 0; j < HL; ++j) {
+#pragma unroll
+      for (int e = 0; e < C; ++e) {
+        v[j][e] = __fmul_rn(v[j][e], had_scale);
+        amax = fmaxf(amax, fabsf(v[j][e]));
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    if constexpr (H::kWarps > 1) {
+      if (lane == 0) red[buf][warp] = amax;
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < H::kWarps; ++i) amax = fmaxf(amax, red[buf][i]);
+    }
+    const float s = token_scale(amax, scale_fp16);
+    if (warp == 0 && lane == 0 && sx != nullptr) sx[row] = s;
+    const float inv_s = __fdiv_rn(1.0f, s);
+    int8_t* crow = codes + row * (S * 128) + at;
+    constexpr int kQ = 8 / C;  // heads per eight values
+#pragma unroll
+    for (int j = 0; j < HL; j += kQ) {
+      float in[8], q[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) in[e] = v[j + e / C][e % C];
+      quant_codes8(in, s, inv_s, q);
+#pragma unroll
+      for (int p = 0; p < 8; p += 4) {
+        const uint32_t w = E4M3 ? pack_codes4_e4m3(q[p], q[p + 1], q[p + 2], q[p + 3])
+                                : pack_codes4(q[p], q[p + 1], q[p + 2], q[p + 3]);
+        if constexpr (C == 4) {
+          *reinterpret_cast<uint32_t*>(crow + (j + p / 4) * 128) = w;
+        } else {
+          *reinterpret_cast<uint16_t*>(crow + (j + p / 2) * 128) = static_cast<uint16_t>(w);
+          *reinterpret_cast<uint16_t*>(crow + (j + p / 2 + 1) * 128) = static_cast<uint16_t>(w >> 16);
+        }
+      }
+    }
   }
 }
 
@@ -595,18 +656,23 @@ int launch_had_fast_t(const XT* x, const XT* up, int64_t ldx, const float* a, co
     HadPlan plan;
     if (plan_fast_hadamard(had, K, &plan)) {
       *taken = true;
-      // across 2 ... 32 heads of 128 values, many rows: the register-only kernel
-      if (had->kind == DQ_HAD_PARTIAL && had->had_dim == 128 && plan.S >= 2 && M >= kHeadsKernelMinRows &&
-          up == nullptr && mode == MODE_CODES && codes != nullptr && (scale_fp16 & 0xFF) != 2) {
-        const int rows_per_cta = (kHeadsKernelThreads / 32) * (plan.S == 32 ? 1 : 2);
-        const dim3 grid((M + rows_per_cta - 1) / rows_per_cta);
+      // across 2 ... 32 heads of 128 values: the register-only kernel
+      if (had->kind == DQ_HAD_PARTIAL && had->had_dim == 128 && plan.S >= 2 && up == nullptr && mode == MODE_CODES &&
+          codes != nullptr && (scale_fp16 & 0xFF) != 2) {
+        DeviceState* st = current_state();
+        if (st == nullptr) return DQ_ERR_NOT_INIT;
 #define DQ_HAD_HEADS(SS)                                                                                            \
-  if ((scale_fp16 & kCodesE4M3) != 0)                                                                               \
-    DQ_CHECK_CUDA(launch_pdl(act_quant_had_heads_kernel<SS, XT, true>, grid, dim3(kHeadsKernelThreads), 0, stream, x, \
-                             ldx, a, M, had->scale, codes, sx, scale_fp16));                                        \
-  else                                                                                                              \
-    DQ_CHECK_CUDA(launch_pdl(act_quant_had_heads_kernel<SS, XT, false>, grid, dim3(kHeadsKernelThreads), 0, stream, x, \
-                             ldx, a, M, had->scale, codes, sx, scale_fp16))
+  {                                                                                                                 \
+    using H = HeadsRow<SS>;                                                                                         \
+    const int ctas = (M + H::kRows - 1) / H::kRows, most = H::kCtas * st->sm_count;                                 \
+    const dim3 grid(ctas < most ? ctas : most);                                                                     \
+    if ((scale_fp16 & kCodesE4M3) != 0)                                                                             \
+      DQ_CHECK_CUDA(launch_pdl(act_quant_had_heads_kernel<SS, XT, true>, grid, dim3(H::kThreads), 0, stream, x,     \
+                               ldx, a, M, had->scale, codes, sx, scale_fp16));                                      \
+    else                                                                                                            \
+      DQ_CHECK_CUDA(launch_pdl(act_quant_had_heads_kernel<SS, XT, false>, grid, dim3(H::kThreads), 0, stream, x,    \
+                               ldx, a, M, had->scale, codes, sx, scale_fp16));                                      \
+  }
         switch (plan.S) {
           case 2: DQ_HAD_HEADS(2); break;
           case 4: DQ_HAD_HEADS(4); break;

@@ -24,12 +24,12 @@ namespace dq {
 // shape, where the kernel is bound by instruction issue and registers are plentiful) instead of
 // being re-expanded from the raw row (few-rows shape, where occupancy hides latency).
 template <int THREADS, int VPT, typename XT, bool KEEP = false>
-__global__ void __launch_bounds__(THREADS, (THREADS >= 512 && VPT <= 2) ? 2048 / THREADS : (VPT >= 4 && !KEEP) ? 1024 / THREADS : 1)
+__global__ void __launch_bounds__(THREADS, (THREADS >= 512 && VPT <= 2) ? (KEEP ? 1 : 2048 / THREADS) : (VPT >= 4 && !KEEP) ? 1024 / THREADS : 1)
 act_quant_rows_kernel(const XT* __restrict__ x, int64_t ldx, const float* __restrict__ a, int K,
                       int8_t* __restrict__ codes, float* __restrict__ sx, float* __restrict__ out,
                       int mode, int scale_fp16, const __nv_bfloat16* __restrict__ norm_w,
                       float norm_eps) {
-  __shared__ float red[THREADS / 32];
+  __shared__ float red[THREADS / 32], red_max[THREADS / 32];
   // the GEMM that consumes the codes may be launched programmatically: let it start streaming
   // its weights now; it waits for this grid before it touches codes / sx
   grid_dep_launch_dependents();
@@ -48,6 +48,15 @@ act_quant_rows_kernel(const XT* __restrict__ x, int64_t ldx, const float* __rest
   }
   const bool norm = norm_eps >= 0.f;
   float inv_rms = 1.f;
+  // few rows: the norm weight and the activation scale come with the row, not behind the reduction
+  constexpr bool kEager = KEEP && VPT == 1;
+  Raw8<__nv_bfloat16> w_raw;
+  float a_raw[8];
+  if constexpr (kEager) {
+    const int idx = threadIdx.x * 8;
+    if (norm_w != nullptr && idx < K) w_raw.load(norm_w + idx);
+    if (a != nullptr && idx < K) load8(a + idx, a_raw);
+  }
   if (norm) {
     float ss = 0.f;
 #pragma unroll
@@ -60,7 +69,7 @@ act_quant_rows_kernel(const XT* __restrict__ x, int64_t ldx, const float* __rest
         for (int e = 0; e < 8; ++e) ss = fmaf(v[e], v[e], ss);
       }
     }
-    ss = block_sum(ss, red, THREADS / 32);
+    ss = block_sum_once(ss, red, THREADS / 32);
     inv_rms = rsqrtf(__fadd_rn(__fdiv_rn(ss, static_cast<float>(K)), norm_eps));
   }
   auto prologue = [&](float* v, int idx) {
@@ -69,7 +78,8 @@ act_quant_rows_kernel(const XT* __restrict__ x, int64_t ldx, const float* __rest
       for (int e = 0; e < 8; ++e) v[e] = bf16_round(__fmul_rn(v[e], inv_rms));
       if (norm_w != nullptr) {
         Raw8<__nv_bfloat16> wr;
-        wr.load(norm_w + idx);
+        if constexpr (kEager) wr = w_raw;
+        else wr.load(norm_w + idx);
         float wv[8];
         wr.expand(wv);
 #pragma unroll
@@ -78,9 +88,9 @@ act_quant_rows_kernel(const XT* __restrict__ x, int64_t ldx, const float* __rest
     }
     if (a != nullptr) {
       float av[8];
-      load8(a + idx, av);
+      if constexpr (!kEager) load8(a + idx, av);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) v[e] = __fmul_rn(v[e], av[e]);
+      for (int e = 0; e < 8; ++e) v[e] = __fmul_rn(v[e], kEager ? a_raw[e] : av[e]);
     }
   };
   float amax = 0.f;
@@ -100,7 +110,7 @@ act_quant_rows_kernel(const XT* __restrict__ x, int64_t ldx, const float* __rest
       }
     }
   }
-  amax = block_max(amax, red, THREADS / 32);
+  amax = block_max_once(amax, red_max, THREADS / 32);
   const float s = token_scale(amax, scale_fp16);
   if (threadIdx.x == 0 && sx != nullptr) sx[row] = s;
   int8_t* crow = (codes != nullptr) ? codes + static_cast<int64_t>(row) * K : nullptr;
@@ -422,17 +432,26 @@ static int launch_act(const XT* x, int64_t ldx, const float* a, const dq_hadamar
                            codes, sx, out, mode, scale_fp16, norm_w, norm_eps))
 #define DQ_ROWS_LAUNCH(T, V) DQ_ROWS_LAUNCH_K(T, V, false)
     constexpr int kBigM = 1024;
+    // Few rows: the loads of norm weight and activation scale go with the row's, its scaled values stay in registers for
+    // the codes, and occupancy is no concern.  Up to 1023 rows; where a row takes 1024 threads, while every row has an SM.
+    // (norm + codes, us: K 4096, 8 rows 3.4 -> 2.7, 400 rows 6.7 -> 5.5; K 8192, 8 rows 4.7 -> 4.2, but 200 rows 7.3 -> 7.5)
+    DeviceState* st = current_state();
+    if (st == nullptr) return DQ_ERR_NOT_INIT;
+    if ((M < kBigM && vec <= 512) || (M <= st->sm_count && vec <= 1024)) {
+      if (vec <= 128) DQ_ROWS_LAUNCH_K(128, 1, true);
+      else if (vec <= 256) DQ_ROWS_LAUNCH_K(256, 1, true);
+      else if (vec <= 512) DQ_ROWS_LAUNCH_K(512, 1, true);
+      else DQ_ROWS_LAUNCH_K(1024, 1, true);
+    }
     // Many rows (prefill): fewer threads per row, each with four 16-byte loads in flight - the
     // kernel is then bound by bytes in flight per SM, not by the per-row latency chain.
-    if (M >= kBigM && vec > 128 && vec <= 512) DQ_ROWS_LAUNCH_K(128, 4, true);
+    else if (M >= kBigM && vec > 128 && vec <= 512) DQ_ROWS_LAUNCH_K(128, 4, true);
     else if (M >= kBigM && vec > 512 && vec <= 1024) DQ_ROWS_LAUNCH_K(256, 4, true);
     // long rows (e.g. 14336): 256 threads with eight vectors each, re-expanded in the code pass, so
     // that four CTAs (four rows) share an SM - 512 threads keeping their values held one row per SM
     // and ran at 1.85 TB/s where this shape reaches 2.7
     else if (M >= kBigM && vec > 1024 && vec <= 2048) DQ_ROWS_LAUNCH_K(256, 8, false);
     else if (vec <= 128) DQ_ROWS_LAUNCH(128, 1);
-    else if (vec <= 256) DQ_ROWS_LAUNCH(256, 1);
-    else if (vec <= 512) DQ_ROWS_LAUNCH(512, 1);
     else if (vec <= 1024) DQ_ROWS_LAUNCH(1024, 1);
     else if (vec <= 2048) DQ_ROWS_LAUNCH(1024, 2);
     else DQ_ROWS_LAUNCH(1024, 4);

@@ -465,3 +465,16 @@ def test_chosen_decode_split_against_the_unsplit_kernel(M, N, K):
     ref = ops.gemm_w4a4_int4(codes, sx, pw, split_k=1)
     assert ((ops.gemm_w4a4_int4(codes, sx, pw) - ref).abs().max() / ref.abs().max()).item() < 1e-6
     _lib.device_status(0)
+
+
+@pytest.mark.parametrize("M,K", [(1, 256), (3, 512), (5, 1024), (7, 2048), (1, 4096), (5923, 256), (1186, 512), (2400, 1024),
+                                 (1185, 2048), (1185, 4096)])
+def test_partial_hadamard_row_ranges_bit_exact(M, K):
+    """One to four rows per CTA, and more rows than CTAs (each CTA walks several, the last ones fewer)."""
+    hd = ops.Hadamard(_lib.HAD_PARTIAL, 1, 128, O.partial_hadamard_scale(K // 128), None)
+    xb = synthetic.make_x(M, K, 13)
+    for a in (None, 1.0 / synthetic.make_scales(8, K, 13)[1]):
+        qx, sx, _ = O.quant_act_int4(xb, a if a is not None else torch.ones(K), ("partial", 128), False)
+        codes, sxg = ops.quant_act_int4(xb.to(DEV), None if a is None else a.to(DEV), hd, False)
+        assert torch.equal(codes.cpu(), qx) and torch.equal(sxg.cpu(), sx)
+    _status_ok()
