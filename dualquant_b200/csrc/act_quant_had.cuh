@@ -372,22 +372,38 @@ act_quant_had_cluster_kernel(const XT* __restrict__ x, const XT* __restrict__ up
   const XT* xr = x + base;
   const XT* ur = (up != nullptr) ? up + base : nullptr;
   const float* ar = (a != nullptr) ? a + static_cast<int64_t>(rank) * SQ * P : nullptr;
+  // the factor's loads are issued first and the row's three operands together: one memory round trip in all
+  constexpr int kCoefs = 1024 / kHadClusterThreads;  // S <= 32
+  float cf[kCoefs];
+#pragma unroll
+  for (int u = 0; u < kCoefs; ++u) {
+    const int i = tid + u * kHadClusterThreads, j = i & 31;
+    cf[u] = (i < S * 32 && j < S) ? had_mat[(i >> 5) * S + j] : 0.f;
+  }
   for (int idx = tid * 8; idx < SQ * P; idx += kHadClusterThreads * 8) {
-    float v[8];
-    load8(xr + idx, v);
-    apply_gate(ur != nullptr ? ur + idx : nullptr, v);
+    Raw8<XT> xw, uw;
+    float v[8], av[8];
+    xw.load(xr + idx);
+    if (ur != nullptr) uw.load(ur + idx);
+    if (ar != nullptr) load8(ar + idx, av);
+    xw.expand(v);
+    if (ur != nullptr) {
+      float u8[8];
+      uw.expand(u8);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = silu_mul_bf16(v[e], u8[e]);
+    }
     if (ar != nullptr) {
-      float av[8];
-      load8(ar + idx, av);
 #pragma unroll
       for (int e = 0; e < 8; ++e) v[e] = __fmul_rn(v[e], av[e]);
     }
     wht8(v);
     row_store8(seg + idx, v);
   }
-  for (int i = tid; i < S * 32; i += kHadClusterThreads) {
-    const int j = i & 31;
-    coef[i] = j < S ? had_mat[(i >> 5) * S + j] : 0.f;
+#pragma unroll
+  for (int u = 0; u < kCoefs; ++u) {
+    const int i = tid + u * kHadClusterThreads;
+    if (i < S * 32) coef[i] = cf[u];
   }
   __syncthreads();
   for (int sgm = warp; sgm < SQ; sgm += kHadClusterThreads / 32) wht_segment_warp<R>(seg + sgm * P, lane, had_scale);
@@ -424,7 +440,7 @@ act_quant_had_cluster_kernel(const XT* __restrict__ x, const XT* __restrict__ up
     amax = fmaxf(amax, fabsf(acc));
   }
   float s = 1.f;
-  amax = block_max(amax, red, kHadClusterThreads / 32);  // (also orders the colv writes before their reads below)
+  amax = block_max_once(amax, red, kHadClusterThreads / 32);  // (also orders the colv writes before their reads below)
   if (tid < kHadClusterCtas)
     dsmem_store_f32(dsmem_map(smem_u32(&pmax[rank]), static_cast<uint32_t>(tid)), amax);
   cluster_sync_all();  // the four partial maxima have landed everywhere; no remote access after this point
