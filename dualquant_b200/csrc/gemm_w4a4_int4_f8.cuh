@@ -389,9 +389,29 @@ gemm_w4a4_e4m3_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
       } else if (n < N) {  // OUT == 0
         const float rn = (r != nullptr) ? r[n] : 1.f;
         const int m0 = t0 + h * kCPW;
+        const int cnt = (M - m0 < kCPW) ? (M - m0) : kCPW;
+        const float* sxp = sx + m0;
+        // A loop for each kind of result, with a pointer that steps: the address arithmetic and the tests of a common
+        // one took 1.6 times the whole kernel (6124 x 2048 -> 18318, fp32: 551 us against 333).
+        if (add.p != nullptr) {
 #pragma unroll
-        for (int j = 0; j < kCPW; ++j)
-          if (m0 + j < M) store_y(y, add, y_bf16, m0 + j, n, N, run[j] * (rn * __ldg(sx + m0 + j)));
+          for (int j = 0; j < kCPW; ++j)
+            if (j < cnt) store_y(y, add, y_bf16, m0 + j, n, N, run[j] * (rn * __ldg(sxp + j)));
+        } else if (y_bf16) {
+          __nv_bfloat16* yp = reinterpret_cast<__nv_bfloat16*>(y) + static_cast<size_t>(m0) * N + n;
+#pragma unroll
+          for (int j = 0; j < kCPW; ++j) {
+            if (j < cnt) *yp = __float2bfloat16_rn(run[j] * (rn * __ldg(sxp + j)));
+            yp += N;
+          }
+        } else {
+          float* yp = reinterpret_cast<float*>(y) + static_cast<size_t>(m0) * N + n;
+#pragma unroll
+          for (int j = 0; j < kCPW; ++j) {
+            if (j < cnt) *yp = run[j] * (rn * __ldg(sxp + j));
+            yp += N;
+          }
+        }
       }
     }
     if constexpr (OUT == 4) __threadfence_system();  // this thread's stores to peers are performed before the kernel ends
