@@ -111,6 +111,7 @@ SIGNATURES = {
     "dq_exchange_sum": (_i, [_vp, _vp, _vp]),
     "dq_exchange_push": (_i, [_vp, _vp, _vp, _vp]),
     "dq_linear_w4a4_int4_scratch_bytes": (_sz, [_i, _i, _i]),
+    "dq_linear_w4a4_int4_byte_form_pays": (_i, [_i, _i, _i]),
     "dq_linear_w4a4_int4_prefill_scratch_bytes": (_sz, [_i, _i, _i]),
     "dq_linear_w4a4_int4": (_i, [_vp, _i64, _vp, _hp, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _i, _i, _vp, _sz, _vp]),
     "dq_linear_w4a4_int4_bias": (_i, [_vp, _i64, _vp, _hp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _i, _i, _vp,

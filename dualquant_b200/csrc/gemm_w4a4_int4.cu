@@ -536,11 +536,11 @@ static int pick_split(int tiles, int total_groups, int tn, int sm_count) {
 // the chip: 3584 -> 4608 at 100 tokens 18.9 us, now 12.0.
 struct Shape {
   int tn, split;
+  float cost;
 };
 static Shape pick_shape(int M, int row_tiles, int total_groups, int sm_count) {
   static const struct { int tn; float group_us; } kTiles[] = {{32, 0.34f}, {64, 0.38f}, {128, 0.435f}};
-  Shape best = {128, 1};
-  float best_cost = 1e30f;
+  Shape best = {128, 1, 1e30f};
   for (const auto& t : kTiles) {
     if (t.tn == 32 && M > 64) continue;
     const int clusters = row_tiles * ((M + t.tn - 1) / t.tn);
@@ -555,13 +555,14 @@ static Shape pick_shape(int M, int row_tiles, int total_groups, int sm_count) {
       const float once = (t.tn == 128 && split > 1 ? 6.5f : 4.0f) + 0.6f * lg;
       const float outside = t.tn == 128 && split == 1 ? once : rounds * once;  // (128 unsplit: persistent CTAs)
       const float cost = rounds * gps * t.group_us * shared + outside;
-      if (cost < best_cost) {
-        best_cost = cost;
-        best = {t.tn, split};
-      }
+      if (cost < best.cost) best = {t.tn, split, cost};
     }
   }
   return best;
+}
+
+float gemm_int4_packed_us(int M, int N, int K, int sm_count) {
+  return pick_shape(M, (N + kBN - 1) / kBN, K / kGroup, sm_count).cost;
 }
 
 template <int TN>
@@ -658,7 +659,7 @@ static int gemm_int4_dispatch(const int8_t* codes, const float* sx, const uint8_
   if (token_tile >= 2000) { forced = 2; token_tile -= 2000; }
   else if (token_tile >= 1000) { forced = 1; token_tile -= 1000; }
   const int row_tiles = (N + kBN - 1) / kBN;
-  Shape shape = {token_tile ? token_tile : pick_token_tile(M), split_k};
+  Shape shape = {token_tile ? token_tile : pick_token_tile(M), split_k, 0.f};
   if (token_tile == 0 && split_k == 0 && !grouped_sx) shape = pick_shape(M, row_tiles, total_groups, st->sm_count);
   const int tn = shape.tn;
   DQ_REQUIRE(tn == 16 || tn == 32 || tn == 64 || tn == 128, DQ_ERR_SHAPE,

@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(256) codes_to_e4m3_kernel(const int8_t* __rest
 // (a group of 256 tokens costs 1.7 times a group of 96, below that a group costs what its weight tile costs), a narrower
 // one leaves less of the last round empty, or spreads a small batch over the chip.  Group times: measured on B200 in
 // long runs at the power cap.
-static int pick_tile(int M, int row_pairs, int ng, int pairs, bool direct) {
+static int pick_tile(int M, int row_pairs, int ng, int pairs, bool direct, float* cost_us = nullptr) {
   static const struct { int tn; float group_us; } kTiles[] = {{256, 0.57f}, {224, 0.53f}, {192, 0.46f}, {160, 0.41f},
                                                               {128, 0.36f}, {96, 0.33f},  {64, 0.31f},  {32, 0.30f}};
   const int forced = tuning(DQ_TUNE_F8_TILE);
@@ -125,6 +125,7 @@ static int pick_tile(int M, int row_pairs, int ng, int pairs, bool direct) {
       best = t.tn;
     }
   }
+  if (cost_us != nullptr) *cost_us = best_cost;
   return best;
 }
 
@@ -240,6 +241,18 @@ extern "C" int dq_gemm_w4a4_int4_e4m3_scatter(const uint8_t* x8, const float* sx
   sc.rot = static_cast<int>(((ctx->rank + 1) % ctx->world) * (ctx->tokens_per_rank / 256));
   return launch_gemm_int4_e4m3_impl(x8, sx, w8, sw_t, r, M, N, K, nullptr, DQ_DTYPE_BF16, Addend{},
                                     static_cast<cudaStream_t>(stream), st, &sc);
+}
+
+// Under 256 tokens the packed weight is the cheaper one to read.  From 512 on the FP8-path GEMM wins everywhere; between,
+// it loses where K is long and the row tiles few, because it does not split K (294 x 14336 -> 1392: 38 us, the packed
+// kernel split four ways 29; 256 x 14336 -> 4096: 49 and 43): there the kernels' own estimates decide, packed by a tenth.
+extern "C" int dq_linear_w4a4_int4_byte_form_pays(int M, int N, int K) {
+  if (M < 256 || N < 1 || K < kGroup || K % kGroup != 0) return 0;
+  DeviceState* st = current_state();
+  if (M >= 512 || st == nullptr) return 1;
+  float bytes_us = 0.f;
+  f8::pick_tile(M, (N + 2 * f8::kBN - 1) / (2 * f8::kBN), K / kGroup, st->sm_count / 2, false, &bytes_us);
+  return gemm_int4_packed_us(M, N, K, st->sm_count) >= 0.9f * bytes_us ? 1 : 0;
 }
 
 extern "C" int dq_expand_w_int4_e4m3(const uint8_t* w_packed, int N, int K, int G, uint8_t* w8, void* stream) {

@@ -35,7 +35,8 @@ namespace {
 #define DQ_FUNCTIONS(X)                                                                              \
   X(dq_quant_act_int4) X(dq_quant_act_int4_f32) X(dq_quant_act_int4_gated) X(dq_quant_act_int4_rmsnorm) \
   X(dq_gemm_w4a4_int4_ex) X(dq_gemm_w4a4_int4_residual) X(dq_gemm_w4a4_int4_e4m3)                      \
-  X(dq_linear_w4a4_int4) X(dq_linear_w4a4_int4_bias) X(dq_linear_w4a4_int4_scratch_bytes)                                         \
+  X(dq_linear_w4a4_int4) X(dq_linear_w4a4_int4_bias) X(dq_linear_w4a4_int4_scratch_bytes) \
+  X(dq_linear_w4a4_int4_byte_form_pays)                                                                                       \
   X(dq_linear_w4a4_int4_prefill_scratch_bytes) X(dq_linear_a16w4) X(dq_linear_a16w4_scratch_bytes)     \
   X(dq_linear_w4a4_fp4) X(dq_linear_w4a4_fp4_scratch_bytes)
 #define DQ_DECLARE(name) decltype(&::name) name = nullptr;
@@ -375,12 +376,10 @@ PyObject* gemm_w4a4_int4_e4m3(PyObject*, PyObject* const* v, Py_ssize_t n) {
 
 // The weight's byte form (ops.PackedInt4Weight.w8, kept with the packed weight once it exists) for a batch that the
 // FP8-path GEMM serves better, or null.  Made by the first such batch: N * K bytes that used to be expanded into scratch
-// on every call.  From 256 tokens on that GEMM is the faster one on every layer shape measured (4096 -> 28672: 88 -> 68 us
-// at 300 tokens, 120 -> 76 at 500; 14336 -> 4096: 58 -> 55).  While a graph is being captured nothing is made: an
+// on every call (4096 -> 28672: 88 -> 68 us at 300 tokens, 120 -> 76 at 500; 14336 -> 4096: 58 -> 55).  While a graph is being captured nothing is made: an
 // expansion recorded there would not have run when the next call reads it.
-constexpr int kByteFormTokens = 256;
-const uint8_t* byte_form(PyObject* pw, int M, int group) {
-  if (M < kByteFormTokens || group != 128) return nullptr;
+const uint8_t* byte_form(PyObject* pw, int M, int N, int K, int group) {
+  if (group != 128 || !abi.dq_linear_w4a4_int4_byte_form_pays(M, N, K)) return nullptr;
   {
     Ref w8(PyObject_GetAttr(pw, names.w8));
     if (w8.p != Py_None) return static_cast<const uint8_t*>(tensor(w8.p, "w8").data_ptr());
@@ -428,7 +427,7 @@ PyObject* linear_w4a4_int4(PyObject*, PyObject* const* v, Py_ssize_t n) {
       throw PyError();
     }
     // a caller's scratch is used as it is when it covers the plain path
-    const uint8_t* w8 = byte_form(v[3], M, w.group);
+    const uint8_t* w8 = byte_form(v[3], M, w.N, K, w.group);
     at::Tensor scratch;
     if (v[7] != Py_None && tensor(v[7], "scratch").numel() >=
                                static_cast<int64_t>(abi.dq_linear_w4a4_int4_scratch_bytes(M, w.N, K)))
@@ -647,7 +646,7 @@ PyObject* perm_forward(PyObject*, PyObject* const* v, Py_ssize_t n) {
     if (bias == nullptr) Py_RETURN_NONE;
     const int idx = prep(x);
     const int M = static_cast<int>(x.numel() / K);
-    const uint8_t* w8 = p->kind == PLAN_INT4 ? byte_form(p->packed, M, p->w4.group) : nullptr;
+    const uint8_t* w8 = p->kind == PLAN_INT4 ? byte_form(p->packed, M, N, K, p->w4.group) : nullptr;
     int64_t need;
     if (p->kind == PLAN_INT4) need = int4_scratch_bytes(w8, M, N, K);
     else if (p->kind == PLAN_FP4) need = fp4_scratch_bytes(M, K, p->w_fp4.fmt);

@@ -492,6 +492,8 @@ DQ_API int dq_gemm_w4a4_int4_acc(const int8_t* codes, const uint8_t* w_packed, i
  * weight call dq_expand_w_int4_e4m3 once and dq_gemm_w4a4_int4_e4m3 directly.
  */
 DQ_API size_t dq_linear_w4a4_int4_scratch_bytes(int M, int N, int K);
+/* 1 if a caller that keeps the weight's byte form (dq_expand_w_int4_e4m3) should use it for M tokens, else 0. */
+DQ_API int dq_linear_w4a4_int4_byte_form_pays(int M, int N, int K);
 DQ_API size_t dq_linear_w4a4_int4_prefill_scratch_bytes(int M, int N, int K);
 DQ_API int dq_linear_w4a4_int4(const void* x_bf16, int64_t ldx, const float* a,
                         const dq_hadamard_desc* had, const uint8_t* w_packed, const void* sw_t,

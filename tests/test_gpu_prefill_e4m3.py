@@ -274,3 +274,20 @@ def test_every_token_tile_equals_the_integer_kernel(tile, M, N, K):
     finally:
         _lib.set_tuning("f8_tile", 0)
     _lib.device_status(0)
+
+
+@pytest.mark.parametrize("M,N,K", [(255, 1392, 2048), (256, 1392, 14336), (294, 1391, 14336), (300, 1024, 8192), (511, 2050, 4096),
+                                   (512, 1391, 1152), (700, 18317, 256)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_linear_picks_weight_form(M, N, K, dtype):
+    """Between 256 and 511 tokens a linear reads the packed weight or its byte form, whichever is estimated faster; rows
+    that are not 16-byte multiples are stored directly.  The result equals the unsplit packed kernel's either way."""
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    pw = ops.pack_w_int4(*ops.quant_w_int4((torch.randn(N, K, generator=g, device=DEV) * 0.02).to(torch.bfloat16)))
+    x = torch.randn(M, K, generator=g, device=DEV).to(torch.bfloat16)
+    codes, sx = ops.quant_act_int4(x)
+    ref = ops.gemm_w4a4_int4(codes, sx, pw, token_tile=1128, split_k=1)
+    y = ops.linear_w4a4_int4(x, None, None, pw, None, out=torch.empty(M, N, dtype=dtype, device=DEV))
+    tol = 1e-6 if dtype == torch.float32 else 4e-3
+    assert ((y.float() - ref).abs().max() / ref.abs().max()).item() < tol
+    _lib.device_status(0)
