@@ -26,6 +26,39 @@ extern "C" size_t dq_linear_w4a4_int4_prefill_scratch_bytes(int M, int N, int K)
   return base + round_up(static_cast<size_t>(N) * static_cast<size_t>(K), 256);
 }
 
+// Quantiser and GEMM with the codes and token scales in the scratch.  The FP8-path GEMM runs with the caller's byte form of
+// the weight (w8), or from kPrefillTokens on with one expanded behind the token scales where the scratch has room for it.
+static int quant_and_gemm(const void* x_bf16, int64_t ldx, const float* a, const dq_hadamard_desc* had,
+                          const uint8_t* w_packed, const uint8_t* w8, const void* sw_t, const float* r, const void* bias,
+                          int M, int N, int K, int G, void* y, int y_dtype, int scale_fp16, void* scratch,
+                          size_t scratch_bytes, void* stream) {
+  uint8_t* base = static_cast<uint8_t*>(scratch);
+  int8_t* codes = static_cast<int8_t*>(scratch);
+  float* sx = reinterpret_cast<float*>(base + round_up(static_cast<size_t>(M) * K, 256));
+  const dq::Addend add = {bias, 0};
+  if (w8 == nullptr && M >= kPrefillTokens && G == dq::kGroup && (scale_fp16 & ~0xFF) == 0 &&
+      scratch_bytes >= dq_linear_w4a4_int4_prefill_scratch_bytes(M, N, K)) {
+    uint8_t* expanded = base + dq_linear_w4a4_int4_scratch_bytes(M, N, K);
+    const int rc = dq_expand_w_int4_e4m3(w_packed, N, K, G, expanded, stream);
+    if (rc != DQ_OK) return rc;
+    w8 = expanded;
+  }
+  const int rc =
+      dq_quant_act_int4(x_bf16, ldx, a, had, M, K, codes, sx, scale_fp16 | (w8 != nullptr ? DQ_CODES_E4M3 : 0), stream);
+  if (rc != DQ_OK) return rc;
+  if (w8 == nullptr)
+    return dq::gemm_w4a4_int4_addend(codes, sx, w_packed, sw_t, r, add, M, N, K, G, y, y_dtype, stream);
+  dq::DeviceState* st = dq::current_state();
+  if (st == nullptr) return DQ_ERR_NOT_INIT;
+  DQ_REQUIRE(sw_t != nullptr && y != nullptr, DQ_ERR_NULL, "null sw_t / y");
+  DQ_REQUIRE(G == dq::kGroup, DQ_ERR_UNSUPPORTED, "weight group size must be %d (got %d)", dq::kGroup, G);
+  DQ_REQUIRE(N >= 1 && K >= dq::kGroup && K % dq::kGroup == 0, DQ_ERR_SHAPE, "bad shape N=%d K=%d", N, K);
+  DQ_REQUIRE(y_dtype == DQ_DTYPE_F32 || y_dtype == DQ_DTYPE_BF16, DQ_ERR_UNSUPPORTED, "unknown y_dtype %d", y_dtype);
+  DQ_REQUIRE(dq::aligned(w8, 16), DQ_ERR_ALIGN, "w8 must be 16-byte aligned");
+  return dq::launch_gemm_int4_e4m3(reinterpret_cast<const uint8_t*>(codes), sx, w8, sw_t, r, M, N, K, y, y_dtype, add,
+                                   static_cast<cudaStream_t>(stream), st);
+}
+
 extern "C" int dq_linear_w4a4_int4(const void* x_bf16, int64_t ldx, const float* a,
                                    const dq_hadamard_desc* had, const uint8_t* w_packed,
                                    const void* sw_t, const float* r, int M, int N, int K, int G,
@@ -50,22 +83,8 @@ extern "C" int dq_linear_w4a4_int4(const void* x_bf16, int64_t ldx, const float*
                                    static_cast<cudaStream_t>(stream), st);
     }
   }
-  int8_t* codes = static_cast<int8_t*>(scratch);
-  float* sx = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) +
-                                       round_up(static_cast<size_t>(M) * K, 256));
-  if (M >= kPrefillTokens && G == dq::kGroup && (scale_fp16 & ~0xFF) == 0 &&
-      scratch_bytes >= dq_linear_w4a4_int4_prefill_scratch_bytes(M, N, K)) {
-    uint8_t* w8 = static_cast<uint8_t*>(scratch) + dq_linear_w4a4_int4_scratch_bytes(M, N, K);
-    int rc = dq_expand_w_int4_e4m3(w_packed, N, K, G, w8, stream);
-    if (rc != DQ_OK) return rc;
-    rc = dq_quant_act_int4(x_bf16, ldx, a, had, M, K, codes, sx, scale_fp16 | DQ_CODES_E4M3, stream);
-    if (rc != DQ_OK) return rc;
-    return dq_gemm_w4a4_int4_e4m3(reinterpret_cast<const uint8_t*>(codes), sx, w8, sw_t, r, M, N, K, G, y, y_dtype,
-                                  nullptr, stream);
-  }
-  int rc = dq_quant_act_int4(x_bf16, ldx, a, had, M, K, codes, sx, scale_fp16, stream);
-  if (rc != DQ_OK) return rc;
-  return dq_gemm_w4a4_int4(codes, sx, w_packed, sw_t, r, M, N, K, G, y, y_dtype, nullptr, 0, stream);
+  return quant_and_gemm(x_bf16, ldx, a, had, w_packed, nullptr, sw_t, r, nullptr, M, N, K, G, y, y_dtype, scale_fp16, scratch,
+                        scratch_bytes, stream);
 }
 
 extern "C" int dq_linear_w4a4_int4_bias(const void* x_bf16, int64_t ldx, const float* a, const dq_hadamard_desc* had,
@@ -79,22 +98,8 @@ extern "C" int dq_linear_w4a4_int4_bias(const void* x_bf16, int64_t ldx, const f
              dq_linear_w4a4_int4_scratch_bytes(M, N, K));
   DQ_REQUIRE(dq::aligned(bias, y_dtype == DQ_DTYPE_BF16 ? 2 : 4), DQ_ERR_ALIGN, "misaligned bias");
   if (M == 0) return DQ_OK;
-  int8_t* codes = static_cast<int8_t*>(scratch);
-  float* sx = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + round_up(static_cast<size_t>(M) * K, 256));
-  const dq::Addend add = {bias, 0};
-  int rc = dq_quant_act_int4(x_bf16, ldx, a, had, M, K, codes, sx, scale_fp16 | (w8 != nullptr ? DQ_CODES_E4M3 : 0), stream);
-  if (rc != DQ_OK) return rc;
-  if (w8 == nullptr)
-    return dq::gemm_w4a4_int4_addend(codes, sx, w_packed, sw_t, r, add, M, N, K, G, y, y_dtype, stream);
-  dq::DeviceState* st = dq::current_state();
-  if (st == nullptr) return DQ_ERR_NOT_INIT;
-  DQ_REQUIRE(sw_t != nullptr && y != nullptr, DQ_ERR_NULL, "null sw_t / y");
-  DQ_REQUIRE(G == dq::kGroup, DQ_ERR_UNSUPPORTED, "weight group size must be %d (got %d)", dq::kGroup, G);
-  DQ_REQUIRE(N >= 1 && K >= dq::kGroup && K % dq::kGroup == 0, DQ_ERR_SHAPE, "bad shape N=%d K=%d", N, K);
-  DQ_REQUIRE(y_dtype == DQ_DTYPE_F32 || y_dtype == DQ_DTYPE_BF16, DQ_ERR_UNSUPPORTED, "unknown y_dtype %d", y_dtype);
-  DQ_REQUIRE(dq::aligned(w8, 16), DQ_ERR_ALIGN, "w8 must be 16-byte aligned");
-  return dq::launch_gemm_int4_e4m3(reinterpret_cast<const uint8_t*>(codes), sx, w8, sw_t, r, M, N, K, y, y_dtype, add,
-                                   static_cast<cudaStream_t>(stream), st);
+  return quant_and_gemm(x_bf16, ldx, a, had, w_packed, w8, sw_t, r, bias, M, N, K, G, y, y_dtype, scale_fp16, scratch,
+                        scratch_bytes, stream);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -506,7 +506,8 @@ DQ_API int dq_linear_w4a4_int4(const void* x_bf16, int64_t ldx, const float* a,
  *   bias [N] of y's element type or null: for bf16 added to the rounded result and rounded again, as "linear(x) + bias"
  *   w8   the weight's byte form from dq_expand_w_int4_e4m3, or null: with it the call runs on the FP8-path GEMM whatever
  *        the batch size, and expands nothing
- * scratch: dq_linear_w4a4_int4_scratch_bytes(M,N,K) bytes.
+ * scratch: dq_linear_w4a4_int4_scratch_bytes(M,N,K) bytes; without w8, room for the byte form behind them
+ * (dq_linear_w4a4_int4_prefill_scratch_bytes) is used as by dq_linear_w4a4_int4.
  */
 DQ_API int dq_linear_w4a4_int4_bias(const void* x_bf16, int64_t ldx, const float* a, const dq_hadamard_desc* had,
                                     const uint8_t* w_packed, const uint8_t* w8, const void* sw_t, const float* r,

@@ -2,6 +2,8 @@
 
 Integer work, so everything here is bit-exact: the byte forms against a table of the sixteen codes,
 the GEMM against the oracle's integer accumulation and epilogue and against the int8-path kernel."""
+import ctypes
+
 import pytest
 import torch
 
@@ -128,6 +130,30 @@ def test_linear_entry_takes_the_fp8_path_with_the_larger_scratch():
                                          scale_fp16=True, scratch=scratch))
     _lib.device_status(0)
     assert torch.equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("M,room", [(1023, True), (1024, False), (1024, True), (1101, True)])
+def test_bias_entry_takes_the_fp8_path_with_the_larger_scratch(M, room):
+    """dq_linear_w4a4_int4_bias without a byte form of the weight: from 1024 tokens on it expands one behind the codes
+    where the scratch has room, and adds the bias to the rounded result either way."""
+    N, K = 520, 1024
+    _, _, pw = _weights(N, K, 17)
+    x = synthetic.make_x(M, K, 18).to(DEV)
+    bias = torch.randn(N, generator=torch.Generator().manual_seed(19)).to(torch.bfloat16).to(DEV)
+    base = ops.linear_scratch_bytes(M, N, K, prefill=False)
+    scratch = torch.full((base + (N * K + 255) // 256 * 256 if room else base,), 0xA5, dtype=torch.uint8, device=DEV)
+    y = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    _lib.check(_lib.load().dq_linear_w4a4_int4_bias(
+        p(x), K, None, None, p(pw.w_packed), None, p(pw.sw_t), None, p(bias), M, N, K, 128, p(y), _lib.DTYPE_BF16, 0,
+        p(scratch), scratch.numel(), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)), "dq_linear_w4a4_int4_bias")
+    _lib.device_status(0)
+    codes, sx = ops.quant_act_int4(x)
+    assert torch.equal(y, ops.gemm_w4a4_int4(codes, sx, pw, None, out_dtype=torch.bfloat16) + bias)
+    if room and M >= 1024:
+        assert torch.equal(scratch[base:base + N * K].view(N, K), ops.expand_w_e4m3(pw))
+    else:
+        assert bool((scratch[base:] == 0xA5).all())
 
 
 def test_decoder_linear_rows_do_not_depend_on_the_batch_they_arrive_in():
