@@ -17,7 +17,6 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/ops/add.h>
 #include <c10/cuda/CUDAFunctions.h>
-#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -35,8 +34,7 @@ namespace {
 #define DQ_FUNCTIONS(X)                                                                              \
   X(dq_quant_act_int4) X(dq_quant_act_int4_f32) X(dq_quant_act_int4_gated) X(dq_quant_act_int4_rmsnorm) \
   X(dq_gemm_w4a4_int4_ex) X(dq_gemm_w4a4_int4_residual) X(dq_gemm_w4a4_int4_e4m3)                      \
-  X(dq_linear_w4a4_int4) X(dq_linear_w4a4_int4_bias) X(dq_linear_w4a4_int4_scratch_bytes) \
-  X(dq_linear_w4a4_int4_byte_form_pays)                                                                                       \
+  X(dq_linear_w4a4_int4) X(dq_linear_w4a4_int4_bias) X(dq_linear_w4a4_int4_scratch_bytes)             \
   X(dq_linear_w4a4_int4_prefill_scratch_bytes) X(dq_linear_a16w4) X(dq_linear_a16w4_scratch_bytes)     \
   X(dq_linear_w4a4_fp4) X(dq_linear_w4a4_fp4_scratch_bytes)
 #define DQ_DECLARE(name) decltype(&::name) name = nullptr;
@@ -52,7 +50,7 @@ uint64_t g_inited = 0;              // devices ensure_init has been called for
 // attribute names, interned once
 #define DQ_NAMES(X)                                                                                   \
   X(kind) X(had_k) X(had_dim) X(scale) X(had_mat) X(w_packed) X(sw_t) X(N) X(K) X(group) X(codes)       \
-  X(sf_atoms) X(tensor_scale) X(w8) X(bytes_e4m3) X(fmt) X(_plan) X(act_quant_enabled) X(online_full_had)                  \
+  X(sf_atoms) X(tensor_scale) X(fmt) X(_plan) X(act_quant_enabled) X(online_full_had)                  \
   X(online_partial_had) X(had_K) X(act_fmt) X(quantize_bmm_input) X(dtype) X(_buffers) X(act_scale)    \
   X(_modules) X(layer) X(_parameters) X(bias) X(_packed) X(_packed_fp4)
 #define DQ_DECLARE(n) PyObject* n = nullptr;
@@ -374,37 +372,24 @@ PyObject* gemm_w4a4_int4_e4m3(PyObject*, PyObject* const* v, Py_ssize_t n) {
   });
 }
 
-// The weight's byte form (ops.PackedInt4Weight.w8, kept with the packed weight once it exists) for a batch that the
-// FP8-path GEMM serves better, or null.  Made by the first such batch: N * K bytes that used to be expanded into scratch
-// on every call (4096 -> 28672: 88 -> 68 us at 300 tokens, 120 -> 76 at 500; 14336 -> 4096: 58 -> 55).  While a graph is being captured nothing is made: an
-// expansion recorded there would not have run when the next call reads it.
-const uint8_t* byte_form(PyObject* pw, int M, int N, int K, int group) {
-  if (group != 128 || !abi.dq_linear_w4a4_int4_byte_form_pays(M, N, K)) return nullptr;
-  {
-    Ref w8(PyObject_GetAttr(pw, names.w8));
-    if (w8.p != Py_None) return static_cast<const uint8_t*>(tensor(w8.p, "w8").data_ptr());
-  }
-  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return nullptr;
-  Ref w8(PyObject_CallMethodNoArgs(pw, names.bytes_e4m3));
-  return static_cast<const uint8_t*>(tensor(w8.p, "w8").data_ptr());
+// Scratch of linear_int4: from 1024 tokens on with room for the weight's byte form, which every call expands anew.  (Kept
+// with the packed weight it would save 5 to 18 us a call, but nothing tells when those bytes are written again, or
+// whether another stream's expansion has finished.  A caller who knows keeps it: ops.PackedInt4Weight.bytes_e4m3.)
+int64_t int4_scratch_bytes(int M, int N, int K) {
+  return std::max<int64_t>(static_cast<int64_t>(abi.dq_linear_w4a4_int4_prefill_scratch_bytes(M, N, K)), 256);
 }
-// Scratch of linear_int4 below.
-int64_t int4_scratch_bytes(const uint8_t* w8, int M, int N, int K) {
-  return static_cast<int64_t>(w8 != nullptr ? abi.dq_linear_w4a4_int4_scratch_bytes(M, N, K)
-                                            : abi.dq_linear_w4a4_int4_prefill_scratch_bytes(M, N, K));
-}
-// Activation quantiser + GEMM of one linear: with the weight's byte form on the FP8 path, else as the library chooses.
+// Activation quantiser + GEMM of one linear.
 void linear_int4(const void* x, int64_t ldx, const float* a, const dq_hadamard_desc* had, const PackedInt4& w,
-                 const uint8_t* w8, const float* r, const void* bias, int M, const at::Tensor& out, int mode,
-                 const at::Tensor& scratch, int idx) {
+                 const float* r, const void* bias, int M, const at::Tensor& out, int mode, const at::Tensor& scratch,
+                 int idx) {
   void* stream = stream_of(idx);
   const size_t bytes = static_cast<size_t>(scratch.numel());
-  if (w8 == nullptr && bias == nullptr)
+  if (bias == nullptr)
     check(abi.dq_linear_w4a4_int4(x, ldx, a, had, w.w_packed, w.sw_t, r, M, w.N, w.K, w.group, out.data_ptr(),
                                   y_dtype_of(out), mode, scratch.data_ptr(), bytes, stream),
           "dq_linear_w4a4_int4");
   else
-    check(abi.dq_linear_w4a4_int4_bias(x, ldx, a, had, w.w_packed, w8, w.sw_t, r, bias, M, w.N, w.K, w.group,
+    check(abi.dq_linear_w4a4_int4_bias(x, ldx, a, had, w.w_packed, nullptr, w.sw_t, r, bias, M, w.N, w.K, w.group,
                                        out.data_ptr(), y_dtype_of(out), mode, scratch.data_ptr(), bytes, stream),
           "dq_linear_w4a4_int4_bias");
 }
@@ -426,18 +411,19 @@ PyObject* linear_w4a4_int4(PyObject*, PyObject* const* v, Py_ssize_t n) {
       PyErr_Format(PyExc_ValueError, "K mismatch: activations %d, weight %d", K, w.K);
       throw PyError();
     }
-    // a caller's scratch is used as it is when it covers the plain path
-    const uint8_t* w8 = byte_form(v[3], M, w.N, K, w.group);
+    // a caller's scratch is used as it is when it covers the plain path; the library takes the FP8-path GEMM for
+    // prefill batches only where it also has room for the weight's byte form
     at::Tensor scratch;
     if (v[7] != Py_None && tensor(v[7], "scratch").numel() >=
                                static_cast<int64_t>(abi.dq_linear_w4a4_int4_scratch_bytes(M, w.N, K)))
       scratch = tensor(v[7], "scratch");
     else
-      scratch = empty({std::max<int64_t>(int4_scratch_bytes(w8, M, w.N, K), 256)}, at::kByte, idx);
+      scratch = empty({int4_scratch_bytes(M, w.N, K)}, at::kByte, idx);
     at::Tensor out = output(v[8], Py_None, v[5], M, w.N, idx);
     const dq_hadamard_desc d = hadamard(v[2]);
-    linear_int4(x.data_ptr(), row_stride(x), static_cast<const float*>(ptr_or_null(v[1], "a")), desc(d), w, w8,
-                static_cast<const float*>(ptr_or_null(v[4], "r")), nullptr, M, out, static_cast<int>(as_long(v[6])), scratch, idx);
+    linear_int4(x.data_ptr(), row_stride(x), static_cast<const float*>(ptr_or_null(v[1], "a")), desc(d), w,
+                static_cast<const float*>(ptr_or_null(v[4], "r")), nullptr, M, out, static_cast<int>(as_long(v[6])), scratch,
+                idx);
     return wrap(std::move(out));
   });
 }
@@ -646,9 +632,8 @@ PyObject* perm_forward(PyObject*, PyObject* const* v, Py_ssize_t n) {
     if (bias == nullptr) Py_RETURN_NONE;
     const int idx = prep(x);
     const int M = static_cast<int>(x.numel() / K);
-    const uint8_t* w8 = p->kind == PLAN_INT4 ? byte_form(p->packed, M, N, K, p->w4.group) : nullptr;
     int64_t need;
-    if (p->kind == PLAN_INT4) need = int4_scratch_bytes(w8, M, N, K);
+    if (p->kind == PLAN_INT4) need = int4_scratch_bytes(M, N, K);
     else if (p->kind == PLAN_FP4) need = fp4_scratch_bytes(M, K, p->w_fp4.fmt);
     else need = static_cast<int64_t>(abi.dq_linear_a16w4_scratch_bytes(M, N, K));
     if (!p->scratch->defined() || p->scratch->numel() < need)
@@ -667,7 +652,7 @@ PyObject* perm_forward(PyObject*, PyObject* const* v, Py_ssize_t n) {
       }
     }
     if (p->kind == PLAN_INT4) {
-      linear_int4(x.data_ptr(), ldx, a, desc(p->had), p->w4, w8, nullptr, bias_ptr, M, out, p->scale_mode, *p->scratch, idx);
+      linear_int4(x.data_ptr(), ldx, a, desc(p->had), p->w4, nullptr, bias_ptr, M, out, p->scale_mode, *p->scratch, idx);
     } else if (p->kind == PLAN_FP4) {
       linear_fp4(x.data_ptr(), false, K, M, a, p->w_fp4, nullptr, bias_ptr, out, *p->scratch, idx);
     } else {

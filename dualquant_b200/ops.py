@@ -455,8 +455,8 @@ def linear_w4a4_int4(x: torch.Tensor, a: Optional[torch.Tensor], had: Optional[H
                      scale_fp16: bool = False, scratch: Optional[torch.Tensor] = None,
                      out: Optional[torch.Tensor] = None, bf16_arith: bool = False) -> torch.Tensor:
     """Whole PermLinear.forward on the int4 path in one call.  A caller's scratch is used as it is when it
-    covers the plain path.  From 256 tokens on it may run on the FP8-path GEMM with the weight's byte form, which
-    the first such call makes and keeps (pw.w8)."""
+    covers the plain path; prefill batches take the FP8-path GEMM when it also has room for the weight's byte
+    form (linear_scratch_bytes)."""
     return _lib.host().linear_w4a4_int4(x, a, had, pw, r, out_dtype, _scale_mode(scale_fp16, bf16_arith), scratch, out)
 
 

@@ -258,3 +258,43 @@ def test_native_forward_equals_the_python_forward_and_follows_changes(name):
         assert torch.equal(pl(x), pl._forward(x))
     twin = copy.deepcopy(pl)
     assert twin._plan is None and torch.equal(twin(x), pl(x))
+
+
+@pytest.mark.parametrize("M", [8, 300, 1100])
+def test_weight_bytes_written_in_place_take_effect(M):
+    """The packed weight is what a call reads: bytes written into it in place count from the next call on, at every
+    batch size and in a captured graph, and a call with the caller's scratch and output allocates nothing."""
+    from dualquant_b200 import ops
+
+    N, K = 520, 1024
+    old, new = (ops.pack_w_int4(*ops.quant_w_int4(synthetic.make_w(N, K, s).to(DEV))) for s in (31, 32))
+    x = synthetic.make_x(M, K, 33).to(DEV)
+    scratch = torch.empty(ops.linear_scratch_bytes(M, N, K), dtype=torch.uint8, device=DEV)
+    y = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    lin = nn.Linear(K, N, bias=False, device=DEV, dtype=torch.bfloat16)
+    pl = PermLinear(lin, formats.make_format("rtn_int4", block_size=-1))
+    pl.pack(ops.unpack_w_int4(old), ops.quant_w_int4(synthetic.make_w(N, K, 31).to(DEV))[1])
+
+    def call(pw):
+        return ops.linear_w4a4_int4(x, None, None, pw, None, scratch=scratch, out=y, bf16_arith=True).clone()
+
+    want = call(new)
+    first = call(old)
+    assert not torch.equal(first, want)
+    for _ in range(2):  # the Python forward, then the native one
+        assert torch.equal(pl(x), first)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = pl(x)
+    for pw in (old, pl._packed):
+        pw.w_packed.copy_(new.w_packed)
+        pw.sw_t.copy_(new.sw_t)
+    assert torch.equal(call(old), want)
+    assert torch.equal(pl(x), want)
+    graph.replay()
+    assert torch.equal(captured, want)
+    torch.cuda.synchronize()
+    held = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    ops.linear_w4a4_int4(x, None, None, old, None, scratch=scratch, out=y, bf16_arith=True)
+    assert torch.cuda.max_memory_allocated() == held
