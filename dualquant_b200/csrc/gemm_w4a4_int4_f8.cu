@@ -203,6 +203,12 @@ static int launch_gemm_int4_e4m3_impl(const uint8_t* x8, const float* sx, const 
   return DQ_OK;
 }
 
+float gemm_int4_bytes_us(int M, int N, int K, int sm_count) {
+  float us = 0.f;
+  f8::pick_tile(M, (N + 2 * f8::kBN - 1) / (2 * f8::kBN), K / kGroup, sm_count / 2, false, &us);
+  return us;
+}
+
 int launch_gemm_int4_e4m3(const uint8_t* x8, const float* sx, const uint8_t* w8, const void* sw_t, const float* r,
                           int M, int N, int K, void* y, int y_dtype, Addend add, cudaStream_t stream,
                           DeviceState* st) {
@@ -250,9 +256,7 @@ extern "C" int dq_linear_w4a4_int4_byte_form_pays(int M, int N, int K) {
   if (M < 256 || N < 1 || K < kGroup || K % kGroup != 0) return 0;
   DeviceState* st = current_state();
   if (M >= 512 || st == nullptr) return 1;
-  float bytes_us = 0.f;
-  f8::pick_tile(M, (N + 2 * f8::kBN - 1) / (2 * f8::kBN), K / kGroup, st->sm_count / 2, false, &bytes_us);
-  return gemm_int4_packed_us(M, N, K, st->sm_count) >= 0.9f * bytes_us ? 1 : 0;
+  return gemm_int4_packed_us(M, N, K, st->sm_count) >= 0.9f * gemm_int4_bytes_us(M, N, K, st->sm_count) ? 1 : 0;
 }
 
 extern "C" int dq_expand_w_int4_e4m3(const uint8_t* w_packed, int N, int K, int G, uint8_t* w8, void* stream) {

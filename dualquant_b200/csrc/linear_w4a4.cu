@@ -1,7 +1,7 @@
 // One-call PermLinear.forward on the real int4 path.  Decode batches (M <= 16, no online Hadamard)
 // may run as ONE kernel that quantises in its prologue; everything else is activation quantiser +
 // GEMM on the caller's stream with the intermediates in caller-provided scratch.  Prefill batches
-// (M >= kPrefillTokens) take the FP8 tensor-core path when the caller's scratch also has room for
+// (expansion_pays) take the FP8 tensor-core path when the caller's scratch also has room for
 // the byte form of the weight: quantiser (E4M3 codes) + weight expansion + GEMM.
 #include "dq_common.h"
 
@@ -16,18 +16,29 @@ extern "C" size_t dq_linear_w4a4_int4_scratch_bytes(int M, int N, int K) {
          round_up(static_cast<size_t>(M) * sizeof(float), 256);
 }
 
-// From this many tokens on the FP8-path GEMM wins even with the weight expanded on every call
-// (the expansion moves 1.5 bytes per weight; measured on B200 it pays from about 1000 tokens).
-static constexpr int kPrefillTokens = 1024;
+// Whether a call does best to expand the weight and run on the FP8-path GEMM: from 1024 tokens on always (quantiser
+// included, 4096 -> 4096 43 us packed, 34 expanded; 14336 -> 1392, the narrowest measured, 80 and 78), from 256 where the
+// kernels' estimates and that of the expansion say so (768 tokens: 18944 -> 3584 157 and 129, 14336 -> 1392 51 and 68;
+// 512 tokens: 4096 -> 6144 44 and 36, 14336 -> 4096 73 and 91).  The estimate of the FP8-path GEMM, whose group times are
+// those of long runs at the power cap, is high for wide outputs (4096 -> 28672 at 768 tokens: 179 and 139, estimated
+// alike), hence the margin there.  Over 95 shapes of 256 to 1000 tokens the choice costs 0.3 % on average, 18 % at worst.
+static bool expansion_pays(int M, int N, int K) {
+  if (M < 256 || N < 1 || K < dq::kGroup || K % dq::kGroup != 0) return false;
+  if (M >= 1024) return true;
+  const dq::DeviceState* st = dq::current_state();
+  const int sms = st != nullptr ? st->sm_count : 148;  // (a size asked for before dq_init)
+  const float expanded = dq::gemm_int4_bytes_us(M, N, K, sms) + dq::expand_w_us(N, K);
+  return dq::gemm_int4_packed_us(M, N, K, sms) >= (M > 384 && N >= 6144 ? 0.75f : 1.0f) * expanded;
+}
 
 extern "C" size_t dq_linear_w4a4_int4_prefill_scratch_bytes(int M, int N, int K) {
   const size_t base = dq_linear_w4a4_int4_scratch_bytes(M, N, K);
-  if (M < kPrefillTokens || N < 1 || K < 1) return base;
+  if (!expansion_pays(M, N, K)) return base;
   return base + round_up(static_cast<size_t>(N) * static_cast<size_t>(K), 256);
 }
 
 // Quantiser and GEMM with the codes and token scales in the scratch.  The FP8-path GEMM runs with the caller's byte form of
-// the weight (w8), or from kPrefillTokens on with one expanded behind the token scales where the scratch has room for it.
+// the weight (w8), or where it pays with one expanded behind the token scales if the scratch has room for it.
 static int quant_and_gemm(const void* x_bf16, int64_t ldx, const float* a, const dq_hadamard_desc* had,
                           const uint8_t* w_packed, const uint8_t* w8, const void* sw_t, const float* r, const void* bias,
                           int M, int N, int K, int G, void* y, int y_dtype, int scale_fp16, void* scratch,
@@ -36,7 +47,7 @@ static int quant_and_gemm(const void* x_bf16, int64_t ldx, const float* a, const
   int8_t* codes = static_cast<int8_t*>(scratch);
   float* sx = reinterpret_cast<float*>(base + round_up(static_cast<size_t>(M) * K, 256));
   const dq::Addend add = {bias, 0};
-  if (w8 == nullptr && M >= kPrefillTokens && G == dq::kGroup && (scale_fp16 & ~0xFF) == 0 &&
+  if (w8 == nullptr && G == dq::kGroup && (scale_fp16 & ~0xFF) == 0 && expansion_pays(M, N, K) &&
       scratch_bytes >= dq_linear_w4a4_int4_prefill_scratch_bytes(M, N, K)) {
     uint8_t* expanded = base + dq_linear_w4a4_int4_scratch_bytes(M, N, K);
     const int rc = dq_expand_w_int4_e4m3(w_packed, N, K, G, expanded, stream);

@@ -372,7 +372,7 @@ PyObject* gemm_w4a4_int4_e4m3(PyObject*, PyObject* const* v, Py_ssize_t n) {
   });
 }
 
-// Scratch of linear_int4: from 1024 tokens on with room for the weight's byte form, which every call expands anew.  (Kept
+// Scratch of linear_int4: for prefill batches with room for the weight's byte form, which every call expands anew.  (Kept
 // with the packed weight it would save 5 to 18 us a call, but nothing tells when those bytes are written again, or
 // whether another stream's expansion has finished.  A caller who knows keeps it: ops.PackedInt4Weight.bytes_e4m3.)
 int64_t int4_scratch_bytes(int M, int N, int K) {

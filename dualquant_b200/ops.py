@@ -442,8 +442,8 @@ def gemm_w4a4_int4_acc(codes: torch.Tensor, pw: PackedInt4Weight) -> torch.Tenso
 
 
 def linear_scratch_bytes(M: int, N: int, K: int, prefill: bool = True) -> int:
-    """Scratch of linear_w4a4_int4; prefill=True includes the room that lets batches of 1024 tokens
-    and more take the FP8-path GEMM (N * K bytes more for those, nothing for smaller batches)."""
+    """Scratch of linear_w4a4_int4; prefill=True includes the room that lets prefill batches take the FP8-path
+    GEMM (N * K bytes more from 1024 tokens on, and from 256 where that is the faster one)."""
     lib = _lib.load()
     if prefill:
         return int(lib.dq_linear_w4a4_int4_prefill_scratch_bytes(M, N, K))

@@ -485,9 +485,10 @@ DQ_API int dq_gemm_w4a4_int4_acc(const int8_t* codes, const uint8_t* w_packed, i
  * One call for a whole PermLinear.forward (activations/perm_linear.py:136-141) on the real
  * int4 path: quantise x (as dq_quant_act_int4) into caller scratch, then the GEMM.
  * scratch must hold dq_linear_w4a4_int4_scratch_bytes(M,N,K) bytes.
- * Prefill batches (1024 tokens and more) run on the FP8-path GEMM (dq_gemm_w4a4_int4_e4m3, same
- * bits, about twice as fast) when the scratch also has room for the byte form of the weight:
- * dq_linear_w4a4_int4_prefill_scratch_bytes(M,N,K) (equal to the plain figure for smaller M).
+ * Prefill batches (1024 tokens and more, and from 256 those for which it is estimated to be faster) run
+ * on the FP8-path GEMM (dq_gemm_w4a4_int4_e4m3, same bits, up to twice as fast) when the scratch also
+ * has room for the byte form of the weight: dq_linear_w4a4_int4_prefill_scratch_bytes(M,N,K) (equal to
+ * the plain figure for other batches).
  * The weight is expanded into the scratch on every call; callers that can keep N*K bytes per
  * weight call dq_expand_w_int4_e4m3 once and dq_gemm_w4a4_int4_e4m3 directly.
  */

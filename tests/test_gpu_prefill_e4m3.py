@@ -132,9 +132,9 @@ def test_linear_entry_takes_the_fp8_path_with_the_larger_scratch():
     assert torch.equal(outs[0], outs[1])
 
 
-@pytest.mark.parametrize("M,room", [(1023, True), (1024, False), (1024, True), (1101, True)])
+@pytest.mark.parametrize("M,room", [(255, True), (1024, False), (1024, True), (1101, True)])
 def test_bias_entry_takes_the_fp8_path_with_the_larger_scratch(M, room):
-    """dq_linear_w4a4_int4_bias without a byte form of the weight: from 1024 tokens on it expands one behind the codes
+    """dq_linear_w4a4_int4_bias without a byte form of the weight: a prefill batch expands one behind the codes
     where the scratch has room, and adds the bias to the rounded result either way."""
     N, K = 520, 1024
     _, _, pw = _weights(N, K, 17)
@@ -303,17 +303,28 @@ def test_every_token_tile_equals_the_integer_kernel(tile, M, N, K):
 
 
 @pytest.mark.parametrize("M,N,K", [(255, 1392, 2048), (256, 1392, 14336), (294, 1391, 14336), (300, 1024, 8192), (511, 2050, 4096),
-                                   (512, 1391, 1152), (700, 18317, 256)])
+                                   (512, 1391, 1152), (640, 4096, 1024), (700, 18317, 256), (1023, 2050, 512), (1024, 136, 256)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_linear_picks_weight_form(M, N, K, dtype):
-    """Between 256 and 511 tokens a linear reads the packed weight or its byte form, whichever is estimated faster; rows
-    that are not 16-byte multiples are stored directly.  The result equals the unsplit packed kernel's either way."""
+    """From 256 tokens on a linear reads the packed weight or expands it into the scratch, whichever is estimated faster;
+    rows that are not 16-byte multiples are stored directly.  The result equals the unsplit packed kernel's: bit for bit
+    where the weight was expanded, to the order of the fp32 sums over the groups where K may have been split."""
     g = torch.Generator(device=DEV).manual_seed(M + N)
     pw = ops.pack_w_int4(*ops.quant_w_int4((torch.randn(N, K, generator=g, device=DEV) * 0.02).to(torch.bfloat16)))
     x = torch.randn(M, K, generator=g, device=DEV).to(torch.bfloat16)
     codes, sx = ops.quant_act_int4(x)
-    ref = ops.gemm_w4a4_int4(codes, sx, pw, token_tile=1128, split_k=1)
-    y = ops.linear_w4a4_int4(x, None, None, pw, None, out=torch.empty(M, N, dtype=dtype, device=DEV))
-    tol = 1e-6 if dtype == torch.float32 else 4e-3
-    assert ((y.float() - ref).abs().max() / ref.abs().max()).item() < tol
+    ref = ops.gemm_w4a4_int4(codes, sx, pw, token_tile=1128, split_k=1, out_dtype=dtype)
+    plain = ops.linear_scratch_bytes(M, N, K, prefill=False)
+    scratch = torch.full((plain + (N * K + 255) // 256 * 256,), 0xA5, dtype=torch.uint8, device=DEV)
+    out = torch.empty(M, N, dtype=dtype, device=DEV)
+    y = ops.linear_w4a4_int4(x, None, None, pw, None, scratch=scratch, out=out)
     _lib.device_status(0)
+    expands = ops.linear_scratch_bytes(M, N, K) > plain
+    assert expands or M < 1024
+    if expands:
+        assert M >= 256 and torch.equal(scratch[plain:plain + N * K].view(N, K), ops.expand_w_e4m3(pw))
+        assert torch.equal(y, ref)
+    else:
+        assert bool((scratch[plain:] == 0xA5).all())
+        tol = 1e-6 if dtype == torch.float32 else 2.0 ** -7  # (bf16: a sum at a rounding boundary steps)
+        assert ((y.float() - ref.float()).abs().max() / ref.float().abs().max()).item() < tol
