@@ -44,7 +44,6 @@ class PermLinear(nn.Module):
         self._packed: Optional[ops.PackedInt4Weight] = None
         self._packed_fp4: Optional[ops.PackedFp4Weight] = None
         self._hadamard_cache = None
-        self._scratch: Optional[torch.Tensor] = None
         # what the native forward needs, made by _make_plan; None = to be made by the next call
         self._plan = None
         # None = not examined yet; False = the weight is not on the W4 grid of the activation
@@ -202,7 +201,6 @@ class PermLinear(nn.Module):
         if packed is not None:
             had = self._hadamard(x.device) if kind == 0 else None
             self._plan = _lib.host().make_plan(self, kind, had, 2 if self._bf16_arith(x2) else 0, self.dtype)
-            self._scratch = None  # the plan keeps its own
 
     def forward(self, x):
         out = _lib.host().perm_forward(self, x)
@@ -221,17 +219,12 @@ class PermLinear(nn.Module):
         if use_int4 and self._packed is not None:
             pw = self._packed
             x2 = x.reshape(-1, x.shape[-1])
-            M = x2.shape[0]
-            need = ops.linear_scratch_bytes(M, pw.N, pw.K)
-            if self._scratch is None or self._scratch.numel() < need or self._scratch.device != x.device:
-                self._scratch = torch.empty(max(need, 256), dtype=torch.uint8, device=x.device)
             out_dtype = self.dtype if self.dtype in (torch.bfloat16, torch.float32) else torch.float32
             if x2.dtype == torch.bfloat16:
                 # without an activation scale and a Hadamard the reference quantises in the input
                 # dtype, i.e. in bf16 arithmetic (perm_linear.py:109-133); same here
                 out = ops.linear_w4a4_int4(x2, self.act_scale, self._hadamard(x.device), pw, None,
-                                           out_dtype=out_dtype, scale_fp16=False, scratch=self._scratch,
-                                           bf16_arith=self._bf16_arith(x2))
+                                           out_dtype=out_dtype, scale_fp16=False, bf16_arith=self._bf16_arith(x2))
             else:
                 # the reference upcasts to fp32 before scaling and quantising (perm_linear.py:119-125):
                 # fp32 / fp16 inputs go through the fp32 quantiser, not through a bf16 rounding

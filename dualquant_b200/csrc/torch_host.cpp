@@ -16,6 +16,7 @@
 #include <ATen/core/grad_mode.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/ops/add.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
@@ -112,6 +113,16 @@ void* stream_of(int idx) {
 at::Tensor empty(at::IntArrayRef sizes, at::ScalarType dtype, int idx) {
   return at::detail::empty_cuda(sizes, dtype, at::Device(at::kCUDA, static_cast<c10::DeviceIndex>(idx)), std::nullopt);
 }
+
+// Scratch of one call, from torch's allocator for the current stream: calls of one module on several streams, and graphs
+// captured through it, keep theirs apart.
+struct Scratch {
+  c10::DataPtr mem;
+  size_t bytes = 0;
+  Scratch() = default;
+  explicit Scratch(int64_t n)
+      : mem(c10::cuda::CUDACachingAllocator::get()->allocate(static_cast<size_t>(n))), bytes(static_cast<size_t>(n)) {}
+};
 
 long as_long(PyObject* o) {
   const long v = PyLong_AsLong(o);
@@ -380,17 +391,16 @@ int64_t int4_scratch_bytes(int M, int N, int K) {
 }
 // Activation quantiser + GEMM of one linear.
 void linear_int4(const void* x, int64_t ldx, const float* a, const dq_hadamard_desc* had, const PackedInt4& w,
-                 const float* r, const void* bias, int M, const at::Tensor& out, int mode, const at::Tensor& scratch,
+                 const float* r, const void* bias, int M, const at::Tensor& out, int mode, void* scratch, size_t bytes,
                  int idx) {
   void* stream = stream_of(idx);
-  const size_t bytes = static_cast<size_t>(scratch.numel());
   if (bias == nullptr)
     check(abi.dq_linear_w4a4_int4(x, ldx, a, had, w.w_packed, w.sw_t, r, M, w.N, w.K, w.group, out.data_ptr(),
-                                  y_dtype_of(out), mode, scratch.data_ptr(), bytes, stream),
+                                  y_dtype_of(out), mode, scratch, bytes, stream),
           "dq_linear_w4a4_int4");
   else
     check(abi.dq_linear_w4a4_int4_bias(x, ldx, a, had, w.w_packed, nullptr, w.sw_t, r, bias, M, w.N, w.K, w.group,
-                                       out.data_ptr(), y_dtype_of(out), mode, scratch.data_ptr(), bytes, stream),
+                                       out.data_ptr(), y_dtype_of(out), mode, scratch, bytes, stream),
           "dq_linear_w4a4_int4_bias");
 }
 
@@ -413,17 +423,23 @@ PyObject* linear_w4a4_int4(PyObject*, PyObject* const* v, Py_ssize_t n) {
     }
     // a caller's scratch is used as it is when it covers the plain path; the library takes the FP8-path GEMM for
     // prefill batches only where it also has room for the weight's byte form
-    at::Tensor scratch;
+    Scratch own;
+    void* scratch = nullptr;
+    size_t bytes = 0;
     if (v[7] != Py_None && tensor(v[7], "scratch").numel() >=
-                               static_cast<int64_t>(abi.dq_linear_w4a4_int4_scratch_bytes(M, w.N, K)))
-      scratch = tensor(v[7], "scratch");
-    else
-      scratch = empty({int4_scratch_bytes(M, w.N, K)}, at::kByte, idx);
+                               static_cast<int64_t>(abi.dq_linear_w4a4_int4_scratch_bytes(M, w.N, K))) {
+      scratch = tensor(v[7], "scratch").data_ptr();
+      bytes = static_cast<size_t>(tensor(v[7], "scratch").numel());
+    } else {
+      own = Scratch(int4_scratch_bytes(M, w.N, K));
+      scratch = own.mem.get();
+      bytes = own.bytes;
+    }
     at::Tensor out = output(v[8], Py_None, v[5], M, w.N, idx);
     const dq_hadamard_desc d = hadamard(v[2]);
     linear_int4(x.data_ptr(), row_stride(x), static_cast<const float*>(ptr_or_null(v[1], "a")), desc(d), w,
-                static_cast<const float*>(ptr_or_null(v[4], "r")), nullptr, M, out, static_cast<int>(as_long(v[6])), scratch,
-                idx);
+                static_cast<const float*>(ptr_or_null(v[4], "r")), nullptr, M, out, static_cast<int>(as_long(v[6])),
+                scratch, bytes, idx);
     return wrap(std::move(out));
   });
 }
@@ -460,10 +476,9 @@ int64_t fp4_scratch_bytes(int M, int K, int fmt) {
   return std::max<int64_t>(static_cast<int64_t>(abi.dq_linear_w4a4_fp4_scratch_bytes(M, K, fmt)), 256);
 }
 void linear_fp4(const void* x, bool f32, int64_t ldx, int M, const float* a, const PackedFp4& w, const float* r,
-                const void* bias, const at::Tensor& out, const at::Tensor& scratch, int idx) {
+                const void* bias, const at::Tensor& out, const Scratch& scratch, int idx) {
   check(abi.dq_linear_w4a4_fp4(x, f32 ? 1 : 0, ldx, a, w.codes, w.sf_atoms, w.tensor_scale, r, bias, M, w.N, w.K, w.fmt,
-                               out.data_ptr(), y_dtype_of(out), scratch.data_ptr(), static_cast<size_t>(scratch.numel()),
-                               stream_of(idx)),
+                               out.data_ptr(), y_dtype_of(out), scratch.mem.get(), scratch.bytes, stream_of(idx)),
         "dq_linear_w4a4_fp4");
 }
 
@@ -483,7 +498,7 @@ PyObject* linear_w4a4_fp4(PyObject*, PyObject* const* v, Py_ssize_t n) {
       PyErr_Format(PyExc_ValueError, "K mismatch: activations %d, weight %d", static_cast<int>(x.size(1)), w.K);
       throw PyError();
     }
-    const at::Tensor scratch = empty({fp4_scratch_bytes(M, w.K, w.fmt)}, at::kByte, idx);
+    const Scratch scratch(fp4_scratch_bytes(M, w.K, w.fmt));
     at::Tensor out = empty({M, w.N}, dtype_arg(v[4]), idx);
     linear_fp4(x.data_ptr(), f32, w.K, M, static_cast<const float*>(ptr_or_null(v[1], "a")), w,
                static_cast<const float*>(ptr_or_null(v[3], "r")), nullptr, out, scratch, idx);
@@ -508,7 +523,6 @@ struct Plan {
   PackedInt4 w4;
   PackedFp4 w_fp4;
   at::ScalarType out_dtype;
-  at::Tensor* scratch;  // grows to the largest batch seen
 };
 
 #define DQ_PLAN_OBJECTS(X)                                                                                      \
@@ -532,7 +546,6 @@ int plan_clear(PyObject* self) {
 void plan_dealloc(PyObject* self) {
   PyObject_GC_UnTrack(self);
   plan_clear(self);
-  delete reinterpret_cast<Plan*>(self)->scratch;
   Py_TYPE(self)->tp_free(self);
 }
 // copies and pickles of a module carry no plan: they make their own
@@ -590,7 +603,6 @@ PyObject* make_plan(PyObject*, PyObject* const* v, Py_ssize_t n) {
     else p->w4 = packed_int4(p->packed);
     Ref wt(PyObject_GetAttr(p->packed, p->kind == PLAN_FP4 ? names.codes : names.w_packed));
     p->device = static_cast<int>(tensor(wt.p, "packed weight").get_device());
-    p->scratch = new at::Tensor();
     Py_INCREF(obj.p);
     return obj.p;
   });
@@ -636,8 +648,7 @@ PyObject* perm_forward(PyObject*, PyObject* const* v, Py_ssize_t n) {
     if (p->kind == PLAN_INT4) need = int4_scratch_bytes(M, N, K);
     else if (p->kind == PLAN_FP4) need = fp4_scratch_bytes(M, K, p->w_fp4.fmt);
     else need = static_cast<int64_t>(abi.dq_linear_a16w4_scratch_bytes(M, N, K));
-    if (!p->scratch->defined() || p->scratch->numel() < need)
-      *p->scratch = empty({std::max<int64_t>(need, 256)}, at::kByte, idx);
+    const Scratch scratch(std::max<int64_t>(need, 256));
     c10::SmallVector<int64_t, 5> sizes(x.sizes().begin(), x.sizes().end());
     sizes.back() = N;
     at::Tensor out = empty(sizes, p->out_dtype, idx);
@@ -652,13 +663,13 @@ PyObject* perm_forward(PyObject*, PyObject* const* v, Py_ssize_t n) {
       }
     }
     if (p->kind == PLAN_INT4) {
-      linear_int4(x.data_ptr(), ldx, a, desc(p->had), p->w4, nullptr, bias_ptr, M, out, p->scale_mode, *p->scratch, idx);
+      linear_int4(x.data_ptr(), ldx, a, desc(p->had), p->w4, nullptr, bias_ptr, M, out, p->scale_mode,
+                  scratch.mem.get(), scratch.bytes, idx);
     } else if (p->kind == PLAN_FP4) {
-      linear_fp4(x.data_ptr(), false, K, M, a, p->w_fp4, nullptr, bias_ptr, out, *p->scratch, idx);
+      linear_fp4(x.data_ptr(), false, K, M, a, p->w_fp4, nullptr, bias_ptr, out, scratch, idx);
     } else {
       check(abi.dq_linear_a16w4(x.data_ptr(), ldx, a, p->w4.w_packed, nullptr, M, N, K, p->w4.group, out.data_ptr(),
-                                y_dtype_of(out), p->scratch->data_ptr(), static_cast<size_t>(p->scratch->numel()),
-                                stream_of(idx)),
+                                y_dtype_of(out), scratch.mem.get(), scratch.bytes, stream_of(idx)),
             "dq_linear_a16w4");
     }
     if (bias != Py_None) return wrap(at::add(out, tensor(bias, "bias")));

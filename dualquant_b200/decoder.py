@@ -66,15 +66,6 @@ class W4A4Linear:
         self.a = 1.0 / c
         self.had = had
         self.N, self.K = N, K
-        self._scratch = {}
-
-    def _scratch_for(self, M: int, device):
-        buf = self._scratch.get(M)
-        if buf is None:
-            buf = torch.empty(max(ops.linear_scratch_bytes(M, self.N, self.K), 256), dtype=torch.uint8,
-                              device=device)
-            self._scratch[M] = buf
-        return buf
 
     # From this many tokens on the linears run on the FP8-path GEMM with the weight's byte form kept
     # next to the 4-bit artefact (N * K bytes more per weight; same results bit for bit, faster on every
@@ -104,8 +95,7 @@ class W4A4Linear:
         if residual is not None or big:
             codes, sx = ops.quant_act_int4(x, self.a, self.had, False, e4m3=big)
             return self._gemm(codes, sx, out_dtype, residual)
-        return ops.linear_w4a4_int4(x, self.a, self.had, self.pw, self.r, out_dtype=out_dtype,
-                                    scale_fp16=False, scratch=self._scratch_for(x.shape[0], x.device))
+        return ops.linear_w4a4_int4(x, self.a, self.had, self.pw, self.r, out_dtype=out_dtype, scale_fp16=False)
 
     def gated(self, gate: torch.Tensor, up: torch.Tensor, out_dtype=torch.bfloat16, ar=None,
               residual=None) -> torch.Tensor:

@@ -298,3 +298,58 @@ def test_weight_bytes_written_in_place_take_effect(M):
     torch.cuda.reset_peak_memory_stats()
     ops.linear_w4a4_int4(x, None, None, old, None, scratch=scratch, out=y, bf16_arith=True)
     assert torch.cuda.max_memory_allocated() == held
+
+
+def _packed_layer(name, K, N):
+    lin = nn.Linear(K, N, bias=False, device=DEV, dtype=torch.bfloat16)
+    lin.weight.data = synthetic.make_w(N, K, 41).to(DEV)
+    if name in ("mxfp4", "nvfp4"):
+        pl = PermLinear(lin, formats.make_format(name, block_size=32 if name == "mxfp4" else 16))
+        pl.pack_fp4(pl._fp4_fmt(), force=True)
+    else:
+        pl = PermLinear(lin, formats.make_format("rtn_int4", block_size=-1))
+        pl.pack(force=True)
+        pl.set_act_quant_enabled(name != "off")
+    pl.set_act_scale(torch.rand(K, generator=torch.Generator().manual_seed(42)).to(DEV) + 0.5)
+    return pl
+
+
+@pytest.mark.parametrize("name", ["rtn_int4", "mxfp4", "nvfp4", "off"])
+def test_graph_captured_through_a_layer_survives_a_larger_batch(name):
+    """A captured call owns its scratch: a larger batch through the same layer frees nothing that a replay writes."""
+    K, N = 1024, 512
+    pl = _packed_layer(name, K, N)
+    x = synthetic.make_x(24, K, 43).to(DEV)
+    pl(x)
+    want = pl(x)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = pl(x)
+    big = pl(synthetic.make_x(900, K, 44).to(DEV))
+    del big
+    # whatever the larger batch released is handed out again here
+    canaries = [torch.zeros(n, dtype=torch.uint8, device=DEV) for n in (256, 24 * K, 24 * K + 512, 48 * K, 64 * K) for _ in range(4)]
+    y.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
+    assert all(not c.any() for c in canaries)
+
+
+@pytest.mark.parametrize("name", ["rtn_int4", "mxfp4", "nvfp4", "off"])
+def test_one_layer_on_two_streams(name):
+    K, N = 2048, 4096
+    pl = _packed_layer(name, K, N)
+    xs = [synthetic.make_x(M, K, 45 + M).to(DEV) for M in (16, 100, 700)]
+    want = [pl(x) for x in xs]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    got = []
+    for i in range(30):
+        for j, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                k = (i + j) % len(xs)
+                got.append((k, pl(xs[k])))
+    torch.cuda.synchronize()
+    for k, y in got:
+        assert torch.equal(y, want[k])
