@@ -68,10 +68,18 @@ class PackedInt4Weight:
                 "group": self.group, "layout_version": 2}
 
     def bytes_e4m3(self) -> torch.Tensor:
-        """The E4M3 byte form of the weight, expanded on first use and kept (N * K bytes)."""
-        if self.w8 is None:
-            self.w8 = expand_w_e4m3(self)
-        return self.w8
+        """The E4M3 byte form of the weight, expanded on first use and kept (N * K bytes) for later calls on any
+        stream: the expansion has finished when it is kept, and one recorded in a graph belongs to that graph.
+        A copy: after w_packed is written again, or to release it, set w8 to None."""
+        if self.w8 is not None:
+            return self.w8
+        w8 = expand_w_e4m3(self)
+        with torch.cuda.device(w8.device):
+            if torch.cuda.is_current_stream_capturing():
+                return w8
+            torch.cuda.current_stream().synchronize()
+        self.w8 = w8
+        return w8
 
 
 def quant_w_int4(w: torch.Tensor, group: int = GROUP):

@@ -156,6 +156,27 @@ def test_bias_entry_takes_the_fp8_path_with_the_larger_scratch(M, room):
         assert bool((scratch[base:] == 0xA5).all())
 
 
+def test_kept_byte_form_is_complete_on_every_stream_and_no_part_of_a_graph():
+    N, K = 512, 1024
+    codes_w, _, pw = _weights(N, K, 21)
+    ops.expand_w_e4m3(pw)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        w8 = pw.bytes_e4m3()
+    assert pw.w8 is None  # nothing has run yet, and the memory is the graph's
+    graph.replay()
+    assert torch.equal(w8, _as_e4m3(codes_w))
+    side = torch.cuda.Stream()
+    busy = torch.randn(4096, 4096, device=DEV)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        for _ in range(20):
+            busy = busy @ busy * 1e-3
+        kept = pw.bytes_e4m3()
+    assert side.query()  # the expansion behind them is done: any stream may read it now
+    assert pw.w8 is kept and pw.bytes_e4m3() is kept and torch.equal(kept, _as_e4m3(codes_w))
+
+
 def test_decoder_linear_rows_do_not_depend_on_the_batch_they_arrive_in():
     """Per-token quantisation makes every output row a function of its input row alone, so a batch
     above the prefill threshold (FP8 path) must reproduce the rows of two batches below it."""
