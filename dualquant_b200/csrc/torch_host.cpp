@@ -652,11 +652,12 @@ PyObject* perm_forward(PyObject*, PyObject* const* v, Py_ssize_t n) {
     c10::SmallVector<int64_t, 5> sizes(x.sizes().begin(), x.sizes().end());
     sizes.back() = N;
     at::Tensor out = empty(sizes, p->out_dtype, idx);
-    // a bias of the output's type is added in the GEMM's epilogue, any other (or one that wants a gradient) by torch
+    // a bias of the output's type and width is added in the GEMM's epilogue, any other (or one that wants a gradient)
+    // by torch, which broadcasts it or says what is wrong with it
     const void* bias_ptr = nullptr;
     if (p->kind != PLAN_A16 && bias != Py_None) {
       const at::Tensor& b = tensor(bias, "bias");
-      if (b.scalar_type() == p->out_dtype && b.dim() == 1 && b.is_contiguous() && b.is_cuda() &&
+      if (b.scalar_type() == p->out_dtype && b.dim() == 1 && b.size(0) == N && b.is_contiguous() && b.is_cuda() &&
           b.get_device() == p->device && !(b.requires_grad() && at::GradMode::is_enabled())) {
         bias_ptr = b.data_ptr();
         bias = Py_None;

@@ -353,3 +353,21 @@ def test_one_layer_on_two_streams(name):
     torch.cuda.synchronize()
     for k, y in got:
         assert torch.equal(y, want[k])
+
+
+@pytest.mark.parametrize("name", ["rtn_int4", "nvfp4", "off"])
+def test_bias_of_another_width_is_torchs_to_add_or_refuse(name):
+    K, N = 512, 256
+    pl = _packed_layer(name, K, N)
+    x = synthetic.make_x(20, K, 47).to(DEV)
+    pl(x)
+    plain = pl(x)
+    one = torch.full((1,), 1.5, dtype=torch.bfloat16, device=DEV)
+    pl.layer.bias = nn.Parameter(one, requires_grad=False)
+    assert pl._plan is not None and torch.equal(pl(x), plain + one)
+    for width in (N - 1, N + 1, 2 * N):
+        pl.layer.bias = nn.Parameter(torch.zeros(width, dtype=torch.bfloat16, device=DEV), requires_grad=False)
+        with pytest.raises(RuntimeError):
+            pl(x)
+    pl.layer.bias = nn.Parameter(torch.full((N,), 1.5, dtype=torch.bfloat16, device=DEV), requires_grad=False)
+    assert torch.equal(pl(x), plain + one)
