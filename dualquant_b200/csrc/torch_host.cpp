@@ -53,7 +53,7 @@ uint64_t g_inited = 0;              // devices ensure_init has been called for
   X(kind) X(had_k) X(had_dim) X(scale) X(had_mat) X(w_packed) X(sw_t) X(N) X(K) X(group) X(codes)       \
   X(sf_atoms) X(tensor_scale) X(fmt) X(_plan) X(act_quant_enabled) X(online_full_had)                  \
   X(online_partial_had) X(had_K) X(act_fmt) X(quantize_bmm_input) X(dtype) X(_buffers) X(act_scale)    \
-  X(_modules) X(layer) X(_parameters) X(bias) X(_packed) X(_packed_fp4)
+  X(_modules) X(layer) X(_parameters) X(bias) X(_packed) X(_packed_fp4) X(name) X(block_size)
 #define DQ_DECLARE(n) PyObject* n = nullptr;
 struct Names {
   DQ_NAMES(DQ_DECLARE)
@@ -133,8 +133,9 @@ long attr_long(PyObject* o, PyObject* name) {
   Ref r(PyObject_GetAttr(o, name));
   return as_long(r.p);
 }
-const void* attr_ptr(PyObject* o, PyObject* name) {
+const void* attr_ptr(PyObject* o, PyObject* name, int* device = nullptr) {
   Ref r(PyObject_GetAttr(o, name));
+  if (device != nullptr) *device = static_cast<int>(tensor(r.p, "packed weight field").get_device());
   return ptr_or_null(r.p, "packed weight field");
 }
 
@@ -158,11 +159,11 @@ const dq_hadamard_desc* desc(const dq_hadamard_desc& d) { return d.kind == DQ_HA
 struct PackedInt4 {
   const uint8_t* w_packed;
   const void* sw_t;
-  int N, K, group;
+  int N, K, group, device;
 };
 PackedInt4 packed_int4(PyObject* o) {
   PackedInt4 w;
-  w.w_packed = static_cast<const uint8_t*>(attr_ptr(o, names.w_packed));
+  w.w_packed = static_cast<const uint8_t*>(attr_ptr(o, names.w_packed, &w.device));
   w.sw_t = attr_ptr(o, names.sw_t);
   w.N = static_cast<int>(attr_long(o, names.N));
   w.K = static_cast<int>(attr_long(o, names.K));
@@ -174,11 +175,11 @@ PackedInt4 packed_int4(PyObject* o) {
 struct PackedFp4 {
   const uint8_t *codes, *sf_atoms;
   const float* tensor_scale;
-  int N, K, fmt;
+  int N, K, fmt, device;
 };
 PackedFp4 packed_fp4(PyObject* o) {
   PackedFp4 w;
-  w.codes = static_cast<const uint8_t*>(attr_ptr(o, names.codes));
+  w.codes = static_cast<const uint8_t*>(attr_ptr(o, names.codes, &w.device));
   w.sf_atoms = static_cast<const uint8_t*>(attr_ptr(o, names.sf_atoms));
   w.tensor_scale = static_cast<const float*>(attr_ptr(o, names.tensor_scale));
   w.N = static_cast<int>(attr_long(o, names.N));
@@ -508,20 +509,20 @@ PyObject* linear_w4a4_fp4(PyObject*, PyObject* const* v, Py_ssize_t n) {
 
 // ------------------------------------------------------------------------------------ PermLinear.forward
 // A Plan is what PermLinear._make_plan found out about a module: which of the packed paths its forward takes
-// and the operands of that path.  perm_forward uses it as long as nothing it was derived from has been
+// and the objects of that path.  perm_forward uses it as long as nothing it was derived from has been
 // replaced since - it compares the objects themselves - and answers None otherwise; the Python forward then
-// does the work and makes a new plan.  The values of act_scale and bias are read from the live tensors.
+// does the work and makes a new plan.  No pointer and no value of a tensor is kept: the packed weight's fields,
+// act_scale, bias and the Hadamard factor are read by every call.
 enum PlanKind { PLAN_INT4 = 0, PLAN_FP4 = 1, PLAN_A16 = 2 };
 
 struct Plan {
   PyObject_HEAD
-  int kind, device, scale_mode;
+  int kind, scale_mode;
   PyObject *act_quant_enabled, *online_full_had, *online_partial_had, *had_K, *K, *had_dim, *act_fmt, *quantize_bmm_input,
       *dtype, *act_scale, *layer, *packed;  // owned; compared by identity
-  PyObject* had_mat;                        // owned: keeps the device copy of the factor alive (None: no factor)
-  dq_hadamard_desc had;
-  PackedInt4 w4;
-  PackedFp4 w_fp4;
+  PyObject *fmt_name, *fmt_block;           // owned: act_fmt's, which may be changed in place
+  PyObject* had_mat;                        // owned: the device copy of the factor (None: no factor)
+  dq_hadamard_desc had;                     // had_mat is filled in by each call
   at::ScalarType out_dtype;
 };
 
@@ -533,6 +534,7 @@ int plan_traverse(PyObject* self, visitproc visit, void* arg) {
   Plan* p = reinterpret_cast<Plan*>(self);
 #define DQ_VISIT(f) Py_VISIT(p->f);
   DQ_PLAN_OBJECTS(DQ_VISIT) DQ_VISIT(act_scale) DQ_VISIT(layer) DQ_VISIT(packed) DQ_VISIT(had_mat)
+  DQ_VISIT(fmt_name) DQ_VISIT(fmt_block)
 #undef DQ_VISIT
   return 0;
 }
@@ -540,6 +542,7 @@ int plan_clear(PyObject* self) {
   Plan* p = reinterpret_cast<Plan*>(self);
 #define DQ_CLEAR(f) Py_CLEAR(p->f);
   DQ_PLAN_OBJECTS(DQ_CLEAR) DQ_CLEAR(act_scale) DQ_CLEAR(layer) DQ_CLEAR(packed) DQ_CLEAR(had_mat)
+  DQ_CLEAR(fmt_name) DQ_CLEAR(fmt_block)
 #undef DQ_CLEAR
   return 0;
 }
@@ -589,20 +592,19 @@ PyObject* make_plan(PyObject*, PyObject* const* v, Py_ssize_t n) {
 #define DQ_KEEP(f) p->f = keep(m.get(names.f));
     DQ_PLAN_OBJECTS(DQ_KEEP)
 #undef DQ_KEEP
+    p->fmt_name = Py_NewRef(Ref(PyObject_GetAttr(p->act_fmt, names.name)).p);
+    p->fmt_block = Py_NewRef(Ref(PyObject_GetAttr(p->act_fmt, names.block_size)).p);
     p->act_scale = keep(m.in(names._buffers, names.act_scale));
     p->layer = keep(m.in(names._modules, names.layer));
     p->packed = keep(m.get(p->kind == PLAN_FP4 ? names._packed_fp4 : names._packed));
     if (p->had.had_mat != nullptr) {
+      p->had.had_mat = nullptr;
       p->had_mat = PyObject_GetAttr(v[2], names.had_mat);
       if (p->had_mat == nullptr) throw PyError();
     } else {
       Py_INCREF(Py_None);
       p->had_mat = Py_None;
     }
-    if (p->kind == PLAN_FP4) p->w_fp4 = packed_fp4(p->packed);
-    else p->w4 = packed_int4(p->packed);
-    Ref wt(PyObject_GetAttr(p->packed, p->kind == PLAN_FP4 ? names.codes : names.w_packed));
-    p->device = static_cast<int>(tensor(wt.p, "packed weight").get_device());
     Py_INCREF(obj.p);
     return obj.p;
   });
@@ -616,16 +618,25 @@ PyObject* perm_forward(PyObject*, PyObject* const* v, Py_ssize_t n) {
     const ModuleDict m(v[0]);
     PyObject* po = m.get(names._plan);
     if (po == nullptr || Py_TYPE(po) != &plan_type) Py_RETURN_NONE;
+    const Ref hold(Py_NewRef(po));  // another thread may replace the module's plan meanwhile
     Plan* p = reinterpret_cast<Plan*>(po);
 #define DQ_SAME(f) if (m.get(names.f) != p->f) Py_RETURN_NONE;
     DQ_PLAN_OBJECTS(DQ_SAME)
 #undef DQ_SAME
+    if (Ref(PyObject_GetAttr(p->act_fmt, names.name)).p != p->fmt_name ||
+        Ref(PyObject_GetAttr(p->act_fmt, names.block_size)).p != p->fmt_block)
+      Py_RETURN_NONE;
     if (m.in(names._buffers, names.act_scale) != p->act_scale || m.in(names._modules, names.layer) != p->layer ||
         m.get(p->kind == PLAN_FP4 ? names._packed_fp4 : names._packed) != p->packed)
       Py_RETURN_NONE;
     const at::Tensor& x = THPVariable_Unpack(v[1]);
-    const int K = p->kind == PLAN_FP4 ? p->w_fp4.K : p->w4.K, N = p->kind == PLAN_FP4 ? p->w_fp4.N : p->w4.N;
-    if (!x.is_cuda() || x.get_device() != p->device || x.scalar_type() != at::kBFloat16 || x.dim() < 1 ||
+    PackedInt4 w4 = {};
+    PackedFp4 w_fp4 = {};
+    if (p->kind == PLAN_FP4) w_fp4 = packed_fp4(p->packed);
+    else w4 = packed_int4(p->packed);
+    const int K = p->kind == PLAN_FP4 ? w_fp4.K : w4.K, N = p->kind == PLAN_FP4 ? w_fp4.N : w4.N;
+    const int device = p->kind == PLAN_FP4 ? w_fp4.device : w4.device;
+    if (!x.is_cuda() || x.get_device() != device || x.scalar_type() != at::kBFloat16 || x.dim() < 1 ||
         x.size(-1) != K || x.numel() == 0)
       Py_RETURN_NONE;
     int64_t ldx = K;
@@ -636,7 +647,7 @@ PyObject* perm_forward(PyObject*, PyObject* const* v, Py_ssize_t n) {
     const float* a = nullptr;
     if (p->act_scale != Py_None) {
       const at::Tensor& s = tensor(p->act_scale, "act_scale");
-      if (!s.is_cuda() || s.get_device() != p->device) Py_RETURN_NONE;
+      if (!s.is_cuda() || s.get_device() != device) Py_RETURN_NONE;
       a = static_cast<const float*>(s.data_ptr());
     }
     const ModuleDict layer(p->layer);
@@ -646,7 +657,7 @@ PyObject* perm_forward(PyObject*, PyObject* const* v, Py_ssize_t n) {
     const int M = static_cast<int>(x.numel() / K);
     int64_t need;
     if (p->kind == PLAN_INT4) need = int4_scratch_bytes(M, N, K);
-    else if (p->kind == PLAN_FP4) need = fp4_scratch_bytes(M, K, p->w_fp4.fmt);
+    else if (p->kind == PLAN_FP4) need = fp4_scratch_bytes(M, K, w_fp4.fmt);
     else need = static_cast<int64_t>(abi.dq_linear_a16w4_scratch_bytes(M, N, K));
     const Scratch scratch(std::max<int64_t>(need, 256));
     c10::SmallVector<int64_t, 5> sizes(x.sizes().begin(), x.sizes().end());
@@ -658,18 +669,20 @@ PyObject* perm_forward(PyObject*, PyObject* const* v, Py_ssize_t n) {
     if (p->kind != PLAN_A16 && bias != Py_None) {
       const at::Tensor& b = tensor(bias, "bias");
       if (b.scalar_type() == p->out_dtype && b.dim() == 1 && b.size(0) == N && b.is_contiguous() && b.is_cuda() &&
-          b.get_device() == p->device && !(b.requires_grad() && at::GradMode::is_enabled())) {
+          b.get_device() == device && !(b.requires_grad() && at::GradMode::is_enabled())) {
         bias_ptr = b.data_ptr();
         bias = Py_None;
       }
     }
     if (p->kind == PLAN_INT4) {
-      linear_int4(x.data_ptr(), ldx, a, desc(p->had), p->w4, nullptr, bias_ptr, M, out, p->scale_mode,
+      dq_hadamard_desc had = p->had;
+      had.had_mat = static_cast<const float*>(ptr_or_null(p->had_mat, "had_mat"));
+      linear_int4(x.data_ptr(), ldx, a, desc(had), w4, nullptr, bias_ptr, M, out, p->scale_mode,
                   scratch.mem.get(), scratch.bytes, idx);
     } else if (p->kind == PLAN_FP4) {
-      linear_fp4(x.data_ptr(), false, K, M, a, p->w_fp4, nullptr, bias_ptr, out, scratch, idx);
+      linear_fp4(x.data_ptr(), false, K, M, a, w_fp4, nullptr, bias_ptr, out, scratch, idx);
     } else {
-      check(abi.dq_linear_a16w4(x.data_ptr(), ldx, a, p->w4.w_packed, nullptr, M, N, K, p->w4.group, out.data_ptr(),
+      check(abi.dq_linear_a16w4(x.data_ptr(), ldx, a, w4.w_packed, nullptr, M, N, K, w4.group, out.data_ptr(),
                                 y_dtype_of(out), scratch.mem.get(), scratch.bytes, stream_of(idx)),
             "dq_linear_a16w4");
     }

@@ -371,3 +371,26 @@ def test_bias_of_another_width_is_torchs_to_add_or_refuse(name):
             pl(x)
     pl.layer.bias = nn.Parameter(torch.full((N,), 1.5, dtype=torch.bfloat16, device=DEV), requires_grad=False)
     assert torch.equal(pl(x), plain + one)
+
+
+@pytest.mark.parametrize("name", ["rtn_int4", "nvfp4", "off"])
+def test_replaced_fields_of_the_packed_weight_and_the_format_take_effect(name):
+    """The native forward keeps no pointer and no value: new tensors in the packed weight's fields, and a format changed
+    in place, count from the next call on."""
+    K, N = 512, 256
+    pl = _packed_layer(name, K, N)
+    x = synthetic.make_x(20, K, 48).to(DEV)
+    pl(x)
+    before = pl(x)
+    other = _packed_layer(name, K, N)
+    other.layer.weight.data = synthetic.make_w(N, K, 49).to(DEV)
+    other.pack_fp4(other._fp4_fmt(), force=True) if name == "nvfp4" else other.pack(force=True)
+    other.set_act_scale(pl.act_scale)
+    want = other(x)
+    mine, new = (pl._packed_fp4, other._packed_fp4) if name == "nvfp4" else (pl._packed, other._packed)
+    for f in ("codes", "sf_atoms", "tensor_scale") if name == "nvfp4" else ("w_packed", "sw_t"):
+        setattr(mine, f, None if getattr(new, f) is None else getattr(new, f).clone())
+    assert pl._plan is not None and torch.equal(pl(x), want) and not torch.equal(want, before)
+    if name == "rtn_int4":
+        pl.act_fmt.block_size = 128  # per group: no longer what the packed path computes
+        assert torch.equal(pl(x), pl._forward(x)) and not torch.equal(pl(x), want)
