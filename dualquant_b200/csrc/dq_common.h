@@ -137,11 +137,9 @@ int gemm_w4a4_int4_addend(const int8_t* codes, const float* sx, const uint8_t* w
                           Addend add, int M, int N, int K, int G, void* y, int y_dtype, void* stream);
 int quant_fp4_activations(const void* x, int x_is_f32, int64_t ldx, const float* a, int M, int K, int fmt, uint8_t* codes,
                           uint8_t* sf_atoms, float* row_scale, cudaStream_t s);
-// Estimated times of the packed-weight GEMM for 17 tokens and more, of the FP8-path GEMM, and of the expansion of a weight
-// in front of it (a launch and 1.5 bytes per weight: 4096 -> 4096 5.4 us, 14336 -> 4096 20, 4096 -> 28672 33).
+// Estimated times of the packed-weight GEMM for 17 tokens and more, and of the FP8-path GEMM.
 float gemm_int4_packed_us(int M, int N, int K, int sm_count);
 float gemm_int4_bytes_us(int M, int N, int K, int sm_count);
-inline float expand_w_us(int N, int K) { return 2.5f + 0.31e-6f * static_cast<float>(N) * static_cast<float>(K); }
 int gemv_pick_split(int tiles, int total_groups, int tok, int sm_count);
 int launch_gemv_int4(const int8_t* codes, const float* sx, const uint8_t* w_packed,
                      const void* sw_t, const float* r, int M, int N, int K, void* y, int y_dtype,

@@ -249,16 +249,6 @@ extern "C" int dq_gemm_w4a4_int4_e4m3_scatter(const uint8_t* x8, const float* sx
                                     static_cast<cudaStream_t>(stream), st, &sc);
 }
 
-// Under 256 tokens the packed weight is the cheaper one to read.  From 512 on the FP8-path GEMM wins everywhere; between,
-// it loses where K is long and the row tiles few, because it does not split K (294 x 14336 -> 1392: 38 us, the packed
-// kernel split four ways 29; 256 x 14336 -> 4096: 49 and 43): there the kernels' own estimates decide, packed by a tenth.
-extern "C" int dq_linear_w4a4_int4_byte_form_pays(int M, int N, int K) {
-  if (M < 256 || N < 1 || K < kGroup || K % kGroup != 0) return 0;
-  DeviceState* st = current_state();
-  if (M >= 512 || st == nullptr) return 1;
-  return gemm_int4_packed_us(M, N, K, st->sm_count) >= 0.9f * gemm_int4_bytes_us(M, N, K, st->sm_count) ? 1 : 0;
-}
-
 extern "C" int dq_expand_w_int4_e4m3(const uint8_t* w_packed, int N, int K, int G, uint8_t* w8, void* stream) {
   DeviceState* st = current_state();
   if (st == nullptr) return DQ_ERR_NOT_INIT;

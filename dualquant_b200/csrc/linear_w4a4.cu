@@ -16,20 +16,30 @@ extern "C" size_t dq_linear_w4a4_int4_scratch_bytes(int M, int N, int K) {
          round_up(static_cast<size_t>(M) * sizeof(float), 256);
 }
 
-// Whether a call does best to expand the weight and run on the FP8-path GEMM: from 1024 tokens on always (quantiser
-// included, 4096 -> 4096 43 us packed, 34 expanded; 14336 -> 1392, the narrowest measured, 80 and 78), from 256 where the
-// kernels' estimates and that of the expansion say so (768 tokens: 18944 -> 3584 157 and 129, 14336 -> 1392 51 and 68;
-// 512 tokens: 4096 -> 6144 44 and 36, 14336 -> 4096 73 and 91).  The estimate of the FP8-path GEMM, whose group times are
-// those of long runs at the power cap, is high for wide outputs (4096 -> 28672 at 768 tokens: 179 and 139, estimated
-// alike), hence the margin there.  Over 95 shapes of 256 to 1000 tokens the choice costs 0.3 % on average, 18 % at worst.
-static bool expansion_pays(int M, int N, int K) {
+// Whether a linear does best on the FP8-path GEMM with the weight's byte form, at extra_us for making it: never under 256
+// tokens, always from 1024, between by the GEMMs' estimates - the FP8-path GEMM does not split K and loses where K is long
+// and the row tiles few.  Its estimate, whose group times are those of long runs at the power cap, is high for wide outputs,
+// hence the margin there.  Microseconds with the quantiser; packed, byte form expanded by the call, byte form kept:
+//   4096 -> 4096     256 tokens  17  27  21    512 tokens  26  30  24     768 tokens   44   34   28    1024 tokens   43   34   29
+//   4096 -> 28672                80  87  52               132 117  86                 179  139  106                224  161  131
+//   14336 -> 4096                45  84  63                73  91  71                 121  100   81                140  111   92
+//   14336 -> 1392                29  58  51                46  64  57                  51   68   61                 80   78   69
+// Over 150 shapes of 256 to 1200 tokens the choice costs 0.4 % on average and 18 % at worst with a byte form expanded by the
+// call, 0.7 and 24 % with one kept.
+static bool byte_form_pays(int M, int N, int K, float extra_us) {
   if (M < 256 || N < 1 || K < dq::kGroup || K % dq::kGroup != 0) return false;
   if (M >= 1024) return true;
   const dq::DeviceState* st = dq::current_state();
   const int sms = st != nullptr ? st->sm_count : 148;  // (a size asked for before dq_init)
-  const float expanded = dq::gemm_int4_bytes_us(M, N, K, sms) + dq::expand_w_us(N, K);
-  return dq::gemm_int4_packed_us(M, N, K, sms) >= (M > 384 && N >= 6144 ? 0.75f : 1.0f) * expanded;
+  return dq::gemm_int4_packed_us(M, N, K, sms) >=
+         (M > 384 && N >= 6144 ? 0.75f : 1.0f) * (dq::gemm_int4_bytes_us(M, N, K, sms) + extra_us);
 }
+// The expansion is a launch and 1.5 bytes per weight: 4096 -> 4096 5.4 us, 14336 -> 4096 20, 4096 -> 28672 33.
+static bool expansion_pays(int M, int N, int K) {
+  return byte_form_pays(M, N, K, 2.5f + 0.31e-6f * static_cast<float>(N) * static_cast<float>(K));
+}
+
+extern "C" int dq_linear_w4a4_int4_byte_form_pays(int M, int N, int K) { return byte_form_pays(M, N, K, 0.f) ? 1 : 0; }
 
 extern "C" size_t dq_linear_w4a4_int4_prefill_scratch_bytes(int M, int N, int K) {
   const size_t base = dq_linear_w4a4_int4_scratch_bytes(M, N, K);

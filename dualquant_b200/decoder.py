@@ -67,10 +67,13 @@ class W4A4Linear:
         self.had = had
         self.N, self.K = N, K
 
-    # From this many tokens on the linears run on the FP8-path GEMM with the weight's byte form kept
-    # next to the 4-bit artefact (N * K bytes more per weight; same results bit for bit, faster on every
-    # linear of a layer).
+    # Batches under this size never run on the FP8-path GEMM
     PREFILL_TOKENS = 256
+
+    def byte_form_pays(self, M: int) -> bool:
+        """Whether M tokens run on the FP8-path GEMM with the weight's byte form, which is then kept next to the
+        4-bit artefact (N * K bytes more per weight; the library's rule for a weight whose byte form is kept)."""
+        return M >= self.PREFILL_TOKENS and bool(_lib.load().dq_linear_w4a4_int4_byte_form_pays(M, self.N, self.K))
 
     def _gemm(self, codes, sx, out_dtype=torch.bfloat16, residual=None):
         if codes.dtype == torch.uint8:
@@ -82,7 +85,7 @@ class W4A4Linear:
                out_dtype=torch.bfloat16) -> torch.Tensor:
         """RMSNorm(x) -> this linear, the norm fused into the activation quantiser."""
         codes, sx = ops.quant_act_int4_rmsnorm(x, norm_weight, eps, self.a, False,
-                                               e4m3=x.shape[0] >= self.PREFILL_TOKENS)
+                                               e4m3=self.byte_form_pays(x.shape[0]))
         return self._gemm(codes, sx, out_dtype)
 
     def __call__(self, x: torch.Tensor, out_dtype=torch.bfloat16, ar=None, residual=None) -> torch.Tensor:
@@ -91,7 +94,7 @@ class W4A4Linear:
         if ar is not None:
             codes, sx = ops.quant_act_int4(x, self.a, self.had, False)
             return ops.gemm_w4a4_int4_ar(codes, sx, self.pw, self.r, ar, out_dtype=out_dtype, residual=residual)
-        big = x.shape[0] >= self.PREFILL_TOKENS
+        big = self.byte_form_pays(x.shape[0])
         if residual is not None or big:
             codes, sx = ops.quant_act_int4(x, self.a, self.had, False, e4m3=big)
             return self._gemm(codes, sx, out_dtype, residual)
@@ -99,7 +102,7 @@ class W4A4Linear:
 
     def gated(self, gate: torch.Tensor, up: torch.Tensor, out_dtype=torch.bfloat16, ar=None,
               residual=None) -> torch.Tensor:
-        big = ar is None and gate.shape[0] >= self.PREFILL_TOKENS
+        big = ar is None and self.byte_form_pays(gate.shape[0])
         codes, sx = ops.quant_act_int4_gated(gate, up, self.a, self.had, False, e4m3=big)
         if ar is not None:
             return ops.gemm_w4a4_int4_ar(codes, sx, self.pw, self.r, ar, out_dtype=out_dtype, residual=residual)
@@ -345,7 +348,7 @@ class Decoder:
 
     def _peer_exchange(self, B: int, S: int) -> bool:
         return (self._token_sharded(B, S) and self.prefill_exchange == "peer" and
-                sharding.peer_exchange_fits(B * S, self.tp, self.cfg.hidden_size, W4A4Linear.PREFILL_TOKENS))
+                sharding.peer_exchange_fits(B * S, self.tp, self.cfg.hidden_size))
 
     def _prefill_body(self, ids: torch.Tensor) -> torch.Tensor:
         """The decoder layers of a prompt pass: kernels on the current stream only - no host
@@ -364,7 +367,8 @@ class Decoder:
         lo, hi = sharding.token_shard(T, self.tp, self.rank)
         Tq = hi - lo
         x = self.embed[ids.reshape(-1)[lo:hi]]
-        e4m3 = T >= W4A4Linear.PREFILL_TOKENS
+        # the gathered codes are the operand of both column-parallel linears
+        e4m3 = self.layers[0].qkv.byte_form_pays(T) and self.layers[0].gate_up.byte_form_pays(T)
         xc = None
         if self._peer_exchange(B, S):
             xc = self._exchange.get(Tq)

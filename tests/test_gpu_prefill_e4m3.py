@@ -199,6 +199,23 @@ def test_decoder_linear_rows_do_not_depend_on_the_batch_they_arrive_in():
     _lib.device_status(0)
 
 
+@pytest.mark.parametrize("M,N,K", [(255, 4096, 1024), (256, 4096, 1024), (700, 1392, 8192), (1023, 136, 4096), (1024, 136, 4096)])
+def test_decoder_linear_follows_the_weight_form_rule(M, N, K):
+    """A decoder linear makes and keeps the weight's byte form exactly where the library's rule says that it pays."""
+    lin = decoder.W4A4Linear(N, K, torch.device(DEV), torch.Generator(device=DEV).manual_seed(5), None)
+    x = synthetic.make_x(M, K, 14).to(DEV)
+    pays = bool(_lib.load().dq_linear_w4a4_int4_byte_form_pays(M, N, K))
+    assert pays == lin.byte_form_pays(M) and (pays or M < 1024) and not (pays and M < 256)
+    res = torch.zeros(M, N, dtype=torch.bfloat16, device=DEV)
+    y = lin(x, residual=res)
+    assert (lin.pw.w8 is not None) == pays
+    codes, sx = ops.quant_act_int4(x, lin.a, None, False)
+    ref = ops.gemm_w4a4_int4(codes, sx, lin.pw, lin.r, token_tile=1128, split_k=1, out_dtype=torch.bfloat16)
+    # unsplit and byte form: the same sums; split over K: a sum at a rounding boundary of bf16 may step
+    assert torch.equal(y, ref) if pays else ((y - ref).abs().max() / ref.abs().max()).item() < 2.0 ** -7
+    _lib.device_status(0)
+
+
 # ------------------------------------------------------------------------------------------
 # the exchange kernels of the token-sharded prompt pass, one rank at a time on one GPU: every
 # "peer" buffer is a local array, and no kernel waits for another
