@@ -139,13 +139,11 @@ template <int R, typename XT, int THREADS, int HS = 0>
 __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 3 : 1)
 act_quant_had_fast_kernel(const XT* __restrict__ x, const XT* __restrict__ up, int64_t ldx,
                           const float* __restrict__ a, int K,
-                          int S, int inner, int matrix, float had_scale,
-                          const float* __restrict__ had_mat, int8_t* __restrict__ codes,
+                          int S, int inner, int matrix, float had_scale, int8_t* __restrict__ codes,
                           float* __restrict__ sx, float* __restrict__ out, int mode, int scale_fp16) {
   extern __shared__ float sm_row[];
   __shared__ float red[THREADS / 32];
   float* row = sm_row;
-  float* hm = sm_row + K;
   grid_dep_launch_dependents();
   grid_dep_wait();
   const int P = K / S;
@@ -190,8 +188,6 @@ act_quant_had_fast_kernel(const XT* __restrict__ x, const XT* __restrict__ up, i
       }
     }
   }
-  (void)hm;
-  (void)had_mat;
   __syncthreads();
 
   if (inner) {
@@ -793,7 +789,7 @@ int launch_had_fast_t(const XT* x, const XT* up, int64_t ldx, const float* a, co
       const bool small_cta = dst != nullptr && M > 2 * dst->sm_count && smem <= 72 * 1024;
 #define DQ_HAD_FAST_T(RR, TT, HH)                                                                      \
   DQ_CHECK_CUDA(launch_pdl(act_quant_had_fast_kernel<RR, XT, TT, HH>, dim3(M), dim3(TT), smem, stream, x, up, \
-                           ldx, a, K, plan.S, plan.inner, plan.matrix, had->scale, had->had_mat, codes, sx,   \
+                           ldx, a, K, plan.S, plan.inner, plan.matrix, had->scale, codes, sx,   \
                            out, mode, scale_fp16))
 #define DQ_HAD_FAST(RR)                                            \
   if (plan.matrix && plan.S == 28 && RR >= 2) {                    \
