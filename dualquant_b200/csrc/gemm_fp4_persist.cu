@@ -116,7 +116,8 @@ gemm_fp4_persist_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_c
     tma_prefetch_desc(&tm_y);
   }
   // No early start for the kernel behind this one: the next quantiser's CTAs, resident and waiting during the K loop, cost
-  // more than the launch they hide (NVFP4 linears, us: 3294 x 4096 -> 11968 132 -> 121, 8192 x 3584 -> 18944 354 -> 327).
+  // more than the launch they hide (NVFP4 linears, us with / without: 3294 x 4096 -> 11968 131 / 126, 8192 x 3584 -> 18944
+  // 362 / 341, 8192 x 3584 -> 37888 667 / 616).
   tc_fence_before();
   __syncthreads();
   tc_fence_after();

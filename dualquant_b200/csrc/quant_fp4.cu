@@ -7,9 +7,10 @@
 //   NVFP4: ts = absmax_row / (6 * 448) (1 for a zero row), or a given per-tensor value;
 //          bs = e4m3(clamp(absmax_block / 6 / ts, 2^-6, 448));    q = e2m1(x32 / (ts * bs))
 // Element and scale conversions use the hardware converters (cvt.rn.satfinite.e2m1x2.f32 /
-// .e4m3x2.f32: round to nearest even, saturating), divisions are IEEE.  One CTA per row, the row
-// in registers, 8 consecutive elements per thread; a block spans 2 (NVFP4) or 4 (MXFP4) lanes.
-// HBM-bound: 2 bytes in, 0.5 byte + scale out per element.
+// .e4m3x2.f32: round to nearest even, saturating).  Codes and scale bytes are those of IEEE divisions; the quotients are
+// estimated with an approximate reciprocal, and only those near a rounding boundary are divided (nvfp4_scale_byte,
+// fp4_emit_vector).  One CTA per row, the row in registers, 8 consecutive elements per thread; a block spans 2 (NVFP4) or
+// 4 (MXFP4) lanes.  2 bytes in, 0.5 byte + scale out per element.
 #include "dq_common.h"
 #include "dq_ptx.cuh"
 
