@@ -348,7 +348,7 @@ def _kernel_class(M: int) -> str:
         return "gemm_w4a4_int4_tm_kernel<32> (tcgen05 kind::i8, weights via tensor memory)"
     if M <= 64:
         return "gemm_w4a4_int4_tm_kernel<64> (tcgen05 kind::i8, weights via tensor memory)"
-    return "gemm_w4a4_int4_kernel<128> (tcgen05 kind::i8, int8 weight tiles in shared memory)"
+    return "gemm_w4a4_int4_kernel<128> / gemm_w4a4_int4_tm_kernel<64> (tcgen05 kind::i8, by estimated cost)"
 
 
 def _traffic_table():
