@@ -366,3 +366,32 @@ def test_linear_picks_weight_form(M, N, K, dtype):
         assert bool((scratch[plain:] == 0xA5).all())
         tol = 1e-6 if dtype == torch.float32 else 2.0 ** -7  # (bf16: a sum at a rounding boundary steps)
         assert ((y.float() - ref.float()).abs().max() / ref.float().abs().max()).item() < tol
+
+
+@pytest.mark.parametrize("M,N", [(700, 4001), (400, 8000), (1100, 1001)])  # all expand the weight; odd N: direct stores
+@pytest.mark.parametrize("had,mode", [(h, m) for h in ("none", "full", "heads") for m in (dict(), dict(scale_fp16=True))]
+                         + [("none", dict(bf16_arith=True))])
+@pytest.mark.parametrize("extras", [False, True])
+def test_expanding_linear_equals_the_packed_kernel_over_its_options(M, N, had, mode, extras):
+    """The one-call linear that expands the weight against quantiser and unsplit packed GEMM: with a Hadamard, with each
+    scale mode, and (extras) with column and row scale, rows that have a gap between them, and fp32 output."""
+    K = 1792
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    pw = ops.pack_w_int4(*ops.quant_w_int4((torch.randn(N, K, generator=g, device=DEV) * 0.02).to(torch.bfloat16)))
+    assert ops.linear_scratch_bytes(M, N, K) > ops.linear_scratch_bytes(M, N, K, prefill=False)
+    x = torch.randn(M, K + 64, generator=g, device=DEV).to(torch.bfloat16)
+    x = x[:, :K] if extras else x[:, :K].contiguous()
+    h = None
+    if had == "full":
+        mat, order = quarot.get_hadK(K)
+        h = ops.Hadamard(_lib.HAD_FULL, order, 0, quarot.full_hadamard_scale(K), mat.to(DEV).contiguous())
+    elif had == "heads":
+        h = ops.Hadamard(_lib.HAD_PARTIAL, 1, 896, quarot.partial_hadamard_scale(2), None)
+    scaled = extras and "bf16_arith" not in mode
+    a = torch.rand(K, generator=g, device=DEV) + 0.5 if scaled else None
+    r = torch.rand(N, generator=g, device=DEV) + 0.5 if extras else None
+    dtype = torch.float32 if extras else torch.bfloat16
+    y = ops.linear_w4a4_int4(x, a, h, pw, r, out_dtype=dtype, **mode)
+    codes, sx = ops.quant_act_int4(x, a, h, **mode)
+    assert torch.equal(y, ops.gemm_w4a4_int4(codes, sx, pw, r, out_dtype=dtype, token_tile=1128, split_k=1))
+    _lib.device_status(0)
