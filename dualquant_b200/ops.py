@@ -116,6 +116,8 @@ def quant_pack_w_int4(w: torch.Tensor, group: int = GROUP) -> PackedInt4Weight:
     """pack_w_int4(*quant_w_int4(w)) in one pass over w (bf16, or fp32 rounded to bf16 on the way in)."""
     lib = _prep(w)
     w = (w if w.dtype in (torch.bfloat16, torch.float32) else w.to(torch.bfloat16)).contiguous()
+    if w.dtype == torch.float32 and w.data_ptr() % 16:  # a view at an odd offset: the kernel reads 16 bytes at a time
+        w = w.clone()
     N, K = w.shape
     w_packed = torch.empty(int(lib.dq_packed_w_bytes(N, K)), dtype=torch.uint8, device=w.device)
     sw_t = torch.empty((N + 127) // 128 * 128 * (K // group), dtype=torch.float16, device=w.device)

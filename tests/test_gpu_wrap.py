@@ -69,3 +69,18 @@ def test_install_from_wrap_matches_oracle():
     ref = oracle.epilogue(oracle.acc_int32(qx, codes), sw, None, sx)
     err = (y - ref).abs().max() / ref.abs().max()
     assert err < 8e-3, err  # bf16 output rounding of the module
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.float64])
+def test_pack_from_dualquant_takes_views_at_any_offset(dtype):
+    from dualquant_b200 import ops, wrap
+    N, K = 130, 256
+    flat = (torch.randn(3 + N * K, generator=torch.Generator().manual_seed(4)) * 0.02).to(dtype).cuda()
+    view = flat[3:].view(N, K)
+    want = ops.pack_w_int4(*ops.quant_w_int4(view.to(torch.bfloat16)))
+    got, _ = wrap.pack_from_dualquant(view)
+    assert torch.equal(got.w_packed, want.w_packed) and torch.equal(got.sw_t.view(torch.int16), want.sw_t.view(torch.int16))
+    wide = torch.zeros(N, K + 1, dtype=dtype, device="cuda")
+    wide[:, 1:] = view
+    assert torch.equal(wrap.pack_from_dualquant(wide[:, 1:])[0].w_packed, want.w_packed)
