@@ -119,9 +119,9 @@ struct Raw8<float> {
   }
 };
 
-__device__ __forceinline__ void emit8(const float* v, float s, int mode, int8_t* codes_row,
+__device__ __forceinline__ void emit8(const float* v, const TokenQuant& tq, int mode, int8_t* codes_row,
                                       float* out_row, int idx, int smode = 0) {
-  const float inv_s = __fdiv_rn(1.0f, s);
+  const float s = tq.s, inv_s = tq.inv_s;
   const bool e4m3 = (smode & kCodesE4M3) != 0;
   smode &= 0xFF;
   if (smode == 2 && mode != MODE_RAW) {
@@ -150,11 +150,7 @@ __device__ __forceinline__ void emit8(const float* v, float s, int mode, int8_t*
     return;
   }
   if (mode == MODE_CODES) {
-    float q[8];
-    quant_codes8(v, s, inv_s, q);
-    const uint32_t lo = e4m3 ? pack_codes4_e4m3(q[0], q[1], q[2], q[3]) : pack_codes4(q[0], q[1], q[2], q[3]);
-    const uint32_t hi = e4m3 ? pack_codes4_e4m3(q[4], q[5], q[6], q[7]) : pack_codes4(q[4], q[5], q[6], q[7]);
-    *reinterpret_cast<uint2*>(codes_row + idx) = make_uint2(lo, hi);
+    *reinterpret_cast<uint2*>(codes_row + idx) = quant_pack8(v, tq, e4m3);
   } else if (mode == MODE_FAKE_BF16) {
     float o[8];
     quant_codes8(v, s, inv_s, o);

@@ -307,11 +307,11 @@ act_quant_had_fast_kernel(const XT* __restrict__ x, const XT* __restrict__ up, i
     }
   }
   }
-  float s = 1.f;
+  TokenQuant tq = {1.f, 1.f, false};
   if (mode != MODE_RAW) {
     amax = block_max(amax, red, THREADS / 32);
-    s = token_scale(amax, scale_fp16);
-    if (threadIdx.x == 0 && sx != nullptr) sx[rr] = s;
+    tq = token_quant(amax, token_scale(amax, scale_fp16));
+    if (threadIdx.x == 0 && sx != nullptr) sx[rr] = tq.s;
   } else {
     __syncthreads();
   }
@@ -320,7 +320,7 @@ act_quant_had_fast_kernel(const XT* __restrict__ x, const XT* __restrict__ up, i
   for (int idx = threadIdx.x * 8; idx < K; idx += THREADS * 8) {
     float v[8];
     row_load8(row + idx, v);
-    emit8(v, s, mode, crow, orow, idx, scale_fp16);
+    emit8(v, tq, mode, crow, orow, idx, scale_fp16);
   }
 }
 
@@ -435,7 +435,7 @@ act_quant_had_cluster_kernel(const XT* __restrict__ x, const XT* __restrict__ up
     colv[i * PC + col] = acc;
     amax = fmaxf(amax, fabsf(acc));
   }
-  float s = 1.f;
+  TokenQuant tq = {1.f, 1.f, false};
   amax = block_max_once(amax, red, kHadClusterThreads / 32);  // (also orders the colv writes before their reads below)
   if (tid < kHadClusterCtas)
     dsmem_store_f32(dsmem_map(smem_u32(&pmax[rank]), static_cast<uint32_t>(tid)), amax);
@@ -444,8 +444,8 @@ act_quant_had_cluster_kernel(const XT* __restrict__ x, const XT* __restrict__ up
     float full = pmax[0];
 #pragma unroll
     for (int c = 1; c < kHadClusterCtas; ++c) full = fmaxf(full, pmax[c]);
-    s = token_scale(full, scale_fp16);
-    if (rank == 0 && tid == 0 && sx != nullptr) sx[rr] = s;
+    tq = token_quant(full, token_scale(full, scale_fp16));
+    if (rank == 0 && tid == 0 && sx != nullptr) sx[rr] = tq.s;
   }
   int8_t* crow = (codes != nullptr) ? codes + static_cast<int64_t>(rr) * K : nullptr;
   float* orow = out_row_ptr(out, rr, K, mode);
@@ -453,7 +453,7 @@ act_quant_had_cluster_kernel(const XT* __restrict__ x, const XT* __restrict__ up
     const int i = u / (PC / 8), piece = u - i * (PC / 8);
     float e8[8];
     row_load8(colv + i * PC + piece * 8, e8);
-    emit8(e8, s, mode, crow, orow, i * P + rank * PC + piece * 8, scale_fp16);
+    emit8(e8, tq, mode, crow, orow, i * P + rank * PC + piece * 8, scale_fp16);
   }
 }
 
@@ -592,21 +592,19 @@ act_quant_had_heads_kernel(const XT* __restrict__ x, int64_t ldx, const float* _
 #pragma unroll
       for (int i = 0; i < H::kWarps; ++i) amax = fmaxf(amax, red[buf][i]);
     }
-    const float s = token_scale(amax, scale_fp16);
-    if (warp == 0 && lane == 0 && sx != nullptr) sx[row] = s;
-    const float inv_s = __fdiv_rn(1.0f, s);
+    const TokenQuant tq = token_quant(amax, token_scale(amax, scale_fp16));
+    if (warp == 0 && lane == 0 && sx != nullptr) sx[row] = tq.s;
     int8_t* crow = codes + row * (S * 128) + at;
     constexpr int kQ = 8 / C;  // heads per eight values
 #pragma unroll
     for (int j = 0; j < HL; j += kQ) {
-      float in[8], q[8];
+      float in[8];
 #pragma unroll
       for (int e = 0; e < 8; ++e) in[e] = v[j + e / C][e % C];
-      quant_codes8(in, s, inv_s, q);
+      const uint2 packed = quant_pack8(in, tq, E4M3);
 #pragma unroll
       for (int p = 0; p < 8; p += 4) {
-        const uint32_t w = E4M3 ? pack_codes4_e4m3(q[p], q[p + 1], q[p + 2], q[p + 3])
-                                : pack_codes4(q[p], q[p + 1], q[p + 2], q[p + 3]);
+        const uint32_t w = p == 0 ? packed.x : packed.y;
         if constexpr (C == 4) {
           *reinterpret_cast<uint32_t*>(crow + (j + p / 4) * 128) = w;
         } else {

@@ -358,6 +358,31 @@ def test_gated_quantiser_matches_bf16_silu_mul():
         assert torch.allclose(sxg.cpu(), sx, rtol=2e-3)
 
 
+# A row whose scale cannot bring its codes into range without the clamp (fp16 scale: overflow to 65504, subnormal, zero),
+# rows with infinities and NaN, a row of exact halves: all against the oracle's division, rounding and clamp.
+@pytest.mark.parametrize("K", [1024, 4096])
+@pytest.mark.parametrize("M", [1, 1030])
+def test_act_quant_extreme_rows(M, K):
+    x = synthetic.make_x(max(M, 8), K, 3).float()
+    x[0] *= 3e7
+    if M > 1:
+        x[1] *= 1e-8
+        x[2] *= 1e-38
+        x[3] = (torch.arange(K) % 29 - 14).float() / 2
+        x[4, 5] = float("inf")
+        x[5, 7] = float("nan")
+    x = x[:M].to(torch.bfloat16)
+    a = torch.ones(K)
+    for fp16 in (False, True):
+        qx, sx, _ = O.quant_act_int4(x, a, None, fp16)
+        codes, sxg = ops.quant_act_int4(x.to(DEV), a.to(DEV), None, fp16)
+        rows = [r for r in range(M) if r not in (4, 5)]
+        assert torch.equal(codes.cpu()[rows], qx[rows]) and torch.equal(sxg.cpu()[rows], sx[rows])
+        x8, _ = ops.quant_act_int4(x.to(DEV), a.to(DEV), None, fp16, e4m3=True)
+        assert torch.equal(x8, ops.codes_to_e4m3(codes))
+    _status_ok()
+
+
 # ------------------------------------------------------------------------------------------
 # RMSNorm fused into the quantiser
 # ------------------------------------------------------------------------------------------
