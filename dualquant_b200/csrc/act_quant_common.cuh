@@ -80,14 +80,29 @@ __device__ __forceinline__ float silu_mul_bf16(float g, float u) {
   const float sgb = __bfloat162float(__float2bfloat16_rn(sg));
   return __bfloat162float(__float2bfloat16_rn(__fmul_rn(sgb, u)));
 }
-template <typename XT>
-__device__ __forceinline__ void apply_gate(const XT* up_ptr, float* v) {
-  if (up_ptr != nullptr) {
-    float u[8];
-    load8(up_ptr, u);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] = silu_mul_bf16(v[e], u[e]);
-  }
+// The same for two bf16 pairs (gate and up as loaded): SiLU as g / (1 + 2^(-g log2 e)) with the hardware's exponential and
+// reciprocal, two elements to an instruction, and the product as one bf16 multiplication (one rounding, like the fp32
+// product's).  A bf16 gate has 65536 values, and this form gives the bf16 result of the one above for each of them (tested);
+// the factors 1/4 keep the reciprocal a normal number where 1 + e^-g nears the end of the range.  With expf and an
+// IEEE division 8192 gated rows of 14336 took 406 us, with this 307.
+__device__ __forceinline__ uint32_t silu_mul_bf16x2(uint32_t g2, uint32_t u2) {
+  const float2 g = make_float2(__uint_as_float(g2 << 16), __uint_as_float(g2 & 0xFFFF0000u));
+  float2 t = __fmul2_rn(g, make_float2(-1.4426950408889634f, -1.4426950408889634f));
+  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(t.x));
+  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(t.y));
+  float2 r = __ffma2_rn(t, make_float2(0.25f, 0.25f), make_float2(0.25f, 0.25f));
+  asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(r.x));
+  asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(r.y));
+  const float2 s = __fmul2_rn(__fmul2_rn(g, make_float2(0.25f, 0.25f)), r);
+  uint32_t out;
+  asm("{\n"
+      ".reg .b32 s;\n"
+      "cvt.rn.bf16x2.f32 s, %2, %1;\n"
+      "mul.rn.bf16x2 %0, s, %3;\n"
+      "}\n"
+      : "=r"(out)
+      : "f"(s.x), "f"(s.y), "r"(u2));
+  return out;
 }
 
 // Eight input elements as loaded (bf16: one 16-byte vector; fp32: two).
@@ -118,6 +133,33 @@ struct Raw8<float> {
     v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
   }
 };
+
+// Eight values of SiLU(gate) * up.
+__device__ __forceinline__ void gated8(const Raw8<__nv_bfloat16>& g, const Raw8<__nv_bfloat16>& u, float* v) {
+  Raw8<__nv_bfloat16> h;
+  h.r = make_uint4(silu_mul_bf16x2(g.r.x, u.r.x), silu_mul_bf16x2(g.r.y, u.r.y), silu_mul_bf16x2(g.r.z, u.r.z),
+                   silu_mul_bf16x2(g.r.w, u.r.w));
+  h.expand(v);
+}
+__device__ __forceinline__ void gated8(const Raw8<float>& g, const Raw8<float>& u, float* v) {
+  float uv[8];
+  g.expand(v);
+  u.expand(uv);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) v[e] = silu_mul_bf16(v[e], uv[e]);
+}
+// Eight values of a row, SiLU(gate) * up where there is an up row.
+template <typename XT>
+__device__ __forceinline__ void load_gated8(const XT* x, const XT* up, float* v) {
+  Raw8<XT> xw, uw;
+  xw.load(x);
+  if (up != nullptr) {
+    uw.load(up);
+    gated8(xw, uw, v);
+  } else {
+    xw.expand(v);
+  }
+}
 
 __device__ __forceinline__ void emit8(const float* v, const TokenQuant& tq, int mode, int8_t* codes_row,
                                       float* out_row, int idx, int smode = 0) {

@@ -170,13 +170,8 @@ act_quant_had_fast_kernel(const XT* __restrict__ x, const XT* __restrict__ up, i
       const int idx = base + i * THREADS * 8;
       if (idx < K) {
         float v[8];
-        xw[i].expand(v);
-        if (ur != nullptr) {
-          float u[8];
-          uw[i].expand(u);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) v[e] = silu_mul_bf16(v[e], u[e]);
-        }
+        if (ur != nullptr) gated8(xw[i], uw[i], v);
+        else xw[i].expand(v);
         if (a != nullptr) {
           float av[8];
           load8(a + idx, av);
@@ -382,13 +377,8 @@ act_quant_had_cluster_kernel(const XT* __restrict__ x, const XT* __restrict__ up
     xw.load(xr + idx);
     if (ur != nullptr) uw.load(ur + idx);
     if (ar != nullptr) load8(ar + idx, av);
-    xw.expand(v);
-    if (ur != nullptr) {
-      float u8[8];
-      uw.expand(u8);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) v[e] = silu_mul_bf16(v[e], u8[e]);
-    }
+    if (ur != nullptr) gated8(xw, uw, v);
+    else xw.expand(v);
     if (ar != nullptr) {
 #pragma unroll
       for (int e = 0; e < 8; ++e) v[e] = __fmul_rn(v[e], av[e]);

@@ -176,8 +176,7 @@ act_quant_had_kernel(const XT* __restrict__ x, const XT* __restrict__ up, int64_
 
   for (int idx = threadIdx.x * 8; idx < K; idx += THREADS * 8) {
     float v[8];
-    load8(xr + idx, v);
-    apply_gate(ur != nullptr ? ur + idx : nullptr, v);
+    load_gated8(xr + idx, ur != nullptr ? ur + idx : nullptr, v);
     if (a != nullptr) {
       float av[8];
       load8(a + idx, av);
@@ -273,8 +272,7 @@ act_quant_had_big_kernel(const XT* __restrict__ x, const XT* __restrict__ up, in
   const XT* ur = (up != nullptr) ? up + static_cast<int64_t>(r) * ldx : nullptr;
   for (int idx = threadIdx.x * 8; idx < K; idx += THREADS * 8) {
     float v[8];
-    load8(xr + idx, v);
-    apply_gate(ur != nullptr ? ur + idx : nullptr, v);
+    load_gated8(xr + idx, ur != nullptr ? ur + idx : nullptr, v);
     if (a != nullptr) {
       float av[8];
       load8(a + idx, av);

@@ -358,6 +358,24 @@ def test_gated_quantiser_matches_bf16_silu_mul():
         assert torch.allclose(sxg.cpu(), sx, rtol=2e-3)
 
 
+def test_gated_quantiser_every_gate_value():
+    """One row per finite bf16 gate value, eight times the same element: the row's scale is |SiLU(gate) * up| / 7 and its
+    codes carry the sign.  fp32 SiLU by torch's division and exponential, rounded to bf16, times up, rounded to bf16."""
+    gate = torch.arange(65536, dtype=torch.int32, device=DEV).to(torch.int16).view(torch.bfloat16)
+    gate = gate[torch.isfinite(gate.float())]
+    g = torch.Generator(device=DEV).manual_seed(5)
+    up = (torch.rand(gate.numel(), generator=g, device=DEV) + 0.5).to(torch.bfloat16)
+    g32 = gate.float()
+    h = (g32 / (1.0 + torch.exp(-g32))).to(torch.bfloat16) * up
+    codes, sx = ops.quant_act_int4_gated(gate.repeat_interleave(8).view(-1, 8), up.repeat_interleave(8).view(-1, 8))
+    h32 = h.float().cpu()  # (on the GPU torch divides by a constant through its reciprocal)
+    assert torch.equal(sx.cpu(), torch.where(h32 == 0, torch.ones_like(h32), h32.abs() / 7.0))
+    # (a subnormal product: absmax / 7 loses bits, its codes are no longer +-7; an infinite one has no codes)
+    normal = (h32.abs() > 1e-30) & torch.isfinite(h32)
+    assert torch.equal(codes.cpu()[normal], (7 * torch.sign(h32[normal])).to(torch.int8).unsqueeze(1).expand(-1, 8))
+    _status_ok()
+
+
 # A row whose scale cannot bring its codes into range without the clamp (fp16 scale: overflow to 65504, subnormal, zero),
 # rows with infinities and NaN, a row of exact halves: all against the oracle's division, rounding and clamp.
 @pytest.mark.parametrize("K", [1024, 4096])
