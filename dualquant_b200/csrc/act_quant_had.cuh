@@ -4,6 +4,7 @@
 // launches its own kernels, so the copies never have to agree.
 #pragma once
 #include "act_quant_common.cuh"
+#include "act_quant_had28.cuh"
 
 namespace dq {
 namespace {
@@ -133,8 +134,8 @@ __device__ __forceinline__ void matrix_rows_dispatch(int qi, const float2* v, fl
 // THREADS = 512: one CTA per SM, the shortest time per row (decode batches, one row per SM at most).
 // THREADS = 256: three CTAs per SM; with many rows one row's load, barrier and store phases overlap
 // another row's arithmetic (two CTAs per SM with more registers each measured 30 % slower).
-// HS: order of the +-1 factor when it is one of the common ones (28: 14336 = 28 * 512 and
-// 28672 = 28 * 1024), so that the matrix stage has no padded terms; 0 = any order up to 32.
+// HS: order of the +-1 factor where it is known (28 for 28672 = 28 * 1024; shorter rows of that order have a kernel of their
+// own, act_quant_had28.cuh), so that the matrix stage has no padded terms; 0 = any order up to 32.
 template <int R, typename XT, int THREADS, int HS = 0>
 __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 3 : 1)
 act_quant_had_fast_kernel(const XT* __restrict__ x, const XT* __restrict__ up, int64_t ldx,
@@ -681,21 +682,20 @@ int init_had_fast_t() {
                              cudaFuncAttributeMaxDynamicSharedMemorySize, kHadMaxSmem);
   DQ_HAD_ATTR(1) DQ_HAD_ATTR(2) DQ_HAD_ATTR(4) DQ_HAD_ATTR(8) DQ_HAD_ATTR(16) DQ_HAD_ATTR(32)
 #undef DQ_HAD_ATTR
-#define DQ_HAD_ATTR28(R)                                                                      \
-  if (e == cudaSuccess)                                                                       \
-    e = cudaFuncSetAttribute(act_quant_had_fast_kernel<R, XT, 512, 28>,                         \
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, kHadMaxSmem);        \
-  if (e == cudaSuccess)                                                                       \
-    e = cudaFuncSetAttribute(act_quant_had_fast_kernel<R, XT, 256, 28>,                         \
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, kHadMaxSmem);
-  DQ_HAD_ATTR28(2) DQ_HAD_ATTR28(4) DQ_HAD_ATTR28(8) DQ_HAD_ATTR28(16) DQ_HAD_ATTR28(32)
-#undef DQ_HAD_ATTR28
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(act_quant_had_fast_kernel<32, XT, 512, 28>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kHadMaxSmem);
 #define DQ_HAD_ATTRC(R)                                                                       \
   if (e == cudaSuccess)                                                                       \
     e = cudaFuncSetAttribute(act_quant_had_cluster_kernel<R, XT>,                               \
                              cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
   DQ_HAD_ATTRC(4) DQ_HAD_ATTRC(8) DQ_HAD_ATTRC(16) DQ_HAD_ATTRC(32)
 #undef DQ_HAD_ATTRC
+#define DQ_HAD_ATTR_28(P)                                                                     \
+  if (e == cudaSuccess)                                                                       \
+    e = cudaFuncSetAttribute(act_quant_had28_kernel<P, XT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Had28<P>::kSmem);
+  DQ_HAD_ATTR_28(64) DQ_HAD_ATTR_28(128) DQ_HAD_ATTR_28(256) DQ_HAD_ATTR_28(512)
+#undef DQ_HAD_ATTR_28
   if (e != cudaSuccess)
     return set_error(DQ_ERR_CUDA, "cudaFuncSetAttribute(act_quant_had fast) failed: %s", cudaGetErrorString(e));
   return DQ_OK;
@@ -768,6 +768,22 @@ int launch_had_fast_t(const XT* x, const XT* up, int64_t ldx, const float* a, co
 #undef DQ_HAD_CLUSTER
         return DQ_OK;
       }
+      // 28 * 64 ... 28 * 512 values and more rows than the cluster kernel takes (28 * 64: any number): from the first row on
+      // it is the faster one (14336, us: 65 rows 14.7 -> 8.1, 300 rows 22.9 -> 15.0; 1792: 70 rows 9.3 -> 7.3)
+      if (plan.matrix && plan.inner && plan.S == 28 && plan.R >= 2 && plan.R <= 16) {
+#define DQ_HAD28(P)                                                                                                    \
+  DQ_CHECK_CUDA(launch_pdl(act_quant_had28_kernel<P, XT>, dim3((M + Had28<P>::kRows - 1) / Had28<P>::kRows),           \
+                           dim3(kHad28Threads), Had28<P>::kSmem, stream, x, up, ldx, a, M, had->scale, had->had_mat,   \
+                           codes, sx, out, mode, scale_fp16))
+        switch (plan.R) {
+          case 2: DQ_HAD28(64); break;
+          case 4: DQ_HAD28(128); break;
+          case 8: DQ_HAD28(256); break;
+          default: DQ_HAD28(512); break;
+        }
+#undef DQ_HAD28
+        return DQ_OK;
+      }
       if (plan.matrix) {
         int rc2 = upload_had_matrix(had->had_mat, plan.S, stream);
         if (rc2 != DQ_OK) return rc2;
@@ -780,10 +796,7 @@ int launch_had_fast_t(const XT* x, const XT* up, int64_t ldx, const float* a, co
                            ldx, a, K, plan.S, plan.inner, plan.matrix, had->scale, codes, sx,   \
                            out, mode, scale_fp16))
 #define DQ_HAD_FAST(RR)                                            \
-  if (plan.matrix && plan.S == 28 && RR >= 2) {                    \
-    if (small_cta) DQ_HAD_FAST_T(RR, 256, 28);                     \
-    else DQ_HAD_FAST_T(RR, 512, 28);                               \
-  } else if (small_cta) {                                          \
+  if (small_cta) {                                                 \
     DQ_HAD_FAST_T(RR, 256, 0);                                     \
   } else {                                                         \
     DQ_HAD_FAST_T(RR, 512, 0);                                     \
@@ -794,7 +807,10 @@ int launch_had_fast_t(const XT* x, const XT* up, int64_t ldx, const float* a, co
         case 4: DQ_HAD_FAST(4); break;
         case 8: DQ_HAD_FAST(8); break;
         case 16: DQ_HAD_FAST(16); break;
-        default: DQ_HAD_FAST(32); break;
+        default:
+          if (plan.matrix && plan.S == 28) DQ_HAD_FAST_T(32, 512, 28);
+          else DQ_HAD_FAST(32);
+          break;
       }
 #undef DQ_HAD_FAST
 #undef DQ_HAD_FAST_T

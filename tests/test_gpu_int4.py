@@ -154,6 +154,28 @@ def test_full_hadamard_many_rows_bit_exact(M, K):
     _status_ok()
 
 
+# 28 * 64 ... 28 * 512 values with a factor other than the table's (its transpose with some columns negated): coefficients
+# from the caller's matrix instead of the compiled-in signs; 1 and 9 rows: the last CTA of eight rows is not full.
+@pytest.mark.parametrize("M,K", [(1, 1792), (9, 1792), (67, 3584), (65, 7168), (66, 14336)])
+@pytest.mark.parametrize("table", [True, False])
+def test_hadamard28_factor_of_the_caller(M, K, table):
+    had, k = O.get_hadK(K)
+    if not table:
+        had = had.T.contiguous()
+        had[:, 3::5] *= -1
+    hd = ops.Hadamard(_lib.HAD_FULL, k, 0, O.full_hadamard_scale(K), had.to(DEV))
+    xb = synthetic.make_x(M, K, 17)
+    got = ops.hadamard_f32(xb.float().to(DEV), hd)
+    assert torch.equal(got.cpu(), O.hadamard_full(xb.float(), had, k))
+    _, c = synthetic.make_scales(8, K, 17)
+    qx, sx, _ = O.quant_act_int4(xb, 1.0 / c, ("full", had, k), True)
+    codes, sxg = ops.quant_act_int4(xb.to(DEV), (1.0 / c).to(DEV), hd, True)
+    assert torch.equal(codes.cpu(), qx) and torch.equal(sxg.cpu(), sx)
+    x8, _ = ops.quant_act_int4(xb.float().to(DEV), (1.0 / c).to(DEV), hd, True, e4m3=True)
+    assert torch.equal(x8, ops.codes_to_e4m3(codes))
+    _status_ok()
+
+
 @pytest.mark.parametrize("K,d", [(4096, 128), (256, 8), (1024, 64), (8192, 128)])
 def test_partial_hadamard_bit_exact(K, d):
     M = 5
