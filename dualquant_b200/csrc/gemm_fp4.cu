@@ -128,9 +128,9 @@ gemm_fp4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     const uint8_t* sfw_tile = sfw + (static_cast<size_t>(n0 / kFBN) * total_st + st_begin) * kSfBytes;
     const uint8_t* sfx_tile = sfx + (static_cast<size_t>(t0 / kFTN) * total_st + st_begin) * kSfBytes;
     const size_t sfx_block = static_cast<size_t>(total_st) * kSfBytes;  // next token block of 128
-    // Only lane 0 works; the other lanes go straight to the end of the role (32 lanes polling a
+    // Only one lane works; the other lanes go straight to the end of the role (32 lanes polling a
     // barrier cost issue slots and barrier-unit bandwidth that the other warps need).
-    if (lane == 0) {
+    if (elect_one()) {
       auto load_w = [&](int i, int s) {
         // the activation box is the CTA's whole token tile (rows past M arrive as zeros and count)
         mbar_expect_tx(&full[s], kFTileBytes + C::kBTileBytes + (1 + nblk) * kSfBytes);
@@ -155,7 +155,7 @@ gemm_fp4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ UMMA issuer
-    if (lane == 0) {  // only lane 0 works (see the producer)
+    if (elect_one()) {  // only one lane works (see the producer)
       for (int i = 0; i < nst; ++i) {
         const int s = i % kFStages;
         // operands landed (full) and their scale factors copied into tensor memory (sf_ready)
@@ -194,7 +194,7 @@ gemm_fp4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     // latency each, took that one thread several times the 271 cycles the UMMAs need to execute.
     // The stage's columns are free again once its previous UMMAs have finished, which the
     // producer has already waited for before refilling the stage (full implies it).
-    if (lane == 0) {
+    if (elect_one()) {
       const bool is_b = (warp == 7);
       const int sf_off = is_b ? C::kOffSFB : C::kOffSFA;
       for (int i = 0; i < nst; ++i) {

@@ -125,7 +125,7 @@ gemm_fp4_persist_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_c
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       const uint64_t pol = l2_policy_evict_last();
       grid_dep_wait();  // the activation codes and scale factors come from the kernel before this one
       int gi = 0;
@@ -153,7 +153,7 @@ gemm_fp4_persist_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_c
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ UMMA issue
-    if (lane == 0) {
+    if (elect_one()) {
       int gi = 0;
       bool ok = true;
       for (int it = 0; it < my_tiles && ok; ++it) {
@@ -187,7 +187,7 @@ gemm_fp4_persist_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_c
   } else if (warp < 4) {
     // ------------------------------------------------------------------ scale-factor copiers
     // warp 2: weight scale factors and those of activation rows 0-127; warp 3: activation rows 128-255
-    if (lane == 0) {
+    if (elect_one()) {
       const bool second = (warp == 3);
       int gi = 0;
       bool ok = true;

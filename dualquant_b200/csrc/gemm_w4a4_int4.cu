@@ -386,9 +386,9 @@ gemm_w4a4_int4_kernel(const uint8_t* __restrict__ w_packed,
     // activation stages, up to SX stages of XC groups ahead of the UMMAs.
     const uint64_t pol_w = w_stream_once ? l2_policy_evict_first() : l2_policy_evict_last();
     const uint64_t pol_x = l2_policy_evict_last();
-    // Only lane 0 works; the other lanes go straight to the end of the role (a waiting warp of
+    // Only one lane works; the other lanes go straight to the end of the role (a waiting warp of
     // 32 polling lanes costs the SM issue slots and barrier-unit bandwidth the other roles need).
-    if (lane == 0) {
+    if (elect_one()) {
       const int pre = (my_groups < C::SP) ? my_groups : C::SP;
       for (int gi = 0; gi < pre; ++gi) {
         mbar_expect_tx(&full_p[gi], kWpBytes);
@@ -417,7 +417,7 @@ gemm_w4a4_int4_kernel(const uint8_t* __restrict__ w_packed,
     const uint32_t x_base = smem_u32(smem + C::kOffX);
     // The (global) groups alternate between the two issuing warps; accumulator b, buffer b and
     // the activation stage of a group are always waited for and released by the same warp.
-    if (lane == 0) {  // only lane 0 works (see the producer)
+    if (elect_one()) {  // only one lane works (see the producer)
       for (int gi = warp - C::kIssuerWarp0; gi < my_groups; gi += C::kIssuers) {
         const int it = gi / ng, i = gi % ng;  // tile iteration, group inside the tile
         const int b = gi % C::NB;

@@ -424,7 +424,7 @@ gemm_w4a4_e4m3_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
     setmaxnreg_dec<kAuxRegs>();
     if (warp == kProducerWarp) {
       // ---------------------------------------------------------------- TMA producer (both CTAs)
-      if (lane == 0) {
+      if (elect_one()) {
         const uint64_t pol = l2_policy_evict_last();
         const uint32_t full_addr = dsmem_map(smem_u32(full), 0);  // the even CTA's
         grid_dep_wait();  // operands may come from the kernels just before this one
@@ -446,7 +446,7 @@ gemm_w4a4_e4m3_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
       }
     } else if (warp >= kIssuerWarp && warp < kIssuerWarp + kIssuers && rank == 0) {
       // ---------------------------------------------------------------- UMMA issue, for both CTAs
-      if (lane == 0 && live) {
+      if (elect_one() && live) {
         constexpr uint32_t idesc = idesc_e4m3(2 * kBN, kTN);
         const int my_groups = my_tiles * ng;
         for (int gi = warp - kIssuerWarp; gi < my_groups; gi += kIssuers) {

@@ -423,9 +423,9 @@ gemm_w4a4_int4_tm_kernel(const uint8_t* __restrict__ w_packed,
                    w_tile + static_cast<size_t>(g_begin + s * kStepGroups) * kTileBytes, bytes,
                    &full_w[sp], pol_w);
     };
-    // Only lane 0 works; the other lanes go straight to the end of the role (a waiting warp of
+    // Only one lane works; the other lanes go straight to the end of the role (a waiting warp of
     // 32 polling lanes costs the SM issue slots and barrier-unit bandwidth the other roles need).
-    if (lane == 0) {
+    if (elect_one()) {
       const int pre = (ns < C::SP) ? ns : C::SP;
       for (int s = 0; s < pre; ++s) issue_w(s);
       grid_dep_wait();
@@ -450,11 +450,10 @@ gemm_w4a4_int4_tm_kernel(const uint8_t* __restrict__ w_packed,
     }
   } else if (warp == C::kIssuerWarp) {
     // ------------------------------------------------------------------ UMMA issuer
-    // Whole warp waits (uniform control flow); lane 0 issues tcgen05.mma / tcgen05.commit.
     constexpr uint32_t idesc = umma_idesc_i8(kBN, TN);
     const uint32_t x_base = smem_u32(smem + C::kOffX);
-    // Only lane 0 works (see the producer).
-    if (lane == 0) {
+    // Only one lane works (see the producer).
+    if (elect_one()) {
       bool ok = true;
       for (int s = 0; s < ns && ok; ++s) {
         const int ab = s % C::NA, sxi = s % C::SX;
