@@ -50,6 +50,8 @@ int make_tmap_2d_u8(CUtensorMap* out, const void* base, uint64_t row_bytes, uint
 // 2-D row-major fp32 / bf16 output matrix for tiled bulk stores (no swizzle).
 int make_tmap_2d_out(CUtensorMap* out, const void* base, int elem_bytes, uint64_t cols, uint64_t rows,
                      uint32_t box_cols, uint32_t box_rows);
+int make_tmap_sf_atoms(CUtensorMap* out, const void* base, int tile_atoms, int tiles, uint32_t box_atoms,
+                       uint32_t box_tiles);
 int make_tmap_x_groups(CUtensorMap* out, const void* base, uint64_t row_bytes, uint64_t rows,
                        uint32_t box_rows, uint32_t box_groups);
 
@@ -115,7 +117,7 @@ int init_gemm_int4_f8_kernels();
 int init_gemm_fp4_persist_kernels();
 int launch_gemm_fp4_persist(const uint8_t* x_codes, const uint8_t* x_sf_atoms, const float* x_scale,
                             const uint8_t* w_codes, const uint8_t* w_sf_atoms, const float* w_scale, const float* r,
-                            const void* bias, int M, int N, int K, int nvfp4, void* y, int y_dtype, int row_tiles, cudaStream_t stream,
+                            const void* bias, int M, int N, int K, int nvfp4, void* y, int y_dtype, cudaStream_t stream,
                             DeviceState* st);
 int launch_gemm_int4_e4m3(const uint8_t* x8, const float* sx, const uint8_t* w8, const void* sw_t, const float* r,
                           int M, int N, int K, void* y, int y_dtype, Addend add, cudaStream_t stream,

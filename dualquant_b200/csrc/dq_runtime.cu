@@ -82,6 +82,24 @@ int make_tmap_2d_out(CUtensorMap* out, const void* base, int elem_bytes, uint64_
   return DQ_OK;
 }
 
+// Scale-factor atoms (512 bytes) in the order the FP4 GEMMs stream, [tile of 128 rows][atom]: a box is `box_atoms`
+// consecutive atoms of `box_tiles` tiles.
+int make_tmap_sf_atoms(CUtensorMap* out, const void* base, int tile_atoms, int tiles, uint32_t box_atoms,
+                       uint32_t box_tiles) {
+  if (g_encode == nullptr) return set_error(DQ_ERR_NOT_INIT, "tensor-map encoder not resolved");
+  cuuint64_t dims[3] = {128, static_cast<cuuint64_t>(tile_atoms), static_cast<cuuint64_t>(tiles)};
+  cuuint64_t strides[2] = {512, static_cast<cuuint64_t>(tile_atoms) * 512};
+  cuuint32_t box[3] = {128, box_atoms, box_tiles};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = g_encode(out, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<void*>(base), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS)
+    return set_error(DQ_ERR_CUDA, "cuTensorMapEncodeTiled (scale factors) failed (%d): base=%p atoms=%d tiles=%d", (int)r,
+                     base, tile_atoms, tiles);
+  return DQ_OK;
+}
+
 // Activation codes [rows][row_bytes] seen as (128-byte group chunk, row, group): one box is
 // `box_groups` consecutive K groups of `box_rows` rows, laid out in shared memory as
 // [group][row][128 B] (each group block is one 128B-swizzled UMMA operand tile).

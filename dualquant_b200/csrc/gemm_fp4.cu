@@ -67,7 +67,7 @@ gemm_fp4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
                 const uint8_t* __restrict__ sfw, const uint8_t* __restrict__ sfx,
                 const float* __restrict__ r, const float* __restrict__ w_scale,
                 const float* __restrict__ x_scale, const void* __restrict__ bias, void* __restrict__ y, int y_bf16, int M, int N,
-                int K, int stages_per_split, int split_k, int tok_fast, int row_tile0, int* status) {
+                int K, int stages_per_split, int split_k, int tok_fast, int* status) {
   using C = FCfg<NT>;
   constexpr int kFStages = C::kStages;
   constexpr int kAtoms = NVFP4 ? 4 : 2;           // scale-factor atoms per operand per stage
@@ -85,7 +85,7 @@ gemm_fp4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // tok_fast: grid x walks the token tiles (CTAs that run together share one weight tile and the
   // whole, smaller, activation matrix stays in L2); otherwise grid x walks the row tiles
-  const int n0 = (static_cast<int>(tok_fast ? blockIdx.y : blockIdx.x) + row_tile0) * kFBN;  // row_tile0: first row tile of this launch
+  const int n0 = static_cast<int>(tok_fast ? blockIdx.y : blockIdx.x) * kFBN;
   const int t0 = (tok_fast ? blockIdx.x : blockIdx.y) * C::kTok;
   // token blocks of this CTA that hold tokens (the last CTA of a ragged M may own only one)
   const int nblk = (NT == 2 && M - t0 > kFTN) ? 2 : 1;
@@ -422,6 +422,36 @@ extern "C" int dq_gemm_w4a4_fp4(const uint8_t* x_codes, const uint8_t* x_sf_atom
                                 fmt, y, y_dtype, 0, stream);  // 0: the library picks the token tile
 }
 
+// Split of K over a cluster in the one-tile kernel.
+static int fp4_split(int M, int N, int stages, int tok, int sm_count) {
+  const int tiles = ((N + kFBN - 1) / kFBN) * ((M + tok - 1) / tok);
+  int split = 1;
+  while (split < 8 && tiles * split * 6 < sm_count * 2 * 5 && stages / (2 * split) >= 2) split *= 2;
+  return split;
+}
+
+// Microseconds of the two kernels above 32 tokens, from their rounds and K loops (stages of 256 k).  Pairs: tiles of 256 x
+// 256, a last round with few tiles run as halves at 0.65 of a round.  One tile per CTA: tiles of 128 x 128, two CTAs per
+// SM; with K split over clusters of 2, 4 or 8 CTAs (places for 148, 66, 36 of them) the direct stores of the partial sums
+// dominate.  Over 162 cases of 48 to 4096 tokens the choice costs 0.6 % on average and 18 % at worst.  us, one tile / pairs:
+//   18944 -> 3584  128 tokens 17 / 29   256  30 / 29   512  40 / 29   1000  64 / 36   4096 176 / 125
+//    3584 -> 4608             12 / 11        22 / 12        19 / 12         13 / 15         47 / 33
+//    3584 -> 37888            18 / 22        31 / 24        50 / 37        105 / 63        381 / 211
+//   14336 -> 1200             13 / 23        14 / 23        24 / 23         32 / 24         61 / 43
+static float fp4_pairs_us(int M, int N, int stages, int sm_count) {
+  const int tiles = ((N + 255) / 256) * ((M + 255) / 256), pairs = sm_count / 2, rest = tiles % pairs;
+  const float rounds = tiles / pairs + (rest == 0 ? 0.f : 2 * rest <= pairs ? 0.65f : 1.f);
+  const float fill = 0.25f * stages;
+  return 6.f + (fill < 3.5f ? fill : 3.5f) + rounds * (0.33f * stages + 0.9f);
+}
+static float fp4_one_tile_us(int M, int N, int stages, int sm_count) {
+  const int tiles = ((N + kFBN - 1) / kFBN) * ((M + kFTN - 1) / kFTN);
+  const int split = fp4_split(M, N, stages, kFTN, sm_count);
+  const int places = (split == 1 ? 296 : split == 2 ? 148 : split == 4 ? 66 : 36) * sm_count / 148;
+  const int rounds = (tiles + places - 1) / places;
+  return split == 1 ? 2.f + rounds * (4.f + 0.52f * stages) : rounds * (9.f + 0.65f * stages / split);
+}
+
 static int gemm_fp4(const uint8_t* x_codes, const uint8_t* x_sf_atoms, const float* x_scale, const uint8_t* w_codes,
                     const uint8_t* w_sf_atoms, const float* w_scale, const float* r, const void* bias, int M, int N, int K,
                     int fmt, void* y, int y_dtype, int token_tile, void* stream) {
@@ -439,44 +469,19 @@ static int gemm_fp4(const uint8_t* x_codes, const uint8_t* x_sf_atoms, const flo
   DQ_REQUIRE(token_tile == 0 || token_tile == 32 || token_tile == 128 || token_tile == 256, DQ_ERR_SHAPE,
              "token_tile must be 0 (library's choice), 32, 128 or 256, got %d", token_tile);
   const int total_st = K / kFKStage;
-  // Prefill-size batches (library's choice of tile, output addressable by the copy engine): the
-  // persistent kernel on as many row tiles as fill whole rounds of one 256-token tile per SM, the
-  // one-tile kernel (with split-K) on the row tiles that are left.  A last round with few tiles
-  // would cost a full tile time: down of the Qwen2.5-7B shapes at M = 4096 is 448 tiles on 148 SMs
-  // - 27 of its 28 row tiles go to the persistent kernel, the last to 256 split-K CTAs (measured
-  // 163 -> 147 us; the same split on o, K = 3584, does not pay for its second launch).
-  int row_tile0 = 0;  // first row tile of the one-tile launch below
-  {
-    const int esz0 = (y_dtype == DQ_DTYPE_BF16) ? 2 : 4;
-    const int rt_all = (N + kFBN - 1) / kFBN, tok256 = (M + 255) / 256;
-    if (token_tile == 0 && M >= 512 && (static_cast<size_t>(N) * esz0) % 16 == 0 && aligned(y, 16)) {
-      const int64_t tiles256 = static_cast<int64_t>(rt_all) * tok256;
-      const int64_t rounds = (tiles256 + st->sm_count - 1) / st->sm_count;
-      int rt_p = 0;
-      if (tiles256 * 100 >= rounds * st->sm_count * 85) rt_p = rt_all;                      // fills its rounds
-      else if (tiles256 >= st->sm_count && K >= 8192)  // long K loops only: a second launch costs ~10 us
-        rt_p = static_cast<int>((tiles256 / st->sm_count) * st->sm_count / tok256);
-      if (rt_p > 0) {
-        int rc0 = launch_gemm_fp4_persist(x_codes, x_sf_atoms, x_scale, w_codes, w_sf_atoms, w_scale, r, bias, M, N, K,
-                                          fmt == DQ_FP4_NVFP4 ? 1 : 0, y, y_dtype, rt_p,
-                                          static_cast<cudaStream_t>(stream), st);
-        if (rc0 != DQ_OK || rt_p == rt_all) return rc0;
-        row_tile0 = rt_p;
-      }
-    }
-  }
+  // The library's choice above a decode batch, where the copy engine can address the output: the persistent kernel on CTA
+  // pairs, unless the one-tile kernel is estimated to be faster.
+  if (token_tile == 0 && M > kFp4DecodeTokens && (static_cast<size_t>(N) * (y_dtype == DQ_DTYPE_BF16 ? 2 : 4)) % 16 == 0 &&
+      aligned(y, 16) && fp4_pairs_us(M, N, total_st, st->sm_count) < fp4_one_tile_us(M, N, total_st, st->sm_count))
+    return launch_gemm_fp4_persist(x_codes, x_sf_atoms, x_scale, w_codes, w_sf_atoms, w_scale, r, bias, M, N, K,
+                                   fmt == DQ_FP4_NVFP4 ? 1 : 0, y, y_dtype, static_cast<cudaStream_t>(stream), st);
   // The library's own choice otherwise: 32-token tiles for decode batches, else 128.  The 256-token tile is
   // not chosen: measured on the Qwen2.5-7B-architecture linears at M = 4096 it is 3 % faster on the
   // longest K loop and 2-15 % slower elsewhere (one CTA and one UMMA-issuing thread per SM).
   const int tile_tok = token_tile ? token_tile : (M <= kFp4DecodeTokens ? 32 : kFTN);
   const int nt = tile_tok == 32 ? 0 : tile_tok / kFTN;
   // split K across a cluster when the output tiles alone leave most SMs idle (decode batches)
-  int split = 1;
-  {
-    const int split_tok = (tile_tok == 32) ? 32 : kFTN;  // the 256-token tile never splits: judged as 128
-    const int tiles1 = ((N + kFBN - 1) / kFBN - row_tile0) * ((M + split_tok - 1) / split_tok);
-    while (split < 8 && tiles1 * split * 6 < st->sm_count * 2 * 5 && total_st / (2 * split) >= 2) split *= 2;
-  }
+  const int split = fp4_split(M, N, total_st, tile_tok == 32 ? 32 : kFTN, st->sm_count);  // (256 never splits: judged as 128)
   DQ_REQUIRE(nt != 0 || M <= 32, DQ_ERR_UNSUPPORTED, "the 32-token tile covers batches of up to 32 tokens, got M=%d", M);
   DQ_REQUIRE(nt != 2 || split == 1, DQ_ERR_UNSUPPORTED,
              "256-token tiles have no split-K path (M=%d N=%d K=%d would split %d ways)", M, N, K, split);
@@ -498,7 +503,7 @@ static int gemm_fp4(const uint8_t* x_codes, const uint8_t* x_sf_atoms, const flo
   }
   const int sps = (total_st + split - 1) / split;
   cudaLaunchConfig_t cfg = {};
-  const int row_tiles = (N + kFBN - 1) / kFBN - row_tile0, tok_tiles = (M + tile_tok - 1) / tile_tok;
+  const int row_tiles = (N + kFBN - 1) / kFBN, tok_tiles = (M + tile_tok - 1) / tile_tok;
   // the smaller operand is the one every CTA wave re-reads; it stays in L2 when grid x walks its tiles
   const int tok_fast = (tok_tiles > 1 && M < N && row_tiles <= 65535) ? 1 : 0;
   cfg.gridDim = tok_fast ? dim3(tok_tiles, row_tiles, split) : dim3(row_tiles, tok_tiles, split);
@@ -520,7 +525,7 @@ static int gemm_fp4(const uint8_t* x_codes, const uint8_t* x_sf_atoms, const flo
                   ? (nt == 2 ? gemm_fp4_kernel<1, 2> : nt == 1 ? gemm_fp4_kernel<1, 1> : gemm_fp4_kernel<1, 0>)
                   : (nt == 2 ? gemm_fp4_kernel<0, 2> : nt == 1 ? gemm_fp4_kernel<0, 1> : gemm_fp4_kernel<0, 0>);
   e = cudaLaunchKernelEx(&cfg, kern, tm_w, tm_x, tm_y, bulk_store, w_sf_atoms, x_sf_atoms, r, w_scale, x_scale, bias, y, bf, M, N,
-                         K, sps, split, tok_fast, row_tile0, st->status_dev);
+                         K, sps, split, tok_fast, st->status_dev);
   if (e != cudaSuccess)
     return set_error(DQ_ERR_CUDA, "gemm_fp4 launch failed (split=%d): %s", split, cudaGetErrorString(e));
   DQ_CHECK_CUDA(cudaGetLastError());

@@ -214,12 +214,9 @@ def test_fp4_gemm_token_tiles_agree(fmt, M, N, K):
     assert err < 1e-3, err
 
 
-# Shapes the library sends to the persistent prefill kernel (at least 512 tokens, 256-token tiles
-# that fill whole rounds of one tile per SM): one tile per CTA and several, a last token tile of 216
+# Shapes the library sends to the persistent prefill kernel: one tile per CTA pair and several, a last token tile of 216
 # tokens (two scale-factor blocks) and one of 100 (a single block), rows past N.
 @pytest.mark.parametrize("fmt", [_lib.FP4_MXFP4, _lib.FP4_NVFP4])
-# (1024 x 5120 and 1000 x 5104 are 160 tiles on 148 SMs: 37 row tiles go to the persistent kernel,
-# the last three to the one-tile kernel with split-K)
 @pytest.mark.parametrize("M,N,K,dtype", [(728, 6272, 512, torch.float32), (612, 6260, 768, torch.bfloat16),
                                          (2048, 9472, 256, torch.bfloat16), (1024, 5120, 8192, torch.bfloat16),
                                          (1000, 5104, 8192, torch.float32)])
@@ -242,6 +239,36 @@ def test_fp4_persistent_kernel_equals_the_one_tile_kernel(fmt, M, N, K, dtype):
     ref = _fp4_reference(x, a.cpu(), w, r, fmt)
     err = ((got.double().cpu() - ref).abs().max() / ref.abs().max()).item()
     assert err < (1e-3 if dtype == torch.float32 else 1e-2), err
+
+
+# Edges of the CTA-pair tiles: a last round of half tiles (some without tokens), an odd number of row tiles (the odd CTA of
+# the last pair has no rows), token tiles of 1, 2 and 128 tokens, more stages than the ring holds and fewer.  Without split-K
+# the one-tile kernel forms the same sums in the same order.
+@pytest.mark.parametrize("fmt", [_lib.FP4_MXFP4, _lib.FP4_NVFP4])
+@pytest.mark.parametrize("M,N,K", [(300, 20008, 512), (130, 38000, 512), (257, 19080, 768), (385, 20000, 256), (1153, 20096, 768)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_fp4_pair_tiles_equal_the_one_tile_kernel(fmt, M, N, K, dtype):
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    x = torch.randn(M, K, generator=g, device=DEV).to(torch.bfloat16)
+    w = (torch.randn(N, K, generator=g, device=DEV) * 0.02).to(torch.bfloat16)
+    r = torch.rand(N, generator=g, device=DEV) + 0.5
+    bias = torch.randn(N, generator=g, device=DEV).to(dtype)
+    pw = ops.pack_w_fp4(w, fmt)
+    codes, sfa, rs = ops.quant_fp4(x, fmt, None, None, atoms=True)
+    want = ops.gemm_w4a4_fp4(codes, sfa, rs, pw, r, out_dtype=dtype, token_tile=128)
+    y = torch.full((M + 1, N), 7.0, dtype=dtype, device=DEV)  # one guard row behind the output
+    ops.gemm_w4a4_fp4(codes, sfa, rs, pw, r, out=y[:M])
+    _lib.device_status(0)
+    assert torch.equal(y[:M], want) and bool((y[M] == 7.0).all())
+    lib = _lib.load()
+    scratch = torch.empty(int(lib.dq_linear_w4a4_fp4_scratch_bytes(M, K, fmt)), dtype=torch.uint8, device=DEV)
+    ptr = lambda t: None if t is None else t.data_ptr()  # noqa: E731
+    ydt = _lib.DTYPE_BF16 if dtype == torch.bfloat16 else _lib.DTYPE_F32
+    _lib.check(lib.dq_linear_w4a4_fp4(ptr(x), 0, K, None, ptr(pw.codes), ptr(pw.sf_atoms), ptr(pw.tensor_scale), ptr(r),
+                                      ptr(bias), M, N, K, fmt, ptr(y), ydt, ptr(scratch), scratch.numel(),
+                                      torch.cuda.current_stream().cuda_stream), "dq_linear_w4a4_fp4")
+    _lib.device_status(0)
+    assert torch.equal(y[:M], want + bias) and bool((y[M] == 7.0).all())
 
 
 @pytest.mark.parametrize("fmt", [_lib.FP4_MXFP4, _lib.FP4_NVFP4])
