@@ -104,6 +104,14 @@ enum {
 };
 int tuning(int key);
 
+int launch_expand_w_e4m3(const uint8_t* w_packed, int N, int K, uint8_t* w8, int per_sm, cudaStream_t stream,
+                         DeviceState* st);
+// dq_quant_act_int4 directly behind launch_expand_w_e4m3 on the same stream, running beside it; whether its kernel for such a
+// call can.
+bool quant_act_int4_can_run_beside(const dq_hadamard_desc* had, int M, int K);
+int quant_act_int4_beside_expansion(const void* x_bf16, int64_t ldx, const float* a, const dq_hadamard_desc* had, int M, int K,
+                                    int8_t* codes, float* sx, int scale_fp16, cudaStream_t stream);
+
 // One-time kernel attribute set-up of each translation unit (called from dq_init).
 int init_gemm_int4_kernels();
 int init_gemv_int4_kernels();

@@ -58,29 +58,42 @@ __device__ __forceinline__ uint32_t low_nibbles(uint32_t v) {
   return (v & 0xFu) | ((v >> 4) & 0xF0u) | ((v >> 8) & 0xF00u) | ((v >> 12) & 0xF000u);
 }
 
-// packed int4 tiles -> E4M3 bytes, row-major [N, K]; one thread per 16-byte chunk (32 codes)
-__global__ void __launch_bounds__(256) expand_w_e4m3_kernel(const uint8_t* __restrict__ w_packed, int N, int K,
-                                                            uint8_t* __restrict__ w8) {
-  grid_dep_launch_dependents();
+// packed int4 tiles -> E4M3 bytes, row-major [N, K]: CTAs walk over the 16-byte chunks (32 codes), AHEAD in flight per
+// thread.  beside: the next kernel is started only once every CTA has seen the kernels before this one finish, so that it
+// need not wait for this one before it works (wait_at_start in act_quant_common.cuh).
+constexpr int kExpandThreads = 256;
+template <int AHEAD>
+__global__ void __launch_bounds__(kExpandThreads) expand_w_e4m3_kernel(const uint8_t* __restrict__ w_packed, int N, int K,
+                                                                       uint8_t* __restrict__ w8, int beside) {
+  if (!beside) grid_dep_launch_dependents();
   grid_dep_wait();
-  const int64_t chunk = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int groups = K / kGroup;
-  const int64_t tiles = (N + 127) / 128;
-  if (chunk >= tiles * groups * 512) return;
-  const int r = static_cast<int>((chunk >> 2) & 127);
-  const int ch = static_cast<int>(chunk & 3) ^ ((r >> 1) & 3);
-  const int64_t tg = chunk >> 9;
-  const int g = static_cast<int>(tg % groups);
-  const int64_t row = (tg / groups) * 128 + r;
-  if (row >= N) return;
-  const uint4 raw = *reinterpret_cast<const uint4*>(w_packed + tg * kTileBytes + (chunk & 511) * 16);
-  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-  uint32_t lo[4], hi[4];
+  if (beside) grid_dep_launch_dependents();
+  const uint32_t groups = static_cast<uint32_t>(K / kGroup);
+  const int64_t total = static_cast<int64_t>((N + 127) / 128) * groups * 512;
+  const int64_t step = static_cast<int64_t>(gridDim.x) * kExpandThreads;
+  for (int64_t c0 = static_cast<int64_t>(blockIdx.x) * kExpandThreads + threadIdx.x; c0 < total; c0 += AHEAD * step) {
+    uint4 raw[AHEAD];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) e4m3_of_word(w[j], lo[j], hi[j]);  // k = 4j .. 4j+3 of the chunk, k = 16 + 4j ..
-  uint8_t* dst = w8 + row * K + (g * 4 + ch) * 32;
-  *reinterpret_cast<uint4*>(dst) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-  *reinterpret_cast<uint4*>(dst + 16) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    for (int i = 0; i < AHEAD; ++i) {
+      const int64_t c = c0 + i * step;
+      if (c < total) raw[i] = *reinterpret_cast<const uint4*>(w_packed + (c >> 9) * kTileBytes + (c & 511) * 16);
+    }
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i) {
+      const int64_t c = c0 + i * step;
+      const uint32_t r = static_cast<uint32_t>(c >> 2) & 127, ch = (static_cast<uint32_t>(c) & 3) ^ ((r >> 1) & 3);
+      const uint32_t tg = static_cast<uint32_t>(c >> 9), tile = tg / groups, g = tg - tile * groups;
+      const int64_t row = static_cast<int64_t>(tile) * 128 + r;
+      if (c >= total || row >= N) continue;
+      const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
+      uint32_t lo[4], hi[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) e4m3_of_word(w[j], lo[j], hi[j]);  // k = 4j .. 4j+3 of the chunk, k = 16 + 4j ..
+      uint8_t* dst = w8 + row * K + (g * 4 + ch) * 32;
+      *reinterpret_cast<uint4*>(dst) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+      *reinterpret_cast<uint4*>(dst + 16) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    }
+  }
 }
 
 // int8 codes (-8..7) [M, K] with row stride ld -> E4M3 bytes [M, K]; one thread per 16 codes
@@ -215,6 +228,17 @@ int launch_gemm_int4_e4m3(const uint8_t* x8, const float* sx, const uint8_t* w8,
   return launch_gemm_int4_e4m3_impl(x8, sx, w8, sw_t, r, M, N, K, y, y_dtype, add, stream, st, nullptr);
 }
 
+// per_sm: CTAs per SM of an expansion with a quantiser beside it; 0: on its own, a thread per chunk.
+int launch_expand_w_e4m3(const uint8_t* w_packed, int N, int K, uint8_t* w8, int per_sm, cudaStream_t stream,
+                         DeviceState* st) {
+  int64_t ctas = (static_cast<int64_t>((N + 127) / 128) * (K / kGroup) * 512 + f8::kExpandThreads - 1) / f8::kExpandThreads;
+  if (per_sm > 0 && ctas > per_sm * st->sm_count) ctas = per_sm * st->sm_count;
+  DQ_CHECK_CUDA(launch_pdl(per_sm > 0 ? f8::expand_w_e4m3_kernel<4> : f8::expand_w_e4m3_kernel<1>,
+                           dim3(static_cast<unsigned>(ctas)), dim3(f8::kExpandThreads), 0, stream, w_packed, N, K, w8,
+                           per_sm > 0 ? 1 : 0));
+  return DQ_OK;
+}
+
 }  // namespace dq
 
 using namespace dq;
@@ -256,10 +280,7 @@ extern "C" int dq_expand_w_int4_e4m3(const uint8_t* w_packed, int N, int K, int 
   DQ_REQUIRE(G == kGroup, DQ_ERR_UNSUPPORTED, "weight group size must be %d (got %d)", kGroup, G);
   DQ_REQUIRE(N >= 1 && K >= kGroup && K % kGroup == 0, DQ_ERR_SHAPE, "bad shape N=%d K=%d", N, K);
   DQ_REQUIRE(aligned(w_packed, 16) && aligned(w8, 16), DQ_ERR_ALIGN, "w_packed and w8 must be 16-byte aligned");
-  const int64_t chunks = static_cast<int64_t>((N + 127) / 128) * (K / kGroup) * 512;
-  DQ_CHECK_CUDA(launch_pdl(f8::expand_w_e4m3_kernel, dim3(static_cast<unsigned>((chunks + 255) / 256)), dim3(256), 0,
-                           static_cast<cudaStream_t>(stream), w_packed, N, K, w8));
-  return DQ_OK;
+  return launch_expand_w_e4m3(w_packed, N, K, w8, 0, static_cast<cudaStream_t>(stream), st);
 }
 
 extern "C" int dq_codes_to_e4m3(const int8_t* codes, int64_t ld, int M, int K, uint8_t* x8, void* stream) {

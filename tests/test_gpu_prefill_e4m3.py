@@ -395,3 +395,34 @@ def test_expanding_linear_equals_the_packed_kernel_over_its_options(M, N, had, m
     codes, sx = ops.quant_act_int4(x, a, h, **mode)
     assert torch.equal(y, ops.gemm_w4a4_int4(codes, sx, pw, r, out_dtype=dtype, token_tile=1128, split_k=1))
     _lib.device_status(0)
+
+
+# The quantiser of these calls runs beside the expansion of the weight - rows in registers (128, 256 and 256 long ones, and 512
+# threads of one vector), 28 * 512 - or behind it (across heads, 2048 = 32 * 64).  Inputs written and scratch read by the
+# kernels just before; the packed path, which expands nothing, gives the same bits.
+@pytest.mark.parametrize("M,K,N,kind", [(1024, 4096, 1024, None), (1030, 8192, 512, None), (1026, 14336, 512, None),
+                                        (700, 4096, 4096, None), (1100, 4096, 4096, "heads"), (1031, 14336, 1024, "full"),
+                                        (1200, 2048, 768, "full")])
+def test_linear_beside_the_expansion_of_its_weight(M, K, N, kind):
+    had = None
+    if kind == "heads":
+        had = ops.Hadamard(_lib.HAD_PARTIAL, 1, 128, quarot.partial_hadamard_scale(K // 128), None)
+    elif kind == "full":
+        mat, order = quarot.get_hadK(K)
+        had = ops.Hadamard(_lib.HAD_FULL, order, 0, quarot.full_hadamard_scale(K), None if mat is None else mat.to(DEV))
+    g = torch.Generator(device=DEV).manual_seed(K + N)
+    pws = [ops.pack_w_int4(*ops.quant_w_int4((torch.randn(N, K, generator=g, device=DEV) * 0.02).to(torch.bfloat16)))
+           for _ in range(2)]
+    a = torch.rand(K, generator=g, device=DEV) + 0.5
+    xs = [torch.randn(M, K, generator=g, device=DEV).to(torch.bfloat16) for _ in range(3)]
+    big = torch.empty(ops.linear_scratch_bytes(M, N, K), dtype=torch.uint8, device=DEV)
+    small = torch.empty(ops.linear_scratch_bytes(M, N, K, prefill=False), dtype=torch.uint8, device=DEV)
+    assert big.numel() >= small.numel() + N * K
+    want = [[ops.linear_w4a4_int4(x, a, had, pw, None, scratch=small) for pw in pws] for x in xs]
+    torch.cuda.synchronize()
+    x, got = torch.empty_like(xs[0]), []
+    for i in range(12):  # nothing between the calls but the copy of the next input
+        x.copy_(xs[i % 3])
+        got.append(ops.linear_w4a4_int4(x, a, had, pws[i % 2], None, scratch=big))
+    _lib.device_status(0)
+    assert all(torch.equal(y, want[i % 3][i % 2]) for i, y in enumerate(got))
