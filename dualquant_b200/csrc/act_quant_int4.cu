@@ -10,6 +10,7 @@
 //   * had_kernel : row staged in shared memory as fp32, butterflies in place, then the same tail.
 // Both are HBM-bound streaming kernels (2 bytes in, 1 byte out per element).
 #include "act_quant_common.cuh"
+#include "act_quant_had_big.cuh"
 
 namespace dq {
 
@@ -252,8 +253,8 @@ act_quant_had_kernel(const XT* __restrict__ x, const XT* __restrict__ up, int64_
 // second buffer of the same size sit in shared memory next to the factor stored as one byte per
 // entry.  Walsh-Hadamard stages over the contiguous segments in place, then one thread per output
 // element: out[i][c] = sum_j H[i][j] * (v[j][c] * scale), j ascending, fp32 - the order of the
-// stand-alone restatement, so codes stay bit-identical.  Used for decode-size batches of models
-// whose intermediate size is not 28 * 2^k (e.g. 11008 = 172 * 64); not a tuned path.
+// stand-alone restatement, so codes stay bit-identical.  Segments of 32, 64 and 128 values have a kernel of their own
+// (act_quant_had_big.cuh); not a tuned path.
 constexpr int kMaxHadKBig = 172;
 
 template <int THREADS, typename XT>
@@ -353,6 +354,13 @@ int init_act_quant_kernels() {
   if (e != cudaSuccess)
     return set_error(DQ_ERR_CUDA, "cudaFuncSetAttribute(act_quant_had) failed: %s",
                      cudaGetErrorString(e));
+  auto allow = [](auto kernel) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024);
+  };
+  e = for_each_wide<__nv_bfloat16>(allow);
+  if (e == cudaSuccess) e = for_each_wide<float>(allow);
+  if (e != cudaSuccess)
+    return set_error(DQ_ERR_CUDA, "cudaFuncSetAttribute(act_quant_had_wide) failed: %s", cudaGetErrorString(e));
   int rc = init_had_fast_bf16();
   if (rc != DQ_OK) return rc;
   return init_had_fast_f32();
@@ -403,7 +411,9 @@ static int launch_act(const XT* x, int64_t ldx, const float* a, const dq_hadamar
   if (use_had || mode == MODE_RAW || K > 32768 || up != nullptr) {  // longer rows than the register path holds
     const int hk = use_had ? had->had_k : 1;
     if (use_had && had->kind == DQ_HAD_FULL && hk > kMaxHadK) {
-      // large +-1 factor: row + result buffer + the factor as bytes
+      if (had_wide_covers(hk, K))
+        return launch_had_wide(x, up, ldx, a, M, K, hk, had->scale, had->had_mat, codes, sx, out, mode, scale_fp16, stream);
+      // other segment lengths: row + result buffer + the factor as bytes
       const size_t big = static_cast<size_t>(K) * 8 + (static_cast<size_t>(hk) * hk + 15) / 16 * 16;
       DQ_REQUIRE(big <= static_cast<size_t>(kHadMaxSmem), DQ_ERR_UNSUPPORTED,
                  "row of K=%d with a Hadamard factor of order %d does not fit in shared memory", K, hk);

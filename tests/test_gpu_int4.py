@@ -231,6 +231,31 @@ def test_full_hadamard_other_orders_bit_exact(K):
     _status_ok()
 
 
+# Factors of more than 32 rows, many token rows: one CTA and clusters of two, four and eight per group of token rows (1, 2 or 4
+# rows a group for segments of 128, 64, 32), groups that are not full, CTAs that walk over several groups.
+@pytest.mark.parametrize("K,M", [(11008, 1), (11008, 31), (11008, 66), (11008, 150), (11008, 301), (13824, 5), (13824, 160),
+                                 (4480, 63), (1152, 130), (6912, 700)])
+def test_wide_hadamard_many_rows_bit_exact(K, M):
+    from dualquant_b200 import quarot
+
+    had, k = quarot.get_hadK(K)
+    hd = ops.Hadamard(_lib.HAD_FULL, k, 0, quarot.full_hadamard_scale(K), had.to(DEV))
+    xb = synthetic.make_x(M, K, 9)
+    got = ops.hadamard_f32(xb.float().to(DEV), hd).cpu()
+    rows = [r for r in sorted({0, 1, 2, M // 2, M - 2, M - 1}) if 0 <= r < M]
+    assert torch.equal(got[rows], O.hadamard_full(xb[rows].float(), had, k))
+    _, c = synthetic.make_scales(8, K, 9)
+    qx, sx, _ = O.quant_act_int4(xb[rows], 1.0 / c, ("full", had, k), True)
+    codes, sxg = ops.quant_act_int4(xb.to(DEV), (1.0 / c).to(DEV), hd, True)
+    assert torch.equal(codes.cpu()[rows], qx) and torch.equal(sxg.cpu()[rows], sx)
+    x8, _ = ops.quant_act_int4(xb.to(DEV), (1.0 / c).to(DEV), hd, True, e4m3=True)
+    assert torch.equal(x8, ops.codes_to_e4m3(codes))
+    # every row the same as on its own (another split)
+    alone, s1 = ops.quant_act_int4(xb[M // 2 : M // 2 + 1].to(DEV), (1.0 / c).to(DEV), hd, True)
+    assert torch.equal(alone[0], codes[M // 2]) and torch.equal(s1[0], sxg[M // 2])
+    _status_ok()
+
+
 def test_hadamard_golden(golden):
     x = torch.from_numpy(golden["hadfull_in"])
     hd, _ = _full_had(896)
