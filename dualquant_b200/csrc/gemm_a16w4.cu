@@ -30,7 +30,9 @@
 //   warps 20, 23 producers: two tiled copies of activations, one bulk copy of packed weights per group.  (One producer
 //                for both, with the tile and ring positions divided out of a group counter, took 0.9 us per group.)
 //   warps 21-22  UMMA issue (of the even CTA, for both); tiles of up to 64 tokens: two warps take alternate groups into
-//                an accumulator each, because issuing a group takes one warp longer than executing it
+//                an accumulator each, because issuing a group takes one warp longer than executing it.  They alternate over
+//                all groups of the CTA, not from a tile's first: a ring slot then stays with one warp also where a tile
+//                has an odd number of groups
 // Persistent CTAs; where the tiles leave the chip idle (decode batches) K is split over the pairs of a larger cluster
 // instead, and the partial tiles are summed in rank order through distributed shared memory.  Every wait is bounded.
 //
@@ -74,6 +76,10 @@ struct Cfg {
   static constexpr int kNumBars = 2 * SP + 2 * SX + 2 * NA + 2 * kAccTiles;
   static constexpr int kSmemBytes = kOffBar + kNumBars * 8 + 16;
   static_assert(kSmemBytes <= 227 * 1024 && SX >= 3 && NA >= 2, "rings");
+  // Waits are by phase parity, so a warp must not be a whole phase ahead of a barrier's previous user: where warps take
+  // groups in turn, every slot of a ring they wait on belongs to one of them.
+  static_assert(SP % kSets == 0 && NA % kSets == 0, "packed tiles and expanded groups: a set of unpack warps per slot");
+  static_assert(NA % kIssuers == 0 && SX % kIssuers == 0, "expanded groups and activations: an issuer per slot");
   static_assert(kXAtom % 1024 == 0, "swizzle atoms on 1 KB boundaries");
   static_assert(TN > 64 || TN * kBN * 4 <= kOffP, "split-K exchange tile");
 };
@@ -229,7 +235,7 @@ gemm_a16w4_kernel(const uint8_t* __restrict__ w_packed, const __grid_constant__ 
     const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
     const uint32_t acc_empty_addr = dsmem_map(smem_u32(acc_empty), even);
     const bool leader = warp == kEpiWarp && lane == 0;
-    const bool second = kIssuers == 2 && ng > 1;  // the second issuer had groups to add up
+    const bool second = kIssuers == 2 && ng > 1;  // both issuers had groups of a tile to add up
     int chunk_no = 0;
     grid_dep_wait();  // what last used y may still be running
     for (int it = 0; it < my_tiles && live; ++it) {
@@ -239,6 +245,7 @@ gemm_a16w4_kernel(const uint8_t* __restrict__ w_packed, const __grid_constant__ 
       const int cols = M - t0 < TN ? (M - t0 + 31) & ~31 : TN;
       const float rn = (n < N && r != nullptr) ? r[n] : 1.f;
       const int set = it % C::kAccTiles;
+      const int only = (kIssuers == 2 && ng == 1) ? it & 1 : 0;  // a tile's only group is in the accumulator of its issuer
       if (TN <= 64 ? !mbar_wait(&acc_full[set], (it / C::kAccTiles) & 1, abort_flag, ASITE_EPI)
                    : !mbar_wait_relaxed(&acc_full[set], (it / C::kAccTiles) & 1, abort_flag, ASITE_EPI))
         break;
@@ -248,7 +255,7 @@ gemm_a16w4_kernel(const uint8_t* __restrict__ w_packed, const __grid_constant__ 
         float v[32];
         {
           uint32_t u[32];
-          const uint32_t at = t_lane + static_cast<uint32_t>(set * kIssuers * TN + c0);
+          const uint32_t at = t_lane + static_cast<uint32_t>((set * kIssuers + only) * TN + c0);
           tmem_ld_x32(at, u);
           tmem_ld_wait();
 #pragma unroll
@@ -358,7 +365,8 @@ gemm_a16w4_kernel(const uint8_t* __restrict__ w_packed, const __grid_constant__ 
       const int set = it % C::kAccTiles;
       const uint32_t d_tmem = tmem_base + static_cast<uint32_t>((set * kIssuers + mine) * TN);
       ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[set], ((it / C::kAccTiles) & 1) ^ 1, abort_flag, ASITE_MMA));
-      for (int i = mine; i < ng && ok; i += kIssuers) {
+      const int first = (mine + it * ng) & (kIssuers - 1);  // of this warp's groups in the tile: gi & 1 == mine
+      for (int i = first; i < ng && ok; i += kIssuers) {
         const int gi = it * ng + i, ab = gi % C::NA, sx = gi % C::SX;
         ok = mbar_wait(&full_x[sx], (gi / C::SX) & 1, abort_flag, ASITE_MMA) &&
              mbar_wait(&a_full[ab], (gi / C::NA) & 1, abort_flag, ASITE_MMA);
@@ -371,7 +379,7 @@ gemm_a16w4_kernel(const uint8_t* __restrict__ w_packed, const __grid_constant__ 
 #pragma unroll
           for (int j = 0; j < 8; ++j)  // eight K = 16 steps: 8 columns of A, 32 bytes along K of B inside an atom
             umma_f16_pair(d_tmem, at + 8 * j, db + (j >> 2) * (C::kXAtom >> 4) + 2 * (j & 3), idesc,
-                          (i != mine || j > 0) ? 1u : 0u);
+                          (i != first || j > 0) ? 1u : 0u);
           umma_commit_pair(&a_free[ab], even);
           umma_commit_pair(&empty_x[sx], even);
         }

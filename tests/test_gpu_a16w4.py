@@ -107,3 +107,28 @@ def test_every_tile_and_split(tile, M, N, K):
     _lib.device_status(0)
     assert ((y.double() - ref).abs().max() / ref.abs().max()).item() < 1e-4
     assert torch.equal(yb, y.to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("M,tile", [(14, 1032), (64, 1064)])
+@pytest.mark.parametrize("groups", [1, 7, 23])
+@pytest.mark.parametrize("N", [19100, 56888])
+def test_odd_group_counts_over_several_tiles(N, groups, M, tile):
+    """More tiles of 256 rows than CTA pairs and an odd number of groups a tile: the two issuing warps go from one tile
+    to the next without exchanging ring slots, and a tile's single group lies in either warp's accumulator."""
+    K = 128 * groups
+    g = torch.Generator(device=DEV).manual_seed(N + K + M)
+    qw, sw = ops.quant_w_int4((torch.randn(N, K, generator=g, device=DEV) * 0.02).to(torch.bfloat16))
+    pw = ops.pack_w_int4(qw, sw)
+    x = torch.randn(M, K, generator=g, device=DEV).to(torch.bfloat16)
+    a, r = torch.rand(K, generator=g, device=DEV) + 0.5, torch.rand(N, generator=g, device=DEV) + 0.5
+    try:
+        _lib.set_tuning("a16_tile", tile)
+        ys = [ops.linear_a16w4(x, a, pw, r, out_dtype=torch.float32) for _ in range(20)]
+        yb = ops.linear_a16w4(x, a, pw, r)
+    finally:
+        _lib.set_tuning("a16_tile", 0)
+    _lib.device_status(0)
+    ref = _restatement(x, a, qw, sw, r)
+    assert ((ys[0].double() - ref).abs().max() / ref.abs().max()).item() < 1e-4
+    assert all(torch.equal(y, ys[0]) for y in ys[1:])
+    assert torch.equal(yb, ys[0].to(torch.bfloat16))
