@@ -33,6 +33,7 @@ act_quant_had_wide_kernel(const XT* __restrict__ x, const XT* __restrict__ up, i
   __shared__ float red[4][kBigWarps], pmax[8][4];
   float* vals = sm;                       // [had_k][128]
   float* coef = sm + had_k * kBigCols;    // [had_k][12][RP]
+  if (split > 1) cluster_arrive();
   grid_dep_launch_dependents();
   grid_dep_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -45,6 +46,7 @@ act_quant_had_wide_kernel(const XT* __restrict__ x, const XT* __restrict__ up, i
     const int i = first_row + w * RPW + r;
     coef[u] = (r < RPW && i < had_k) ? had_mat[i * had_k + j] : 0.f;
   }
+  if (split > 1) cluster_wait();  // the peers have started: their shared memory may be written (the rows' maxima)
   const int groups = (M + T - 1) / T;
   for (int grp = blockIdx.x / split; grp < groups; grp += gridDim.x / split) {
     const int row0 = grp * T;

@@ -425,10 +425,22 @@ __device__ __forceinline__ void grid_dep_wait() {
 // ---------------------------------------------------------------------------------------
 // thread-block clusters
 // ---------------------------------------------------------------------------------------
+// (The .aligned forms want the warp's threads together, also behind a branch that some of them took.)
 __device__ __forceinline__ void cluster_sync_all() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n"
                "barrier.cluster.wait.acquire.aligned;" ::
                    : "memory");
+}
+// The same barrier in two steps.  A CTA's shared memory may be written by a peer only once it is known to have started:
+// kernels whose first remote access is a store arrive when they start and wait in front of that store.
+__device__ __forceinline__ void cluster_arrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;

@@ -232,9 +232,19 @@ def test_full_hadamard_other_orders_bit_exact(K):
 
 
 # Factors of more than 32 rows, many token rows: one CTA and clusters of two, four and eight per group of token rows (1, 2 or 4
-# rows a group for segments of 128, 64, 32), groups that are not full, CTAs that walk over several groups.
-@pytest.mark.parametrize("K,M", [(11008, 1), (11008, 31), (11008, 66), (11008, 150), (11008, 301), (13824, 5), (13824, 160),
-                                 (4480, 63), (1152, 130), (6912, 700)])
+# rows a group for segments of 128, 64, 32), groups that are not full, CTAs that walk over several groups.  On 148 SMs up to 15
+# groups go to clusters of eight, 33 to four, 74 to two.  Output rows of the factor per warp, of 2, 4, 5, 8, 9, 13 and 15: two
+# in every cluster of eight, then
+@pytest.mark.parametrize("K,M", [
+    (11008, 1), (13824, 5),                      # clusters of eight
+    (11008, 31), (11008, 66), (1152, 130),       # of four: 4, 4 and 2 (a factor of 36 leaves the last CTA without rows)
+    (11008, 150),                                # of one from 75 groups on: 15
+    (11008, 100), (9984, 67), (8960, 147),       # of two: 8, 8 (156 * 64), 8 (140 * 64)
+    (3456, 201), (1664, 160), (1152, 290),       # of two, segments of 32: 5 (108), 4 (52), 2 (36)
+    (13824, 160), (6912, 700), (11008, 301),     # of one: 9, 9, 15
+    (4480, 63), (8960, 149), (9984, 301),        # 140 * 32 on clusters of four; 13, 13
+    (3328, 151), (3840, 700), (5120, 77),        # of one: 5 (52, 60), 4 (40 * 128)
+])
 def test_wide_hadamard_many_rows_bit_exact(K, M):
     from dualquant_b200 import quarot
 
@@ -250,6 +260,13 @@ def test_wide_hadamard_many_rows_bit_exact(K, M):
     assert torch.equal(codes.cpu()[rows], qx) and torch.equal(sxg.cpu()[rows], sx)
     x8, _ = ops.quant_act_int4(xb.to(DEV), (1.0 / c).to(DEV), hd, True, e4m3=True)
     assert torch.equal(x8, ops.codes_to_e4m3(codes))
+    # SiLU(gate) * up in front
+    gate = synthetic.make_x(M, K, 10).to(DEV)
+    g32 = gate[rows].float()
+    h = (g32 / (1.0 + torch.exp(-g32))).to(torch.bfloat16).cpu() * xb[rows]
+    qh, sh, _ = O.quant_act_int4(h, 1.0 / c, ("full", had, k), True)
+    gcodes, gsx = ops.quant_act_int4_gated(gate, xb.to(DEV), (1.0 / c).to(DEV), hd, True)
+    assert torch.equal(gcodes.cpu()[rows], qh) and torch.equal(gsx.cpu()[rows], sh)
     # every row the same as on its own (another split)
     alone, s1 = ops.quant_act_int4(xb[M // 2 : M // 2 + 1].to(DEV), (1.0 / c).to(DEV), hd, True)
     assert torch.equal(alone[0], codes[M // 2]) and torch.equal(s1[0], sxg[M // 2])
