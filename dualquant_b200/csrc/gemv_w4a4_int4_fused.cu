@@ -159,6 +159,7 @@ gemv_fused_kernel(const uint8_t* __restrict__ w_packed, const __nv_bfloat16* __r
   }
   grid_dep_launch_dependents();
   __syncthreads();
+  cluster_arrive();  // waited for in front of the first store to a peer
 
   if (warp == kComputeWarps) {
     // ------------------------------------------------------------------ producer warp
@@ -177,7 +178,8 @@ gemv_fused_kernel(const uint8_t* __restrict__ w_packed, const __nv_bfloat16* __r
       }
     }
     __syncwarp();
-    // the two cluster barriers of the quantisation phase (every thread of the cluster arrives)
+    // the cluster barriers of the quantisation phase (every thread of the cluster arrives): started, maxima, codes
+    cluster_wait();
     cluster_sync_all();
     cluster_sync_all();
     if (lane == 0) {
@@ -240,6 +242,7 @@ gemv_fused_kernel(const uint8_t* __restrict__ w_packed, const __nv_bfloat16* __r
       // the TPR lanes of a row are consecutive lanes of one warp
 #pragma unroll
       for (int o = TPR / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+      cluster_wait();  // every CTA of the cluster has started: its shared memory may be written
       // partial maximum of (this CTA, row) -> slot [my_rank][row] of every CTA of the cluster
       if (lr < csize) {
         const uint32_t slot = smem_u32(pmax + my_rank * TOK + row);
