@@ -4,6 +4,7 @@
 #include "dq_common.h"
 #include "dq_ptx.cuh"
 #include "dq_quant.cuh"
+#include "expand_w_e4m3.cuh"
 
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -12,18 +13,15 @@ namespace dq {
 
 enum { MODE_CODES = 0, MODE_FAKE = 1, MODE_RAW = 2, MODE_FAKE_BF16 = 3 };
 
-// How a quantiser orders itself behind the kernel in front of it.  BESIDE: that kernel is the expansion of a weight
-// (expand_w_e4m3_kernel), which neither writes what the quantiser reads nor reads what it writes and lets it start only once
-// the kernels before it have finished; the quantiser waits for it at its end, so that the GEMM behind finds both finished.
-// (A template parameter: behind a run-time condition, a branch or a predicate, loads were moved to in front of the wait.)
-template <bool BESIDE>
-__device__ __forceinline__ void wait_at_start() {
-  if constexpr (!BESIDE) grid_dep_wait();
-}
-template <bool BESIDE>
-__device__ __forceinline__ void wait_at_end() {
-  if constexpr (BESIDE) grid_dep_wait();
-}
+// The expansion of a weight that a quantiser's launch is asked to take along; `done`: it has.
+struct Along {
+  WeightExpansion e;
+  bool done;
+  unsigned take(int threads, int64_t rows, ExpansionShare* s) {
+    done = true;
+    return take_along(e, threads, rows, s);
+  }
+};
 
 // Row `row` of the de-quantised output: fp32 elements, or bf16 elements for MODE_FAKE_BF16 (the
 // pointer type stays float*; emit8 casts it back).

@@ -709,7 +709,7 @@ int init_had_fast_t() {
 template <typename XT>
 int launch_had_fast_t(const XT* x, const XT* up, int64_t ldx, const float* a, const dq_hadamard_desc* had, int M, int K,
                       size_t smem, int8_t* codes, float* sx, float* out, int mode, int scale_fp16,
-                      cudaStream_t stream, bool* taken, bool beside_expansion) {
+                      cudaStream_t stream, bool* taken, Along* along) {
   *taken = false;
     HadPlan plan;
     if (plan_fast_hadamard(had, K, &plan)) {
@@ -775,10 +775,16 @@ int launch_had_fast_t(const XT* x, const XT* up, int64_t ldx, const float* a, co
       // it is the faster one (14336, us: 65 rows 14.7 -> 8.1, 300 rows 22.9 -> 15.0; 1792: 70 rows 9.3 -> 7.3)
       if (plan.matrix && plan.inner && plan.S == 28 && plan.R >= 2 && plan.R <= 16) {
 #define DQ_HAD28(P)                                                                                                    \
-  DQ_CHECK_CUDA(launch_pdl(beside_expansion ? act_quant_had28_kernel<P, XT, sizeof(XT) == 2>                           \
-                                            : act_quant_had28_kernel<P, XT>, dim3((M + Had28<P>::kRows - 1) / Had28<P>::kRows),           \
-                           dim3(kHad28Threads), Had28<P>::kSmem, stream, x, up, ldx, a, M, had->scale, had->had_mat,   \
-                           codes, sx, out, mode, scale_fp16))
+  {                                                                                                                    \
+    constexpr bool kExpand = sizeof(XT) == 2;                                                                          \
+    ExpansionShare ex = {};                                                                                            \
+    const bool both = kExpand && along != nullptr;                                                                     \
+    const int ctas = (M + Had28<P>::kRows - 1) / Had28<P>::kRows;                                                      \
+    const unsigned grid = both ? along->take(kHad28Threads, ctas, &ex) : static_cast<unsigned>(ctas);                  \
+    DQ_CHECK_CUDA(launch_pdl(both ? act_quant_had28_kernel<P, XT, kExpand> : act_quant_had28_kernel<P, XT>,            \
+                             dim3(grid), dim3(kHad28Threads), Had28<P>::kSmem, stream, x, up, ldx, a, M, had->scale,   \
+                             had->had_mat, codes, sx, out, mode, scale_fp16, ex));                                     \
+  }
         switch (plan.R) {
           case 2: DQ_HAD28(64); break;
           case 4: DQ_HAD28(128); break;

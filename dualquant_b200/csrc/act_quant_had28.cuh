@@ -84,19 +84,22 @@ struct Had28 {
 // and the codes, four neighbours a thread at a time.  Element o of a segment sits at o ^ ((o & 32) >> 3), so that the 16-byte
 // accesses of eight lanes, two vectors apart in the load pass, touch every bank once.
 // The factor is compiled in; a CTA compares the caller's matrix with it and takes coefficients from memory if they differ.
-template <int P, typename XT, bool BESIDE = false>
+// EXPAND: some of the CTAs expand a weight instead (expand_w_e4m3.cuh).
+template <int P, typename XT, bool EXPAND = false>
 __global__ void __launch_bounds__(kHad28Threads, 3)
 act_quant_had28_kernel(const XT* __restrict__ x, const XT* __restrict__ up, int64_t ldx, const float* __restrict__ a, int M,
                        float had_scale, const float* __restrict__ had_mat, int8_t* __restrict__ codes,
-                       float* __restrict__ sx, float* __restrict__ out, int mode, int scale_fp16) {
+                       float* __restrict__ sx, float* __restrict__ out, int mode, int scale_fp16, const ExpansionShare ex) {
   using H = Had28<P>;
   constexpr int T = kHad28Threads, K = 28 * P, V = P / 8;
   extern __shared__ float sm_row[];
   __shared__ float red[T / 32];
   grid_dep_launch_dependents();
-  wait_at_start<BESIDE>();
+  grid_dep_wait();
   const int tid = threadIdx.x;
-  const int row0 = blockIdx.x * H::kRows;
+  const int cta = EXPAND ? quantiser_cta<T>(ex) : static_cast<int>(blockIdx.x);
+  if (EXPAND && cta < 0) return;
+  const int row0 = cta * H::kRows;
 
   bool known = true;
 #pragma unroll
@@ -231,8 +234,6 @@ act_quant_had28_kernel(const XT* __restrict__ x, const XT* __restrict__ up, int6
       emit8(v, tq, mode, crow, orow, o, scale_fp16);
     }
   }
-  // (a CTA's first row exists, so some of its threads get here)
-  wait_at_end<BESIDE>();
 }
 
 }  // namespace

@@ -7,8 +7,8 @@ int init_had_fast_f32() { return init_had_fast_t<float>(); }
 
 int launch_had_fast(const float* x, const float* up, int64_t ldx, const float* a, const dq_hadamard_desc* had,
                     int M, int K, size_t smem, int8_t* codes, float* sx, float* out, int mode, int scale_fp16,
-                    cudaStream_t stream, bool* taken, bool beside_expansion) {
-  return launch_had_fast_t<float>(x, up, ldx, a, had, M, K, smem, codes, sx, out, mode, scale_fp16, stream, taken, beside_expansion);
+                    cudaStream_t stream, bool* taken, Along* along) {
+  return launch_had_fast_t<float>(x, up, ldx, a, had, M, K, smem, codes, sx, out, mode, scale_fp16, stream, taken, along);
 }
 
 }  // namespace dq

@@ -26,19 +26,21 @@ namespace dq {
 // being re-expanded from the raw row (few-rows shape, where occupancy hides latency).  Four vectors a thread: 1024 threads
 // of 64 registers per SM; at the 76 that the compiler takes by itself a tenth fewer rows are in flight and 2048 rows need a
 // third round (2048 rows of 4096 with RMSNorm 14.2 -> 11.5 us, 8192 rows 41.7 -> 35.3).
-template <int THREADS, int VPT, typename XT, bool KEEP = false, bool BESIDE = false>
+// EXPAND: some of the CTAs expand a weight instead (expand_w_e4m3.cuh).
+template <int THREADS, int VPT, typename XT, bool KEEP = false, bool EXPAND = false>
 __global__ void __launch_bounds__(THREADS, (THREADS >= 512 && VPT <= 2) ? (KEEP ? 1 : 2048 / THREADS) : VPT >= 4 ? 1024 / THREADS : 1)
 act_quant_rows_kernel(const XT* __restrict__ x, int64_t ldx, const float* __restrict__ a, int K,
                       int8_t* __restrict__ codes, float* __restrict__ sx, float* __restrict__ out,
                       int mode, int scale_fp16, const __nv_bfloat16* __restrict__ norm_w,
-                      float norm_eps) {
+                      float norm_eps, const ExpansionShare ex) {
   __shared__ float red[THREADS / 32], red_max[THREADS / 32];
   // the GEMM that consumes the codes may be launched programmatically: let it start streaming
   // its weights now; it waits for this grid before it touches codes / sx
   grid_dep_launch_dependents();
   // x may come from the kernel before this one; codes / sx may still be read by it
-  wait_at_start<BESIDE>();
-  const int row = blockIdx.x;
+  grid_dep_wait();
+  const int row = EXPAND ? quantiser_cta<THREADS>(ex) : static_cast<int>(blockIdx.x);
+  if (EXPAND && row < 0) return;
   const XT* xr = x + static_cast<int64_t>(row) * ldx;
   // The row is held in registers in its input width (bf16: 4 registers per 8 elements) and
   // expanded once per pass - sum of squares (with a norm), absmax, codes - with identical
@@ -134,7 +136,6 @@ act_quant_rows_kernel(const XT* __restrict__ x, int64_t ldx, const float* __rest
       }
     }
   }
-  wait_at_end<BESIDE>();
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -328,10 +329,10 @@ act_quant_had_big_kernel(const XT* __restrict__ x, const XT* __restrict__ up, in
 // type): their unrolled matrix stages dominate the build time.
 int launch_had_fast(const __nv_bfloat16* x, const __nv_bfloat16* up, int64_t ldx, const float* a,
                     const dq_hadamard_desc* had, int M, int K, size_t smem, int8_t* codes, float* sx, float* out,
-                    int mode, int scale_fp16, cudaStream_t stream, bool* taken, bool beside_expansion);
+                    int mode, int scale_fp16, cudaStream_t stream, bool* taken, Along* along);
 int launch_had_fast(const float* x, const float* up, int64_t ldx, const float* a, const dq_hadamard_desc* had,
                     int M, int K, size_t smem, int8_t* codes, float* sx, float* out, int mode, int scale_fp16,
-                    cudaStream_t stream, bool* taken, bool beside_expansion);
+                    cudaStream_t stream, bool* taken, Along* along);
 int init_had_fast_bf16();
 int init_had_fast_f32();
 
@@ -392,7 +393,7 @@ template <typename XT>
 static int launch_act(const XT* x, int64_t ldx, const float* a, const dq_hadamard_desc* had, int M,
                       int K, int8_t* codes, float* sx, float* out, int mode, int scale_fp16,
                       cudaStream_t stream, const XT* up = nullptr,
-                      const __nv_bfloat16* norm_w = nullptr, float norm_eps = -1.f, bool beside_expansion = false) {
+                      const __nv_bfloat16* norm_w = nullptr, float norm_eps = -1.f, Along* along = nullptr) {
   DQ_REQUIRE(x != nullptr, DQ_ERR_NULL, "x is null");
   DQ_REQUIRE(M >= 0 && K >= 8 && K % 8 == 0, DQ_ERR_SHAPE, "bad shape M=%d K=%d (K %% 8 != 0)", M, K);
   DQ_REQUIRE(ldx >= K && ldx % 8 == 0, DQ_ERR_ALIGN, "ldx=%lld must be >= K and a multiple of 8",
@@ -428,7 +429,7 @@ static int launch_act(const XT* x, int64_t ldx, const float* a, const dq_hadamar
                "row of K=%d does not fit in shared memory", K);
     if (use_had) {
       bool taken = false;
-      const int rc2 = launch_had_fast(x, up, ldx, a, had, M, K, smem, codes, sx, out, mode, scale_fp16, stream, &taken, beside_expansion);
+      const int rc2 = launch_had_fast(x, up, ldx, a, had, M, K, smem, codes, sx, out, mode, scale_fp16, stream, &taken, along);
       if (taken) return rc2;
     }
     DQ_CHECK_CUDA(launch_pdl(act_quant_had_kernel<kHadThreads, XT>, dim3(M), dim3(kHadThreads), smem,
@@ -440,14 +441,16 @@ static int launch_act(const XT* x, int64_t ldx, const float* a, const dq_hadamar
     // thread holds few elements and many warps are resident to hide the load -> reduce -> store
     // latency chain
     const int vec = K / 8;
-    // (beside an expansion: see quant_act_int4_can_run_beside)
+    // (an expansion goes with the launch shapes of a prefill batch)
 #define DQ_ROWS_LAUNCH_K(T, V, KP)                                                                                       \
   do {                                                                                                                   \
-    constexpr bool kCanBeside = sizeof(XT) == 2 && ((V) >= 4 || ((KP) && (T) <= 512));                                   \
-    DQ_CHECK_CUDA(launch_pdl(beside_expansion ? act_quant_rows_kernel<T, V, XT, KP, kCanBeside>                          \
-                                              : act_quant_rows_kernel<T, V, XT, KP, false>,                              \
-                             dim3(M), dim3(T), 0, stream, x, ldx, a, K, codes, sx, out, mode, scale_fp16, norm_w,        \
-                             norm_eps));                                                                                 \
+    constexpr bool kExpand = sizeof(XT) == 2 && ((V) >= 4 || ((KP) && (T) <= 512));                                      \
+    ExpansionShare ex = {};                                                                                              \
+    const bool both = kExpand && along != nullptr;                                                                       \
+    const unsigned grid = both ? along->take(T, M, &ex) : static_cast<unsigned>(M);                                      \
+    DQ_CHECK_CUDA(launch_pdl(both ? act_quant_rows_kernel<T, V, XT, KP, kExpand> : act_quant_rows_kernel<T, V, XT, KP>,  \
+                             dim3(grid), dim3(T), 0, stream, x, ldx, a, K, codes, sx, out, mode, scale_fp16, norm_w,     \
+                             norm_eps, ex));                                                                             \
   } while (false)
 #define DQ_ROWS_LAUNCH(T, V) DQ_ROWS_LAUNCH_K(T, V, false)
     constexpr int kBigM = 1024;
@@ -481,20 +484,18 @@ static int launch_act(const XT* x, int64_t ldx, const float* a, const dq_hadamar
   return DQ_OK;
 }
 
-// Rows in registers in the launch shapes of a prefill batch, and 28 * 64 ... 28 * 512 values with the online Hadamard.  (Across
-// heads the kernel fills the SM by itself: 2048 rows of 4096 lost 1 % beside an expansion.)
-bool quant_act_int4_can_run_beside(const dq_hadamard_desc* had, int M, int K) {
-  const int vec = K / 8;
-  if (had == nullptr || had->kind == DQ_HAD_NONE) return M >= 1024 ? vec > 128 && vec <= 2048 : vec <= 512;
-  return had->kind == DQ_HAD_FULL && had->had_k == 28 && K % 28 == 0 && K / 28 >= 64 && K / 28 <= 512 && M > 64;
-}
-
-int quant_act_int4_beside_expansion(const void* x_bf16, int64_t ldx, const float* a, const dq_hadamard_desc* had, int M, int K,
-                                    int8_t* codes, float* sx, int scale_fp16, cudaStream_t stream) {
+// Rows in registers in the launch shapes of a prefill batch, and 28 * 64 ... 28 * 512 values with the online Hadamard, take the
+// expansion along; behind any other quantiser it is a launch of its own.  (Across heads the kernel fills the SM by itself: 2048
+// rows of 4096 lost 1 % beside an expansion.)
+int quant_act_int4_and_expand(const void* x_bf16, int64_t ldx, const float* a, const dq_hadamard_desc* had, int M, int K,
+                              int8_t* codes, float* sx, int scale_fp16, const WeightExpansion& e, cudaStream_t stream) {
   if (current_state() == nullptr) return DQ_ERR_NOT_INIT;
   DQ_REQUIRE(codes != nullptr && sx != nullptr, DQ_ERR_NULL, "codes / sx is null");
-  return launch_act(static_cast<const __nv_bfloat16*>(x_bf16), ldx, a, had, M, K, codes, sx, nullptr, MODE_CODES, scale_fp16,
-                    stream, static_cast<const __nv_bfloat16*>(nullptr), static_cast<const __nv_bfloat16*>(nullptr), -1.f, true);
+  Along along = {e, false};
+  const int rc = launch_act(static_cast<const __nv_bfloat16*>(x_bf16), ldx, a, had, M, K, codes, sx, nullptr, MODE_CODES,
+                            scale_fp16, stream, static_cast<const __nv_bfloat16*>(nullptr),
+                            static_cast<const __nv_bfloat16*>(nullptr), -1.f, &along);
+  return rc != DQ_OK || along.done ? rc : launch_expand_w_e4m3(e, stream);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -104,13 +104,16 @@ enum {
 };
 int tuning(int key);
 
-int launch_expand_w_e4m3(const uint8_t* w_packed, int N, int K, uint8_t* w8, int per_sm, cudaStream_t stream,
-                         DeviceState* st);
-// dq_quant_act_int4 directly behind launch_expand_w_e4m3 on the same stream, running beside it; whether its kernel for such a
-// call can.
-bool quant_act_int4_can_run_beside(const dq_hadamard_desc* had, int M, int K);
-int quant_act_int4_beside_expansion(const void* x_bf16, int64_t ldx, const float* a, const dq_hadamard_desc* had, int M, int K,
-                                    int8_t* codes, float* sx, int scale_fp16, cudaStream_t stream);
+// The byte form of a packed weight, made by a linear for the GEMM behind its quantiser.
+struct WeightExpansion {
+  const uint8_t* w_packed;
+  uint8_t* w8;
+  int N, K;
+};
+int launch_expand_w_e4m3(const WeightExpansion& e, cudaStream_t stream);
+// dq_quant_act_int4 and an expansion: one kernel that does both where the quantiser's can take the expansion along.
+int quant_act_int4_and_expand(const void* x_bf16, int64_t ldx, const float* a, const dq_hadamard_desc* had, int M, int K,
+                              int8_t* codes, float* sx, int scale_fp16, const WeightExpansion& e, cudaStream_t stream);
 
 // One-time kernel attribute set-up of each translation unit (called from dq_init).
 int init_gemm_int4_kernels();

@@ -18,6 +18,7 @@
 // The kernel (gemm_w4a4_int4_f8.cuh) works on tiles of 256 weight rows x TN tokens on a pair of CTAs; this file
 // holds the operand conversions, the choice of TN and the C entry points.
 #include "gemm_w4a4_int4_f8.cuh"
+#include "expand_w_e4m3.cuh"
 
 namespace dq {
 namespace f8 {
@@ -34,66 +35,17 @@ cudaError_t init_out2();
 cudaError_t init_out3();
 cudaError_t init_out5();
 
-// Four two's-complement nibbles (bits 0-15 of sel) -> four E4M3 bytes of the same integers.
-// Non-negative codes 0..7: 00 38 40 44 48 4A 4C 4E; negative codes -8..-1: D0 CE CC CA C8 C4 C0 B8.
-// The byte permute takes the nibbles as selectors: its low three bits look up a magnitude, and where the fourth (the
-// sign) is set it replicates the sign bit of the byte looked up - so one permute over bytes of 0x80 gives 0x80 for a
-// non-negative code and 0xFF for a negative one, and that selects between the two tables and makes the sign bit.
-__device__ __forceinline__ uint32_t e4m3x4_of_nibbles(uint32_t sel) {
-  const uint32_t s3 = sel & 0x7777u;
-  const uint32_t pos = __byte_perm(0x44403800u, 0x4E4C4A48u, s3);
-  const uint32_t neg = __byte_perm(0x4A4C4E50u, 0x38404448u, s3);  // magnitudes
-  uint32_t r;
-  asm("prmt.b32 %0, %1, %1, %2;" : "=r"(r) : "r"(0x80808080u), "r"(sel));
-  return (pos & ~r) | (neg & r & 0x7F7F7F7Fu) | ((r << 7) & 0x80808080u);
-}
-// A packed word of the artefact (low nibbles: four consecutive k, high nibbles: the four sixteen further on) -> both fours
-__device__ __forceinline__ void e4m3_of_word(uint32_t w, uint32_t& lo, uint32_t& hi) {
-  const uint32_t a = e4m3x4_of_nibbles(w), b = e4m3x4_of_nibbles(w >> 16);  // lo0 hi0 lo1 hi1 | lo2 hi2 lo3 hi3
-  lo = __byte_perm(a, b, 0x6420);
-  hi = __byte_perm(a, b, 0x7531);
-}
 // the low nibbles of the four bytes of v, packed into bits 0-15
 __device__ __forceinline__ uint32_t low_nibbles(uint32_t v) {
   return (v & 0xFu) | ((v >> 4) & 0xF0u) | ((v >> 8) & 0xF00u) | ((v >> 12) & 0xF000u);
 }
 
-// packed int4 tiles -> E4M3 bytes, row-major [N, K]: CTAs walk over the 16-byte chunks (32 codes), AHEAD in flight per
-// thread.  beside: the next kernel is started only once every CTA has seen the kernels before this one finish, so that it
-// need not wait for this one before it works (wait_at_start in act_quant_common.cuh).
+// An expansion on its own: a thread per chunk.
 constexpr int kExpandThreads = 256;
-template <int AHEAD>
-__global__ void __launch_bounds__(kExpandThreads) expand_w_e4m3_kernel(const uint8_t* __restrict__ w_packed, int N, int K,
-                                                                       uint8_t* __restrict__ w8, int beside) {
-  if (!beside) grid_dep_launch_dependents();
+__global__ void __launch_bounds__(kExpandThreads) expand_w_e4m3_kernel(const WeightExpansion e) {
+  grid_dep_launch_dependents();
   grid_dep_wait();
-  if (beside) grid_dep_launch_dependents();
-  const uint32_t groups = static_cast<uint32_t>(K / kGroup);
-  const int64_t total = static_cast<int64_t>((N + 127) / 128) * groups * 512;
-  const int64_t step = static_cast<int64_t>(gridDim.x) * kExpandThreads;
-  for (int64_t c0 = static_cast<int64_t>(blockIdx.x) * kExpandThreads + threadIdx.x; c0 < total; c0 += AHEAD * step) {
-    uint4 raw[AHEAD];
-#pragma unroll
-    for (int i = 0; i < AHEAD; ++i) {
-      const int64_t c = c0 + i * step;
-      if (c < total) raw[i] = *reinterpret_cast<const uint4*>(w_packed + (c >> 9) * kTileBytes + (c & 511) * 16);
-    }
-#pragma unroll
-    for (int i = 0; i < AHEAD; ++i) {
-      const int64_t c = c0 + i * step;
-      const uint32_t r = static_cast<uint32_t>(c >> 2) & 127, ch = (static_cast<uint32_t>(c) & 3) ^ ((r >> 1) & 3);
-      const uint32_t tg = static_cast<uint32_t>(c >> 9), tile = tg / groups, g = tg - tile * groups;
-      const int64_t row = static_cast<int64_t>(tile) * 128 + r;
-      if (c >= total || row >= N) continue;
-      const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
-      uint32_t lo[4], hi[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) e4m3_of_word(w[j], lo[j], hi[j]);  // k = 4j .. 4j+3 of the chunk, k = 16 + 4j ..
-      uint8_t* dst = w8 + row * K + (g * 4 + ch) * 32;
-      *reinterpret_cast<uint4*>(dst) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-      *reinterpret_cast<uint4*>(dst + 16) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-    }
-  }
+  expand_chunks<kExpandThreads, 1>(e, blockIdx.x);
 }
 
 // int8 codes (-8..7) [M, K] with row stride ld -> E4M3 bytes [M, K]; one thread per 16 codes
@@ -228,14 +180,9 @@ int launch_gemm_int4_e4m3(const uint8_t* x8, const float* sx, const uint8_t* w8,
   return launch_gemm_int4_e4m3_impl(x8, sx, w8, sw_t, r, M, N, K, y, y_dtype, add, stream, st, nullptr);
 }
 
-// per_sm: CTAs per SM of an expansion with a quantiser beside it; 0: on its own, a thread per chunk.
-int launch_expand_w_e4m3(const uint8_t* w_packed, int N, int K, uint8_t* w8, int per_sm, cudaStream_t stream,
-                         DeviceState* st) {
-  int64_t ctas = (static_cast<int64_t>((N + 127) / 128) * (K / kGroup) * 512 + f8::kExpandThreads - 1) / f8::kExpandThreads;
-  if (per_sm > 0 && ctas > per_sm * st->sm_count) ctas = per_sm * st->sm_count;
-  DQ_CHECK_CUDA(launch_pdl(per_sm > 0 ? f8::expand_w_e4m3_kernel<4> : f8::expand_w_e4m3_kernel<1>,
-                           dim3(static_cast<unsigned>(ctas)), dim3(f8::kExpandThreads), 0, stream, w_packed, N, K, w8,
-                           per_sm > 0 ? 1 : 0));
+int launch_expand_w_e4m3(const WeightExpansion& e, cudaStream_t stream) {
+  DQ_CHECK_CUDA(launch_pdl(f8::expand_w_e4m3_kernel, dim3(static_cast<unsigned>(expand_ctas(e.N, e.K, f8::kExpandThreads))),
+                           dim3(f8::kExpandThreads), 0, stream, e));
   return DQ_OK;
 }
 
@@ -280,7 +227,7 @@ extern "C" int dq_expand_w_int4_e4m3(const uint8_t* w_packed, int N, int K, int 
   DQ_REQUIRE(G == kGroup, DQ_ERR_UNSUPPORTED, "weight group size must be %d (got %d)", kGroup, G);
   DQ_REQUIRE(N >= 1 && K >= kGroup && K % kGroup == 0, DQ_ERR_SHAPE, "bad shape N=%d K=%d", N, K);
   DQ_REQUIRE(aligned(w_packed, 16) && aligned(w8, 16), DQ_ERR_ALIGN, "w_packed and w8 must be 16-byte aligned");
-  return launch_expand_w_e4m3(w_packed, N, K, w8, 0, static_cast<cudaStream_t>(stream), st);
+  return launch_expand_w_e4m3({w_packed, w8, N, K}, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int dq_codes_to_e4m3(const int8_t* codes, int64_t ld, int M, int K, uint8_t* x8, void* stream) {

@@ -57,31 +57,20 @@ static int quant_and_gemm(const void* x_bf16, int64_t ldx, const float* a, const
   int8_t* codes = static_cast<int8_t*>(scratch);
   float* sx = reinterpret_cast<float*>(base + round_up(static_cast<size_t>(M) * K, 256));
   const dq::Addend add = {bias, 0};
-  uint8_t* expanded = nullptr;
-  bool beside = false;
   if (w8 == nullptr && G == dq::kGroup && (scale_fp16 & ~0xFF) == 0 && expansion_pays(M, N, K) &&
       scratch_bytes >= dq_linear_w4a4_int4_prefill_scratch_bytes(M, N, K)) {
-    expanded = base + dq_linear_w4a4_int4_scratch_bytes(M, N, K);
-    DQ_REQUIRE(w_packed != nullptr && dq::aligned(w_packed, 16), DQ_ERR_ALIGN, "w_packed is null or not 16-byte aligned");
-    dq::DeviceState* st = dq::current_state();
-    if (st == nullptr) return DQ_ERR_NOT_INIT;
-    // The quantiser may run beside the expansion, which streams memory where the quantiser computes.  Where the expansion is
-    // the smaller part it gets two CTAs per SM and the quantiser the rest; for a weight much wider than the batch it is most
-    // of the time and goes first.  us, one after the other / beside with two / with eight CTAs per SM:
-    //   1200 x 14336 ->  4096  147 / 127 / 139    1024 x 4096 ->  4096  33.0 / 30.1 / 31.4    2048 x 4096 -> 4096  49.5 / 47.8
-    //   1531 x 14336 ->  4096, Hadamard  160 / 157    768 x 4096 -> 4096  32.8 / 37.6 / 31.4    1024 x 4096 -> 8192  55 / 53 / 50
-    //    768 x 4096 -> 28672  135 / 171 / 140     900 x 4096 -> 12288  89.7 / 105 / 92.7    1300 x 4096 -> 18944  130 / 142 / 138
-    beside = N <= 12 * static_cast<int64_t>(M) && dq::quant_act_int4_can_run_beside(had, M, K);
-    const int rc = dq::launch_expand_w_e4m3(w_packed, N, K, expanded, !beside ? 0 : N <= 4 * static_cast<int64_t>(M) ? 2 : 8,
-                                            static_cast<cudaStream_t>(stream), st);
+    uint8_t* expanded = base + dq_linear_w4a4_int4_scratch_bytes(M, N, K);
+    DQ_REQUIRE(w_packed != nullptr, DQ_ERR_NULL, "w_packed is null");
+    DQ_REQUIRE(dq::aligned(w_packed, 16), DQ_ERR_ALIGN, "w_packed must be 16-byte aligned");
+    const int rc = dq::quant_act_int4_and_expand(x_bf16, ldx, a, had, M, K, codes, sx, scale_fp16 | DQ_CODES_E4M3,
+                                                 {w_packed, expanded, N, K}, static_cast<cudaStream_t>(stream));
     if (rc != DQ_OK) return rc;
     w8 = expanded;
+  } else {
+    const int rc = dq_quant_act_int4(x_bf16, ldx, a, had, M, K, codes, sx,
+                                     scale_fp16 | (w8 != nullptr ? DQ_CODES_E4M3 : 0), stream);
+    if (rc != DQ_OK) return rc;
   }
-  const int mode = scale_fp16 | (w8 != nullptr ? DQ_CODES_E4M3 : 0);
-  const int rc = beside ? dq::quant_act_int4_beside_expansion(x_bf16, ldx, a, had, M, K, codes, sx, mode,
-                                                              static_cast<cudaStream_t>(stream))
-                        : dq_quant_act_int4(x_bf16, ldx, a, had, M, K, codes, sx, mode, stream);
-  if (rc != DQ_OK) return rc;
   if (w8 == nullptr)
     return dq::gemm_w4a4_int4_addend(codes, sx, w_packed, sw_t, r, add, M, N, K, G, y, y_dtype, stream);
   dq::DeviceState* st = dq::current_state();

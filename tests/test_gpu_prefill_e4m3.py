@@ -397,12 +397,16 @@ def test_expanding_linear_equals_the_packed_kernel_over_its_options(M, N, had, m
     _lib.device_status(0)
 
 
-# The quantiser of these calls runs beside the expansion of the weight - rows in registers (128, 256 and 256 long ones, and 512
-# threads of one vector), 28 * 512 - or behind it (across heads, 2048 = 32 * 64).  Inputs written and scratch read by the
-# kernels just before; the packed path, which expands nothing, gives the same bits.
+# The quantisers of these calls take the expansion of the weight along - rows in registers (128 threads, 256, 256 for long rows;
+# under 1024 rows 512 and 256 threads of one vector), 28 * 512, 28 * 64 with eight rows a CTA - or leave it to a launch of its own
+# (across heads, 2048 = 32 * 64).  Weights of one row, one tile and two: fewer CTAs expand than there are SMs; 18000 rows: most
+# of them do.  Inputs written and scratch read by the kernels just before; the packed path, which expands nothing, gives the
+# same bits.
 @pytest.mark.parametrize("M,K,N,kind", [(1024, 4096, 1024, None), (1030, 8192, 512, None), (1026, 14336, 512, None),
-                                        (700, 4096, 4096, None), (1100, 4096, 4096, "heads"), (1031, 14336, 1024, "full"),
-                                        (1200, 2048, 768, "full")])
+                                        (700, 4096, 4096, None), (600, 2048, 8192, None), (1100, 4096, 4096, "heads"),
+                                        (1031, 14336, 1024, "full"), (1200, 2048, 768, "full"), (1024, 1792, 300, "full"),
+                                        (1025, 4096, 1, None), (1090, 14336, 128, None), (1024, 8192, 130, None),
+                                        (1029, 14336, 256, "full"), (1027, 1792, 16, "full"), (1024, 1152, 18000, None)])
 def test_linear_beside_the_expansion_of_its_weight(M, K, N, kind):
     had = None
     if kind == "heads":
@@ -426,3 +430,21 @@ def test_linear_beside_the_expansion_of_its_weight(M, K, N, kind):
         got.append(ops.linear_w4a4_int4(x, a, had, pws[i % 2], None, scratch=big))
     _lib.device_status(0)
     assert all(torch.equal(y, want[i % 3][i % 2]) for i, y in enumerate(got))
+
+
+def test_one_call_linear_refuses_an_expansion_of_nothing():
+    """A batch whose weight is expanded: a null packed weight and a misaligned one are refused by their own codes."""
+    M, K, N = 1024, 1792, 256
+    x = torch.randn(M, K, device=DEV).to(torch.bfloat16)
+    sw_t = torch.ones(K // 128, N, dtype=torch.float16, device=DEV)
+    w = torch.zeros(N * K, dtype=torch.uint8, device=DEV)
+    y = torch.full((M, N), 3.0, device=DEV)
+    scratch = torch.empty(ops.linear_scratch_bytes(M, N, K), dtype=torch.uint8, device=DEV)
+    lib, stream = _lib.load(), torch.cuda.current_stream().cuda_stream
+    for packed, error in ((None, "DQ_ERR_NULL"), (w.data_ptr() + 8, "DQ_ERR_ALIGN")):
+        rc = lib.dq_linear_w4a4_int4(x.data_ptr(), K, None, None, packed, sw_t.data_ptr(), None, M, N, K, 128, y.data_ptr(),
+                                     _lib.DTYPE_F32, 0, scratch.data_ptr(), scratch.numel(), stream)
+        with pytest.raises((ValueError, RuntimeError), match=error):
+            _lib.check(rc, "dq_linear_w4a4_int4")
+    _lib.device_status(0)
+    assert bool((y == 3.0).all())
