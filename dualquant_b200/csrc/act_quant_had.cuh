@@ -138,8 +138,8 @@ __device__ __forceinline__ void matrix_rows_dispatch(int qi, const float2* v, fl
 // own, act_quant_had28.cuh), so that the matrix stage has no padded terms; 0 = any order up to 32.
 template <int R, typename XT, int THREADS, int HS = 0>
 __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 3 : 1)
-act_quant_had_fast_kernel(const XT* __restrict__ x, const XT* __restrict__ up, int64_t ldx,
-                          const float* __restrict__ a, int K,
+act_quant_had_fast_kernel(const XT* x, const XT* up, int64_t ldx,
+                          const float* a, int K,
                           int S, int inner, int matrix, float had_scale, int8_t* __restrict__ codes,
                           float* __restrict__ sx, float* __restrict__ out, int mode, int scale_fp16) {
   extern __shared__ float sm_row[];
@@ -340,8 +340,8 @@ constexpr int kHadClusterMaxRows = 64;
 
 template <int R, typename XT>
 __global__ void __launch_bounds__(kHadClusterThreads, 1)
-act_quant_had_cluster_kernel(const XT* __restrict__ x, const XT* __restrict__ up, int64_t ldx,
-                             const float* __restrict__ a, int S, float had_scale, const float* __restrict__ had_mat,
+act_quant_had_cluster_kernel(const XT* x, const XT* up, int64_t ldx,
+                             const float* a, int S, float had_scale, const float* had_mat,
                              int8_t* __restrict__ codes, float* __restrict__ sx, float* __restrict__ out, int mode,
                              int scale_fp16) {
   constexpr int P = 32 * R;                   // segment length
@@ -475,7 +475,7 @@ struct HeadsRow {
 
 template <int S, typename XT, bool E4M3>
 __global__ void __launch_bounds__(HeadsRow<S>::kThreads, HeadsRow<S>::kCtas)
-act_quant_had_heads_kernel(const XT* __restrict__ x, int64_t ldx, const float* __restrict__ a, int M, float had_scale,
+act_quant_had_heads_kernel(const XT* x, int64_t ldx, const float* a, int M, float had_scale,
                            int8_t* __restrict__ codes, float* __restrict__ sx, int scale_fp16) {
   using H = HeadsRow<S>;
   constexpr int HL = H::kHeads, C = H::kCols, CL = H::kLanes;

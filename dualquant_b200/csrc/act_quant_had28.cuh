@@ -87,8 +87,8 @@ struct Had28 {
 // EXPAND: some of the CTAs expand a weight instead (expand_w_e4m3.cuh).
 template <int P, typename XT, bool EXPAND = false>
 __global__ void __launch_bounds__(kHad28Threads, 3)
-act_quant_had28_kernel(const XT* __restrict__ x, const XT* __restrict__ up, int64_t ldx, const float* __restrict__ a, int M,
-                       float had_scale, const float* __restrict__ had_mat, int8_t* __restrict__ codes,
+act_quant_had28_kernel(const XT* x, const XT* up, int64_t ldx, const float* a, int M,
+                       float had_scale, const float* had_mat, int8_t* __restrict__ codes,
                        float* __restrict__ sx, float* __restrict__ out, int mode, int scale_fp16, const ExpansionShare ex) {
   using H = Had28<P>;
   constexpr int T = kHad28Threads, K = 28 * P, V = P / 8;
@@ -188,7 +188,7 @@ act_quant_had28_kernel(const XT* __restrict__ x, const XT* __restrict__ up, int6
         float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
         for (int j = 0; j < 28; ++j) {
-          const float h = __ldg(had_mat + i * 28 + j);
+          const float h = had_mat[i * 28 + j];
           acc = __ffma2_rn(make_float2(h, h), v[j], acc);
         }
         *reinterpret_cast<float2*>(col + i * H::kPitch) = acc;

@@ -24,8 +24,8 @@ __host__ __device__ constexpr int big_smem(int had_k, int rpw) { return had_k * 
 // 1108 -> 248; 13824, 8 rows 68 -> 12.5, 2048 954 -> 226; 5120 = 40 * 128, 2048 rows 195 -> 74.
 template <int RPW, typename XT>
 __global__ void __launch_bounds__(kBigThreads, 1)
-act_quant_had_wide_kernel(const XT* __restrict__ x, const XT* __restrict__ up, int64_t ldx, const float* __restrict__ a, int M,
-                          int K, int had_k, float had_scale, const float* __restrict__ had_mat, int split,
+act_quant_had_wide_kernel(const XT* x, const XT* up, int64_t ldx, const float* a, int M,
+                          int K, int had_k, float had_scale, const float* had_mat, int split,
                           int8_t* __restrict__ codes, float* __restrict__ sx, float* __restrict__ out, int mode,
                           int scale_fp16) {
   constexpr int RP = (RPW + 3) / 4 * 4, kPitch = big_pitch(RPW);

@@ -29,9 +29,9 @@ namespace dq {
 // EXPAND: some of the CTAs expand a weight instead (expand_w_e4m3.cuh).
 template <int THREADS, int VPT, typename XT, bool KEEP = false, bool EXPAND = false>
 __global__ void __launch_bounds__(THREADS, (THREADS >= 512 && VPT <= 2) ? (KEEP ? 1 : 2048 / THREADS) : VPT >= 4 ? 1024 / THREADS : 1)
-act_quant_rows_kernel(const XT* __restrict__ x, int64_t ldx, const float* __restrict__ a, int K,
+act_quant_rows_kernel(const XT* x, int64_t ldx, const float* a, int K,
                       int8_t* __restrict__ codes, float* __restrict__ sx, float* __restrict__ out,
-                      int mode, int scale_fp16, const __nv_bfloat16* __restrict__ norm_w,
+                      int mode, int scale_fp16, const __nv_bfloat16* norm_w,
                       float norm_eps, const ExpansionShare ex) {
   __shared__ float red[THREADS / 32], red_max[THREADS / 32];
   // the GEMM that consumes the codes may be launched programmatically: let it start streaming
@@ -163,10 +163,10 @@ constexpr int kMaxHadK = 32;
 
 template <int THREADS, typename XT>
 __global__ void __launch_bounds__(THREADS)
-act_quant_had_kernel(const XT* __restrict__ x, const XT* __restrict__ up, int64_t ldx,
-                     const float* __restrict__ a, int K,
+act_quant_had_kernel(const XT* x, const XT* up, int64_t ldx,
+                     const float* a, int K,
                      int had_kind, int had_k, int had_dim, float had_scale,
-                     const float* __restrict__ had_mat, int8_t* __restrict__ codes,
+                     const float* had_mat, int8_t* __restrict__ codes,
                      float* __restrict__ sx, float* __restrict__ out, int mode, int scale_fp16) {
   extern __shared__ float sm_row[];
   __shared__ float red[THREADS / 32];
@@ -260,9 +260,9 @@ constexpr int kMaxHadKBig = 172;
 
 template <int THREADS, typename XT>
 __global__ void __launch_bounds__(THREADS)
-act_quant_had_big_kernel(const XT* __restrict__ x, const XT* __restrict__ up, int64_t ldx,
-                         const float* __restrict__ a, int K, int had_k, float had_scale,
-                         const float* __restrict__ had_mat, int8_t* __restrict__ codes,
+act_quant_had_big_kernel(const XT* x, const XT* up, int64_t ldx,
+                         const float* a, int K, int had_k, float had_scale,
+                         const float* had_mat, int8_t* __restrict__ codes,
                          float* __restrict__ sx, float* __restrict__ out, int mode, int scale_fp16) {
   extern __shared__ float sm_row[];
   __shared__ float red[THREADS / 32];
@@ -506,7 +506,7 @@ int quant_act_int4_and_expand(const void* x_bf16, int64_t ldx, const float* a, c
 // variant is not on the measured path).  round_away = 1 rounds halves away from zero like the
 // Triton kernel's libdevice.round, 0 rounds them to even like torch.round.
 __global__ void __launch_bounds__(256)
-act_quant_grouped_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, const float* __restrict__ a,
+act_quant_grouped_kernel(const __nv_bfloat16* x, int64_t ldx, const float* a,
                          int M, int K, int8_t* __restrict__ codes, float* __restrict__ sxg,
                          int scale_fp16, int round_away) {
   grid_dep_launch_dependents();

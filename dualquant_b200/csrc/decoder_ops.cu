@@ -27,10 +27,10 @@ __device__ __forceinline__ unsigned short float_to_bf16_bits(float v) {
 // grid: (B * S, heads = hq + 2 * hkv); block: head_dim / 2 threads (thread i owns elements i, i + d/2).
 // Token (b, s) sits in row b * S + s of qkv and goes to cache position pos0 + s, pos0 = *pos_ptr when
 // a device pointer is given (decode inside a captured graph), else the host value.
-__global__ void rope_kv_append_kernel(const unsigned short* __restrict__ qkv, int64_t ld_qkv,
-                                      const unsigned short* __restrict__ cos_tab,
-                                      const unsigned short* __restrict__ sin_tab,
-                                      const long long* __restrict__ pos_ptr, long long pos_host, int S,
+__global__ void rope_kv_append_kernel(const unsigned short* qkv, int64_t ld_qkv,
+                                      const unsigned short* cos_tab,
+                                      const unsigned short* sin_tab,
+                                      const long long* pos_ptr, long long pos_host, int S,
                                       int hq, int hkv, int hd, int max_len,
                                       unsigned short* __restrict__ q_out,
                                       unsigned short* __restrict__ k_cache,
@@ -80,10 +80,10 @@ __device__ __forceinline__ void unpack_bf16x8(const uint4& v, float (&f)[8]) {
 }
 
 __global__ void __launch_bounds__(128)
-rope_kv_append_vec_kernel(const unsigned short* __restrict__ qkv, int64_t ld_qkv,
-                          const unsigned short* __restrict__ cos_tab,
-                          const unsigned short* __restrict__ sin_tab,
-                          const long long* __restrict__ pos_ptr, long long pos_host, int S, int hq,
+rope_kv_append_vec_kernel(const unsigned short* qkv, int64_t ld_qkv,
+                          const unsigned short* cos_tab,
+                          const unsigned short* sin_tab,
+                          const long long* pos_ptr, long long pos_host, int S, int hq,
                           int hkv, int hd, int max_len, unsigned short* __restrict__ q_out,
                           unsigned short* __restrict__ k_cache, unsigned short* __restrict__ v_cache) {
   grid_dep_launch_dependents();

@@ -418,6 +418,10 @@ __device__ __forceinline__ void grid_dep_launch_dependents() {
 }
 // Blocks until every kernel this one depends on has completed and its writes are visible.
 // A no-op for kernels launched without the attribute.
+// What is read behind the wait must not be a `const __restrict__` parameter nor go through __ldg: such loads count as constant
+// for the whole kernel, and the compiler may place them in front (seen behind a wait under a run-time condition).  Output
+// pointers keep their __restrict__, which is what lets ordinary loads pass the stores; the packed weight is read before the
+// wait on purpose; and warps that never wait themselves read the token scales behind a barrier that the waiting warp leads to.
 __device__ __forceinline__ void grid_dep_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }

@@ -117,7 +117,7 @@ __device__ __forceinline__ uint32_t nib2_to_f16x2(uint32_t t, __half2 s2) {
 template <int TN>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_a16w4_kernel(const uint8_t* __restrict__ w_packed, const __grid_constant__ CUtensorMap tm_x,
-                  const __grid_constant__ CUtensorMap tm_y, int bulk_store, const float* __restrict__ r,
+                  const __grid_constant__ CUtensorMap tm_y, int bulk_store, const float* r,
                   void* __restrict__ y, int y_bf16, int M, int N, int K, int row_pairs, int tok_tiles, int tok_block,
                   int split, int groups_per_split, int* status) {
   using C = Cfg<TN>;
@@ -428,8 +428,8 @@ gemm_a16w4_kernel(const uint8_t* __restrict__ w_packed, const __grid_constant__ 
 
 // xs[m, k] = fp16(float(x[m, k]) * a[k]) (a may be null), saturating at the fp16 range; inside every four k the order is
 // 0, 2, 1, 3 (see the unpack warps)
-__global__ void __launch_bounds__(256) scale_cols_f16_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx,
-                                                             const float* __restrict__ a, int M, int K,
+__global__ void __launch_bounds__(256) scale_cols_f16_kernel(const __nv_bfloat16* x, int64_t ldx,
+                                                             const float* a, int M, int K,
                                                              __half* __restrict__ xs) {
   grid_dep_launch_dependents();
   grid_dep_wait();

@@ -111,8 +111,8 @@ template <int NVFP4, bool BIAS, bool BF16>
 __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1)
 gemm_fp4_persist_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
                         const __grid_constant__ CUtensorMap tm_y, const __grid_constant__ CUtensorMap tm_sfw,
-                        const __grid_constant__ CUtensorMap tm_sfx, const float* __restrict__ r,
-                        const float* __restrict__ w_scale, const float* __restrict__ x_scale, const void* __restrict__ bias,
+                        const __grid_constant__ CUtensorMap tm_sfx, const float* r,
+                        const float* w_scale, const float* x_scale, const void* bias,
                         int M, int N, int K, const Tiles tiles, int* status) {
   using C = PCfg<BF16>;
   constexpr int kStages = C::kStages;
@@ -320,7 +320,7 @@ gemm_fp4_persist_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_c
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
             const int m = t0 + c0 + j;
-            const float tx = (x_scale != nullptr && m < M) ? __ldg(x_scale + m) : 1.f;
+            const float tx = (x_scale != nullptr && m < M) ? x_scale[m] : 1.f;
             const float val = __uint_as_float(v[k][j]) * (rn * tx);
             if constexpr (BF16)
               reinterpret_cast<__nv_bfloat16*>(buf)[j * kFBN + q * 32 + lane] = bf16_with_bias(val, BIAS ? bias : nullptr, bias_n);

@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(kExpandThreads) expand_w_e4m3_kernel(const Wei
 }
 
 // int8 codes (-8..7) [M, K] with row stride ld -> E4M3 bytes [M, K]; one thread per 16 codes
-__global__ void __launch_bounds__(256) codes_to_e4m3_kernel(const int8_t* __restrict__ codes, int64_t ld, int M,
+__global__ void __launch_bounds__(256) codes_to_e4m3_kernel(const int8_t* codes, int64_t ld, int M,
                                                             int K, uint8_t* __restrict__ x8) {
   grid_dep_launch_dependents();
   grid_dep_wait();

@@ -103,8 +103,8 @@ template <int TN, int OUT>
 __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1)
 gemm_w4a4_e4m3_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
                       const __grid_constant__ CUtensorMap tm_y, const __grid_constant__ CUtensorMap tm_res,
-                      const __half* __restrict__ sw_t, const float* __restrict__ r,
-                      const float* __restrict__ sx, void* __restrict__ y, int y_bf16,
+                      const __half* __restrict__ sw_t, const float* r,
+                      const float* sx, void* __restrict__ y, int y_bf16,
                       const Addend add, int M, int N, int K, int row_pairs, int tok_tiles,
                       int tok_block, int* status, const __grid_constant__ ScatterDst sc) {
   using C = Cfg<TN>;
@@ -242,7 +242,7 @@ gemm_w4a4_e4m3_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
       tile_of(it, row_tile, tok_tile);
       const int n = row_tile * kBN + q * 32 + lane;
       const int t0 = tok_tile * kTN;
-      if (bulk_out && tid < kTN) sx_sm[(it & 1) * kTN + tid] = (t0 + tid < M) ? __ldg(sx + t0 + tid) : 0.f;
+      if (bulk_out && tid < kTN) sx_sm[(it & 1) * kTN + tid] = (t0 + tid < M) ? sx[t0 + tid] : 0.f;
 #pragma unroll
       for (int j = 0; j < kCPW; ++j) run[j] = 0.f;
       // (a row tile past the last one is computed on zeros and not stored: any scales will do)

@@ -94,7 +94,7 @@ __device__ __forceinline__ uint32_t cluster_ctaid_z() {
 }
 
 // 8 bf16 (one 16-byte vector) -> 8 floats, times 8 entries of the column scale (or 1)
-__device__ __forceinline__ void expand_scale8(const uint4& raw, const float* __restrict__ a_ptr,
+__device__ __forceinline__ void expand_scale8(const uint4& raw, const float* a_ptr,
                                               float* v) {
   const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
@@ -103,8 +103,8 @@ __device__ __forceinline__ void expand_scale8(const uint4& raw, const float* __r
     v[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
   }
   if (a_ptr != nullptr) {
-    const float4 a0 = __ldg(reinterpret_cast<const float4*>(a_ptr));
-    const float4 a1 = __ldg(reinterpret_cast<const float4*>(a_ptr + 4));
+    const float4 a0 = *reinterpret_cast<const float4*>(a_ptr);
+    const float4 a1 = *reinterpret_cast<const float4*>(a_ptr + 4);
     v[0] = __fmul_rn(v[0], a0.x); v[1] = __fmul_rn(v[1], a0.y);
     v[2] = __fmul_rn(v[2], a0.z); v[3] = __fmul_rn(v[3], a0.w);
     v[4] = __fmul_rn(v[4], a1.x); v[5] = __fmul_rn(v[5], a1.y);
@@ -116,8 +116,8 @@ __device__ __forceinline__ void expand_scale8(const uint4& raw, const float* __r
 // registers between the absmax pass and the code pass.
 template <int NT, int U>
 __global__ void __launch_bounds__(kThreads, (U <= 2) ? 3 : 2)
-gemv_fused_kernel(const uint8_t* __restrict__ w_packed, const __nv_bfloat16* __restrict__ x,
-                  int64_t ldx, const float* __restrict__ a, const float* __restrict__ r,
+gemv_fused_kernel(const uint8_t* __restrict__ w_packed, const __nv_bfloat16* x,
+                  int64_t ldx, const float* a, const float* r,
                   void* __restrict__ y, int y_bf16, const Addend add, int M, int N,
                   int K, int groups_per_split, int split_k, int cx, int stages, int scale_fp16,
                   int* status) {
@@ -219,7 +219,7 @@ gemv_fused_kernel(const uint8_t* __restrict__ w_packed, const __nv_bfloat16* __r
         if (live && unit < units_per_row) {
           const uint4* p = reinterpret_cast<const uint4*>(xrow + unit * 32);
 #pragma unroll
-          for (int q = 0; q < 4; ++q) raw[u][q] = __ldg(p + q);
+          for (int q = 0; q < 4; ++q) raw[u][q] = p[q];
         } else {
 #pragma unroll
           for (int q = 0; q < 4; ++q) raw[u][q] = make_uint4(0u, 0u, 0u, 0u);

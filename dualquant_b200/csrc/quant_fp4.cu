@@ -194,8 +194,8 @@ struct Fp4Raw<float> {
 // again in the second pass (from L1).  PER_SM CTAs' worth of registers.
 template <int THREADS, int VPT, int PER_SM, typename XT>
 __global__ void __launch_bounds__(THREADS, PER_SM)
-quant_fp4_kernel(const XT* __restrict__ x, int64_t ldx, const float* __restrict__ a, int K, int fmt,
-                 const float* __restrict__ tensor_scale, uint8_t* __restrict__ codes,
+quant_fp4_kernel(const XT* x, int64_t ldx, const float* a, int K, int fmt,
+                 const float* tensor_scale, uint8_t* __restrict__ codes,
                  uint8_t* __restrict__ sf, float* __restrict__ row_scale, float* __restrict__ out,
                  int mode, int M, int sf_atoms, int activations) {
   // THREADS bounds the launch; the CTA may be smaller (a multiple of 32): vectors are dealt out

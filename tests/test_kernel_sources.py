@@ -30,6 +30,8 @@ STARTS_EARLY = sorted(k for k, (_, body) in KERNELS.items() if "grid_dep_launch_
 # Kernels whose first loads of what an earlier kernel wrote stand right behind the wait.  (The others' stand behind a barrier
 # as well, whose phase the thread that has waited completes.)
 READS_AT_ONCE = ("act_quant", "quant_fp4", "scale_cols", "codes_to", "expand_w", "rope_kv")
+LOADS_ORDERED = READS_AT_ONCE + ("gemv_fused", "gemm_w4a4_e4m3", "gemm_a16w4", "gemm_fp4_persist", "column_stat",
+                                 "iteration", "finish")
 
 
 def test_the_kernels_are_found():
@@ -47,3 +49,12 @@ def test_a_kernel_that_starts_the_next_one_early_waits_itself(kernel):
         before = body[: body.index(CALL)]
         assert before.count("{") == before.count("}"), "the wait is conditional"
         assert not re.search(r"\bif\s*\([^)]*\)\s*$", before), "the wait is conditional"
+
+
+@pytest.mark.parametrize("kernel", [k for k in STARTS_EARLY if k.startswith(LOADS_ORDERED)])
+def test_loads_behind_the_wait_are_ordinary_ones(kernel):
+    """A `const __restrict__` parameter and __ldg say that the memory is constant while the kernel runs; the compiler may then
+    place the load in front of the wait.  Only what the packed weight holds is read that way."""
+    params, body = KERNELS[kernel]
+    assert set(re.findall(r"const\s+[\w ]+\*\s*__restrict__\s+(\w+)", params)) <= {"w_packed", "sw_t"}
+    assert set(re.findall(r"__ldg\((\w+)", body)) <= {"sw_row", "sxp"}  # sxp: behind the last group's barrier
