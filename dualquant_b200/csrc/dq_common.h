@@ -100,7 +100,8 @@ enum {
   DQ_TUNE_AR_WAIT_LOG2 = 4,     // fused all-reduce: a peer's flag is waited for 2^value SM cycles (0 = 30)
   DQ_TUNE_F8_TILE = 5,          // token tile of the FP8-path GEMM (32 .. 256 in steps of 32)
   DQ_TUNE_A16_TILE = 6,         // token tile of the A16W4 GEMM (+ 1000 x split of K)
-  DQ_TUNE_COUNT = 7
+  DQ_TUNE_FP4_KERNEL = 7,       // FP4 GEMM above 32 tokens: 1 = one tile per CTA, 2 = persistent on CTA pairs
+  DQ_TUNE_COUNT = 8
 };
 int tuning(int key);
 

@@ -334,8 +334,8 @@ __device__ __forceinline__ void tmem_st_wait() {
 // warp computes alike in uniform registers, where tcgen05 instructions and TMA copies want their operands.  The loops that
 // issue them are chains of one thread: in a probe of 16 KB copies an iteration took 181 ns under this branch and 220 under
 // `lane == 0`, and the GEMMs whose producers and issuers changed over gained (us, cold L2): FP8 path 8192 x 4096 -> 28672
-// 753 -> 715, 2048 x 4096 -> 4096 36.6 -> 35.3; FP4 persistent 4096 x 3584 -> 37888 285 -> 262, NVFP4 4096 x 18944 -> 3584
-// 156 -> 147; tensor-memory int4 kernel 32 x 4096 -> 28672 18.9 -> 15.9; kind::i8 kernel 128 x 4096 -> 28672 35.3 -> 34.3.
+// 753 -> 715, 2048 x 4096 -> 4096 36.6 -> 35.3; FP4 persistent (then on single CTAs) 4096 x 3584 -> 37888 285 -> 262, NVFP4
+// 4096 x 18944 -> 3584 156 -> 147; tensor-memory int4 kernel 32 x 4096 -> 28672 18.9 -> 15.9; kind::i8 kernel 128 x 4096 -> 28672 35.3 -> 34.3.
 // (The decode GEMM's producer, two copies a stage of 17 KB, lost 1.5 % and keeps the lane test.)
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;

@@ -131,7 +131,8 @@ extern "C" int dq_abi_version(void) { return 2; }
 
 extern "C" int dq_set_tuning(const char* name, int value) {
   static const char* const names[DQ_TUNE_COUNT] = {"linear_fused", "fused_stages", "fused_split",
-                                                   "fused_extra_cta", "ar_wait_log2", "f8_tile", "a16_tile"};
+                                                   "fused_extra_cta", "ar_wait_log2", "f8_tile", "a16_tile",
+                                                   "fp4_kernel"};
   DQ_REQUIRE(name != nullptr, DQ_ERR_NULL, "null tuning name");
   for (int i = 0; i < DQ_TUNE_COUNT; ++i) {
     if (strcmp(name, names[i]) == 0) {

@@ -471,8 +471,10 @@ static int gemm_fp4(const uint8_t* x_codes, const uint8_t* x_sf_atoms, const flo
   const int total_st = K / kFKStage;
   // The library's choice above a decode batch, where the copy engine can address the output: the persistent kernel on CTA
   // pairs, unless the one-tile kernel is estimated to be faster.
+  const int forced = tuning(DQ_TUNE_FP4_KERNEL);
   if (token_tile == 0 && M > kFp4DecodeTokens && (static_cast<size_t>(N) * (y_dtype == DQ_DTYPE_BF16 ? 2 : 4)) % 16 == 0 &&
-      aligned(y, 16) && fp4_pairs_us(M, N, total_st, st->sm_count) < fp4_one_tile_us(M, N, total_st, st->sm_count))
+      aligned(y, 16) && forced != 1 &&
+      (forced == 2 || fp4_pairs_us(M, N, total_st, st->sm_count) < fp4_one_tile_us(M, N, total_st, st->sm_count)))
     return launch_gemm_fp4_persist(x_codes, x_sf_atoms, x_scale, w_codes, w_sf_atoms, w_scale, r, bias, M, N, K,
                                    fmt == DQ_FP4_NVFP4 ? 1 : 0, y, y_dtype, static_cast<cudaStream_t>(stream), st);
   // The library's own choice otherwise: 32-token tiles for decode batches, else 128.  The 256-token tile is

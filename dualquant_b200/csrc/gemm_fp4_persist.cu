@@ -400,7 +400,7 @@ int launch_gemm_fp4_persist(const uint8_t* x_codes, const uint8_t* x_sf_atoms, c
   t.row_pairs = (N + 2 * kFBN - 1) / (2 * kFBN);
   t.tok_tiles = (M + fp4p::kTok - 1) / fp4p::kTok;
   const int pairs = st->sm_count / 2, all = t.row_pairs * t.tok_tiles, rest = all % pairs;
-  // few tiles in the last round: twice as many half ones, in half the time
+  // few tiles in the last round: twice as many half ones, in about 0.65 of the time (a half tile's copies are a whole one's)
   const bool halves = rest > 0 && 2 * rest <= pairs;
   t.full = halves ? all - rest : all;
   t.units = halves ? all + rest : all;

@@ -90,7 +90,9 @@ DQ_API int dq_abi_version(void);
  * (0 = the library's own choice), "ar_wait_log2" (the fused all-reduce waits 2^value SM cycles for a
  * peer before it gives up with DQ_ERR_TIMEOUT; 0 = 30, about half a second), "f8_tile" (token tile of the
  * FP8-path GEMM, 32 .. 256 in steps of 32; 0 = the library's own choice), "a16_tile" (token tile of the A16W4 GEMM, 32 /
- * 64 / 128 / 192 / 256, plus 1000 x its split of K for tiles up to 64; 0 = the library's own choice).  Process-wide, not thread-safe against concurrent launches. */
+ * 64 / 128 / 192 / 256, plus 1000 x its split of K for tiles up to 64; 0 = the library's own choice), "fp4_kernel" (FP4 GEMM above 32 tokens
+ * where the token tile is left to the library: 1 = one tile per CTA, 2 = CTA pairs, which need an output that bulk stores can
+ * address; 0 = the library's own choice).  Process-wide, not thread-safe against concurrent launches. */
 DQ_API int dq_set_tuning(const char* name, int value);
 
 /* Tensor-core ceiling probe: launches, on every SM, a loop of `iters` x 4 tcgen05.mma instructions

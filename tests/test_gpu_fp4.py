@@ -214,13 +214,21 @@ def test_fp4_gemm_token_tiles_agree(fmt, M, N, K):
     assert err < 1e-3, err
 
 
-# Shapes the library sends to the persistent prefill kernel: one tile per CTA pair and several, a last token tile of 216
-# tokens (two scale-factor blocks) and one of 100 (a single block), rows past N.
+@pytest.fixture
+def pair_kernel():
+    """The FP4 GEMM above 32 tokens on CTA pairs, whatever the library's estimate says."""
+    _lib.set_tuning("fp4_kernel", 2)
+    yield
+    _lib.set_tuning("fp4_kernel", 0)
+
+
+# The persistent kernel: one tile per CTA pair and several, a last token tile of 216 tokens (two scale-factor blocks) and one of
+# 100 (a single block), rows past N.  At these sizes the one-tile kernel does not split K: the same sums in the same order.
 @pytest.mark.parametrize("fmt", [_lib.FP4_MXFP4, _lib.FP4_NVFP4])
-@pytest.mark.parametrize("M,N,K,dtype", [(728, 6272, 512, torch.float32), (612, 6260, 768, torch.bfloat16),
-                                         (2048, 9472, 256, torch.bfloat16), (1024, 5120, 8192, torch.bfloat16),
-                                         (1000, 5104, 8192, torch.float32)])
-def test_fp4_persistent_kernel_equals_the_one_tile_kernel(fmt, M, N, K, dtype):
+@pytest.mark.parametrize("M,N,K,dtype", [(728, 6272, 512, torch.float32), (612, 6260, 768, torch.float32),
+                                         (612, 6264, 768, torch.bfloat16), (2048, 9472, 256, torch.bfloat16),
+                                         (1024, 5120, 8192, torch.bfloat16), (1000, 5104, 8192, torch.float32)])
+def test_fp4_persistent_kernel_equals_the_one_tile_kernel(fmt, M, N, K, dtype, pair_kernel):
     x = synthetic.make_x(M, K, M + 1)
     w = synthetic.make_w(N, K, N + 2)
     r, c = synthetic.make_scales(N, K, 3)
@@ -230,15 +238,39 @@ def test_fp4_persistent_kernel_equals_the_one_tile_kernel(fmt, M, N, K, dtype):
     sfa = ops.fp4_sf_to_atoms(sf, K, fmt)
     want = ops.gemm_w4a4_fp4(codes, sfa, rs, pw, r.to(DEV), out_dtype=dtype, token_tile=128)
     got = torch.full((M, N), float("nan"), dtype=dtype, device=DEV)
-    ops.gemm_w4a4_fp4(codes, sfa, rs, pw, r.to(DEV), out=got)  # library's choice: the persistent kernel
+    ops.gemm_w4a4_fp4(codes, sfa, rs, pw, r.to(DEV), out=got)
     _lib.device_status(0)
-    # (rows finished by a split-K launch sum their fp32 partial sums in another order)
-    assert torch.allclose(got.float(), want.float(), rtol=2e-6 if dtype == torch.float32 else 2 ** -7, atol=1e-6)
-    if N in (6272, 6260, 9472):
-        assert torch.equal(got, want)
+    assert torch.equal(got, want)
     ref = _fp4_reference(x, a.cpu(), w, r, fmt)
     err = ((got.double().cpu() - ref).abs().max() / ref.abs().max()).item()
     assert err < (1e-3 if dtype == torch.float32 else 1e-2), err
+
+
+# Up to 128 tokens: one block of activation scale factors where the copy's box has two, fewer tokens than a CTA's half of the
+# tile, half tiles.  From 247 row tiles on the one-tile kernel does not split K and the sums are the same; else its partial
+# sums are added in another order: at most K / 64 roundings of 2^-24 apart at the size of the largest output, with a factor 4
+# for partial sums larger than the result.
+@pytest.mark.parametrize("fmt", [_lib.FP4_MXFP4, _lib.FP4_NVFP4])
+@pytest.mark.parametrize("M", [33, 64, 100, 128])
+@pytest.mark.parametrize("N,K", [(32000, 512), (8192, 1024), (28672, 4096), (1032, 2304)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_fp4_pair_kernel_small_batches(fmt, M, N, K, dtype, pair_kernel):
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    x = torch.randn(M, K, generator=g, device=DEV).to(torch.bfloat16)
+    pw = ops.pack_w_fp4((torch.randn(N, K, generator=g, device=DEV) * 0.02).to(torch.bfloat16), fmt)
+    r = torch.rand(N, generator=g, device=DEV) + 0.5
+    codes, sfa, rs = ops.quant_fp4(x, fmt, None, None, atoms=True)
+    want = ops.gemm_w4a4_fp4(codes, sfa, rs, pw, r, out_dtype=dtype, token_tile=128)
+    y = torch.full((M + 1, N), 7.0, dtype=dtype, device=DEV)  # one guard row behind the output
+    ops.gemm_w4a4_fp4(codes, sfa, rs, pw, r, out=y[:M])
+    _lib.device_status(0)
+    assert bool((y[M] == 7.0).all())
+    if (N + 127) // 128 >= 247:
+        assert torch.equal(y[:M], want)
+    else:
+        apart = 4 * K / 64 * 2.0**-24 * want.abs().max().item()
+        step = 2.0**-7 * want.float().abs() if dtype == torch.bfloat16 else 0.0
+        assert bool(((y[:M].float() - want.float()).abs() <= apart + step).all())
 
 
 # Edges of the CTA-pair tiles: a last round of half tiles (some without tokens), an odd number of row tiles (the odd CTA of
@@ -247,7 +279,7 @@ def test_fp4_persistent_kernel_equals_the_one_tile_kernel(fmt, M, N, K, dtype):
 @pytest.mark.parametrize("fmt", [_lib.FP4_MXFP4, _lib.FP4_NVFP4])
 @pytest.mark.parametrize("M,N,K", [(300, 20008, 512), (130, 38000, 512), (257, 19080, 768), (385, 20000, 256), (1153, 20096, 768)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-def test_fp4_pair_tiles_equal_the_one_tile_kernel(fmt, M, N, K, dtype):
+def test_fp4_pair_tiles_equal_the_one_tile_kernel(fmt, M, N, K, dtype, pair_kernel):
     g = torch.Generator(device=DEV).manual_seed(M + N)
     x = torch.randn(M, K, generator=g, device=DEV).to(torch.bfloat16)
     w = (torch.randn(N, K, generator=g, device=DEV) * 0.02).to(torch.bfloat16)

@@ -26,7 +26,7 @@ def _kernels():
 
 
 KERNELS = _kernels()
-STARTS_EARLY = sorted(k for k, (_, body) in KERNELS.items() if "grid_dep_launch_dependents" in body)
+STARTS_EARLY = sorted(k for k, (_, body) in KERNELS.items() if "grid_dep_launch_dependents" in body or CALL in body)
 # Kernels whose first loads of what an earlier kernel wrote stand right behind the wait.  (The others' stand behind a barrier
 # as well, whose phase the thread that has waited completes.)
 READS_AT_ONCE = ("act_quant", "quant_fp4", "scale_cols", "codes_to", "expand_w", "rope_kv")
