@@ -433,7 +433,9 @@ static int fp4_split(int M, int N, int stages, int tok, int sm_count) {
 // Microseconds of the two kernels above 32 tokens, from their rounds and K loops (stages of 256 k).  Pairs: tiles of 256 x
 // 256, a last round with few tiles run as halves at 0.65 of a round.  One tile per CTA: tiles of 128 x 128, two CTAs per
 // SM; with K split over clusters of 2, 4 or 8 CTAs (places for 148, 66, 36 of them) the direct stores of the partial sums
-// dominate.  Over 162 cases of 48 to 4096 tokens the choice costs 0.6 % on average and 18 % at worst.  us, one tile / pairs:
+// dominate.  Over 360 linears (33 to 2048 tokens, twelve weights, both formats) the choice costs 0.4 % on average and 24 % at
+// worst (MXFP4, 320 x 4096 -> 6144: 19.7 where pairs take 15.9); all are as fast as, or faster than, with the kernels and the
+// rule before pairs (19.9 there).  us, one tile / pairs:
 //   18944 -> 3584  128 tokens 17 / 29   256  30 / 29   512  40 / 29   1000  64 / 36   4096 176 / 125
 //    3584 -> 4608             12 / 11        22 / 12        19 / 12         13 / 15         47 / 33
 //    3584 -> 37888            18 / 22        31 / 24        50 / 37        105 / 63        381 / 211

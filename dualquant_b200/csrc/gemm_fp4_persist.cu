@@ -173,7 +173,9 @@ gemm_fp4_persist_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_c
   }
   // No early start for the kernel behind this one: the next quantiser's CTAs, resident and waiting during the K loop, cost
   // more than the launch they hide (NVFP4 linears on single CTAs, us with / without: 3294 x 4096 -> 11968 131 / 126, 8192 x
-  // 3584 -> 18944 362 / 341, 8192 x 3584 -> 37888 667 / 616).
+  // 3584 -> 18944 362 / 341, 8192 x 3584 -> 37888 667 / 616; on pairs, chains of linears at 640 to 1000 tokens: up to 10 %
+  // slower, 1.5 % on average, NVFP4 1000 x 4096 -> 4096 26.0 / 23.7).  Up to 511 tokens it would gain 3 to 6 % on average (MXFP4
+  // 256 x 4096 -> 4096 11.6 / 12.8) and lose 4 % at worst.
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();  // the peer's barriers are initialised before anything arrives on them
