@@ -17,9 +17,11 @@ enum { MODE_CODES = 0, MODE_FAKE = 1, MODE_RAW = 2, MODE_FAKE_BF16 = 3 };
 struct Along {
   WeightExpansion e;
   bool done;
-  unsigned take(int threads, int64_t rows, ExpansionShare* s) {
+  int sm_count;
+  // rows: the quantiser's CTAs; they come first if there are at most per_sm for an SM
+  unsigned take(int threads, int64_t rows, int per_sm, ExpansionShare* s) {
     done = true;
-    return take_along(e, threads, rows, s);
+    return take_along(e, threads, rows, static_cast<int64_t>(per_sm) * sm_count, s);
   }
 };
 

@@ -780,7 +780,7 @@ int launch_had_fast_t(const XT* x, const XT* up, int64_t ldx, const float* a, co
     ExpansionShare ex = {};                                                                                            \
     const bool both = kExpand && along != nullptr;                                                                     \
     const int ctas = (M + Had28<P>::kRows - 1) / Had28<P>::kRows;                                                      \
-    const unsigned grid = both ? along->take(kHad28Threads, ctas, &ex) : static_cast<unsigned>(ctas);                  \
+    const unsigned grid = both ? along->take(kHad28Threads, ctas, 3, &ex) : static_cast<unsigned>(ctas);               \
     DQ_CHECK_CUDA(launch_pdl(both ? act_quant_had28_kernel<P, XT, kExpand> : act_quant_had28_kernel<P, XT>,            \
                              dim3(grid), dim3(kHad28Threads), Had28<P>::kSmem, stream, x, up, ldx, a, M, had->scale,   \
                              had->had_mat, codes, sx, out, mode, scale_fp16, ex));                                     \

@@ -441,13 +441,14 @@ static int launch_act(const XT* x, int64_t ldx, const float* a, const dq_hadamar
     // thread holds few elements and many warps are resident to hide the load -> reduce -> store
     // latency chain
     const int vec = K / 8;
-    // (an expansion goes with the launch shapes of a prefill batch)
+    // (an expansion goes with the launch shapes of a prefill batch, always between the rows: rows first where they find places
+    // at once was slower, 1100 x 3584 -> 4608 40.0 -> 41.8, 1150 x 4096 -> 12288 83.0 -> 86.5, and equal under 1024 rows)
 #define DQ_ROWS_LAUNCH_K(T, V, KP)                                                                                       \
   do {                                                                                                                   \
     constexpr bool kExpand = sizeof(XT) == 2 && ((V) >= 4 || ((KP) && (T) <= 512));                                      \
     ExpansionShare ex = {};                                                                                              \
     const bool both = kExpand && along != nullptr;                                                                       \
-    const unsigned grid = both ? along->take(T, M, &ex) : static_cast<unsigned>(M);                                      \
+    const unsigned grid = both ? along->take(T, M, 0, &ex) : static_cast<unsigned>(M);                                   \
     DQ_CHECK_CUDA(launch_pdl(both ? act_quant_rows_kernel<T, V, XT, KP, kExpand> : act_quant_rows_kernel<T, V, XT, KP>,  \
                              dim3(grid), dim3(T), 0, stream, x, ldx, a, K, codes, sx, out, mode, scale_fp16, norm_w,     \
                              norm_eps, ex));                                                                             \
@@ -486,12 +487,17 @@ static int launch_act(const XT* x, int64_t ldx, const float* a, const dq_hadamar
 
 // Rows in registers in the launch shapes of a prefill batch, and 28 * 64 ... 28 * 512 values with the online Hadamard, take the
 // expansion along; behind any other quantiser it is a launch of its own.  (Across heads the kernel fills the SM by itself: 2048
-// rows of 4096 lost 1 % beside an expansion.)
+// rows of 4096 lost 1 % beside an expansion.)  The expansion streams memory where the quantiser computes.  Linears in a chain,
+// us, expansion and quantiser one after the other (the better order) / in one launch: 1200 x 14336 -> 4096 135 / 127, 2048 x
+// 4096 -> 4096 47.2 / 45.0, 1300 x 4096 -> 18944 127 / 123, 1030 x 14336 -> 512 44.4 / 42.1, 1531 x 14336 -> 4096 with the
+// Hadamard 158 / 157, 8192 x 14336 -> 4096 with it 622 / 609, 1100 x 1792 -> 4096 with it (single calls) 25.8 / 25.5; under 1024 rows from 4 % slower (700 x 4096 -> 4096 27.1 / 28.1) to
+// 4 % faster (single calls of 400 x 2048 -> 8192 20.2 / 19.4).
 int quant_act_int4_and_expand(const void* x_bf16, int64_t ldx, const float* a, const dq_hadamard_desc* had, int M, int K,
                               int8_t* codes, float* sx, int scale_fp16, const WeightExpansion& e, cudaStream_t stream) {
-  if (current_state() == nullptr) return DQ_ERR_NOT_INIT;
+  const DeviceState* st = current_state();
+  if (st == nullptr) return DQ_ERR_NOT_INIT;
   DQ_REQUIRE(codes != nullptr && sx != nullptr, DQ_ERR_NULL, "codes / sx is null");
-  Along along = {e, false};
+  Along along = {e, false, st->sm_count};
   const int rc = launch_act(static_cast<const __nv_bfloat16*>(x_bf16), ldx, a, had, M, K, codes, sx, nullptr, MODE_CODES,
                             scale_fp16, stream, static_cast<const __nv_bfloat16*>(nullptr),
                             static_cast<const __nv_bfloat16*>(nullptr), -1.f, &along);

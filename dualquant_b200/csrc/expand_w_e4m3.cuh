@@ -57,25 +57,36 @@ inline int64_t expand_ctas(int N, int K, int chunks_per_cta) {
   return (static_cast<int64_t>((N + 127) / 128) * (K / kGroup) * 512 + chunks_per_cta - 1) / chunks_per_cta;
 }
 
-// A quantiser's launch of `rows` CTAs with an expansion taken along: `ctas` more of them, spread evenly.  Of the first b CTAs
-// floor(b * share / 2^32) expand; share is ctas * 2^32 / (rows + ctas) rounded up, so that with rows >= 1 it fits 32 bits, no
-// CTA counts twice, and the whole grid (fewer than 2^32 CTAs: the rounding adds less than one) has exactly `ctas` of them.
+// A quantiser's launch of `rows` CTAs with an expansion taken along: `ctas` more of them.  Long quantiser CTAs that all find a
+// place at once (up to `resident`) come first, spread over the SMs as on their own (28 * P with the Hadamard, linears, us: 1100 x
+// 1792 -> 4096 28.6 -> 25.5, 1024 x 1792 -> 2048 19.5 -> 16.7, 1100 x 3584 -> 4096 40.3 -> 37.4); else the others lie evenly
+// between them: of the first b CTAs floor(b * share / 2^32) expand.  share is ctas * 2^32 / (rows + ctas) rounded up, so that with rows >= 1 it
+// fits 32 bits and is not 0, no CTA counts twice, and the whole grid (fewer than 2^32 CTAs: the rounding adds less than one) has
+// exactly `ctas` of them.
 struct ExpansionShare {
   WeightExpansion e;
-  uint32_t share;
+  uint32_t rows, share;  // share 0: the quantiser's CTAs first
 };
 constexpr int kShareAhead = 4;
-inline unsigned take_along(const WeightExpansion& e, int threads, int64_t rows, ExpansionShare* s) {
+inline unsigned take_along(const WeightExpansion& e, int threads, int64_t rows, int64_t resident, ExpansionShare* s) {
   const int64_t ctas = expand_ctas(e.N, e.K, threads * kShareAhead), total = rows + ctas;
   s->e = e;
-  s->share = static_cast<uint32_t>(((static_cast<uint64_t>(ctas) << 32) + static_cast<uint64_t>(total) - 1) / static_cast<uint64_t>(total));
+  s->rows = static_cast<uint32_t>(rows);
+  s->share = rows <= resident ? 0
+                              : static_cast<uint32_t>(((static_cast<uint64_t>(ctas) << 32) + static_cast<uint64_t>(total) - 1) /
+                                                      static_cast<uint64_t>(total));
   return static_cast<unsigned>(total);
 }
 // This CTA's index among the quantiser's; or, after its part of the expansion, -1.
 template <int THREADS>
 __device__ __forceinline__ int quantiser_cta(const ExpansionShare& s) {
-  const uint32_t before = __umulhi(blockIdx.x, s.share);
-  if (__umulhi(blockIdx.x + 1, s.share) == before) return static_cast<int>(blockIdx.x - before);
+  uint32_t before = __umulhi(blockIdx.x, s.share);
+  bool expands = __umulhi(blockIdx.x + 1, s.share) != before;
+  if (s.share == 0) {
+    expands = blockIdx.x >= s.rows;
+    if (expands) before = blockIdx.x - s.rows;
+  }
+  if (!expands) return static_cast<int>(blockIdx.x - before);
   expand_chunks<THREADS, kShareAhead>(s.e, before);
   return -1;
 }

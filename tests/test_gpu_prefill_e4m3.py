@@ -400,13 +400,14 @@ def test_expanding_linear_equals_the_packed_kernel_over_its_options(M, N, had, m
 # The quantisers of these calls take the expansion of the weight along - rows in registers (128 threads, 256, 256 for long rows;
 # under 1024 rows 512 and 256 threads of one vector), 28 * 512, 28 * 64 with eight rows a CTA - or leave it to a launch of its own
 # (across heads, 2048 = 32 * 64).  Weights of one row, one tile and two: fewer CTAs expand than there are SMs; 18000 rows: most
-# of them do.  Inputs written and scratch read by the kernels just before; the packed path, which expands nothing, gives the
+# of them do.  28 * 64: up to 444 quantiser CTAs (on 148 SMs) come first, more of them with the others between.  Inputs written and scratch read by the kernels just before; the packed path, which expands nothing, gives the
 # same bits.
 @pytest.mark.parametrize("M,K,N,kind", [(1024, 4096, 1024, None), (1030, 8192, 512, None), (1026, 14336, 512, None),
                                         (700, 4096, 4096, None), (600, 2048, 8192, None), (1100, 4096, 4096, "heads"),
                                         (1031, 14336, 1024, "full"), (1200, 2048, 768, "full"), (1024, 1792, 300, "full"),
                                         (1025, 4096, 1, None), (1090, 14336, 128, None), (1024, 8192, 130, None),
-                                        (1029, 14336, 256, "full"), (1027, 1792, 16, "full"), (1024, 1152, 18000, None)])
+                                        (1029, 14336, 256, "full"), (1027, 1792, 16, "full"), (1024, 1152, 18000, None),
+                                        (3552, 1792, 256, "full"), (3553, 1792, 256, "full")])
 def test_linear_beside_the_expansion_of_its_weight(M, K, N, kind):
     had = None
     if kind == "heads":
